@@ -86,6 +86,152 @@ __device__ __forceinline__ bool robust_loss(double s, int loss, double scale, do
     return true;
 }
 
+// ---------------------------------------------------------------- the objective in few FP64 operations
+// A warp-wide FP64 operation (a conversion from or to FP32 included) holds a sub-partition's FP64
+// pipe for 64 cycles on this part, 76 for an addition, so the objective kernels are bound by the
+// number of FP64 operations per observation: about 159 with project64, robust_loss, the divisions
+// and log1p of the CUDA library; about 48 in the form below (pb_gpu_objective_noalloc over 4 000 000
+// observations, Cauchy: 1021 -> 347 us a call).
+//   - comparisons and finiteness tests look at the bit patterns on the integer pipe;
+//   - the reciprocal and the square root take one third-order Householder step from the 20-bit
+//     hardware approximation of the operand's high word (error below 2^-59 before the last rounding);
+//   - the principal point is subtracted from the pixel before the focal product is added;
+//   - a Cauchy sum takes one log1p per run of observations: sum log1p(x_i) = log1p(prod (1 + x_i) - 1),
+//     with the product kept as q = prod - 1 (q <- q + x (1 + q), relative precision also for tiny x).
+
+__device__ __forceinline__ unsigned hi_word(double v) { return static_cast<unsigned>(__double2hiint(v)); }
+// finite and not negative (a negative zero counts as zero)
+__device__ __forceinline__ bool bits_nonneg_finite(double v) {
+    const unsigned h = hi_word(v);
+    return h < 0x7ff00000u || (h == 0x80000000u && __double2loint(v) == 0);
+}
+
+// v < 0 (not a negative zero, not a NaN)
+__device__ __forceinline__ bool bits_negative(double v) {
+    const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v));
+    return b > 0x8000000000000000ull && b <= 0xfff0000000000000ull;
+}
+
+// 1 / z, z of any sign: within 1 ulp for exponents in (-1000, 1000), the IEEE quotient otherwise.
+__device__ __forceinline__ double rcp64(double z) {
+    const unsigned ex = (hi_word(z) >> 20) & 0x7ffu;
+    if (ex - 24u > 1998u) return 1.0 / z;
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(z));
+    const double e = fma(-z, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+// sqrt(s) of a positive finite s: within 1 ulp for exponents in (-900, 900).
+__device__ __forceinline__ double sqrt64(double s) {
+    const unsigned ex = (hi_word(s) >> 20) & 0x7ffu;
+    if (ex - 124u > 1798u) return sqrt(s);
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
+    const double n = s * y;
+    const double e = fma(-n, y, 1.0);
+    return fma(n, e * fma(0.375, e, 0.5), n);
+}
+
+// A camera record as the objective reads it (records of 32 doubles).  VEC: the records start on a
+// 16-byte boundary, two doubles per load (lanes read different cameras, so a load costs a line per
+// lane whatever its width).
+template <bool VEC>
+__device__ __forceinline__ void load_cam_objective(const double* __restrict__ c, DCam& k) {
+    double v[24];
+    if (VEC) {
+#pragma unroll
+        for (int i = 0; i < 12; ++i) {
+            const double2 d = __ldg(reinterpret_cast<const double2*>(c) + i);
+            v[2 * i] = d.x;
+            v[2 * i + 1] = d.y;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 24; ++i) v[i] = __ldg(c + i);
+    }
+#pragma unroll
+    for (int i = 0; i < 9; ++i) k.R[i] = v[i];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) k.C[i] = v[9 + i];
+    k.cx = v[14]; k.cy = v[15];
+    k.k1 = v[16]; k.k2 = v[17]; k.k3 = v[18]; k.p1 = v[19]; k.p2 = v[20];
+    // the axis signs (negative entries flip) go into the focal lengths by their sign bit
+    k.fx = __hiloint2double(__double2hiint(v[12]) ^ (bits_negative(v[21]) ? 0x80000000 : 0), __double2loint(v[12]));
+    k.fy = __hiloint2double(__double2hiint(v[13]) ^ (bits_negative(v[22]) ? 0x80000000 : 0), __double2loint(v[13]));
+    k.su = k.sv = 1.0;
+    k.flip = (__double_as_longlong(v[23]) << 1) != 0;
+}
+
+// w (r_u^2 + r_v^2) of one observation: false where project64 and robust_loss reject it (not in
+// front of the camera, not finite, negative).  `c` from load_cam_objective.
+__device__ __forceinline__ bool weighted_square64(const DCam& c, double X0, double X1, double X2, double u, double v,
+                                                  double w, double& s) {
+    const double d0 = X0 - c.C[0], d1 = X1 - c.C[1], d2 = X2 - c.C[2];
+    const double xc = fma(c.R[6], d2, fma(c.R[3], d1, c.R[0] * d0));
+    const double yc = fma(c.R[7], d2, fma(c.R[4], d1, c.R[1] * d0));
+    const double zc = fma(c.R[8], d2, fma(c.R[5], d1, c.R[2] * d0));
+    // forward depth above 1e-9 (a NaN passes here and fails the test of s)
+    const long long fwd = __double_as_longlong(zc) ^ (c.flip ? 0x8000000000000000ll : 0ll);
+    if (fwd <= __double_as_longlong(1e-9)) return false;
+    const double iz = rcp64(zc);
+    const double x = xc * iz, y = yc * iz;
+    const double r2 = fma(y, y, x * x);
+    const double radial = fma(r2, fma(r2, fma(r2, c.k3, c.k2), c.k1), 1.0);
+    // x radial + 2 p1 x y + p2 (r2 + 2 x^2) = x (radial + 2 (p1 y + p2 x)) + p2 r2, and likewise in y
+    const double h = fma(2.0, fma(c.p1, y, c.p2 * x), radial);
+    const double xd = fma(x, h, c.p2 * r2);
+    const double yd = fma(y, h, c.p1 * r2);
+    const double r0 = fma(c.fx, xd, c.cx - u), r1 = fma(c.fy, yd, c.cy - v);
+    s = w * fma(r1, r1, r0 * r0);
+    return bits_nonneg_finite(s);
+}
+
+// Robust costs of one thread's observations (evaluateImageRobustLoss,
+// BundleAdjustPlaMatrixProjection.cpp:75-109), in the order they are added.
+struct RobustSum {
+    double sum = 0.0;  // costs (Cauchy: of the finished runs, in units of c^2 / 2)
+    double q = 0.0;    // Cauchy: product of the open run's (1 + s / c^2), less one
+    // c2 = scale^2, ic2 = 1 / c2; `plain`: scale^2 and its reciprocal are finite and positive.
+    __device__ __forceinline__ bool add(double s, int loss, double scale, double c2, double ic2, bool plain) {
+        if (loss == 0) {
+            sum = fma(0.5, s, sum);
+            return true;
+        }
+        if (!plain) {
+            double cost, rw;
+            if (!robust_loss(s, loss, scale, cost, rw) || !isfinite(cost)) return false;
+            sum += cost;
+            return true;
+        }
+        if (loss == 1) {
+            if (__double_as_longlong(s) <= __double_as_longlong(c2)) {
+                sum = fma(0.5, s, sum);
+                return true;
+            }
+            const double cost = fma(scale, sqrt64(s), -0.5 * c2);
+            if (!bits_nonneg_finite(cost)) return false;
+            sum += cost;
+            return true;
+        }
+        const double x = s * ic2;
+        if (!bits_nonneg_finite(x)) return false;
+        // 2^400: a run is closed long before its product overflows
+        if (hi_word(x) >= 0x58f00000u || hi_word(q) >= 0x58f00000u) {
+            sum += log1p(q);
+            q = 0.0;
+            if (hi_word(x) >= 0x58f00000u) {
+                sum += log1p(x);
+                return true;
+            }
+        }
+        q = fma(x, 1.0 + q, q);
+        return true;
+    }
+    __device__ __forceinline__ double value(int loss, double c2, bool plain) const {
+        return loss == 2 && plain ? 0.5 * c2 * (sum + log1p(q)) : sum;
+    }
+};
+
 // First and second derivatives d1 = rho'(s), d2 = rho''(s) of the robust cost of robust_loss
 // (the normal weight is 2 rho'(s)).  Used by the exact Hessian of the backward pass.
 __device__ __forceinline__ void robust_derivatives(double s, int loss, double scale, double& d1, double& d2) {

@@ -7,6 +7,7 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <type_traits>
 
 #include "pb_device.cuh"
@@ -349,107 +350,96 @@ __global__ void k_trial_cameras(Shape S, DevPtrs D, const double* __restrict__ s
                  D.cams_trial + (static_cast<size_t>(a) * S.nc + c) * kCamStride);
 }
 
-// Objective of the trial states: image costs (FP64) per step length, block partials.
-__global__ void __launch_bounds__(256) k_cost_batch(Shape S, DevPtrs D, const double* __restrict__ step_p,
-                                                    const double* __restrict__ alphas, int n_alpha, int use_trial,
-                                                    double* __restrict__ part) {
-    __shared__ double s_c[kMaxAlpha][8];
-    __shared__ int s_bad[kMaxAlpha];
-    const long long o = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (threadIdx.x < kMaxAlpha) s_bad[threadIdx.x] = 0;
-    __syncthreads();
-    double c[kMaxAlpha];
-    for (int a = 0; a < kMaxAlpha; ++a) c[a] = 0.0;
-    if (o < S.nop) {
+// Objective of the trial states: image costs (FP64) per step length (blockIdx.y), block partials.
+// FP64-pipe-bound: see the objective in pb_device.cuh for the form of a term.  A thread takes every
+// (grid.x x block)-th observation; part holds the sums of step length a at a * gridDim.x and, from
+// kMaxAlpha * gridDim.x on, the blocks' invalid-projection marks in the same order.
+constexpr int kCostThreads = 128;
+__global__ void __launch_bounds__(kCostThreads) k_cost_batch(Shape S, DevPtrs D, const double* __restrict__ step_p,
+                                                             const double* __restrict__ alphas, int use_trial, double c2,
+                                                             double ic2, int plain, double* __restrict__ part) {
+    __shared__ double s_c[kCostThreads / 32];
+    __shared__ int s_bad[kCostThreads / 32];
+    const int a = blockIdx.y;
+    const double* cams = use_trial ? D.cams_trial + static_cast<size_t>(a) * S.nc * kCamStride : D.cams_eff;
+    const double alpha = use_trial ? alphas[a] : 0.0;
+    RobustSum acc;
+    double targets = 0.0;  // control-point costs
+    int bad = 0;
+    const long long stride = static_cast<long long>(gridDim.x) * kCostThreads;
+    for (long long o = static_cast<long long>(blockIdx.x) * kCostThreads + threadIdx.x; o < S.nop; o += stride) {
         const int cam = D.obs_cam[o], trk = D.obs_trk[o];
         const double* X = D.points + static_cast<size_t>(trk) * 3;
-        const double u = D.obs_u[o], v = D.obs_v[o], w = D.obs_w[o];
-        const bool moves = use_trial && D.trk_free[trk];
-        const double s = moves ? D.pscale[trk] : 0.0;
-        const double* dp = moves ? step_p + static_cast<size_t>(trk) * 3 : nullptr;
-        for (int a = 0; a < n_alpha; ++a) {
-            DCam k;
-            load_cam((use_trial ? D.cams_trial + (static_cast<size_t>(a) * S.nc) * kCamStride : D.cams_eff) +
-                         static_cast<size_t>(cam) * kCamStride,
-                     k);
-            double X0 = X[0], X1 = X[1], X2 = X[2];
-            if (moves) {
-                const double f = s * alphas[a];
-                X0 += f * dp[0];
-                X1 += f * dp[1];
-                X2 += f * dp[2];
+        double X0 = X[0], X1 = X[1], X2 = X[2];
+        if (use_trial && D.trk_free[trk]) {
+            const double* dp = step_p + static_cast<size_t>(trk) * 3;
+            const double f = D.pscale[trk] * alpha;
+            X0 = fma(f, dp[0], X0);
+            X1 = fma(f, dp[1], X1);
+            X2 = fma(f, dp[2], X2);
+        }
+        DCam k;
+        load_cam_objective<true>(cams + static_cast<size_t>(cam) * kCamStride, k);
+        double s;
+        if (!weighted_square64(k, X0, X1, X2, D.obs_u[o], D.obs_v[o], D.obs_w[o], s) ||
+            !acc.add(s, S.loss, S.loss_scale, c2, ic2, plain != 0)) {
+            bad = 1;
+            continue;
+        }
+        if (S.ncp > 0 && o == D.trk_obs_begin[trk]) {
+            // the track's control points, once per track (its first observation's thread); a
+            // term that is not finite is skipped (BundleAdjustPlaMatrixAssembly.cpp:674-690)
+            for (int q = D.trk_cp_begin[trk]; q < D.trk_cp_begin[trk + 1]; ++q) {
+                double r[3], cc, cw;
+                if (cp_eval(D.cp_rec + static_cast<size_t>(q) * 12, X0, X1, X2, S.cp_huber, r, cc, cw)) targets += cc;
             }
-            Proj p;
-            double cost = 0.0, rw;
-            bool good = project64(k, X0, X1, X2, p);
-            if (good) {
-                const double r0 = p.px - u, r1 = p.py - v;
-                good = robust_loss(w * (r0 * r0 + r1 * r1), S.loss, S.loss_scale, cost, rw) && isfinite(cost);
-            }
-            if (good && S.ncp > 0 && o == D.trk_obs_begin[trk]) {
-                // the track's control points, once per track (its first observation's thread); a
-                // term that is not finite is skipped (BundleAdjustPlaMatrixAssembly.cpp:674-690)
-                for (int q = D.trk_cp_begin[trk]; q < D.trk_cp_begin[trk + 1]; ++q) {
-                    double r[3], cc, cw;
-                    if (cp_eval(D.cp_rec + static_cast<size_t>(q) * 12, X0, X1, X2, S.cp_huber, r, cc, cw)) cost += cc;
-                }
-            }
-            if (!good) atomicOr(&s_bad[a], 1);
-            else c[a] = cost;
         }
     }
+    __syncwarp();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int a = 0; a < n_alpha; ++a) {
-        const double v = warp_sum(c[a]);
-        if (lane == 0) s_c[a][wid] = v;
+    double v = acc.value(S.loss, c2, plain != 0);
+    if (S.ncp > 0) v += targets;
+    v = warp_sum(v);
+    bad = __any_sync(0xffffffffu, bad);
+    if (lane == 0) {
+        s_c[wid] = v;
+        s_bad[wid] = bad;
     }
     __syncthreads();
-    if (threadIdx.x < n_alpha) {
-        double t = 0.0;
-        for (int w2 = 0; w2 < static_cast<int>(blockDim.x >> 5); ++w2) t += s_c[threadIdx.x][w2];
-        part[static_cast<size_t>(blockIdx.x) * kMaxAlpha * 2 + threadIdx.x] = t;
-        part[static_cast<size_t>(blockIdx.x) * kMaxAlpha * 2 + kMaxAlpha + threadIdx.x] = s_bad[threadIdx.x];
+    if (threadIdx.x == 0) {
+        const size_t at = static_cast<size_t>(a) * gridDim.x + blockIdx.x;
+        part[at] = (s_c[0] + s_c[1]) + (s_c[2] + s_c[3]);
+        part[static_cast<size_t>(kMaxAlpha) * gridDim.x + at] = s_bad[0] | s_bad[1] | s_bad[2] | s_bad[3];
     }
 }
+static_assert(kCostThreads == 128, "k_cost_batch adds the sums of four warps");
 
-// Final objective per step length: block partials in fixed order plus the intrinsic priors of the
-// trial groups (assemblePrimaryPriors cost, BundleAdjustPlaMatrixAssemblySurvey.cpp:43-91).
-__global__ void k_cost_final(Shape S, DevPtrs D, const double* __restrict__ part, int nblocks, int n_alpha,
-                             int use_trial, double* __restrict__ out) {
-    __shared__ double s_v[256];
-    __shared__ int s_b[256];
-    for (int a = 0; a < n_alpha; ++a) {
-        double v = 0.0;
-        int bad = 0;
-        for (int i = threadIdx.x; i < nblocks; i += blockDim.x) {
-            v += part[static_cast<size_t>(i) * kMaxAlpha * 2 + a];
-            bad |= part[static_cast<size_t>(i) * kMaxAlpha * 2 + kMaxAlpha + a] != 0.0;
-        }
-        s_v[threadIdx.x] = v;
-        s_b[threadIdx.x] = bad;
-        __syncthreads();
-        for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-            if (threadIdx.x < st) {
-                s_v[threadIdx.x] += s_v[threadIdx.x + st];
-                s_b[threadIdx.x] |= s_b[threadIdx.x + st];
-            }
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) {
-            double cost = s_v[0];
-            for (int g = 0; g < S.ng; ++g) {
-                const double* G = (use_trial ? D.groups_trial + static_cast<size_t>(a) * S.ng * kGroupRec : D.groups) +
-                                  static_cast<size_t>(g) * kGroupRec;
-                for (int c = 0; c < S.ni; ++c) {
-                    const int p = S.int_cols[c];
-                    const double r = G[2 * kP + p] * (G[p] - G[kP + p]);
-                    cost += 0.5 * r * r;
-                }
-            }
-            out[a] = s_b[0] ? __longlong_as_double(0x7ff0000000000000ll) : cost;
-        }
-        __syncthreads();
+// Final objective per step length, one warp each: block partials in fixed order plus the intrinsic
+// priors of the trial groups (assemblePrimaryPriors cost, BundleAdjustPlaMatrixAssemblySurvey.cpp:43-91).
+__global__ void __launch_bounds__(32 * kMaxAlpha) k_cost_final(Shape S, DevPtrs D, const double* __restrict__ part,
+                                                               int nblocks, int n_alpha, int use_trial,
+                                                               double* __restrict__ out) {
+    const int a = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (a >= n_alpha) return;
+    const double* sums = part + static_cast<size_t>(a) * nblocks;
+    const double* marks = part + static_cast<size_t>(kMaxAlpha + a) * nblocks;
+    double v = 0.0;
+    bool bad = false;
+#pragma unroll 8
+    for (int i = lane; i < nblocks; i += 32) {
+        v += sums[i];
+        bad |= __double_as_longlong(marks[i]) != 0;
     }
+    for (int e = lane; e < S.nb; e += 32) {
+        const int g = e / S.ni, p = S.int_cols[e - g * S.ni];
+        const double* G = (use_trial ? D.groups_trial + static_cast<size_t>(a) * S.ng * kGroupRec : D.groups) +
+                          static_cast<size_t>(g) * kGroupRec;
+        const double r = G[2 * kP + p] * (G[p] - G[kP + p]);
+        v = fma(0.5 * r, r, v);
+    }
+    v = warp_sum(v);
+    bad = __any_sync(0xffffffffu, bad);
+    if (lane == 0) out[a] = bad ? __longlong_as_double(0x7ff0000000000000ll) : v;
 }
 
 // Back-substitution (recoverReferencePointSteps, ...ReferenceSchur.cpp:982-1082), one thread per
@@ -789,6 +779,14 @@ void launch_effective(const Shape& S, const DevPtrs& D, cudaStream_t st) {
     k_effective<<<(n + 127) / 128, 128, 0, st>>>(S, D);
 }
 
+// Blocks per step length of k_cost_batch: eight resident blocks on each of 152 SMs share the batch;
+// beyond, a thread takes several observations (one log1p per thread of a Cauchy sum, and at most
+// 1216 partials a step length for the final sum).
+static int cost_blocks(long long nop, int n_alpha) {
+    const long long need = (nop + kCostThreads - 1) / kCostThreads;
+    return static_cast<int>(std::max<long long>(1, std::min<long long>(need, std::max(152, kCostMaxBlocks / n_alpha))));
+}
+
 void launch_cost(const Shape& S, const DevPtrs& D, const double* step_c, const double* step_p, const double* alphas,
                  int n_alpha, int use_trial, double* part, double* out, cudaStream_t st, const RigDev* rig) {
     if (use_trial) {
@@ -797,9 +795,11 @@ void launch_cost(const Shape& S, const DevPtrs& D, const double* step_c, const d
         // rig cameras: poses composed from the trial captures and sensors
         if (rig) launch_rig_trial(*rig, S.nc, alphas, n_alpha, D.cams_trial, st);
     }
-    const int nblk = static_cast<int>(std::max<long long>(1, (S.nop + 255) / 256));
-    k_cost_batch<<<nblk, 256, 0, st>>>(S, D, step_p, alphas, n_alpha, use_trial, part);
-    k_cost_final<<<1, 256, 0, st>>>(S, D, part, nblk, n_alpha, use_trial, out);
+    const int nblk = cost_blocks(S.nop, n_alpha);
+    const double c2 = S.loss_scale * S.loss_scale, ic2 = 1.0 / c2;
+    const int plain = S.loss != 0 && std::isnormal(c2) && std::isnormal(ic2) ? 1 : 0;
+    k_cost_batch<<<dim3(nblk, n_alpha), kCostThreads, 0, st>>>(S, D, step_p, alphas, use_trial, c2, ic2, plain, part);
+    k_cost_final<<<1, 32 * kMaxAlpha, 0, st>>>(S, D, part, nblk, n_alpha, use_trial, out);
 }
 
 void launch_accept(const Shape& S, const DevPtrs& D, const double* step_p, double alpha, int a, cudaStream_t st) {

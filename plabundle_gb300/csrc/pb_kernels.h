@@ -11,6 +11,7 @@
 namespace pb {
 
 constexpr int kMaxAlpha = 8;  // trial step lengths evaluated per objective pass
+constexpr int kCostMaxBlocks = 152 * 8;  // partials per step length of an objective pass, at most
 
 // Outputs of the assembly kernel (per-chunk partials) and per-track / per-observation data kept
 // for the back-substitution.  Partials are the accumulator pairs of Acc<T>: (hi, lo) float pairs

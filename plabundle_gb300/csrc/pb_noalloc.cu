@@ -1,16 +1,15 @@
 // pb_noalloc.cu -- allocation-free robust objective of caller-owned device arrays.
 //
-// pb_gpu_objective_noalloc is the per-observation cost kernel of the LM line search
-// (k_cost_batch / k_cost_final: FP64 projection, robust loss, per-block partial sums reduced in a
-// fixed order) for callers that own their device buffers and may not allocate.  Its per-block
-// partials live in one file-scope device array of fixed size instead of context memory, so a
-// call launches two kernels, copies three numbers back and allocates nothing.
+// pb_gpu_objective_noalloc is the objective of the LM line search (k_cost_batch: FP64 projection,
+// robust loss, per-block partial sums reduced in a fixed order) for callers that own their device
+// buffers and may not allocate.  Its per-block partials live in one file-scope device array of
+// fixed size instead of context memory, so a call launches one or two kernels, copies three
+// numbers back and allocates nothing.
 //
 // Limits and rules (also stated in include/pb_gpu.h):
-//   - at most PB_NOALLOC_MAX_OBS observations (one 256-thread block per 256 observations, one
-//     partial per block); larger inputs are rejected before any launch;
-//   - every element of the scratch array that the final kernel reads is written by the first
-//     kernel of the same call, so nothing has to start at zero;
+//   - at most PB_NOALLOC_MAX_OBS observations; larger inputs are rejected before any launch;
+//   - every element of the scratch array that the final sum reads is written earlier in the same
+//     call, so nothing has to start at zero;
 //   - the array is shared by all callers on a device: calls that overlap in time on one device
 //     race; callers serialise them (one stream, or host-side ordering);
 //   - the array's device address is resolved with cudaGetSymbolAddress on the first call on each
@@ -19,61 +18,98 @@
 //     cudaDeviceReset);
 //   - an error already pending on the calling thread is left for its owner: the call returns
 //     PB_ERR_CUDA without launching, and every status it reads afterwards is its own.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "pb_device.cuh"
 
 namespace pb {
 
-constexpr int kNoAllocThreads = 256;
-constexpr int kNoAllocMaxBlocks = static_cast<int>(PB_NOALLOC_MAX_OBS / kNoAllocThreads);
+constexpr int kNoAllocThreads = 128;
+// Eight blocks on each of 152 SMs: 155 648 threads fill the FP64 pipes, and beyond that a thread takes
+// several observations, so that a Cauchy sum needs one log1p per thread and the final sum covers at
+// most 1216 partials.
+constexpr int kNoAllocMaxBlocks = 152 * 8;
+constexpr int kClusterBlocks = 8, kClusterThreads = 256;
+// Up to two observations per thread of the cluster, one launch beats two (a call, 4 096 observations:
+// 35.0 against 36.7 us; 8 192: 46.3 against 37.0, eight SMs are then too few).
+constexpr long long kClusterMaxObs = 2LL * kClusterBlocks * kClusterThreads;
 constexpr int kNoAllocMaxDevices = 64;
 
 // [0, B): cost partials; [B, 2B): invalid projections; [2B, 3B): index errors; [3B, 3B + 3): totals
-// (B = 16384 blocks: 384 KB per device)
+// (B = 1216 blocks, eight per SM)
 static __device__ __align__(256) double g_noalloc_scratch[3 * kNoAllocMaxBlocks + 3];
 
 namespace {
 
-__global__ void __launch_bounds__(kNoAllocThreads)
-    k_objective_part(const double* __restrict__ cameras, int n_cameras, const double* __restrict__ points,
-                     int n_points, const int* __restrict__ obs_camera, const int* __restrict__ obs_point,
-                     const double* __restrict__ obs_u, const double* __restrict__ obs_v,
-                     const double* __restrict__ obs_w, long long n_obs, int loss, double scale,
-                     double* __restrict__ scratch) {
-    __shared__ double s_red[3][kNoAllocThreads / 32];
-    const long long o = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    double cost = 0.0, bad = 0.0, oob = 0.0;
-    if (o < n_obs) {
-        const int cam = obs_camera[o], pt = obs_point[o];
-        if (cam < 0 || cam >= n_cameras || pt < 0 || pt >= n_points) {
-            oob = 1.0;  // the access is skipped; the host reports PB_ERR_BOUNDS
-        } else {
-            DCam c;
-            load_cam(cameras + static_cast<size_t>(cam) * kCamStride, c);
-            const double* X = points + static_cast<size_t>(pt) * 3;
-            Proj p;
-            double cst = 0.0, rw;
-            bool good = project64(c, X[0], X[1], X[2], p);
-            if (good) {
-                const double r0 = p.px - obs_u[o], r1 = p.py - obs_v[o];
-                good = robust_loss(obs_w[o] * (r0 * r0 + r1 * r1), loss, scale, cst, rw) && isfinite(cst);
-            }
-            if (good) cost = cst;
-            else bad = 1.0;
+struct ObjectiveArgs {
+    const double* cameras;
+    const double* points;
+    const int* obs_camera;
+    const int* obs_point;
+    const double* obs_u;
+    const double* obs_v;
+    const double* obs_w;
+    long long n_obs;
+    int n_cameras, n_points, loss, plain;
+    double scale, c2, ic2;
+};
+
+struct ObjectiveSums {
+    double cost;
+    int bad, oob;  // invalid projections, indices out of range
+};
+
+// The calling warp's observations first, first + stride, ... (one per lane and turn), summed over the
+// warp.
+template <bool VEC>
+__device__ __forceinline__ ObjectiveSums objective_warp(const ObjectiveArgs& A, long long first, long long stride) {
+    RobustSum acc;
+    ObjectiveSums r{0.0, 0, 0};
+    for (long long o = first; o < A.n_obs; o += stride) {
+        const int cam = A.obs_camera[o], pt = A.obs_point[o];
+        if (cam < 0 || cam >= A.n_cameras || pt < 0 || pt >= A.n_points) {
+            ++r.oob;  // the access is skipped; the host reports PB_ERR_BOUNDS
+            continue;
         }
+        DCam c;
+        load_cam_objective<VEC>(A.cameras + static_cast<size_t>(cam) * kCamStride, c);
+        const double* X = A.points + static_cast<size_t>(pt) * 3;
+        double s;
+        if (!weighted_square64(c, X[0], X[1], X[2], A.obs_u[o], A.obs_v[o], A.obs_w[o], s) ||
+            !acc.add(s, A.loss, A.scale, A.c2, A.ic2, A.plain != 0))
+            ++r.bad;
     }
-    const double v[3] = {warp_sum(cost), warp_sum(bad), warp_sum(oob)};
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0)
-        for (int k = 0; k < 3; ++k) s_red[k][warp] = v[k];
+    __syncwarp();
+    r.cost = warp_sum(acc.value(A.loss, A.c2, A.plain != 0));
+    r.bad = __reduce_add_sync(0xffffffffu, r.bad);
+    r.oob = __reduce_add_sync(0xffffffffu, r.oob);
+    return r;
+}
+
+// One partial triple per block; a thread takes every (grid x block)-th observation.  FP64-pipe-bound
+// (see the objective in pb_device.cuh).
+template <bool VEC>
+__global__ void __launch_bounds__(kNoAllocThreads) k_objective_part(ObjectiveArgs A, double* __restrict__ scratch) {
+    __shared__ ObjectiveSums s_sum[kNoAllocThreads / 32];
+    const ObjectiveSums r = objective_warp<VEC>(A, static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x,
+                                                static_cast<long long>(gridDim.x) * blockDim.x);
+    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = r;
     __syncthreads();
-    if (threadIdx.x < 3) {
-        double t = 0.0;
-        for (int w = 0; w < kNoAllocThreads / 32; ++w) t += s_red[threadIdx.x][w];
-        scratch[static_cast<size_t>(threadIdx.x) * kNoAllocMaxBlocks + blockIdx.x] = t;
+    if (threadIdx.x == 0) {
+        ObjectiveSums t = s_sum[0];
+        for (int w = 1; w < kNoAllocThreads / 32; ++w) {
+            t.cost += s_sum[w].cost;
+            t.bad += s_sum[w].bad;
+            t.oob += s_sum[w].oob;
+        }
+        scratch[blockIdx.x] = t.cost;
+        scratch[kNoAllocMaxBlocks + blockIdx.x] = t.bad;
+        scratch[2 * kNoAllocMaxBlocks + blockIdx.x] = t.oob;
     }
 }
 
@@ -82,16 +118,49 @@ __global__ void __launch_bounds__(kNoAllocThreads) k_objective_final(int nblocks
     __shared__ double s_red[3][kNoAllocThreads];
     for (int k = 0; k < 3; ++k) {
         double t = 0.0;
-        for (int b = threadIdx.x; b < nblocks; b += blockDim.x) t += scratch[static_cast<size_t>(k) * kNoAllocMaxBlocks + b];
+        for (int b = threadIdx.x; b < nblocks; b += kNoAllocThreads) t += scratch[k * kNoAllocMaxBlocks + b];
         s_red[k][threadIdx.x] = t;
     }
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s)
-            for (int k = 0; k < 3; ++k) s_red[k][threadIdx.x] += s_red[k][threadIdx.x + s];
-        __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp < 3) {  // one warp per total
+        double t = s_red[warp][lane];
+        for (int i = lane + 32; i < kNoAllocThreads; i += 32) t += s_red[warp][i];
+        t = warp_sum(t);
+        if (lane == 0) scratch[3 * kNoAllocMaxBlocks + warp] = t;
     }
-    if (threadIdx.x < 3) scratch[3 * static_cast<size_t>(kNoAllocMaxBlocks) + threadIdx.x] = s_red[threadIdx.x][0];
+}
+
+// Small inputs in one launch: a cluster of eight blocks, whose partials the first block reads from
+// the others' shared memory.
+template <bool VEC>
+__global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(kClusterThreads)
+    k_objective_cluster(ObjectiveArgs A, double* __restrict__ scratch) {
+    __shared__ ObjectiveSums s_sum[kClusterThreads / 32];
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const ObjectiveSums r = objective_warp<VEC>(A, static_cast<long long>(blockIdx.x) * kClusterThreads + threadIdx.x,
+                                                static_cast<long long>(kClusterBlocks) * kClusterThreads);
+    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = r;
+    cluster.sync();
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
+        double cost = 0.0;
+        int bad = 0, oob = 0;
+        for (int i = threadIdx.x; i < kClusterBlocks * (kClusterThreads / 32); i += 32) {
+            const ObjectiveSums* p = cluster.map_shared_rank(&s_sum[i % (kClusterThreads / 32)], i / (kClusterThreads / 32));
+            cost += p->cost;
+            bad += p->bad;
+            oob += p->oob;
+        }
+        cost = warp_sum(cost);
+        bad = __reduce_add_sync(0xffffffffu, bad);
+        oob = __reduce_add_sync(0xffffffffu, oob);
+        if (threadIdx.x == 0) {
+            scratch[3 * kNoAllocMaxBlocks] = cost;
+            scratch[3 * kNoAllocMaxBlocks + 1] = bad;
+            scratch[3 * kNoAllocMaxBlocks + 2] = oob;
+        }
+    }
+    cluster.sync();  // the other blocks' shared memory stays until it has been read
 }
 
 // Device address of the scratch array on the current device, resolved once per device.
@@ -135,13 +204,21 @@ extern "C" pb_status pb_gpu_objective_noalloc(const double* cameras, int32_t n_c
     double* scratch = noalloc_scratch();
     if (!scratch) return PB_ERR_CUDA;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int nblocks = static_cast<int>((n_obs + kNoAllocThreads - 1) / kNoAllocThreads);
-    k_objective_part<<<nblocks, kNoAllocThreads, 0, st>>>(cameras, n_cameras, points, n_points, obs_camera, obs_point,
-                                                          obs_u, obs_v, obs_w, static_cast<long long>(n_obs),
-                                                          robust_loss, robust_loss_scale, scratch);
-    if (cudaGetLastError() != cudaSuccess) return PB_ERR_CUDA;
-    k_objective_final<<<1, kNoAllocThreads, 0, st>>>(nblocks, scratch);
-    if (cudaGetLastError() != cudaSuccess) return PB_ERR_CUDA;
+    const int nblocks = static_cast<int>(std::min<int64_t>((n_obs + kNoAllocThreads - 1) / kNoAllocThreads, kNoAllocMaxBlocks));
+    const double c2 = robust_loss_scale * robust_loss_scale, ic2 = 1.0 / c2;
+    const int plain = robust_loss != 0 && std::isnormal(c2) && std::isnormal(ic2) ? 1 : 0;
+    const ObjectiveArgs args{cameras, points, obs_camera, obs_point, obs_u, obs_v, obs_w, static_cast<long long>(n_obs),
+                             n_cameras, n_points, robust_loss, plain, robust_loss_scale, c2, ic2};
+    const bool vec = (reinterpret_cast<uintptr_t>(cameras) & 15) == 0;
+    if (n_obs <= kClusterMaxObs) {
+        (vec ? k_objective_cluster<true> : k_objective_cluster<false>)<<<kClusterBlocks, kClusterThreads, 0, st>>>(args, scratch);
+        if (cudaGetLastError() != cudaSuccess) return PB_ERR_CUDA;
+    } else {
+        (vec ? k_objective_part<true> : k_objective_part<false>)<<<nblocks, kNoAllocThreads, 0, st>>>(args, scratch);
+        if (cudaGetLastError() != cudaSuccess) return PB_ERR_CUDA;
+        k_objective_final<<<1, kNoAllocThreads, 0, st>>>(nblocks, scratch);
+        if (cudaGetLastError() != cudaSuccess) return PB_ERR_CUDA;
+    }
     double totals[3] = {0.0, 0.0, 0.0};
     if (cudaMemcpyAsync(totals, scratch + 3 * static_cast<size_t>(kNoAllocMaxBlocks), sizeof totals,
                         cudaMemcpyDeviceToHost, st) != cudaSuccess ||

@@ -385,8 +385,7 @@ void upload_structure(pb_gpu_ctx* c) {
     c->bs_part = A.alloc<double>(2 * static_cast<size_t>(bs_blocks));
     c->bs_terms = A.alloc<double>(3 * static_cast<size_t>(std::max<long long>(1, nop)));
     c->bs_out = A.alloc<double>(4);
-    const long long cost_blocks = std::max<long long>(1, (nop + 255) / 256);
-    c->cost_part = A.alloc<double>(static_cast<size_t>(cost_blocks) * kMaxAlpha * 2);
+    c->cost_part = A.alloc<double>(static_cast<size_t>(kCostMaxBlocks) * kMaxAlpha * 2);
     c->cost_out = A.alloc<double>(kMaxAlpha);
     c->alphas_d = A.alloc<double>(kMaxAlpha);
     c->pcg_res = A.alloc<PcgResult>(1);
