@@ -195,39 +195,9 @@ __device__ void diag_factor_inverse(T* __restrict__ A, T* __restrict__ Dinv, int
     constexpr int PW = 16;   // panel width
     __syncthreads();
     for (int c0 = 0; c0 < TS; c0 += PW) {
-        // (a) the panel's diagonal block, warp 0.  FP32: in registers, lane r holds columns 0-7 of
-        // row c0 + r, lane r + 16 its columns 8-15, and pivot entries reach the other lanes by
-        // shuffle.  FP64: in shared memory, each lane updating its own few of the block's 120
-        // elements, which issues a quarter of the FP64 instructions of the register form (every
-        // lane of that form steps through every column).
-        if (warp == 0 && sizeof(T) == 8) {
-            int ri[4], rl[4];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                const int e = lane + 32 * t;  // e < 120: row r, column e - r (r - 1) / 2 + 1
-                int r = 1;
-                while (r * (r + 1) / 2 <= e) ++r;
-                ri[t] = e < 120 ? r : -1;
-                rl[t] = e < 120 ? e - r * (r - 1) / 2 + 1 : 0x7fff;
-            }
-            for (int j = c0; j < c0 + PW; ++j) {
-                __syncwarp();
-                const T d = sA[j * TP + j];
-                if (!(d > T(0))) {
-                    if (lane == 0) atomicOr(status, 2);
-                }
-                const T inv = d > T(0) ? T(1) / d : T(0);
-                if (lane == 0) s_inv[j] = inv;
-                const int rj = j - c0;
-#pragma unroll
-                for (int t = 0; t < 4; ++t)
-                    if (rl[t] > rj && ri[t] >= 0) {
-                        const int i = c0 + ri[t], l = c0 + rl[t];
-                        sA[i * TP + l] = fma(-(sA[i * TP + j] * sA[l * TP + j]), inv, sA[i * TP + l]);
-                    }
-            }
-            __syncwarp();
-        } else if (warp == 0) {
+        // (a) the panel's diagonal block, warp 0, in registers: lane r holds columns 0-7 of row
+        // c0 + r, lane r + 16 its columns 8-15, and pivot entries reach the other lanes by shuffle
+        if (warp == 0) {
             const int ri = lane & 15, half = lane >> 4;
             T a[PW / 2];
 #pragma unroll
@@ -440,6 +410,288 @@ __global__ void __launch_bounds__(256) k_potrf_coop(T* __restrict__ A, T* __rest
             const int r = e / TS, c = e % TS;
             dst[static_cast<size_t>(r) * np + c] = sA[r * TP + c];
         }
+        __syncthreads();
+    }
+}
+
+// ---- FP64 factorisation: 32 x 32 tiles
+// A warp-wide FP64 FMA takes 64 cycles of a sub-partition, so a 64 x 64 x 64 tile product keeps an SM
+// busy for 63 us and a system of a few hundred unknowns spends its time on a few SMs, one step after
+// another.  Tiles of 32 cut a product to 8 us (4 where one factor is triangular, with the rows or
+// columns of a warp chosen so that every warp sums 66 products) and spread the same work over four
+// times as many SMs; the diagonal tile's chain (below) is a quarter of the 64 x 64 one.  A whole FP64
+// step, of which this is the largest part: 114 unknowns 811 -> 451 us, 600 unknowns 3.56 -> 1.71 ms, 1216
+// unknowns 9.8 -> 4.5 ms, 3010 unknowns 29.5 -> 20.6 ms (the FP64 pipes of all SMs are the bound there).
+// The FP32 factor keeps its tiles of 64: its products are cheap and fewer steps cost fewer barriers.
+namespace {
+constexpr int TD = 32, TDP = TD + 1;
+constexpr int kPotrf64Threads = 256;
+constexpr size_t kPotrf64Smem = (3 * static_cast<size_t>(TD) * TDP + TD * 9 + 3 * TD) * sizeof(double);
+}  // namespace
+
+// Inverse of the 8 x 8 diagonal block b of the tile's factor from its unscaled columns, by one warp
+// (lane c < 8 a column): with L_ik = a_ik rs_k and z_k = rs_k x_k, x_i = -rs_i sum_k a_ik z_k.
+__device__ __forceinline__ void inverse8(const double* sC, double* sX, const double* s_d, double* s_sd, double* s_rs,
+                                         int b) {
+    const int lane = threadIdx.x & 31, c = lane & 7, o = 8 * b;
+    const double d = s_d[o + c];
+    const double sd = d > 0.0 ? sqrt64(d) : 1.0;
+    const double rs = rcp64(sd);
+    if (lane < 8) {
+        s_sd[o + c] = sd;
+        s_rs[o + c] = rs;
+    }
+    double z[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        double t = 0.0;
+#pragma unroll
+        for (int k = 0; k < i; ++k) t = fma(sC[(o + i) * TDP + o + k], z[k], t);
+        const double ri = __shfl_sync(0xffffffffu, rs, i);
+        const double x = i == c ? ri : (i > c ? -ri * t : 0.0);
+        z[i] = ri * x;
+        if (lane < 8) sX[(o + i) * TDP + o + c] = x;
+    }
+}
+
+// The diagonal tile in sC (lower triangle): L_kk into A (zeros above the diagonal) and D_k = L_kk^-1
+// into Dinv.  Unscaled elimination in four panels of eight columns: warp 0 takes the panel, a lane per
+// row with its eight columns in registers and the pivots passed by shuffle (a pivot costs a reciprocal
+// of three FP64 operations, a product and the updates: ~450 cycles a column, the chain that bounds the
+// tile), every warp then applies the panel to the rest; warp 1 inverts the previous panel's 8 x 8 block
+// meanwhile.  The square roots come once at the end, and the inverse grows from the 8 x 8 blocks by
+// doubling: X21 = -X22 (L21 X11).
+__device__ void diag_factor_inverse64(double* __restrict__ Akk, int np, double* __restrict__ D, double* sC, double* sX,
+                                      double* sP, double* sT, double* s_d, int* __restrict__ status) {
+    double* s_sd = s_d + TD;
+    double* s_rs = s_sd + TD;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int e = tid; e < TD * TDP; e += kPotrf64Threads) sX[e] = 0.0;
+    __syncthreads();
+    for (int b = 0; b < 4; ++b) {
+        const int c0 = 8 * b;
+        if (warp == 0) {
+            const int i = c0 + lane;
+            double a[8];
+#pragma unroll
+            for (int l = 0; l < 8; ++l) a[l] = i < TD ? sC[i * TDP + c0 + l] : 0.0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const double d = __shfl_sync(0xffffffffu, a[j], j);
+                const bool pos = d > 0.0;
+                const double inv = pos ? rcp64(d) : 0.0;
+                if (lane == j) {
+                    s_d[c0 + j] = d;
+                    if (!pos) atomicOr(status, 2);
+                }
+                const double t = a[j] * inv;
+                if (i < TD) sT[i * 9 + j] = t;
+#pragma unroll
+                for (int l = j + 1; l < 8; ++l) {
+                    const double alj = __shfl_sync(0xffffffffu, a[j], l);
+                    a[l] = fma(-t, alj, a[l]);
+                }
+            }
+            if (i < TD)
+#pragma unroll
+                for (int l = 0; l < 8; ++l) sC[i * TDP + c0 + l] = a[l];
+        } else if (warp == 1 && b > 0) {
+            inverse8(sC, sX, s_d, s_sd, s_rs, b - 1);
+        }
+        __syncthreads();
+        const int m = TD - 8 - c0;
+        for (int e = tid; e < m * (m + 1) / 2; e += kPotrf64Threads) {
+            const int t = tri_row(e);
+            const int i = c0 + 8 + t, l = c0 + 8 + e - t * (t + 1) / 2;
+            double a = sC[i * TDP + l];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) a = fma(-sT[i * 9 + j], sC[l * TDP + c0 + j], a);
+            sC[i * TDP + l] = a;
+        }
+        __syncthreads();
+    }
+    if (warp == 1) inverse8(sC, sX, s_d, s_sd, s_rs, 3);
+    __syncthreads();
+    // L: columns times 1 / sqrt(pivot); the 8 x 8 blocks of the inverse are final already
+    for (int e = tid; e < TD * TD; e += kPotrf64Threads) {
+        const int i = e / TD, j = e % TD;
+        const double v = i > j ? sC[i * TDP + j] * s_rs[j] : (i == j ? s_sd[j] : 0.0);
+        sC[i * TDP + j] = v;
+        Akk[static_cast<size_t>(i) * np + j] = v;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 8; h <= 16; h *= 2) {
+        // pairs of h x h blocks: rows r0 + h .. r0 + 2h - 1, columns r0 .. r0 + h - 1
+        const int per = h * h, pairs = TD / (2 * h);
+        const int pr = tid / per, e = tid % per, r = e / h, c = e % h, r0 = pr * 2 * h;
+        if (pr < pairs) {
+            double t = 0.0;
+#pragma unroll
+            for (int k = 0; k < h; ++k) t = fma(sC[(r0 + h + r) * TDP + r0 + k], sX[(r0 + k) * TDP + r0 + c], t);
+            sP[(r0 + r) * TDP + c] = t;
+        }
+        __syncthreads();
+        if (pr < pairs) {
+            double t = 0.0;
+#pragma unroll
+            for (int k = 0; k < h; ++k) t = fma(sX[(r0 + h + r) * TDP + r0 + h + k], sP[(r0 + k) * TDP + c], t);
+            sX[(r0 + h + r) * TDP + r0 + c] = -t;
+        }
+        __syncthreads();
+    }
+    for (int e = tid; e < TD * TD; e += kPotrf64Threads) D[e] = sX[(e / TD) * TDP + e % TD];
+    (void)lane;
+}
+
+// Global 32 x 32 tile (row stride ld, 16-byte aligned rows) into shared memory, row-major.
+__device__ __forceinline__ void tile32_load(const double* __restrict__ g, int ld, double* __restrict__ s) {
+#pragma unroll
+    for (int e = threadIdx.x; e < TD * TD / 2; e += kPotrf64Threads) {
+        const int r = e >> 4, c = 2 * (e & 15);
+        const double2 v = *reinterpret_cast<const double2*>(g + static_cast<size_t>(r) * ld + c);
+        s[r * TDP + c] = v.x;
+        s[r * TDP + c + 1] = v.y;
+    }
+}
+// Rows (or columns) of a warp in a product with a triangular factor: four whose lengths add up to 66.
+__device__ __forceinline__ int balanced32(int warp, int m) {
+    return m == 0 ? warp : m == 1 ? 15 - warp : m == 2 ? 16 + warp : 31 - warp;
+}
+
+// A (lower triangle, np x np with identity padding) -> X = L^-1 in X and X^T in the upper triangle of A;
+// nt tiles of 32.  The steps of k_potrf_coop: panel and inverse row, barrier, trailing and inverse
+// update with the next diagonal tile factored by the block that updates it, barrier.
+__global__ void __launch_bounds__(kPotrf64Threads) k_potrf64_coop(double* __restrict__ A, double* __restrict__ X,
+                                                                  double* __restrict__ Dinv, int np, int nt,
+                                                                  int* __restrict__ status) {
+    cgk::grid_group grid = cgk::this_grid();
+    extern __shared__ __align__(16) double smem64[];
+    double* sA = smem64;
+    double* sB = sA + TD * TDP;
+    double* sC = sB + TD * TDP;
+    double* sT = sC + TD * TDP;
+    double* s_d = sT + TD * 9;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    auto tile = [np](double* M, int i, int j) { return M + static_cast<size_t>(i) * TD * np + static_cast<size_t>(j) * TD; };
+    // R = 0 below the diagonal tiles (X_kk is D_k itself)
+    for (int r = blockIdx.x; r < nt * TD; r += gridDim.x)
+        for (int c = tid; c < (r / TD) * TD; c += kPotrf64Threads) X[static_cast<size_t>(r) * np + c] = 0.0;
+    if (blockIdx.x == 0) {
+        tile32_load(A, np, sC);
+        __syncthreads();
+        diag_factor_inverse64(A, np, Dinv, sC, sA, sB, sT, s_d, status);
+    }
+    grid.sync();
+    for (int k = 0; k < nt; ++k) {
+        const int m = nt - 1 - k;
+        const double* Dk = Dinv + static_cast<size_t>(k) * TD * TD;
+        for (int it = blockIdx.x; it < m + k + 1; it += gridDim.x) {
+            tile32_load(Dk, TD, sB);
+            if (it < m) {
+                // L_ik = A_ik D_k^T: a lane per row, columns of equal total length per warp
+                double* Aik = tile(A, k + 1 + it, k);
+                tile32_load(Aik, np, sA);
+                __syncthreads();
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int c = balanced32(warp, q);
+                    double t = 0.0;
+#pragma unroll 8
+                    for (int l = 0; l <= c; ++l) t = fma(sA[lane * TDP + l], sB[c * TDP + l], t);
+                    sC[lane * TDP + c] = t;
+                }
+                __syncthreads();
+                for (int e = tid; e < TD * TD; e += kPotrf64Threads)
+                    Aik[static_cast<size_t>(e / TD) * np + e % TD] = sC[(e / TD) * TDP + e % TD];
+            } else {
+                // X_kj = D_k R_kj: a lane per column; X_kk = D_k
+                const int j = it - m;
+                double* Xkj = tile(X, k, j);
+                if (j < k) tile32_load(Xkj, np, sA);
+                __syncthreads();
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int r = balanced32(warp, q);
+                    double t = 0.0;
+                    if (j == k) t = sB[r * TDP + lane];
+                    else
+#pragma unroll 8
+                        for (int l = 0; l <= r; ++l) t = fma(sB[r * TDP + l], sA[l * TDP + lane], t);
+                    Xkj[static_cast<size_t>(r) * np + lane] = t;
+                }
+            }
+            __syncthreads();
+        }
+        grid.sync();
+        // trailing update and R update; item 0 is the next diagonal tile, updated and factored by
+        // block 0 while the other blocks share the rest
+        const int ntrail = m * (m + 1) / 2;
+        const int nitems = ntrail + m * (k + 1);
+        const int first_it = blockIdx.x == 0 ? 0 : (gridDim.x > 1 ? blockIdx.x : 1);
+        const int stride = gridDim.x > 1 ? static_cast<int>(gridDim.x) - 1 : 1;
+        for (int it = first_it; it < nitems; it = (it == 0 && gridDim.x > 1) ? nitems : it + stride) {
+            if (it == 0) {
+                const double* Lk = tile(A, k + 1, k);
+                double* Akk = tile(A, k + 1, k + 1);
+                tile32_load(Lk, np, sA);
+                tile32_load(Akk, np, sC);
+                __syncthreads();
+                // the lower triangle alone: 528 elements
+                for (int e = tid; e < TD * (TD + 1) / 2; e += kPotrf64Threads) {
+                    const int r = tri_row(e), c = e - r * (r + 1) / 2;
+                    double t = sC[r * TDP + c];
+#pragma unroll 8
+                    for (int l = 0; l < TD; ++l) t = fma(-sA[r * TDP + l], sA[c * TDP + l], t);
+                    sC[r * TDP + c] = t;
+                }
+                __syncthreads();
+                diag_factor_inverse64(Akk, np, Dinv + static_cast<size_t>(k + 1) * TD * TD, sC, sA, sB, sT, s_d, status);
+                __syncthreads();
+                continue;
+            }
+            double* dst;
+            const bool trail = it < ntrail;
+            if (trail) {
+                // A_ij -= L_ik L_jk^T
+                const int t = tri_row(it);
+                const int i = k + 1 + t, j = k + 1 + (it - t * (t + 1) / 2);
+                tile32_load(tile(A, i, k), np, sA);
+                tile32_load(tile(A, j, k), np, sB);
+                dst = tile(A, i, j);
+            } else {
+                // R_ij -= L_ik X_kj
+                const int q = it - ntrail;
+                const int i = k + 1 + q / (k + 1), j = q % (k + 1);
+                tile32_load(tile(A, i, k), np, sA);
+                tile32_load(tile(X, k, j), np, sB);
+                dst = tile(X, i, j);
+            }
+            double acc[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[q] = dst[static_cast<size_t>(warp + 8 * q) * np + lane];
+            __syncthreads();
+            const double* b = sB + (trail ? lane * TDP : lane);
+            const int bs = trail ? 1 : TDP;
+#pragma unroll 8
+            for (int l = 0; l < TD; ++l) {
+                const double bv = b[l * bs];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[q] = fma(-sA[(warp + 8 * q) * TDP + l], bv, acc[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) dst[static_cast<size_t>(warp + 8 * q) * np + lane] = acc[q];
+            __syncthreads();
+        }
+        grid.sync();
+    }
+    for (int it = blockIdx.x; it < nt * (nt + 1) / 2; it += gridDim.x) {
+        const int i = tri_row(it), j = it - i * (i + 1) / 2;
+        tile32_load(tile(X, i, j), np, sA);
+        __syncthreads();
+        double* dst = tile(A, j, i);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) dst[static_cast<size_t>(warp + 8 * q) * np + lane] = sA[lane * TDP + warp + 8 * q];
         __syncthreads();
     }
 }
@@ -782,7 +1034,8 @@ int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, cu
     const int n = W.n, np = W.np, nt = W.nt;
     const size_t two_tiles = 2 * static_cast<size_t>(TS) * TP * sizeof(T);
     static std::once_flag attrs;
-    std::call_once(attrs, [&] { set_smem<T>(reinterpret_cast<const void*>(&k_potrf_coop<T>), two_tiles); });
+    if constexpr (sizeof(T) == 4)
+        std::call_once(attrs, [&] { set_smem<T>(reinterpret_cast<const void*>(&k_potrf_coop<T>), two_tiles); });
     int L = 0;
     cudaMemsetAsync(W.status, 0, sizeof(int), st);
     cudaMemsetAsync(W.A, 0, static_cast<size_t>(np) * np * sizeof(T), st);
@@ -792,25 +1045,29 @@ int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, cu
     if (nfill > 0) k_dense_fill<T><<<static_cast<unsigned>((nfill + 255) / 256), 256, 0, st>>>(sys, W.dscale, W.A, np);
     k_dense_diag<T><<<(np + 255) / 256, 256, 0, st>>>(W.A, n, np, shift);
     L += 3;
+    constexpr bool f64 = sizeof(T) == 8;
+    const void* kernel;
+    if constexpr (f64) kernel = reinterpret_cast<const void*>(&k_potrf64_coop);
+    else kernel = reinterpret_cast<const void*>(&k_potrf_coop<T>);
+    const int threads = f64 ? kPotrf64Threads : 256;
+    const size_t smem = f64 ? kPotrf64Smem : two_tiles;
     if (W.fact_grid == 0) {
         int dev = 0, sms = 0, per_sm = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_potrf_coop<T>, 256, two_tiles);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
         W.fact_grid = std::max(1, std::min(per_sm, 2) * sms);
     }
     {
         T* A = W.A;
         T* X = W.X;
         T* Dv = W.Dinv;
-        int npv = np, ntv = nt;
+        int npv = np, ntv = f64 ? (n + TD - 1) / TD : nt;
         int* stv = W.status;
         void* args[] = {&A, &X, &Dv, &npv, &ntv, &stv};
         // one block per lower tile at most: small systems take a small grid
-        const int fgrid = std::max(1, std::min(W.fact_grid, nt * (nt + 1) / 2));
-        if (cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&k_potrf_coop<T>), dim3(fgrid), dim3(256),
-                                        args, two_tiles, st) != cudaSuccess)
-            return -1;
+        const int fgrid = std::max(1, std::min(W.fact_grid, ntv * (ntv + 1) / 2));
+        if (cudaLaunchCooperativeKernel(kernel, dim3(fgrid), dim3(threads), args, smem, st) != cudaSuccess) return -1;
         ++L;
     }
     if (launches) *launches += L;
