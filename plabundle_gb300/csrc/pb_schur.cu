@@ -15,12 +15,12 @@
 //     Jacobi-scaled S (FP64, or FP32 when mixed precision is requested), to
 //     |b - S x| <= max(relative_tolerance |b|, absolute_tolerance);
 //   - the eliminated steps are y_e = V_e^-1 (-g_e - W_e^T x).
-// Kernels: one thread per eliminated block for the inverses and Y = W V^-1; one thread per row of
-// each upper primary block of S, summing its terms over a host-built list of coupling pairs in a
-// fixed order (no atomics: the result is deterministic); one thread per primary row for b; the
-// dense factor and CG of pb_dense.cu on S held as a dense block (ncb = 0, nb = n); one thread per
-// eliminated block for the back-substitution.  The pattern (coupling order, pair lists) is built
-// once per structure and reused while the structure hash is unchanged.
+// Kernels: one thread per coupling for Y = W V^-1 (and one per eliminated block for its inverse); one
+// CTA per segment of the host-built list of coupling pairs of an upper primary block of S, then one
+// thread per entry of S adding the segments in order (no atomics: the result is deterministic); one CTA
+// per primary block for b; the dense factor and CG of pb_dense.cu on S held as a dense block (ncb = 0,
+// nb = n); four lanes per eliminated block for the back-substitution.  The pattern (coupling order, pair
+// lists) is built once per structure and reused while the structure hash is unchanged.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -49,121 +49,194 @@ void bne_couplings(const pb_bne* q, const std::vector<int>** elim, const std::ve
 namespace {
 
 constexpr int kEb = 3;
-constexpr int kMaxPb = PB_BNE_MAX_PRIMARY_BLOCK_SIZE;
+constexpr int kGatherThreads = 192;  // of the 169 elements of a pair of 13-column blocks, 88 % of the lanes work
+constexpr int kSegItems = 64;        // coupling pairs of one block that one CTA sums
 
-// Eliminated blocks: damped inverse, q = V^-1 g_e, and Y_c = W_c V^-1 for each coupling of e.
-__global__ void k_schur_eliminate(int E, int pb, double damping, const double* __restrict__ hee,
-                                  const int* __restrict__ e_begin, const double* __restrict__ cpl,
-                                  double* __restrict__ vinv, double* __restrict__ Y, int* __restrict__ flags) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E) return;
+// Damped inverse of an eliminated block (row-major); false when singular.
+__device__ __forceinline__ bool damped_inverse(const double* __restrict__ h, double damping, double* inv) {
     double V[9];
-    for (int i = 0; i < 9; ++i) V[i] = hee[static_cast<size_t>(e) * 9 + i];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) V[i] = h[i];
+#pragma unroll
     for (int d = 0; d < 3; ++d) V[d * 4] *= 1.0 + damping;
     const double c00 = V[4] * V[8] - V[5] * V[7], c01 = V[5] * V[6] - V[3] * V[8], c02 = V[3] * V[7] - V[4] * V[6];
     const double det = V[0] * c00 + V[1] * c01 + V[2] * c02;
-    double inv[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     if (!(fabs(det) > 1e-15) || !isfinite(det)) {
-        atomicOr(flags, 1);
-    } else {
-        const double id = 1.0 / det;
-        inv[0] = c00 * id;
-        inv[1] = (V[2] * V[7] - V[1] * V[8]) * id;
-        inv[2] = (V[1] * V[5] - V[2] * V[4]) * id;
-        inv[3] = c01 * id;
-        inv[4] = (V[0] * V[8] - V[2] * V[6]) * id;
-        inv[5] = (V[2] * V[3] - V[0] * V[5]) * id;
-        inv[6] = c02 * id;
-        inv[7] = (V[1] * V[6] - V[0] * V[7]) * id;
-        inv[8] = (V[0] * V[4] - V[1] * V[3]) * id;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) inv[i] = 0.0;
+        return false;
     }
-    for (int i = 0; i < 9; ++i) vinv[static_cast<size_t>(e) * 9 + i] = inv[i];
-    for (int c = e_begin[e]; c < e_begin[e + 1]; ++c) {
-        const double* W = cpl + static_cast<size_t>(c) * pb * kEb;
-        double* y = Y + static_cast<size_t>(c) * pb * kEb;
-        for (int a = 0; a < pb; ++a)
-            for (int k = 0; k < kEb; ++k)
-                y[a * kEb + k] = W[a * kEb] * inv[k] + W[a * kEb + 1] * inv[3 + k] + W[a * kEb + 2] * inv[6 + k];
+    const double id = 1.0 / det;
+    inv[0] = c00 * id;
+    inv[1] = (V[2] * V[7] - V[1] * V[8]) * id;
+    inv[2] = (V[1] * V[5] - V[2] * V[4]) * id;
+    inv[3] = c01 * id;
+    inv[4] = (V[0] * V[8] - V[2] * V[6]) * id;
+    inv[5] = (V[2] * V[3] - V[0] * V[5]) * id;
+    inv[6] = c02 * id;
+    inv[7] = (V[1] * V[6] - V[0] * V[7]) * id;
+    inv[8] = (V[0] * V[4] - V[1] * V[3]) * id;
+    return true;
+}
+
+// Threads 0 .. E - 1: the damped inverse of their eliminated block.  Threads E .. E + ncpl - 1: Y_c = W_c V^-1
+// of their coupling, with the inverse formed again (about 50 FP64 operations next to the 117 of the
+// product).  A thread per coupling instead of one per eliminated block: a block's couplings no longer
+// wait for each other on the few warps that the blocks fill.
+__global__ void __launch_bounds__(128) k_schur_eliminate(int E, int ncpl, int pb, double damping,
+                                                         const double* __restrict__ hee, const int* __restrict__ cpl_elim,
+                                                         const double* __restrict__ cpl, double* __restrict__ vinv,
+                                                         double* __restrict__ Y, int* __restrict__ flags) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= E + ncpl) return;
+    const int c = t - E, e = c < 0 ? t : cpl_elim[c];
+    double inv[9];
+    const bool ok = damped_inverse(hee + static_cast<size_t>(e) * 9, damping, inv);
+    if (c < 0) {
+        if (!ok) atomicOr(flags, 1);
+#pragma unroll
+        for (int i = 0; i < 9; ++i) vinv[static_cast<size_t>(e) * 9 + i] = inv[i];
+        return;
+    }
+    const double* W = cpl + static_cast<size_t>(c) * pb * kEb;
+    double* y = Y + static_cast<size_t>(c) * pb * kEb;
+#pragma unroll 4
+    for (int a = 0; a < pb; ++a) {
+        const double w0 = W[a * kEb], w1 = W[a * kEb + 1], w2 = W[a * kEb + 2];
+#pragma unroll
+        for (int k = 0; k < kEb; ++k) y[a * kEb + k] = w0 * inv[k] + w1 * inv[3 + k] + w2 * inv[6 + k];
     }
 }
 
-// Row a of upper block (bi, bj) of S: damped H_pp minus the Schur terms of its coupling pairs.
-__global__ void k_schur_gather(int nblocks, int pb, int n, double damping, const int* __restrict__ blk_i,
-                               const int* __restrict__ blk_j, const int* __restrict__ blk_src,
-                               const int* __restrict__ item_begin, const int2* __restrict__ items,
-                               const double* __restrict__ diag, const double* __restrict__ off,
-                               const double* __restrict__ Y, const double* __restrict__ cpl, double* __restrict__ S) {
-    const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= static_cast<long long>(nblocks) * pb) return;
-    const int blk = static_cast<int>(t / pb), a = static_cast<int>(t - static_cast<long long>(blk) * pb);
-    const int bi = blk_i[blk], bj = blk_j[blk], src = blk_src[blk];
-    double acc[kMaxPb];
-    const double* H = nullptr;
-    if (bi == bj) H = diag + static_cast<size_t>(bi) * pb * pb;
-    else if (src >= 0) H = off + static_cast<size_t>(src) * pb * pb;
-#pragma unroll
-    for (int b = 0; b < kMaxPb; ++b) acc[b] = (b < pb && H) ? H[a * pb + b] : 0.0;
-    if (bi == bj) {
-        // damping of the primary diagonal (a structurally empty entry becomes 1)
-#pragma unroll
-        for (int b = 0; b < kMaxPb; ++b)
-            if (b == a) acc[b] = acc[b] != 0.0 ? acc[b] * (1.0 + damping) : 1.0;
-    }
-    for (int it = item_begin[blk]; it < item_begin[blk + 1]; ++it) {
-        const int2 cc = items[it];
-        const double* y = Y + static_cast<size_t>(cc.x) * pb * kEb + a * kEb;
-        const double y0 = y[0], y1 = y[1], y2 = y[2];
-        const double* W = cpl + static_cast<size_t>(cc.y) * pb * kEb;
-#pragma unroll
-        for (int b = 0; b < kMaxPb; ++b)
-            if (b < pb) acc[b] -= y0 * W[b * kEb] + y1 * W[b * kEb + 1] + y2 * W[b * kEb + 2];
-    }
-    const size_t row = static_cast<size_t>(bi) * pb + a;
-#pragma unroll
-    for (int b = 0; b < kMaxPb; ++b) {
-        if (b >= pb) break;
-        const size_t col = static_cast<size_t>(bj) * pb + b;
-        S[row * n + col] = acc[b];
-        if (bi != bj) S[col * n + row] = acc[b];
-    }
-}
-
-// b = -g_p + sum_c Y_c g_e(c) per primary row; couplings of each primary block in p_list.
-__global__ void k_schur_rhs(int n, int pb, const double* __restrict__ gp, const int* __restrict__ p_begin,
-                            const int* __restrict__ p_list, const int* __restrict__ cpl_elim,
-                            const double* __restrict__ Y, const double* __restrict__ ge, double* __restrict__ b) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n) return;
-    const int blk = r / pb, a = r - blk * pb;
-    double v = -gp[r];
-    for (int k = p_begin[blk]; k < p_begin[blk + 1]; ++k) {
-        const int c = p_list[k];
-        const double* y = Y + static_cast<size_t>(c) * pb * kEb + a * kEb;
-        const double* g = ge + static_cast<size_t>(cpl_elim[c]) * kEb;
-        v += y[0] * g[0] + y[1] * g[1] + y[2] * g[2];
-    }
-    b[r] = v;
-}
-
-// y_e = V_e^-1 (-g_e - sum_c W_c^T x_prim(c)).
-__global__ void k_schur_backsub(int E, int pb, const int* __restrict__ e_begin, const int* __restrict__ cpl_prim,
-                                const double* __restrict__ cpl, const double* __restrict__ vinv,
-                                const double* __restrict__ ge, const double* __restrict__ x, double* __restrict__ y) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E) return;
-    double r[3] = {-ge[static_cast<size_t>(e) * 3], -ge[static_cast<size_t>(e) * 3 + 1], -ge[static_cast<size_t>(e) * 3 + 2]};
-    for (int c = e_begin[e]; c < e_begin[e + 1]; ++c) {
-        const double* W = cpl + static_cast<size_t>(c) * pb * kEb;
-        const double* xp = x + static_cast<size_t>(cpl_prim[c]) * pb;
-        for (int a = 0; a < pb; ++a) {
-            const double xa = xp[a];
-            r[0] -= W[a * kEb] * xa;
-            r[1] -= W[a * kEb + 1] * xa;
-            r[2] -= W[a * kEb + 2] * xa;
+// Partial sums of the Schur terms sum Y_c1 W_c2^T of one segment (at most kSegItems consecutive
+// coupling pairs of one upper block), a thread per element of the block (of its upper triangle for a
+// diagonal block) and the pairs dealt to as many thread groups as fit, whose sums are added in
+// order.  FP64-bound: three FMAs per element and pair.
+__global__ void __launch_bounds__(kGatherThreads) k_schur_gather(int pb, const int* __restrict__ seg_blk,
+                                                                 const int* __restrict__ seg_begin,
+                                                                 const int* __restrict__ blk_i,
+                                                                 const int* __restrict__ blk_j,
+                                                                 const int2* __restrict__ items,
+                                                                 const double* __restrict__ Y,
+                                                                 const double* __restrict__ cpl,
+                                                                 double* __restrict__ part) {
+    __shared__ double s_acc[kGatherThreads + 64];
+    const int seg = blockIdx.x, blk = seg_blk[seg];
+    const bool diag = blk_i[blk] == blk_j[blk];
+    const int ne = diag ? pb * (pb + 1) / 2 : pb * pb;
+    const int groups = max(1, kGatherThreads / ne);
+    const int i0 = seg_begin[seg], i1 = seg_begin[seg + 1];
+    for (int e0 = 0; e0 < ne; e0 += kGatherThreads) {  // (once, up to thirteen columns)
+        const int g = threadIdx.x / ne, e = e0 + (groups > 1 ? threadIdx.x - g * ne : threadIdx.x);
+        const bool mine = (groups == 1 || g < groups) && e < ne;
+        double acc = 0.0;
+        int a = 0, b = 0;
+        if (mine) {
+            if (diag) {  // e-th element of the upper triangle, column by column
+                while ((b + 1) * (b + 2) / 2 <= e) ++b;
+                a = e - b * (b + 1) / 2;
+            } else {
+                a = e / pb;
+                b = e - a * pb;
+            }
+#pragma unroll 4
+            for (int it = i0 + (groups > 1 ? g : 0); it < i1; it += groups) {
+                const int2 cc = items[it];
+                const double* y = Y + (static_cast<size_t>(cc.x) * pb + a) * kEb;
+                const double* W = cpl + (static_cast<size_t>(cc.y) * pb + b) * kEb;
+                acc = fma(y[2], W[2], fma(y[1], W[1], fma(y[0], W[0], acc)));
+            }
+        }
+        if (groups > 1) {
+            s_acc[threadIdx.x] = acc;
+            __syncthreads();
+            if (threadIdx.x < ne)
+                for (int q = 1; q < groups; ++q) acc += s_acc[q * ne + threadIdx.x];
+        }
+        if (mine && (groups == 1 || g == 0)) {
+            double* p = part + static_cast<size_t>(seg) * pb * pb;
+            p[a * pb + b] = acc;
+            if (diag) p[b * pb + a] = acc;
         }
     }
-    const double* iv = vinv + static_cast<size_t>(e) * 9;
-    for (int k = 0; k < 3; ++k) y[static_cast<size_t>(e) * 3 + k] = iv[k * 3] * r[0] + iv[k * 3 + 1] * r[1] + iv[k * 3 + 2] * r[2];
+}
+
+// Upper blocks of S (and their transposes): damped H_pp minus the block's segments, in order.
+__global__ void __launch_bounds__(256) k_schur_sum(int nblocks, int pb, int n, double damping, const int* __restrict__ blk_i,
+                                                   const int* __restrict__ blk_j, const int* __restrict__ blk_src,
+                                                   const int* __restrict__ blk_seg, const double* __restrict__ diag,
+                                                   const double* __restrict__ off, const double* __restrict__ part,
+                                                   double* __restrict__ S) {
+    const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int pp = pb * pb;
+    if (t >= static_cast<long long>(nblocks) * pp) return;
+    const int blk = static_cast<int>(t / pp), e = static_cast<int>(t - static_cast<long long>(blk) * pp);
+    const int a = e / pb, b = e - a * pb;
+    const int bi = blk_i[blk], bj = blk_j[blk], src = blk_src[blk];
+    double v = 0.0;
+    if (bi == bj) v = diag[static_cast<size_t>(bi) * pp + e];
+    else if (src >= 0) v = off[static_cast<size_t>(src) * pp + e];
+    // damping of the primary diagonal (a structurally empty entry becomes 1)
+    if (bi == bj && a == b) v = v != 0.0 ? v * (1.0 + damping) : 1.0;
+#pragma unroll 4
+    for (int s = blk_seg[blk]; s < blk_seg[blk + 1]; ++s) v -= part[static_cast<size_t>(s) * pp + e];
+    const size_t row = static_cast<size_t>(bi) * pb + a, col = static_cast<size_t>(bj) * pb + b;
+    S[row * n + col] = v;
+    if (bi != bj) S[col * n + row] = v;
+}
+
+// b = -g_p + sum_c Y_c g_e(c): one block per primary block, its couplings dealt to thread groups of pb
+// rows, the groups' sums added in order.
+__global__ void __launch_bounds__(256) k_schur_rhs(int pb, const double* __restrict__ gp, const int* __restrict__ p_begin,
+                                                   const int* __restrict__ p_list, const int* __restrict__ cpl_elim,
+                                                   const double* __restrict__ Y, const double* __restrict__ ge,
+                                                   double* __restrict__ b) {
+    __shared__ double s_acc[256];
+    const int blk = blockIdx.x, groups = 256 / pb;
+    const int g = threadIdx.x / pb, a = threadIdx.x - g * pb;
+    double v = 0.0;
+    if (g < groups)
+#pragma unroll 4
+        for (int k = p_begin[blk] + g; k < p_begin[blk + 1]; k += groups) {
+            const int c = p_list[k];
+            const double* y = Y + (static_cast<size_t>(c) * pb + a) * kEb;
+            const double* q = ge + static_cast<size_t>(cpl_elim[c]) * kEb;
+            v = fma(y[2], q[2], fma(y[1], q[1], fma(y[0], q[0], v)));
+        }
+    s_acc[threadIdx.x] = v;
+    __syncthreads();
+    if (threadIdx.x < pb) {
+        double t = -gp[static_cast<size_t>(blk) * pb + threadIdx.x];
+        for (int q = 0; q < groups; ++q) t += s_acc[q * pb + threadIdx.x];
+        b[static_cast<size_t>(blk) * pb + threadIdx.x] = t;
+    }
+}
+
+// y_e = V_e^-1 (-g_e - sum_c W_c^T x_prim(c)): four lanes per eliminated block, lane k < 3 its k-th
+// component (neighbouring lanes read neighbouring columns of W).
+__global__ void __launch_bounds__(128) k_schur_backsub(int E, int pb, const int* __restrict__ e_begin,
+                                                       const int* __restrict__ cpl_prim, const double* __restrict__ cpl,
+                                                       const double* __restrict__ vinv, const double* __restrict__ ge,
+                                                       const double* __restrict__ x, double* __restrict__ y) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, e = t >> 2, k = t & 3, kk = min(k, 2);
+    const int base = threadIdx.x & 28;
+    double r = 0.0;
+    if (e < E) {
+        r = -ge[static_cast<size_t>(e) * 3 + kk];
+        for (int c = e_begin[e]; c < e_begin[e + 1]; ++c) {
+            const double* W = cpl + static_cast<size_t>(c) * pb * kEb + kk;
+            const double* xp = x + static_cast<size_t>(cpl_prim[c]) * pb;
+#pragma unroll 8
+            for (int a = 0; a < pb; ++a) r = fma(-W[a * kEb], xp[a], r);
+        }
+    }
+    __syncwarp();
+    const double r0 = __shfl_sync(0xffffffffu, r, base), r1 = __shfl_sync(0xffffffffu, r, base + 1),
+                 r2 = __shfl_sync(0xffffffffu, r, base + 2);
+    if (e < E && k < 3) {
+        const double* iv = vinv + static_cast<size_t>(e) * 9 + k * 3;
+        y[static_cast<size_t>(e) * 3 + k] = iv[0] * r0 + iv[1] * r1 + iv[2] * r2;
+    }
 }
 
 // r = b - S x0 (dense FP64 rows, one warp per row) for a warm start; out[0] = |r|^2 partials per row
@@ -209,7 +282,10 @@ struct SchurWork {
     Arena pattern, values, dense;
     // pattern
     int *e_begin = nullptr, *cpl_prim = nullptr, *cpl_elim = nullptr, *p_begin = nullptr, *p_list = nullptr;
-    int *blk_i = nullptr, *blk_j = nullptr, *blk_src = nullptr, *item_begin = nullptr, *zero = nullptr;
+    int *blk_i = nullptr, *blk_j = nullptr, *blk_src = nullptr, *blk_seg = nullptr, *seg_blk = nullptr,
+        *seg_begin = nullptr, *zero = nullptr;
+    int nseg = 0;
+    double* part = nullptr;  // Schur terms of the segments
     int2* items = nullptr;
     // values and work
     double *diag = nullptr, *off = nullptr, *gp = nullptr, *hee = nullptr, *ge = nullptr, *cpl = nullptr;
@@ -349,12 +425,19 @@ void build_pattern(SchurWork* w, const pb_bne* q) {
             for (int c2 = c1; c2 < e_begin[e + 1]; ++c2) add_item(block_of(sprim[c1], sprim[c2]), make_int2(c1, c2));
     w->nblocks = static_cast<int>(bi.size());
     blk_items.resize(w->nblocks);
-    std::vector<int> item_begin(w->nblocks + 1, 0);
+    // segments of at most kSegItems consecutive items of one block
+    std::vector<int> blk_seg(1, 0), seg_blk, seg_begin(1, 0);
     std::vector<int2> items;
     for (int k = 0; k < w->nblocks; ++k) {
-        items.insert(items.end(), blk_items[k].begin(), blk_items[k].end());
-        item_begin[k + 1] = static_cast<int>(items.size());
+        for (size_t i = 0; i < blk_items[k].size(); i += kSegItems) {
+            const size_t i1 = std::min(blk_items[k].size(), i + kSegItems);
+            items.insert(items.end(), blk_items[k].begin() + i, blk_items[k].begin() + i1);
+            seg_blk.push_back(k);
+            seg_begin.push_back(static_cast<int>(items.size()));
+        }
+        blk_seg.push_back(static_cast<int>(seg_blk.size()));
     }
+    w->nseg = static_cast<int>(seg_blk.size());
     w->nitems = static_cast<int>(items.size());
     auto up = [&](auto& arena, const auto& v) {
         using T = typename std::decay_t<decltype(v)>::value_type;
@@ -370,7 +453,9 @@ void build_pattern(SchurWork* w, const pb_bne* q) {
     w->blk_i = up(w->pattern, bi);
     w->blk_j = up(w->pattern, bj);
     w->blk_src = up(w->pattern, bsrc);
-    w->item_begin = up(w->pattern, item_begin);
+    w->blk_seg = up(w->pattern, blk_seg);
+    w->seg_blk = up(w->pattern, seg_blk);
+    w->seg_begin = up(w->pattern, seg_begin);
     w->items = up(w->pattern, items);
     w->zero = up(w->pattern, std::vector<int>{0});
     const size_t n = static_cast<size_t>(w->n);
@@ -382,6 +467,7 @@ void build_pattern(SchurWork* w, const pb_bne* q) {
     w->cpl = w->values.alloc<double>(static_cast<size_t>(w->ncpl) * pbs * kEb);
     w->vinv = w->values.alloc<double>(static_cast<size_t>(E) * 9);
     w->Y = w->values.alloc<double>(static_cast<size_t>(w->ncpl) * pbs * kEb);
+    w->part = w->values.alloc<double>(static_cast<size_t>(w->nseg) * pbs * pbs);
     w->S = w->values.alloc<double>(n * n);
     w->b = w->values.alloc<double>(n);
     w->x = w->values.alloc<double>(n);
@@ -490,15 +576,17 @@ int schur_solve(SchurWork* w, int device, cudaStream_t st, const pb_bne* q, doub
     cudaMemsetAsync(w->S, 0, static_cast<size_t>(n) * n * sizeof(double), st);
     cudaEventRecord(w->ev[0], st);
     if (E > 0)
-        k_schur_eliminate<<<(E + 127) / 128, 128, 0, st>>>(E, pbs, damping, w->hee, w->e_begin, w->cpl, w->vinv, w->Y,
-                                                          w->flags);
+        k_schur_eliminate<<<(E + w->ncpl + 127) / 128, 128, 0, st>>>(E, w->ncpl, pbs, damping, w->hee, w->cpl_elim, w->cpl,
+                                                                    w->vinv, w->Y, w->flags);
     cudaEventRecord(w->ev[1], st);
-    const long long rows = static_cast<long long>(w->nblocks) * pbs;
-    if (rows > 0)
-        k_schur_gather<<<static_cast<unsigned>((rows + 127) / 128), 128, 0, st>>>(
-            w->nblocks, pbs, n, damping, w->blk_i, w->blk_j, w->blk_src, w->item_begin, w->items, w->diag, w->off, w->Y,
-            w->cpl, w->S);
-    if (n > 0) k_schur_rhs<<<(n + 127) / 128, 128, 0, st>>>(n, pbs, w->gp, w->p_begin, w->p_list, w->cpl_elim, w->Y, w->ge, w->b);
+    if (w->nseg > 0)
+        k_schur_gather<<<w->nseg, kGatherThreads, 0, st>>>(pbs, w->seg_blk, w->seg_begin, w->blk_i, w->blk_j, w->items, w->Y,
+                                                          w->cpl, w->part);
+    const long long entries = static_cast<long long>(w->nblocks) * pbs * pbs;
+    if (entries > 0)
+        k_schur_sum<<<static_cast<unsigned>((entries + 255) / 256), 256, 0, st>>>(
+            w->nblocks, pbs, n, damping, w->blk_i, w->blk_j, w->blk_src, w->blk_seg, w->diag, w->off, w->part, w->S);
+    if (n > 0) k_schur_rhs<<<P, 256, 0, st>>>(pbs, w->gp, w->p_begin, w->p_list, w->cpl_elim, w->Y, w->ge, w->b);
     cudaEventRecord(w->ev[2], st);
     if (cudaGetLastError() != cudaSuccess) {
         *err = "block-Schur assembly launch failed";
@@ -522,7 +610,7 @@ int schur_solve(SchurWork* w, int device, cudaStream_t st, const pb_bne* q, doub
     if (n == 0) {
         rep->converged = 1;
         if (E > 0) {
-            k_schur_backsub<<<(E + 127) / 128, 128, 0, st>>>(E, pbs, w->e_begin, w->cpl_prim, w->cpl, w->vinv, w->ge, w->x, w->y);
+            k_schur_backsub<<<(4 * E + 127) / 128, 128, 0, st>>>(E, pbs, w->e_begin, w->cpl_prim, w->cpl, w->vinv, w->ge, w->x, w->y);
             cudaMemcpyAsync(eliminated_step, w->y, static_cast<size_t>(E) * 3 * sizeof(double), cudaMemcpyDeviceToHost, st);
         }
         cudaStreamSynchronize(st);
@@ -560,7 +648,7 @@ int schur_solve(SchurWork* w, int device, cudaStream_t st, const pb_bne* q, doub
     cudaMemcpyAsync(hb.data(), w->r0, static_cast<size_t>(n) * sizeof(double), cudaMemcpyDeviceToHost, st);
     cudaEventRecord(w->ev[6], st);
     if (E > 0)
-        k_schur_backsub<<<(E + 127) / 128, 128, 0, st>>>(E, pbs, w->e_begin, w->cpl_prim, w->cpl, w->vinv, w->ge, w->x, w->y);
+        k_schur_backsub<<<(4 * E + 127) / 128, 128, 0, st>>>(E, pbs, w->e_begin, w->cpl_prim, w->cpl, w->vinv, w->ge, w->x, w->y);
     cudaEventRecord(w->ev[7], st);
     if (primary_step)
         cudaMemcpyAsync(primary_step, w->x, static_cast<size_t>(n) * sizeof(double), cudaMemcpyDeviceToHost, st);
