@@ -52,10 +52,202 @@ __device__ __forceinline__ int info_group(int info) { return ((info >> 2) & 7) -
 // per-observation track record: first observation (8 bits) | chunk track slot (8) | length (16)
 __device__ __forceinline__ int trk_slot(int v) { return (v >> 8) & 0xFF; }
 
+// The six sums of an owned row in phase D.  The FP32 path keeps them as three packed pairs: a term of a
+// coupling is 108 packed operations and 15 loads instead of 216 and 21, each half rounded as the scalar
+// operations round it, in the same order (100 cameras, 780 000 observations, two groups of eight
+// intrinsics: 1555 -> 1416 us a launch).
+template <typename T>
+struct RowAcc;
+template <>
+struct RowAcc<double> {
+    Acc<double> a[6];
+    // += J0 u0 + J1 u1 for the pose columns of two Jacobian rows
+    __device__ __forceinline__ void jacobian(const double* J0, const double* J1, double u0, double u1) {
+#pragma unroll
+        for (int y = 0; y < 6; ++y) {
+            acc_fma(a[y], J0[y], u0);
+            acc_fma(a[y], J1[y], u1);
+        }
+    }
+    // += G (g0, g1, g2)^T (LEFT: g is the left factor of the products)
+    template <bool LEFT>
+    __device__ __forceinline__ void coupling(const double* G, double g0, double g1, double g2) {
+#pragma unroll
+        for (int y = 0; y < 6; ++y) {
+            acc_fma(a[y], g0, G[3 * y]);
+            acc_fma(a[y], g1, G[3 * y + 1]);
+            acc_fma(a[y], g2, G[3 * y + 2]);
+        }
+    }
+    __device__ __forceinline__ void add(const double* g) {
+#pragma unroll
+        for (int y = 0; y < 6; ++y) a[y].add(g[y]);
+    }
+    __device__ __forceinline__ double part(int y) const { return a[y].part(); }
+};
+template <>
+struct RowAcc<float> {
+    Acc2 a[3];
+    __device__ __forceinline__ void jacobian(const float* J0, const float* J1, ff u0, ff u1) {
+        const f2 h0 = f2_both(u0.hi), nh0 = f2_both(-u0.hi), nl0 = f2_both(-u0.lo);
+        const f2 h1 = f2_both(u1.hi), nh1 = f2_both(-u1.hi), nl1 = f2_both(-u1.lo);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            a[q].fma_f(f2_pack(J0[2 * q], J0[2 * q + 1]), h0, nh0, nl0);
+            a[q].fma_f(f2_pack(J1[2 * q], J1[2 * q + 1]), h1, nh1, nl1);
+        }
+    }
+    template <bool LEFT>
+    __device__ __forceinline__ void coupling(const float4* G, ff g0, ff g1, ff g2) {
+        const ulonglong2* G2 = reinterpret_cast<const ulonglong2*>(G);
+        const ff g[3] = {g0, g1, g2};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const f2 h = f2_both(g[k].hi), nh = f2_both(-g[k].hi), nl = f2_both(-g[k].lo);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const ulonglong2 v = G2[k * 3 + q];
+                a[q].template fma_ff<LEFT>(h, nh, nl, v.x, v.y);
+            }
+        }
+    }
+    __device__ __forceinline__ void add(const ff* g) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            a[q].add(f2_pack(g[2 * q].hi, g[2 * q + 1].hi));
+            a[q].lo = f2_add(a[q].lo, f2_pack(g[2 * q].lo, g[2 * q + 1].lo));
+        }
+    }
+    __device__ __forceinline__ float2 part(int y) const {
+        const float2 h = f2_parts(a[y >> 1].hi), l = f2_parts(a[y >> 1].lo);
+        return y & 1 ? make_float2(h.y, l.y) : make_float2(h.x, l.x);
+    }
+};
+
+// Two neighbouring columns of a track's K: sums of a0 y0 + a1 y1 over its observations.
+template <typename T>
+struct ColumnPair;
+template <>
+struct ColumnPair<double> {
+    double s0 = 0.0, s1 = 0.0;
+    __device__ __forceinline__ void add(double a0, double b0, double y0, double a1, double b1, double y1) {
+        s0 = s0 + (a0 * y0 + a1 * y1);
+        s1 = s1 + (b0 * y0 + b1 * y1);
+    }
+    __device__ __forceinline__ double first() const { return s0; }
+    __device__ __forceinline__ double second() const { return s1; }
+};
+template <>
+struct ColumnPair<float> {
+    ff2p s{0ull, 0ull};
+    __device__ __forceinline__ void add(float a0, float b0, ff y0, float a1, float b1, ff y1) {
+        s = s + (f2_pack(a0, b0) * y0 + f2_pack(a1, b1) * y1);
+    }
+    __device__ __forceinline__ ff first() const { return {f2_parts(s.hi).x, f2_parts(s.lo).x}; }
+    __device__ __forceinline__ ff second() const { return {f2_parts(s.hi).y, f2_parts(s.lo).y}; }
+};
+
+// Four neighbouring entries of a row of the intrinsic block (or of its gradient).  Four at a time read
+// the row's own factors, the weight and the group marks once, and the FP32 path sums them as two packed
+// pairs: with a warp per entry the phase took 64 000 of a chunk's 190 000 cycles (same launch, this and
+// ColumnPair: 1416 -> 1200 us).
+template <typename T>
+struct QuadAcc;
+template <>
+struct QuadAcc<double> {
+    Acc<double> a[4];
+    __device__ __forceinline__ void weighted(double w, double r, double b0, double b1, double b2, double b3) {
+        acc_fma(a[0], w, r * b0);
+        acc_fma(a[1], w, r * b1);
+        acc_fma(a[2], w, r * b2);
+        acc_fma(a[3], w, r * b3);
+    }
+    __device__ __forceinline__ void minus(double r, double b0, double b1, double b2, double b3) {
+        acc_fma(a[0], -r, b0);
+        acc_fma(a[1], -r, b1);
+        acc_fma(a[2], -r, b2);
+        acc_fma(a[3], -r, b3);
+    }
+    __device__ __forceinline__ void jacobian(double b0, double b1, double b2, double b3, double r) { minus(-r, b0, b1, b2, b3); }
+    __device__ __forceinline__ void add(double b0, double b1, double b2, double b3) {
+        a[0].add(b0);
+        a[1].add(b1);
+        a[2].add(b2);
+        a[3].add(b3);
+    }
+    __device__ __forceinline__ void split(Acc<double>* q) const {
+        for (int i = 0; i < 4; ++i) q[i] = a[i];
+    }
+};
+template <>
+struct QuadAcc<float> {
+    Acc2 a[2];
+    // += w (r b): the product r b exact, acc_fma of w and it
+    __device__ __forceinline__ void weighted(ff w, float r, float b0, float b1, float b2, float b3) {
+        const f2 wh = f2_both(w.hi), nwh = f2_both(-w.hi), nwl = f2_both(-w.lo), rr = f2_both(r), nr = f2_both(-r);
+        const f2 b[2] = {f2_pack(b0, b1), f2_pack(b2, b3)};
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const f2 h = f2_mul(rr, b[q]), nl = f2_fma(nr, b[q], h);  // r b = h - nl
+            const f2 p = f2_mul(wh, h);
+            const f2 ne = f2_fma(nwl, h, f2_fma(wh, nl, f2_fma(nwh, h, p)));
+            a[q].add(p);
+            a[q].lo = f2_sub(a[q].lo, ne);
+        }
+    }
+    // += (-r) b
+    __device__ __forceinline__ void minus(ff r, ff b0, ff b1, ff b2, ff b3) {
+        const f2 h = f2_both(-r.hi), nh = f2_both(r.hi), nl = f2_both(r.lo);
+        a[0].template fma_ff<true>(h, nh, nl, f2_pack(b0.hi, b1.hi), f2_pack(b0.lo, b1.lo));
+        a[1].template fma_ff<true>(h, nh, nl, f2_pack(b2.hi, b3.hi), f2_pack(b2.lo, b3.lo));
+    }
+    __device__ __forceinline__ void jacobian(float b0, float b1, float b2, float b3, ff r) {
+        const f2 h = f2_both(r.hi), nh = f2_both(-r.hi), nl = f2_both(-r.lo);
+        a[0].fma_f(f2_pack(b0, b1), h, nh, nl);
+        a[1].fma_f(f2_pack(b2, b3), h, nh, nl);
+    }
+    __device__ __forceinline__ void add(ff b0, ff b1, ff b2, ff b3) {
+        a[0].add(f2_pack(b0.hi, b1.hi));
+        a[0].lo = f2_add(a[0].lo, f2_pack(b0.lo, b1.lo));
+        a[1].add(f2_pack(b2.hi, b3.hi));
+        a[1].lo = f2_add(a[1].lo, f2_pack(b2.lo, b3.lo));
+    }
+    __device__ __forceinline__ void split(Acc<float>* q) const {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float2 h = f2_parts(a[i].hi), l = f2_parts(a[i].lo);
+            q[2 * i].hi = h.x;
+            q[2 * i].lo = l.x;
+            q[2 * i + 1].hi = h.y;
+            q[2 * i + 1].lo = l.y;
+        }
+    }
+};
+
+// A fixed shuffle tree (lane l takes lane l + 16's value, then l + 8's, ...) for four values at once: at
+// the first two levels a lane gives half of its values away and keeps the other half, in either case
+// merging the higher lane's value into the lower lane's.  The total of value x ends in lane 8x.
+template <typename T>
+__device__ __forceinline__ Acc<T> quad_merge(Acc<T>* q) {
+    const int lane = threadIdx.x & 31;
+    Acc<T> two[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) two[i] = exchange_merge(q[i], q[2 + i], 16, (lane & 16) != 0);
+    Acc<T> one = exchange_merge(two[0], two[1], 8, (lane & 8) != 0);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) one.merge_part(shfl_down_part(one.part(), o));
+    return one;
+}
+
+// 256 threads per chunk whatever its observation count (at most 256): threads beyond the chunk's
+// observations idle in phases A-C and take their share of the gathers of phase D.
+constexpr int kAssembleThreads = 256;
+static_assert(kAssembleThreads == 32 * kAssembleWarps, "the owner-gather schedule is planned for 8 warps");
+
 }  // namespace
 
 template <typename T>
-__global__ void __launch_bounds__(256, 2) k_assemble(Shape S, DevPtrs D, AsmOutT<T> O, double damping) {
+__global__ void __launch_bounds__(kAssembleThreads, 2) k_assemble(Shape S, DevPtrs D, AsmOutT<T> O, double damping) {
     using P = typename Acc<T>::part_type;
     using Val = ValueOf<T>;
     using VT = typename Val::type;
@@ -72,6 +264,9 @@ __global__ void __launch_bounds__(256, 2) k_assemble(Shape S, DevPtrs D, AsmOutT
     double* s_V = carve<double>(ptr, static_cast<size_t>(MO) * 9);  // point normal terms, then the track factor
     T* s_A = carve<T>(ptr, static_cast<size_t>(MO) * sA);
     VT* s_G = carve<VT>(ptr, static_cast<size_t>(MO) * sG);
+    // FP32 path: G in packed pairs of rows, G4[k * 3 + q] = (hi, hi, lo, lo) of G[2q][k] and G[2q + 1][k],
+    // nine 16-byte words per observation (the lanes of a quarter-warp hit distinct banks)
+    float4* s_G4 = reinterpret_cast<float4*>(s_G);
     VT* s_Y = carve<VT>(ptr, static_cast<size_t>(MO) * sY);
     VT* s_M = carve<VT>(ptr, static_cast<size_t>(MO) * sM);
     VT* s_D = carve<VT>(ptr, static_cast<size_t>(MO) * sD);
@@ -285,13 +480,28 @@ __global__ void __launch_bounds__(256, 2) k_assemble(Shape S, DevPtrs D, AsmOutT
         }
         s_cpc[tslot] = cc_sum;
     }
-    if (telim) {
-        double V[6] = {cpV[0], cpV[1], cpV[2], cpV[3], cpV[4], cpV[5]}, rhs[3] = {cpg[0], cpg[1], cpg[2]};
-        for (int j = 0; j < tk; ++j) {
-            const double* v = s_V + static_cast<size_t>(tfirst + j) * 9;
-            for (int i = 0; i < 6; ++i) V[i] += v[i];
-            for (int i = 0; i < 3; ++i) rhs[i] += v[6 + i];
+    // sums of the track's nine point terms over its observations, in observation order: a thread per
+    // track and term (a thread per track kept 10 of 32 lanes busy through 58 FP64 additions); the sums
+    // and their start, the control points' terms, take the place of G, which phase C writes
+    double* s_sum = reinterpret_cast<double*>(s_G);
+    if (S.ncp > 0) {
+        if (tact) {
+            for (int i = 0; i < 6; ++i) s_sum[tslot * 9 + i] = cpV[i];
+            for (int i = 0; i < 3; ++i) s_sum[tslot * 9 + 6 + i] = cpg[i];
         }
+        __syncthreads();
+    }
+    for (int e = tid; e < 9 * ntc; e += kAssembleThreads) {
+        const int t = e / 9, i = e - 9 * t, j0 = s_tfirst[t], j1 = s_tfirst[t + 1];
+        double v = S.ncp > 0 ? s_sum[e] : 0.0;
+        for (int j = j0; j < j1; ++j) v += s_V[static_cast<size_t>(j) * 9 + i];
+        s_sum[e] = v;
+    }
+    __syncthreads();
+    if (telim) {
+        double V[6], rhs[3];
+        for (int i = 0; i < 6; ++i) V[i] = s_sum[tslot * 9 + i];
+        for (int i = 0; i < 3; ++i) rhs[i] = s_sum[tslot * 9 + 6 + i];
         V[0] *= 1.0 + damping;
         V[3] *= 1.0 + damping;
         V[5] *= 1.0 + damping;
@@ -338,6 +548,7 @@ __global__ void __launch_bounds__(256, 2) k_assemble(Shape S, DevPtrs D, AsmOutT
     if (active) {
         if (!start) s_trk[tid] = s_trk[first];
         VT* G = s_G + static_cast<size_t>(tid) * sG;
+        float4* G4 = s_G4 + static_cast<size_t>(tid) * 9;
         VT* Ys = s_Y + static_cast<size_t>(tid) * sY;
         VT* Mo = s_M + static_cast<size_t>(tid) * sM;
         if (ok) {
@@ -351,7 +562,7 @@ __global__ void __launch_bounds__(256, 2) k_assemble(Shape S, DevPtrs D, AsmOutT
                     const double i00 = st[0], i10 = st[1], i11 = st[2], i20 = st[3], i21 = st[4], i22 = st[5];
                     q[0] = st[6]; q[1] = st[7]; q[2] = st[8];
                     for (int pa = 0; pa < 2; ++pa) {
-                        const double p0 = jpT[pa * 3], p1 = jpT[pa * 3 + 1], p2 = jpT[pa * 3 + 2];
+                        const double p0 = f64_of(jpT[pa * 3]), p1 = f64_of(jpT[pa * 3 + 1]), p2 = f64_of(jpT[pa * 3 + 2]);
                         Y[pa][0] = w * (i00 * p0);
                         Y[pa][1] = w * (i10 * p0 + i11 * p1);
                         Y[pa][2] = w * (i20 * p0 + i21 * p1 + i22 * p2);
@@ -367,43 +578,69 @@ __global__ void __launch_bounds__(256, 2) k_assemble(Shape S, DevPtrs D, AsmOutT
             }
             for (int i = 0; i < 6; ++i) Ys[i] = y[i];
             const T* A = s_A + static_cast<size_t>(tid) * sA;
-            // back-substitution record of the observation: A rows, then Y
-            T* rec = O.obs_rec + static_cast<size_t>(o) * (2 * nA + 6);
-            for (int i = 0; i < 2 * nA; ++i) rec[i] = A[i];
-            for (int i = 0; i < 6; ++i) {
-                if constexpr (kMixed) rec[2 * nA + i] = y[i].hi;  // RN of the FP64 value
-                else rec[2 * nA + i] = y[i];
-            }
-            for (int a = 0; a < 6; ++a) {
-                const T ja0 = A[a], ja1 = A[nA + a];
-                G[a * 3 + 0] = ja0 * y[0] + ja1 * y[3];
-                G[a * 3 + 1] = ja0 * y[1] + ja1 * y[4];
-                G[a * 3 + 2] = ja0 * y[2] + ja1 * y[5];
+            if constexpr (kMixed) {
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+#pragma unroll
+                    for (int k3 = 0; k3 < 3; ++k3) {
+                        const ff e = A[2 * q] * y[k3] + A[nA + 2 * q] * y[3 + k3];
+                        const ff f = A[2 * q + 1] * y[k3] + A[nA + 2 * q + 1] * y[3 + k3];
+                        G4[k3 * 3 + q] = make_float4(e.hi, f.hi, e.lo, f.lo);
+                    }
+            } else {
+                for (int a = 0; a < 6; ++a) {
+                    const T ja0 = A[a], ja1 = A[nA + a];
+                    G[a * 3 + 0] = ja0 * y[0] + ja1 * y[3];
+                    G[a * 3 + 1] = ja0 * y[1] + ja1 * y[4];
+                    G[a * 3 + 2] = ja0 * y[2] + ja1 * y[5];
+                }
             }
         } else {
-            T* rec = O.obs_rec + static_cast<size_t>(o) * (2 * nA + 6);
-            for (int i = 0; i < 2 * nA + 6; ++i) rec[i] = T(0);
             for (int i = 0; i < 6; ++i) Mo[i] = Val::zero();
             for (int i = 0; i < 6; ++i) Ys[i] = Val::zero();
-            for (int i = 0; i < 18; ++i) G[i] = Val::zero();
+            if constexpr (kMixed) {
+                for (int i = 0; i < 9; ++i) G4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            } else {
+                for (int i = 0; i < 18; ++i) G[i] = Val::zero();
+            }
         }
     }
     __syncthreads();
-    // ---- K: per track and group, K[(g, c), k] = sum_(o in track, group g) (J_intr^T Y)[c, k]
+    // back-substitution records of the chunk's observations: A rows, then Y (rounded to T), a warp per
+    // observation (a thread per observation wrote 32 lines per store)
+    {
+        const int rl = 2 * nA + 6;
+        for (int ob = wid; ob < nobs; ob += kAssembleWarps) {
+            T* rec = O.obs_rec + static_cast<size_t>(obs0 + ob) * rl;
+            const T* A = s_A + static_cast<size_t>(ob) * sA;
+            const VT* Y = s_Y + static_cast<size_t>(ob) * sY;
+            for (int i = lane; i < rl; i += 32) {
+                T v;
+                if (i < 2 * nA) v = A[i];
+                else if constexpr (kMixed) v = Y[i - 2 * nA].hi;  // RN of the FP64 value
+                else v = Y[i - 2 * nA];
+                rec[i] = v;
+            }
+        }
+    }
+    // ---- K: per track and group, K[(g, c), k] = sum_(o in track, group g) (J_intr^T Y)[c, k]; a thread per
+    // track, group, pair of columns and k
     if (nb > 0) {
-        const int per = nb * 3;
-        for (int it = tid; it < ntc * per; it += blockDim.x) {
+        const int npc = (ni + 1) / 2, per = ng * npc * 3;
+        for (int it = tid; it < ntc * per; it += kAssembleThreads) {
             const int t = it / per, r = it - t * per;
             const int gc = r / 3, kk = r - gc * 3;
-            const int g = gc / ni, c = gc - g * ni;
-            VT acc = Val::zero();
+            const int g = gc / npc, c = 2 * (gc - g * npc), c1 = min(c + 1, ni - 1);
+            ColumnPair<T> acc;
             for (int ob = s_tfirst[t]; ob < s_tfirst[t + 1]; ++ob) {
                 if (info_group(s_info[ob]) != g) continue;
-                const T* A = s_A + static_cast<size_t>(ob) * sA;
+                const T* A = s_A + static_cast<size_t>(ob) * sA + 6;
                 const VT* Y = s_Y + static_cast<size_t>(ob) * sY;
-                acc = acc + (A[6 + c] * Y[kk] + A[nA + 6 + c] * Y[3 + kk]);
+                acc.add(A[c], A[c1], Y[kk], A[nA + c], A[nA + c1], Y[3 + kk]);
             }
-            s_K[static_cast<size_t>(t) * sK + r] = acc;
+            VT* K = s_K + static_cast<size_t>(t) * sK + (g * ni + c) * 3 + kk;
+            K[0] = acc.first();
+            if (c + 1 < ni) K[3] = acc.second();
         }
         __syncthreads();
     }
@@ -426,7 +663,7 @@ __global__ void __launch_bounds__(256, 2) k_assemble(Shape S, DevPtrs D, AsmOutT
             const int s = wk / 6, x = wk - s * 6;
             const int pk = D.ch_pairs[pair0 + s];
             const bool diag = (pk & 0xFFFF) == (pk >> 16);
-            Acc<T> acc[6];
+            RowAcc<T> acc;
             const int i1 = D.slot_item_begin[pair0 + s + 1];
             for (int it = D.slot_item_begin[pair0 + s]; it < i1; ++it) {
                 const unsigned item = D.slot_items[it];
@@ -438,31 +675,25 @@ __global__ void __launch_bounds__(256, 2) k_assemble(Shape S, DevPtrs D, AsmOutT
                     const T ax0 = A[x], ax1 = A[nA + x];
                     const VT u0 = ax0 * M[0] + ax1 * M[1];
                     const VT u1 = ax0 * M[1] + ax1 * M[2];
-#pragma unroll
-                    for (int y = 0; y < 6; ++y) {
-                        acc_fma(acc[y], A[y], u0);
-                        acc_fma(acc[y], A[nA + y], u1);
-                    }
+                    acc.jacobian(A, A + nA, u0, u1);
+                } else if constexpr (kMixed) {
+                    const float4* Ga = s_G4 + static_cast<size_t>(oa) * 9;
+                    const float* Gx = reinterpret_cast<const float*>(Ga + (x >> 1)) + (x & 1);
+                    acc.template coupling<true>(s_G4 + static_cast<size_t>(ob) * 9, ff{-Gx[0], -Gx[2]}, ff{-Gx[12], -Gx[14]},
+                                                 ff{-Gx[24], -Gx[26]});
                 } else {
                     const VT* Ga = s_G + static_cast<size_t>(oa) * sG + 3 * x;
-                    const VT* Gb = s_G + static_cast<size_t>(ob) * sG;
-                    const VT g0 = -Ga[0], g1 = -Ga[1], g2 = -Ga[2];
-#pragma unroll
-                    for (int y = 0; y < 6; ++y) {
-                        acc_fma(acc[y], g0, Gb[3 * y]);
-                        acc_fma(acc[y], g1, Gb[3 * y + 1]);
-                        acc_fma(acc[y], g2, Gb[3 * y + 2]);
-                    }
+                    acc.template coupling<true>(s_G + static_cast<size_t>(ob) * sG, -Ga[0], -Ga[1], -Ga[2]);
                 }
             }
             P* out = O.part_pair + static_cast<size_t>(pair0 + s) * 36;
 #pragma unroll
             for (int y = 0; y < 6; ++y) {
                 if (!diag) {
-                    out[x * 6 + y] = acc[y].part();
+                    out[x * 6 + y] = acc.part(y);
                 } else if (y >= x) {
-                    out[x * 6 + y] = acc[y].part();
-                    out[y * 6 + x] = acc[y].part();
+                    out[x * 6 + y] = acc.part(y);
+                    out[y * 6 + x] = acc.part(y);
                 }
             }
         } else if (wk < w_pair + w_cam) {
@@ -470,28 +701,21 @@ __global__ void __launch_bounds__(256, 2) k_assemble(Shape S, DevPtrs D, AsmOutT
             const int l = r / crow, row = r - l * crow;
             const int b0 = D.lcam_obs_begin[cam0 + l], b1 = D.lcam_obs_begin[cam0 + l + 1];
             P* out = O.part_cam + static_cast<size_t>(cam0 + l) * camrec;
-            Acc<T> acc[6];
+            RowAcc<T> acc;
             if (row < 2) {
                 // gradient rows: the reduced gradient -J_pose^T (w r + Y q) and the direct
                 // gradient -J_pose^T w r (the point term with the rounded Jacobian)
                 for (int it = b0; it < b1; ++it) {
                     const int ob = D.lcam_obs[it];
-                    const VT* Dg = s_D + static_cast<size_t>(ob) * sD;
-#pragma unroll
-                    for (int a = 0; a < 6; ++a) acc[a].add(Dg[a]);
+                    acc.add(s_D + static_cast<size_t>(ob) * sD);
                     if (row == 0) {
                         const T* A = s_A + static_cast<size_t>(ob) * sA;
                         const VT* M = s_M + static_cast<size_t>(ob) * sM;
-                        const VT m0 = -M[3], m1 = -M[4];
-#pragma unroll
-                        for (int a = 0; a < 6; ++a) {
-                            acc_fma(acc[a], A[a], m0);
-                            acc_fma(acc[a], A[nA + a], m1);
-                        }
+                        acc.jacobian(A, A + nA, -M[3], -M[4]);
                     }
                 }
 #pragma unroll
-                for (int a = 0; a < 6; ++a) out[row * 6 + a] = acc[a].part();
+                for (int a = 0; a < 6; ++a) out[row * 6 + a] = acc.part(a);
             } else {
                 // border column (g, c2) of the camera's pose rows
                 const int gc = row - 2, g = gc / ni, c2 = gc - g * ni;
@@ -501,89 +725,109 @@ __global__ void __launch_bounds__(256, 2) k_assemble(Shape S, DevPtrs D, AsmOutT
                     const T* A = s_A + static_cast<size_t>(ob) * sA;
                     if (info_group(info) == g) {
                         const VT w = s_M[static_cast<size_t>(ob) * sM + 5];
-                        const VT u0 = A[6 + c2] * w, u1 = A[nA + 6 + c2] * w;
-#pragma unroll
-                        for (int a = 0; a < 6; ++a) {
-                            acc_fma(acc[a], A[a], u0);
-                            acc_fma(acc[a], A[nA + a], u1);
-                        }
+                        acc.jacobian(A, A + nA, A[6 + c2] * w, A[nA + 6 + c2] * w);
                     }
                     const int ts = trk_slot(s_trk[ob]);
                     if ((info & kElim) && ts < ntc && ((s_tmask[ts] >> g) & 1)) {
                         const VT* Kt = s_K + static_cast<size_t>(ts) * sK + gc * 3;
-                        const VT k0 = -Kt[0], k1 = -Kt[1], k2 = -Kt[2];
-                        const VT* Go = s_G + static_cast<size_t>(ob) * sG;
-#pragma unroll
-                        for (int a = 0; a < 6; ++a) {
-                            acc_fma(acc[a], Go[3 * a], k0);
-                            acc_fma(acc[a], Go[3 * a + 1], k1);
-                            acc_fma(acc[a], Go[3 * a + 2], k2);
-                        }
+                        if constexpr (kMixed)
+                            acc.template coupling<false>(s_G4 + static_cast<size_t>(ob) * 9, -Kt[0], -Kt[1], -Kt[2]);
+                        else
+                            acc.template coupling<false>(s_G + static_cast<size_t>(ob) * sG, -Kt[0], -Kt[1], -Kt[2]);
                     }
                 }
 #pragma unroll
-                for (int a = 0; a < 6; ++a) out[12 + (g * 6 + a) * ni + c2] = acc[a].part();
+                for (int a = 0; a < 6; ++a) out[12 + (g * 6 + a) * ni + c2] = acc.part(a);
             }
         }
     }
-    // Intrinsic block entries (i, j), i <= j, and intrinsic gradient entries: one warp per entry,
-    // its lanes striding over the chunk's observations and tracks, then a fixed shuffle tree (the
-    // entries sum over every observation of the chunk, so a thread per entry would be the
-    // chunk's critical path).  Warps that finish their rows above start here at once.
-    {
+    // Intrinsic block entries (i, j), i <= j, and intrinsic gradient entries: a warp takes up to four
+    // entries of one row, its lanes striding over the chunk's observations and tracks, then a fixed
+    // shuffle tree (the entries sum over every observation of the chunk, so a thread per entry would be
+    // the chunk's critical path).  Warps that finish their rows above start here at once.
+    if (nb > 0) {
         P* out = O.part_chunk + static_cast<size_t>(chunk) * chrec;
-        // a warp takes the next entry when it is free (an entry is summed the same way by any
-        // warp, so the order of taking changes no result)
+        // units of up to four columns: of a row within its own group (from the diagonal on), of a row
+        // with a later group, of the reduced and of the direct gradient
+        const int nq = (ni + 3) / 4;
+        int own = 0;  // units of one group's own rows
+        for (int c = 0; c < ni; ++c) own += (ni - c + 3) / 4;
+        const int u_own = ng * own, u_cross = ng * (ng - 1) / 2 * ni * nq, u_all = u_own + u_cross + 2 * ng * nq;
+        // a warp takes the next unit when it is free (an entry is summed the same way by any warp, so
+        // the order of taking changes no result)
         for (;;) {
             int e = 0;
             if (lane == 0) e = atomicAdd(s_next_entry, 1);
             e = __shfl_sync(0xffffffffu, e, 0);
-            if (e >= chrec) break;
-            Acc<T> acc;
-            if (e < nb * nb) {
-                const int i = e / nb, j = e - i * nb;
-                if (i > j) continue;
-                const int g1 = i / ni, c1 = i - g1 * ni, g2 = j / ni, c2 = j - g2 * ni;
-                if (g1 == g2) {
+            if (e >= u_all) break;
+            QuadAcc<T> acc;
+            int at = 0, row = -1, col = 0, c0 = 0;  // first entry; row and column of the block (row < 0: gradient)
+            if (e < u_own + u_cross) {
+                int g1, c1, g2;
+                if (e < u_own) {
+                    g1 = g2 = e / own;
+                    int r = e - g1 * own;
+                    for (c1 = 0; r >= (ni - c1 + 3) / 4; ++c1) r -= (ni - c1 + 3) / 4;
+                    c0 = c1 + 4 * r;
+                } else {
+                    int r = e - u_own;
+                    const int pr = r / (ni * nq);
+                    r -= pr * (ni * nq);
+                    c1 = r / nq;
+                    c0 = 4 * (r - c1 * nq);
+                    g1 = 0;
+                    int left = pr;
+                    while (left >= ng - 1 - g1) left -= ng - 1 - g1++;
+                    g2 = g1 + 1 + left;
+                }
+                row = g1 * ni + c1;
+                col = g2 * ni + c0;
+                at = row * nb + col;
+                // columns beyond the group's last one repeat it and are not written
+                const int k1 = min(c0 + 1, ni - 1), k2 = min(c0 + 2, ni - 1), k3 = min(c0 + 3, ni - 1);
+                if (g1 == g2)
                     for (int ob = lane; ob < nobs; ob += 32) {
                         if (info_group(s_info[ob]) != g1) continue;
-                        const T* A = s_A + static_cast<size_t>(ob) * sA;
+                        const T* A = s_A + static_cast<size_t>(ob) * sA + 6;
                         const VT w = s_M[static_cast<size_t>(ob) * sM + 5];
-                        acc_fma(acc, w, two_prod(A[6 + c1], A[6 + c2]));
-                        acc_fma(acc, w, two_prod(A[nA + 6 + c1], A[nA + 6 + c2]));
+                        acc.weighted(w, A[c1], A[c0], A[k1], A[k2], A[k3]);
+                        acc.weighted(w, A[nA + c1], A[nA + c0], A[nA + k1], A[nA + k2], A[nA + k3]);
                     }
-                }
                 const int need = (1 << g1) | (1 << g2);
                 for (int t = lane; t < ntc; t += 32) {
                     if ((s_tmask[t] & need) != need) continue;
-                    const VT* K1 = s_K + static_cast<size_t>(t) * sK + i * 3;
-                    const VT* K2 = s_K + static_cast<size_t>(t) * sK + j * 3;
-                    acc_fma(acc, -K1[0], K2[0]);
-                    acc_fma(acc, -K1[1], K2[1]);
-                    acc_fma(acc, -K1[2], K2[2]);
-                }
-                warp_merge(acc);
-                if (lane == 0) {
-                    out[e] = acc.part();
-                    if (i != j) out[j * nb + i] = acc.part();
+                    const VT* K1 = s_K + static_cast<size_t>(t) * sK + row * 3;
+                    const VT* K2 = s_K + static_cast<size_t>(t) * sK + g2 * ni * 3;
+#pragma unroll
+                    for (int kk = 0; kk < 3; ++kk)
+                        acc.minus(K1[kk], K2[c0 * 3 + kk], K2[k1 * 3 + kk], K2[k2 * 3 + kk], K2[k3 * 3 + kk]);
                 }
             } else {
-                const int idx = e - nb * nb;
-                const bool reduced = idx < nb;
-                const int col = reduced ? idx : idx - nb;
-                const int g = col / ni, c = col - g * ni;
+                const int r = e - u_own - u_cross, half = r / (ng * nq);
+                const int g = (r - half * ng * nq) / nq;
+                c0 = 4 * (r - half * ng * nq - g * nq);
+                at = nb * nb + half * nb + g * ni + c0;
+                const int k1 = min(c0 + 1, ni - 1), k2 = min(c0 + 2, ni - 1), k3 = min(c0 + 3, ni - 1);
                 for (int ob = lane; ob < nobs; ob += 32) {
                     if (info_group(s_info[ob]) != g) continue;
-                    acc.add(s_D[static_cast<size_t>(ob) * sD + 6 + c]);
-                    if (reduced) {
-                        const T* A = s_A + static_cast<size_t>(ob) * sA;
+                    const VT* Dg = s_D + static_cast<size_t>(ob) * sD + 6;
+                    acc.add(Dg[c0], Dg[k1], Dg[k2], Dg[k3]);
+                    if (half == 0) {  // the reduced gradient
+                        const T* A = s_A + static_cast<size_t>(ob) * sA + 6;
                         const VT* M = s_M + static_cast<size_t>(ob) * sM;
-                        acc_fma(acc, A[6 + c], -M[3]);
-                        acc_fma(acc, A[nA + 6 + c], -M[4]);
+                        acc.jacobian(A[c0], A[k1], A[k2], A[k3], -M[3]);
+                        acc.jacobian(A[nA + c0], A[nA + k1], A[nA + k2], A[nA + k3], -M[4]);
                     }
                 }
-                warp_merge(acc);
-                if (lane == 0) out[e] = acc.part();
+            }
+            __syncwarp();
+            Acc<T> q[4];
+            acc.split(q);
+            const Acc<T> v = quad_merge(q);
+            const int x = lane >> 3;  // the entry whose total this lane's group of eight holds
+            if ((lane & 7) == 0 && c0 + x < ni) {
+                out[at + x] = v.part();
+                if (row >= 0 && row != col + x) out[(col + x) * nb + row] = v.part();
             }
         }
     }
@@ -603,11 +847,6 @@ static AsmOutT<T> typed_out(const AsmOut& o) {
     return {static_cast<P*>(o.part_pair_v), static_cast<P*>(o.part_cam_v), static_cast<P*>(o.part_chunk_v),
             o.part_cost, o.part_flags, static_cast<double*>(o.trk_data_v), static_cast<T*>(o.obs_rec_v)};
 }
-
-// 256 threads per chunk whatever its observation count (at most 256): threads beyond the chunk's
-// observations idle in phases A-C and take their share of the gathers of phase D.
-constexpr int kAssembleThreads = 256;
-static_assert(kAssembleThreads == 32 * kAssembleWarps, "the owner-gather schedule is planned for 8 warps");
 
 template <typename T>
 void launch_assemble(const Shape& S, const DevPtrs& D, const AsmOut& O, double damping, size_t smem, cudaStream_t st) {

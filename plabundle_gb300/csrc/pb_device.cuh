@@ -451,6 +451,36 @@ __device__ __forceinline__ ff ff_make(double d) {
     const float h = static_cast<float>(d);
     return {h, static_cast<float>(d - static_cast<double>(h))};
 }
+// Conversions between FP64 and FP32 on the integer pipe, bit for bit those of the conversion
+// instructions, which take the FP64 pipe for 64 cycles a warp (the form below about ten).  Zero apart,
+// values outside the range of normal FP32 numbers go to the instruction.
+__device__ __forceinline__ double f64_of(float f) {
+    const unsigned u = __float_as_uint(f), mag = u & 0x7fffffffu;
+    if (mag - 1u < 0x007fffffu || mag >= 0x7f800000u) return static_cast<double>(f);  // denormal, infinite, NaN
+    const unsigned hi = mag == 0u ? u : ((u & 0x80000000u) | ((mag >> 3) + 0x38000000u));
+    return __hiloint2double(static_cast<int>(hi), static_cast<int>(u << 29));
+}
+__device__ __forceinline__ double f64_of(double d) { return d; }
+// hi = RN(d), lo = RN(d - hi).  For 2^-74 <= |d| < 2^127 the difference is an integer of at most 29 bits
+// times 2^(e - 52) (e the exponent of d), rounded by its conversion to FP32; scaling it is exact.
+__device__ __forceinline__ ff ff_make_bits(double d) {
+    const unsigned hw = hi_word(d), lw = static_cast<unsigned>(__double2loint(d));
+    const unsigned ex = (hw >> 20) & 0x7ffu;
+    if (ex - 949u > 200u) {
+        const float h = static_cast<float>(d);
+        return {h, static_cast<float>(d - static_cast<double>(h))};
+    }
+    // sign, exponent - 896 and the upper 23 bits of the fraction, rounded to nearest even
+    unsigned u = (__funnelshift_l(lw, hw, 3) + 0x40000000u) | (hw & 0x80000000u);
+    int rest = static_cast<int>(lw & 0x1fffffffu);
+    if (rest + static_cast<int>(u & 1u) > 0x10000000) {
+        rest -= 0x20000000;
+        ++u;
+    }
+    if (hw & 0x80000000u) rest = -rest;
+    const float lo = static_cast<float>(rest) * __uint_as_float((ex - 948u) << 23);
+    return {__uint_as_float(u), lo};
+}
 // __fmul_rn / __fadd_rn are never contracted into an FMA, which the error-free transformations
 // below depend on.
 __device__ __forceinline__ ff ff_norm(float s, float e) {
@@ -484,7 +514,7 @@ struct ValueOf;
 template <>
 struct ValueOf<float> {
     using type = ff;
-    __device__ static __forceinline__ ff make(double d) { return ff_make(d); }
+    __device__ static __forceinline__ ff make(double d) { return ff_make_bits(d); }
     __device__ static __forceinline__ ff zero() { return {0.f, 0.f}; }
 };
 template <>
@@ -545,6 +575,95 @@ struct Acc<float> {
     __device__ __forceinline__ float2 part() const { return make_float2(hi, lo); }
 };
 
+// Two FP32 numbers in one 64-bit register and the packed operations on them: each half is rounded as
+// the scalar operation rounds it.  A packed operation takes the FP32 pipe as long as two scalar ones and
+// half their issue slots.
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 f2_pack(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_both(float a) { return f2_pack(a, a); }
+__device__ __forceinline__ float2 f2_parts(f2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_sub(f2 a, f2 b) {
+    f2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// Two float-float numbers side by side: products with a common float-float factor and sums, rounded as
+// the operators of ff round them.
+struct ff2p {
+    f2 hi, lo;
+};
+__device__ __forceinline__ ff2p ff2_norm(f2 s, f2 e) {
+    const f2 h = f2_add(s, e);
+    return {h, f2_sub(e, f2_sub(h, s))};
+}
+__device__ __forceinline__ ff2p operator*(f2 a, ff b) {
+    const f2 bh = f2_both(b.hi);
+    const f2 p = f2_mul(a, bh);
+    const f2 ne = f2_fma(a, f2_both(-b.lo), f2_fma(a, f2_both(-b.hi), p));  // less the rounding error
+    const f2 h = f2_sub(p, ne);
+    return {h, f2_sub(f2_sub(p, h), ne)};
+}
+__device__ __forceinline__ ff2p operator+(ff2p a, ff2p b) {
+    const f2 s = f2_add(a.hi, b.hi);
+    const f2 bp = f2_sub(s, a.hi);
+    const f2 e = f2_add(f2_add(f2_sub(a.hi, f2_sub(s, bp)), f2_sub(b.hi, bp)), f2_add(a.lo, b.lo));
+    return ff2_norm(s, e);
+}
+
+// Two accumulators Acc<float> side by side.
+struct Acc2 {
+    f2 hi = 0ull, lo = 0ull;
+    __device__ __forceinline__ void add(f2 v) {
+        const f2 s = f2_add(hi, v);
+        const f2 bp = f2_sub(s, hi);
+        const f2 e = f2_add(f2_sub(hi, f2_sub(s, bp)), f2_sub(v, bp));
+        hi = s;
+        lo = f2_add(lo, e);
+    }
+    // acc_fma of (a, alo) b with the negated factors na = -a, nalo = -alo (LEFT), or of b (a, alo): the
+    // order of the two cross products.  The product's rounding error is carried with its sign changed
+    // and subtracted.
+    template <bool LEFT>
+    __device__ __forceinline__ void fma_ff(f2 a, f2 na, f2 nalo, f2 bhi, f2 blo) {
+        const f2 p = f2_mul(a, bhi);
+        const f2 e = f2_fma(na, bhi, p);
+        const f2 ne = LEFT ? f2_fma(nalo, bhi, f2_fma(na, blo, e)) : f2_fma(na, blo, f2_fma(nalo, bhi, e));
+        add(p);
+        lo = f2_sub(lo, ne);
+    }
+    // acc_fma of the floats a and the float-float b (nb = -b)
+    __device__ __forceinline__ void fma_f(f2 a, f2 bhi, f2 nbhi, f2 nblo) {
+        const f2 p = f2_mul(a, bhi);
+        const f2 ne = f2_fma(a, nblo, f2_fma(a, nbhi, p));
+        add(p);
+        lo = f2_sub(lo, ne);
+    }
+};
+
 // acc += a * b, the product's rounding error carried into the compensation term (FP32 path) /
 // one FMA (FP64 path).
 __device__ __forceinline__ void acc_fma(Acc<float>& acc, ff a, ff b) {
@@ -564,18 +683,28 @@ __device__ __forceinline__ void acc_fma(Acc<float>& acc, float a, ff b) {
 }
 __device__ __forceinline__ void acc_fma(Acc<double>& acc, double a, double b) { acc.s = fma(a, b, acc.s); }
 
-// Sum of the accumulators of a warp into lane 0 by a fixed shuffle tree (deterministic order).
-__device__ __forceinline__ void warp_merge(Acc<double>& acc) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc.s += __shfl_down_sync(0xffffffffu, acc.s, o);
+// Pieces of fixed shuffle trees over the accumulators of a warp.
+__device__ __forceinline__ double shfl_down_part(double v, int o) { return __shfl_down_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ float2 shfl_down_part(float2 v, int o) {
+    return make_float2(__shfl_down_sync(0xffffffffu, v.x, o), __shfl_down_sync(0xffffffffu, v.y, o));
 }
-__device__ __forceinline__ void warp_merge(Acc<float>& acc) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float h = __shfl_down_sync(0xffffffffu, acc.hi, o);
-        const float l = __shfl_down_sync(0xffffffffu, acc.lo, o);
-        acc.merge_part(make_float2(h, l));
-    }
+// The lanes of bit `o` clear (up == false) keep `a` and receive their partner's `a`; the others keep `b`.
+// The result is the higher lane's value merged into the lower lane's.
+__device__ __forceinline__ Acc<double> exchange_merge(Acc<double> a, Acc<double> b, int o, bool up) {
+    const double got = __shfl_xor_sync(0xffffffffu, up ? a.s : b.s, o);
+    Acc<double> r;
+    r.s = (up ? b.s : a.s) + got;
+    return r;
+}
+__device__ __forceinline__ Acc<float> exchange_merge(Acc<float> a, Acc<float> b, int o, bool up) {
+    const float gh = __shfl_xor_sync(0xffffffffu, up ? a.hi : b.hi, o);
+    const float gl = __shfl_xor_sync(0xffffffffu, up ? a.lo : b.lo, o);
+    const Acc<float>& own = up ? b : a;
+    Acc<float> low;
+    low.hi = up ? gh : own.hi;
+    low.lo = up ? gl : own.lo;
+    low.merge_part(make_float2(up ? own.hi : gh, up ? own.lo : gl));
+    return low;
 }
 
 // exact product of two floats as a float-float
