@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <mutex>
 #include <type_traits>
 
 #include "pb_device.cuh"
@@ -18,7 +19,9 @@ namespace pb {
 // The three fixed-order sums below are independent of one another and each is latency-bound on
 // a small grid (the chunk-record sum has one CTA per 32 record entries), so one launch runs them
 // side by side over block ranges [pose pairs | cameras | chunk records + cost].  Each keeps the
-// summation order of its own loop; the loads of a loop are issued ahead of its merge chain.
+// summation order of its own loop.  A list's merges are a serial chain of a few FP32 additions (one FP64
+// addition) each, and the lists are long (hundreds to thousands of chunks touch a camera), so the records
+// in flight per list decide.
 template <typename T>
 struct ReduceArgs {
     using part_t = typename Acc<T>::part_type;
@@ -28,46 +31,118 @@ struct ReduceArgs {
     const double* part_cost;
     const int* part_flags;
     double *vals, *rhs, *direct, *border, *border_t, *Cm, *result;
-    unsigned pair_blocks, cam_blocks;
+    unsigned chunk_blocks;
 };
 
-// Sum of the chunk partials of every upper pose block, written to both CSR orientations.
-template <typename T>
-__device__ __forceinline__ void reduce_pairs(const Shape& S, const DevPtrs& D, const ReduceArgs<T>& R, unsigned blk) {
-    const long long idx = static_cast<long long>(blk) * blockDim.x + threadIdx.x;
-    if (idx >= static_cast<long long>(S.nupper) * 36) return;
-    const int u = static_cast<int>(idx / 36), e = static_cast<int>(idx - static_cast<long long>(u) * 36);
-    Acc<T> acc;
-    const int c1 = D.up_contrib_begin[u + 1];
-#pragma unroll 4
-    for (int c = D.up_contrib_begin[u]; c < c1; ++c)
-        acc.merge_part(R.part_pair[static_cast<size_t>(D.up_contrib[c]) * 36 + e]);
-    const double v = acc.value64();
-    R.vals[static_cast<size_t>(D.up_csr[u]) * 36 + e] = v;
-    const int t = D.up_csr_t[u];
-    if (t >= 0) R.vals[static_cast<size_t>(t) * 36 + (e % 6) * 6 + e / 6] = v;
+// A warp sums up to 36 neighbouring entries of one list's records (lane l entries l and 32 + l) in the
+// order of the list.  The records stream through a ring of six stages of eight in shared memory by
+// asynchronous copies, their list indices loaded a vector of 32 ahead.  (A thread per entry with four
+// loads ahead left the longest lists waiting: 100 cameras, 4982 chunks, mixed 307 -> 160 us a launch; 500
+// cameras, 8301 chunks 211 -> 160 us; 40 cameras, FP64 47 -> 29 us.)
+constexpr int kRedWarps = 8, kRedEntries = 36, kRedStages = 6, kRedSlots = 8;
+constexpr int kRedPieces = kRedEntries / 2;  // 16-byte pieces of a full record tile
+constexpr size_t kRedSmem = static_cast<size_t>(kRedWarps) * kRedStages * kRedSlots * kRedEntries * 8;
+
+__device__ __forceinline__ void copy16_async(void* dst, const void* src) {
+    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
 }
 
-// Sum of the per-camera partials: rhs, direct rhs and the intrinsic border rows.
+// records: the tile's first entry of record 0; stride: entries from one record to the next (even);
+// entries: width of the tile (even, at most 36).
 template <typename T>
-__device__ __forceinline__ void reduce_cams(const Shape& S, const DevPtrs& D, const ReduceArgs<T>& R, unsigned blk) {
-    const int camrec = 12 + S.ng * 6 * S.ni;
-    const long long idx = static_cast<long long>(blk) * blockDim.x + threadIdx.x;
-    if (idx >= static_cast<long long>(S.ncb) * camrec) return;
-    const int i = static_cast<int>(idx / camrec), e = static_cast<int>(idx - static_cast<long long>(i) * camrec);
-    Acc<T> acc;
-    const int c1 = D.cam_contrib_begin[i + 1];
-#pragma unroll 4
-    for (int c = D.cam_contrib_begin[i]; c < c1; ++c)
-        acc.merge_part(R.part_cam[static_cast<size_t>(D.cam_contrib[c]) * camrec + e]);
-    const double v = acc.value64();
-    if (e < 6) R.rhs[i * 6 + e] = v;
-    else if (e < 12) R.direct[i * 6 + e - 6] = v;
-    else {
-        const int f = e - 12;  // (g * 6 + a) * ni + c
-        const int g = f / (6 * S.ni), rem = f - g * 6 * S.ni, a = rem / S.ni, c = rem - a * S.ni;
-        R.border[(static_cast<size_t>(i) * 6 + a) * S.nb + g * S.ni + c] = v;
-        R.border_t[static_cast<size_t>(g * S.ni + c) * 6 * S.ncb + i * 6 + a] = v;
+__device__ __forceinline__ void reduce_list(Acc<T>* acc, const typename Acc<T>::part_type* __restrict__ records,
+                                            size_t stride, int entries, const int* __restrict__ list, int c0, int c1,
+                                            typename Acc<T>::part_type* ring) {
+    const int lane = threadIdx.x & 31, pieces = entries / 2;
+    const int n = c1 - c0, stages = (n + kRedSlots - 1) / kRedSlots;
+    int now = lane < n ? list[c0 + lane] : 0, next = 32 + lane < n ? list[c0 + 32 + lane] : 0;
+    auto issue = [&](int st) {
+        if (st < stages) {
+            if (st > 0 && (st & 3) == 0) {
+                const int ahead = 8 * st + 32 + lane;
+                now = next;
+                next = ahead < n ? list[c0 + ahead] : 0;
+            }
+            typename Acc<T>::part_type* to = ring + static_cast<size_t>(st % kRedStages) * kRedSlots * kRedEntries;
+#pragma unroll
+            for (int k = 0; k < kRedSlots * kRedPieces / 32 + (kRedSlots * kRedPieces % 32 ? 1 : 0); ++k) {
+                const int p = lane + 32 * k, sl = p / kRedPieces, q = p - sl * kRedPieces;
+                const int rec = __shfl_sync(0xffffffffu, now, (8 * (st & 3) + min(sl, kRedSlots - 1)) & 31);
+                if (sl < kRedSlots && q < pieces && kRedSlots * st + sl < n)
+                    copy16_async(to + sl * kRedEntries + 2 * q, records + static_cast<size_t>(rec) * stride + 2 * q);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int st = 0; st < kRedStages - 1; ++st) issue(st);
+    for (int st = 0; st < stages; ++st) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kRedStages - 2) : "memory");
+        __syncwarp();
+        const typename Acc<T>::part_type* v = ring + static_cast<size_t>(st % kRedStages) * kRedSlots * kRedEntries;
+        const int m = min(kRedSlots, n - kRedSlots * st);
+        if (m == kRedSlots && entries == kRedEntries) {
+#pragma unroll
+            for (int i = 0; i < kRedSlots; ++i) {
+                acc[0].merge_part(v[i * kRedEntries + lane]);
+                if (lane < kRedEntries - 32) acc[1].merge_part(v[i * kRedEntries + 32 + lane]);
+            }
+        } else {
+            for (int i = 0; i < m; ++i) {
+                if (lane < entries) acc[0].merge_part(v[i * kRedEntries + lane]);
+                if (32 + lane < entries) acc[1].merge_part(v[i * kRedEntries + 32 + lane]);
+            }
+        }
+        __syncwarp();
+        issue(st + kRedStages - 1);
+    }
+}
+
+// Sums of the chunk partials of every upper pose block, written to both CSR orientations, and of the
+// per-camera partials (rhs, direct rhs and the intrinsic border rows, in tiles of 36 entries): one warp
+// per block or tile.
+template <typename T>
+__device__ __forceinline__ void reduce_lists(const Shape& S, const DevPtrs& D, const ReduceArgs<T>& R, unsigned blk,
+                                             unsigned char* smem) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    auto* ring = reinterpret_cast<typename Acc<T>::part_type*>(smem) +
+                 static_cast<size_t>(wid) * kRedStages * kRedSlots * kRedEntries;
+    const int camrec = 12 + S.ng * 6 * S.ni, tiles = (camrec + kRedEntries - 1) / kRedEntries;
+    const int unit = static_cast<int>(blk) * kRedWarps + wid;
+    Acc<T> acc[2];
+    if (unit < S.nupper) {
+        const int u = unit;
+        reduce_list<T>(acc, R.part_pair, 36, 36, D.up_contrib, D.up_contrib_begin[u], D.up_contrib_begin[u + 1], ring);
+        const int t = D.up_csr_t[u];
+        double* vals = R.vals + static_cast<size_t>(D.up_csr[u]) * 36;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int e = 32 * k + lane;
+            if (e >= 36) continue;
+            const double v = acc[k].value64();
+            vals[e] = v;
+            if (t >= 0) R.vals[static_cast<size_t>(t) * 36 + (e % 6) * 6 + e / 6] = v;
+        }
+    } else if (unit < S.nupper + S.ncb * tiles) {
+        const int i = (unit - S.nupper) / tiles, tile = unit - S.nupper - i * tiles, e0 = tile * kRedEntries;
+        const int width = min(kRedEntries, camrec - e0);
+        reduce_list<T>(acc, R.part_cam + e0, camrec, width, D.cam_contrib, D.cam_contrib_begin[i], D.cam_contrib_begin[i + 1],
+                       ring);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int e = e0 + 32 * k + lane;
+            if (32 * k + lane >= width) continue;
+            const double v = acc[k].value64();
+            if (e < 6) R.rhs[i * 6 + e] = v;
+            else if (e < 12) R.direct[i * 6 + e - 6] = v;
+            else {
+                const int f = e - 12;  // (g * 6 + a) * ni + c
+                const int g = f / (6 * S.ni), rem = f - g * 6 * S.ni, a = rem / S.ni, c = rem - a * S.ni;
+                R.border[(static_cast<size_t>(i) * 6 + a) * S.nb + g * S.ni + c] = v;
+                R.border_t[static_cast<size_t>(g * S.ni + c) * 6 * S.ncb + i * 6 + a] = v;
+            }
+        }
     }
 }
 
@@ -87,8 +162,27 @@ __device__ __forceinline__ void reduce_chunks(const Shape& S, const ReduceArgs<T
         const int e = blk * 32 + lane;
         Acc<T> acc;
         if (e < chrec) {
+            // sixteen records in registers while the next sixteen are on their way
+            constexpr int kAhead = 16;
+            const typename Acc<T>::part_type* src = R.part_chunk + e;
+            typename Acc<T>::part_type v[kAhead];
+            int c = wid;
+            const int step = kAhead * nw;
+            if (c + step - nw < S.nchunks)
+#pragma unroll
+                for (int i = 0; i < kAhead; ++i) v[i] = src[static_cast<size_t>(c + i * nw) * chrec];
+            for (; c + step - nw < S.nchunks; c += step) {
+                typename Acc<T>::part_type w[kAhead];
+                if (c + 2 * step - nw < S.nchunks)
+#pragma unroll
+                    for (int i = 0; i < kAhead; ++i) w[i] = src[static_cast<size_t>(c + step + i * nw) * chrec];
+#pragma unroll
+                for (int i = 0; i < kAhead; ++i) acc.merge_part(v[i]);
+#pragma unroll
+                for (int i = 0; i < kAhead; ++i) v[i] = w[i];
+            }
 #pragma unroll 4
-            for (int c = wid; c < S.nchunks; c += nw) acc.merge_part(R.part_chunk[static_cast<size_t>(c) * chrec + e]);
+            for (; c < S.nchunks; c += nw) acc.merge_part(src[static_cast<size_t>(c) * chrec]);
         }
         s_acc[wid][lane] = acc.part();
         __syncthreads();
@@ -127,13 +221,13 @@ __device__ __forceinline__ void reduce_chunks(const Shape& S, const ReduceArgs<T
 }
 
 // 256 threads per block (the chunk-record sum's warp count and cost buffers assume it); the block
-// range decides the sum, uniformly per block.
+// range decides the sum, uniformly per block: the chunk records first, they take longest.
 template <typename T>
 __global__ void __launch_bounds__(256) k_reduce_sums(Shape S, DevPtrs D, ReduceArgs<T> R) {
+    extern __shared__ __align__(16) unsigned char reduce_smem[];
     const unsigned b = blockIdx.x;
-    if (b < R.pair_blocks) reduce_pairs<T>(S, D, R, b);
-    else if (b < R.pair_blocks + R.cam_blocks) reduce_cams<T>(S, D, R, b - R.pair_blocks);
-    else reduce_chunks<T>(S, R, b - R.pair_blocks - R.cam_blocks);
+    if (b < R.chunk_blocks) reduce_chunks<T>(S, R, b);
+    else reduce_lists<T>(S, D, R, b - R.chunk_blocks, reduce_smem);
 }
 
 // Intrinsic priors (assembleReferencePriors, ...ReferenceSchur.cpp:492-536) and
@@ -149,24 +243,28 @@ __global__ void k_finalize(Shape S, DevPtrs D, double* __restrict__ vals, double
         const double v = *d;
         *d = v != 0.0 ? v * (1.0 + damping) : 1.0;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0 && S.ng > 0) {
-        double cost = 0.0;
-        for (int g = 0; g < S.ng; ++g) {
-            const double* G = D.groups + static_cast<size_t>(g) * kGroupRec;
-            for (int c = 0; c < S.ni; ++c) {
-                const int p = S.int_cols[c];
+    // priors of the intrinsic columns, a lane each (one thread after the other took 18 us for 16 columns);
+    // their costs are added in column order
+    if (blockIdx.x == 0 && threadIdx.x < 32 && S.nb > 0) {
+        double total = 0.0;
+        for (int c0 = 0; c0 < S.nb; c0 += 32) {
+            const int col = c0 + threadIdx.x;
+            double cost = 0.0;
+            if (col < S.nb) {
+                const int g = col / S.ni, p = S.int_cols[col - g * S.ni];
+                const double* G = D.groups + static_cast<size_t>(g) * kGroupRec;
                 const double w = G[2 * kP + p];
                 const double r = w * (G[p] - G[kP + p]);
-                cost += 0.5 * r * r;
-                const int col = g * S.ni + c;
+                cost = 0.5 * r * r;
                 double* cd = Cm + col * S.nb + col;
                 const double v = *cd + w * w;
                 *cd = v != 0.0 ? v * (1.0 + damping) : 1.0;
                 rhs_b[col] -= w * r;
                 direct_b[col] -= w * r;
             }
+            for (int i = 0; i < min(32, S.nb - c0); ++i) total += __shfl_sync(0xffffffffu, cost, i);
         }
-        result[0] += cost;
+        if (threadIdx.x == 0) result[0] += total;
     }
 }
 
@@ -414,24 +512,25 @@ __global__ void __launch_bounds__(kCostThreads) k_cost_batch(Shape S, DevPtrs D,
 }
 static_assert(kCostThreads == 128, "k_cost_batch adds the sums of four warps");
 
-// Final objective per step length, one warp each: block partials in fixed order plus the intrinsic
-// priors of the trial groups (assemblePrimaryPriors cost, BundleAdjustPlaMatrixAssemblySurvey.cpp:43-91).
-__global__ void __launch_bounds__(32 * kMaxAlpha) k_cost_final(Shape S, DevPtrs D, const double* __restrict__ part,
-                                                               int nblocks, int n_alpha, int use_trial,
-                                                               double* __restrict__ out) {
-    const int a = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (a >= n_alpha) return;
+// Final objective of step length blockIdx.x: block partials in fixed order plus the intrinsic priors of
+// the trial groups (assemblePrimaryPriors cost, BundleAdjustPlaMatrixAssemblySurvey.cpp:43-91).
+constexpr int kCostFinalThreads = 256;
+__global__ void __launch_bounds__(kCostFinalThreads) k_cost_final(Shape S, DevPtrs D, const double* __restrict__ part,
+                                                                  int nblocks, int use_trial, double* __restrict__ out) {
+    __shared__ double s_v[kCostFinalThreads / 32];
+    __shared__ int s_b[kCostFinalThreads / 32];
+    const int a = blockIdx.x, tid = threadIdx.x;
     const double* sums = part + static_cast<size_t>(a) * nblocks;
     const double* marks = part + static_cast<size_t>(kMaxAlpha + a) * nblocks;
     double v = 0.0;
-    bool bad = false;
-#pragma unroll 8
-    for (int i = lane; i < nblocks; i += 32) {
+    int bad = 0;
+#pragma unroll 5
+    for (int i = tid; i < nblocks; i += kCostFinalThreads) {
         v += sums[i];
         bad |= __double_as_longlong(marks[i]) != 0;
     }
-    for (int e = lane; e < S.nb; e += 32) {
-        const int g = e / S.ni, p = S.int_cols[e - g * S.ni];
+    if (tid < S.nb) {  // (at most 36 columns)
+        const int g = tid / S.ni, p = S.int_cols[tid - g * S.ni];
         const double* G = (use_trial ? D.groups_trial + static_cast<size_t>(a) * S.ng * kGroupRec : D.groups) +
                           static_cast<size_t>(g) * kGroupRec;
         const double r = G[2 * kP + p] * (G[p] - G[kP + p]);
@@ -439,8 +538,20 @@ __global__ void __launch_bounds__(32 * kMaxAlpha) k_cost_final(Shape S, DevPtrs 
     }
     v = warp_sum(v);
     bad = __any_sync(0xffffffffu, bad);
-    if (lane == 0) out[a] = bad ? __longlong_as_double(0x7ff0000000000000ll) : v;
+    if ((tid & 31) == 0) {
+        s_v[tid >> 5] = v;
+        s_b[tid >> 5] = bad;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < kCostFinalThreads / 32; ++w) {
+            v += s_v[w];
+            bad |= s_b[w];
+        }
+        out[a] = bad ? __longlong_as_double(0x7ff0000000000000ll) : v;
+    }
 }
+static_assert(kMaxNB <= kCostFinalThreads, "a thread per intrinsic column");
 
 // Back-substitution (recoverReferencePointSteps, ...ReferenceSchur.cpp:982-1082), one thread per
 // track:  dp = R^-T (q - R^-1 u),  u = sum_o w J_p^T (J_o dc).
@@ -712,13 +823,17 @@ void launch_reduce_sums(const Shape& S, const DevPtrs& D, const AsmOut& O, const
     A.border_t = R.border_t;
     A.Cm = R.Cm;
     A.result = R.result;
-    const long long np = static_cast<long long>(S.nupper) * 36;
-    const long long nc = static_cast<long long>(S.ncb) * (12 + S.ng * 6 * S.ni);
-    A.pair_blocks = static_cast<unsigned>((np + 255) / 256);
-    A.cam_blocks = static_cast<unsigned>((nc + 255) / 256);
+    const int tiles = (12 + S.ng * 6 * S.ni + kRedEntries - 1) / kRedEntries;
     const int chrec = S.nb * S.nb + 2 * S.nb;
-    const unsigned chunk_blocks = static_cast<unsigned>((chrec + 31) / 32) + 1;
-    k_reduce_sums<T><<<A.pair_blocks + A.cam_blocks + chunk_blocks, 256, 0, st>>>(S, D, A);
+    A.chunk_blocks = static_cast<unsigned>((chrec + 31) / 32) + 1;
+    const unsigned list_blocks = static_cast<unsigned>((S.nupper + S.ncb * tiles + kRedWarps - 1) / kRedWarps);
+    static std::once_flag once[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::call_once(once[dev & 63], [] {
+        cudaFuncSetAttribute(k_reduce_sums<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRedSmem));
+    });
+    k_reduce_sums<T><<<A.chunk_blocks + list_blocks, 256, kRedSmem, st>>>(S, D, A);
 }
 
 template <typename T>
@@ -799,7 +914,7 @@ void launch_cost(const Shape& S, const DevPtrs& D, const double* step_c, const d
     const double c2 = S.loss_scale * S.loss_scale, ic2 = 1.0 / c2;
     const int plain = S.loss != 0 && std::isnormal(c2) && std::isnormal(ic2) ? 1 : 0;
     k_cost_batch<<<dim3(nblk, n_alpha), kCostThreads, 0, st>>>(S, D, step_p, alphas, use_trial, c2, ic2, plain, part);
-    k_cost_final<<<1, 32 * kMaxAlpha, 0, st>>>(S, D, part, nblk, n_alpha, use_trial, out);
+    k_cost_final<<<n_alpha, kCostFinalThreads, 0, st>>>(S, D, part, nblk, use_trial, out);
 }
 
 void launch_accept(const Shape& S, const DevPtrs& D, const double* step_p, double alpha, int a, cudaStream_t st) {
