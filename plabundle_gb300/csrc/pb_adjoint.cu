@@ -24,10 +24,12 @@
 //   k_adj_rhs       dL/dz of the primary variables added to the reduced right-hand side.
 //   (the reduced system is then solved by the forward path's dense Cholesky-preconditioned CG
 //    or block-Jacobi PCG)
-//   k_adj_gradient  one thread per track: point back-substitution mu_p = V^-1 (b_p - W^T mu_c),
-//                   dL/d(u, v) = W2 J mu per observation, cross terms of fixed cameras and
-//                   tracks, and the gauge terms (anchor centre, baseline) from the scale camera's
-//                   observations in the Euclidean centre chart.
+//   k_adj_terms     one thread per observation: W^T mu_c;
+//   k_adj_points    one thread per track: point back-substitution mu_p = V^-1 (b_p - W^T mu_c), cross
+//                   terms of fixed tracks;
+//   k_adj_gradient  one thread per observation: dL/d(u, v) = W2 J mu, cross terms of fixed cameras;
+//   k_adj_gauge     the gauge terms (anchor centre, baseline) from the scale camera's observations in
+//                   the Euclidean centre chart.
 // Every sum of the reduced system and of dL/d(u, v) has a fixed order; only the initial-pose cross
 // terms of fixed cameras and of the gauge pair are accumulated with FP64 atomics.
 #include <cuda_runtime.h>
@@ -44,8 +46,10 @@ namespace {
 // distorted normalised point (xd, yd) over (x, y) = (X / Z, Y / Z), chained through the
 // perspective division; the intrinsics enter bilinearly (focal x distortion), so their own
 // block is non-zero only in the focal and aspect rows.
-__host__ __device__ __forceinline__ void lam_pixel_derivatives(const DCam& c, const double* xc, double lam0, double lam1, int ni,
+template <int NI>
+__device__ __forceinline__ void lam_pixel_derivatives(const DCam& c, const double* xc, double lam0, double lam1, int n_int,
                                                       const int* cols, double* gx, double* Hm) {
+    const int ni = NI < 0 ? n_int : NI;
     const int M = 3 + ni;
     const double iz = 1.0 / xc[2];
     const double x = xc[0] * iz, y = xc[1] * iz;
@@ -140,127 +144,207 @@ __device__ __forceinline__ int sym6(int a, int b) { return a * 6 - a * (a - 1) /
 __device__ __forceinline__ int sym3(int a, int b) { return a * 3 - a * (a - 1) / 2 + (b - a); }
 __device__ __forceinline__ int symn(int n, int a, int b) { return a * n - a * (a - 1) / 2 + (b - a); }
 
-__device__ __forceinline__ void cross3(const double* a, const double* b, double* o) {
-    o[0] = a[1] * b[2] - a[2] * b[1];
-    o[1] = a[2] * b[0] - a[0] * b[2];
-    o[2] = a[0] * b[1] - a[1] * b[0];
-}
-
 // Exact per-observation Hessian record (layout AdjLayout) in the chart of the observation's
 // camera: tangent (gauge scale camera, centre columns 3 and 4 along the world basis gb) or
 // Euclidean.  nvec / baseline: unit direction anchor -> scale camera and the gauge baseline.
-// Returns false on an invalid projection or loss.
-__device__ bool adj_obs_hessian(const DCam& c, const double* X, double s, double u, double v, double wobs, int loss,
-                                double lscale, bool tangent, const double* gb, const double* nvec, double baseline,
-                                int ni, const int* cols, const AdjLayout& Lo, double* rec) {
-    Lin<double> L;
-    if (!linearize_obs<double>(c, X[0], X[1], X[2], s, u, v, wobs, loss, lscale, tangent, false, gb, ni, cols, true, L))
-        return false;
-    const double r0 = L.rd0, r1 = L.rd1;
+// Returns false on an invalid projection or loss.  NI: the number of intrinsic columns when it is known at
+// compile time (0: no column, so that every intermediate lives in registers), or -1.
+//
+// Every pose and point column acts through the world displacement d = X - C: the rotation columns are
+// v_i = s_i e_i x d (s = (1, -1, -1)), the centre columns -e_k, the point columns s(X) e_k.  So all blocks
+// follow from the gradient gw and the 3 x 3 Hessian Hw = Jw^T W2 Jw + R (lam^T d2 pi) R^T over d and, per
+// intrinsic column, one world vector: H(rot, d) = Hw v_i plus the rotation's own curvature, H(rot, rot) =
+// v_i^T Hw v_j plus it, and the centre and point blocks are Hw scaled.  About 300 FP64 operations per
+// observation without intrinsics; products of the full 9-column Jacobians took 1100
+// (105 000 observations: 195 -> 99 us).
+template <int NI>
+__device__ __forceinline__ bool adj_obs_hessian(const DCam& c, const double* X, double s, double u, double v, double wobs,
+                                                int loss, double lscale, bool tangent, const double* gb, const double* nvec,
+                                                double baseline, int n_int, const int* cols, double* rec) {
+    const int ni = NI < 0 ? n_int : NI;
+    constexpr int kNI = NI < 0 ? kMaxNI : NI;
+    AdjLayout Lo;
+    Lo.ni = ni;
+    Proj p;
+    if (!project64(c, X[0], X[1], X[2], p)) return false;
+    const double r0 = p.px - u, r1 = p.py - v;
+    const double sq = wobs * (r0 * r0 + r1 * r1);
+    if (!bits_nonneg_finite(sq)) return false;
     double d1, d2;
-    robust_derivatives(wobs * (r0 * r0 + r1 * r1), loss, lscale, d1, d2);
+    robust_derivatives(sq, loss, lscale, d1, d2);
     const double wa = 2.0 * d1 * wobs, wb = 4.0 * d2 * wobs * wobs;
+    if (!isfinite(wa) || !isfinite(wb) || (loss == 2 && !isfinite(lscale * lscale))) return false;
     const double W00 = wa + wb * r0 * r0, W01 = wb * r0 * r1, W11 = wa + wb * r1 * r1;
     const double lam0 = wa * r0, lam1 = wa * r1;
-    // world displacement d = X - C and the camera-frame point x_c = C2W^T d
-    const double d[3] = {X[0] - c.C[0], X[1] - c.C[1], X[2] - c.C[2]};
-    double xc[3];
-    for (int m = 0; m < 3; ++m) xc[m] = c.R[m] * d[0] + c.R[3 + m] * d[1] + c.R[6 + m] * d[2];
-    // second derivatives of lam^T pi over (x_c, kappa)
+    const double d[3] = {p.d0, p.d1, p.d2};
+    // gradient and second derivatives of lam^T pi over the camera-frame point and the intrinsics
     const int M = 3 + ni;
     double gx[3];
-    double Hm[(3 + kMaxNI) * (3 + kMaxNI)];
-    lam_pixel_derivatives(c, xc, lam0, lam1, ni, cols, gx, Hm);
-    // camera-frame point Jacobian over (w0..2, centre 0..2, dX 0..2), columns of Jx[m][col]
-    const double sg[3] = {1.0, -1.0, -1.0};
-    double Jx[3][9];
-    for (int i = 0; i < 3; ++i) {
-        const double e[3] = {i == 0 ? 1.0 : 0.0, i == 1 ? 1.0 : 0.0, i == 2 ? 1.0 : 0.0};
-        double a[3];
-        cross3(e, d, a);
-        for (int m = 0; m < 3; ++m) {
-            Jx[m][i] = sg[i] * (c.R[m] * a[0] + c.R[3 + m] * a[1] + c.R[6 + m] * a[2]);
-            Jx[m][6 + i] = s * c.R[3 * i + m];
-            if (tangent)
-                Jx[m][3 + i] = i < 2 ? -(c.R[m] * gb[3 * i] + c.R[3 + m] * gb[3 * i + 1] + c.R[6 + m] * gb[3 * i + 2]) : 0.0;
-            else
-                Jx[m][3 + i] = -c.R[3 * i + m];
+    double Hm[(3 + kNI) * (3 + kNI)];
+    {
+        double xc[3];
+#pragma unroll
+        for (int m = 0; m < 3; ++m) xc[m] = c.R[m] * d[0] + c.R[3 + m] * d[1] + c.R[6 + m] * d[2];
+        lam_pixel_derivatives<NI>(c, xc, lam0, lam1, ni, cols, gx, Hm);
+    }
+    // Jacobian of the pixel over the camera-frame point, then over the world displacement (2 x 3)
+    double Jw[2][3];
+    {
+        const double dr = c.k1 + p.r2 * (2.0 * c.k2 + 3.0 * c.k3 * p.r2);
+        const double xx = p.radial + 2.0 * p.x * p.x * dr + 2.0 * c.p1 * p.y + 6.0 * c.p2 * p.x;
+        const double xy = 2.0 * (p.x * p.y * dr + c.p1 * p.x + c.p2 * p.y);
+        const double yy = p.radial + 2.0 * p.y * p.y * dr + 6.0 * c.p1 * p.y + 2.0 * c.p2 * p.x;
+        const double fx = c.su * c.fx * p.iz, fy = c.sv * c.fy * p.iz;
+        const double a[2][2] = {{fx * xx, fx * xy}, {fy * xy, fy * yy}};
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const double az = -(a[r][0] * p.x + a[r][1] * p.y);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) Jw[r][j] = a[r][0] * c.R[3 * j] + a[r][1] * c.R[3 * j + 1] + az * c.R[3 * j + 2];
         }
     }
-    // g_w = C2W g_x: gradient of lam^T pi w.r.t. the world displacement d
-    double gw[3];
-    for (int j = 0; j < 3; ++j) gw[j] = c.R[3 * j] * gx[0] + c.R[3 * j + 1] * gx[1] + c.R[3 * j + 2] * gx[2];
-    const double gd = gw[0] * d[0] + gw[1] * d[1] + gw[2] * d[2];
-    // T: lam^T (d pi / d x_c) d2 x_c over the pose and point columns (upper 9x9)
-    double T[9][9];
-    for (int a = 0; a < 9; ++a)
-        for (int b = 0; b < 9; ++b) T[a][b] = 0.0;
-    for (int i = 0; i < 3; ++i)
-        for (int j = i; j < 3; ++j)  // d2 E / dw_i dw_j = G_i G_j (i <= j, product order Rx Ry Rz)
-            T[i][j] = sg[i] * sg[j] * (gw[j] * d[i] - (i == j ? gd : 0.0));
-    for (int i = 0; i < 3; ++i) {
-        const double e[3] = {i == 0 ? 1.0 : 0.0, i == 1 ? 1.0 : 0.0, i == 2 ? 1.0 : 0.0};
-        double ge[3];  // g_w x e_i, so that g_w . (e_i x b) = b . (g_w x e_i)
-        cross3(gw, e, ge);
-        for (int k = 0; k < 3; ++k) {
-            T[i][6 + k] = s * sg[i] * ge[k];
-            if (tangent)
-                T[i][3 + k] = k < 2 ? -sg[i] * (ge[0] * gb[3 * k] + ge[1] * gb[3 * k + 1] + ge[2] * gb[3 * k + 2]) : 0.0;
-            else
-                T[i][3 + k] = -sg[i] * ge[k];
-        }
+    // gw = R gx; Hw = R Hxx R^T + Jw^T W2 Jw
+    double gw[3], Hw[3][3], WJ[2][3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        gw[j] = c.R[3 * j] * gx[0] + c.R[3 * j + 1] * gx[1] + c.R[3 * j + 2] * gx[2];
+        WJ[0][j] = W00 * Jw[0][j] + W01 * Jw[1][j];
+        WJ[1][j] = W01 * Jw[0][j] + W11 * Jw[1][j];
     }
-    if (tangent) {
-        const double tt = (gw[0] * nvec[0] + gw[1] * nvec[1] + gw[2] * nvec[2]) / baseline;
-        T[3][3] = tt;
-        T[4][4] = tt;
+    {
+        double A[3][3];  // R Hxx
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+            for (int m = 0; m < 3; ++m)
+                A[j][m] = c.R[3 * j] * Hm[m] + c.R[3 * j + 1] * Hm[M + m] + c.R[3 * j + 2] * Hm[2 * M + m];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = i; j < 3; ++j) {
+                const double h = A[i][0] * c.R[3 * j] + A[i][1] * c.R[3 * j + 1] + A[i][2] * c.R[3 * j + 2] +
+                                 Jw[0][i] * WJ[0][j] + Jw[1][i] * WJ[1][j];
+                Hw[i][j] = h;
+                Hw[j][i] = h;
+            }
     }
-    // full local Jacobian rows and W2 J
-    const int nl = 9 + ni;
-    double Jf[2][9 + kMaxNI], WJ[2][9 + kMaxNI];
-    for (int r = 0; r < 2; ++r) {
-        for (int a = 0; a < 6; ++a) Jf[r][a] = L.Jc[r * 6 + a];
-        for (int a = 0; a < 3; ++a) Jf[r][6 + a] = L.Jp[r * 3 + a];
-        for (int k = 0; k < ni; ++k) Jf[r][9 + k] = L.Ji[r * kMaxNI + k];
-    }
-    for (int a = 0; a < nl; ++a) {
-        WJ[0][a] = W00 * Jf[0][a] + W01 * Jf[1][a];
-        WJ[1][a] = W01 * Jf[0][a] + W11 * Jf[1][a];
-    }
-    // HJ = Hxx Jx (3 x 9)
-    double HJ[3][9];
-    for (int m = 0; m < 3; ++m)
-        for (int a = 0; a < 9; ++a)
-            HJ[m][a] = Hm[m * M + 0] * Jx[0][a] + Hm[m * M + 1] * Jx[1][a] + Hm[m * M + 2] * Jx[2][a];
-    auto h99 = [&](int a, int b) {  // a <= b < 9
-        return Jf[0][a] * WJ[0][b] + Jf[1][a] * WJ[1][b] + Jx[0][a] * HJ[0][b] + Jx[1][a] * HJ[1][b] +
-               Jx[2][a] * HJ[2][b] + T[a][b];
+    // v_i = s_i e_i x d: v_0 = (0, -d2, d1), v_1 = -(d2, 0, -d0), v_2 = -(-d1, d0, 0); a . v_i below
+    auto dot_v = [&](int i, const double* a) {
+        return i == 0 ? a[2] * d[1] - a[1] * d[2] : i == 1 ? a[2] * d[0] - a[0] * d[2] : a[0] * d[1] - a[1] * d[0];
     };
+    // rows rot_i over the displacement: Hw v_i and the rotation's curvature s_i (gw x e_i)
+    double Hrd[3][3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        Hrd[0][k] = dot_v(0, Hw[k]);
+        Hrd[1][k] = dot_v(1, Hw[k]);
+        Hrd[2][k] = dot_v(2, Hw[k]);
+    }
+    double Hrr[6];  // upper rot x rot, with d2 E / dw_i dw_j = G_i G_j (i <= j, product order Rx Ry Rz)
+    {
+        const double gd = gw[0] * d[0] + gw[1] * d[1] + gw[2] * d[2];
+        Hrr[0] = dot_v(0, Hrd[0]) + (gw[0] * d[0] - gd);
+        Hrr[1] = dot_v(1, Hrd[0]) - gw[1] * d[0];
+        Hrr[2] = dot_v(2, Hrd[0]) - gw[2] * d[0];
+        Hrr[3] = dot_v(1, Hrd[1]) + (gw[1] * d[1] - gd);
+        Hrr[4] = dot_v(2, Hrd[1]) + gw[2] * d[1];
+        Hrr[5] = dot_v(2, Hrd[2]) + (gw[2] * d[2] - gd);
+    }
+    // s_i (gw x e_i): (0, g2, -g1), -(-g2, 0, g0), -(g1, -g0, 0)
+    Hrd[0][1] += gw[2];
+    Hrd[0][2] -= gw[1];
+    Hrd[1][0] += gw[2];
+    Hrd[1][2] -= gw[0];
+    Hrd[2][0] -= gw[1];
+    Hrd[2][1] += gw[0];
     double* hcc = rec + Lo.hcc();
     double* hcp = rec + Lo.hcp();
     double* hpp = rec + Lo.hpp();
     double* hck = rec + Lo.hck();
     double* hpk = rec + Lo.hpk();
     double* hkk = rec + Lo.hkk();
-    for (int a = 0; a < 6; ++a)
-        for (int b = a; b < 6; ++b) hcc[sym6(a, b)] = h99(a, b);
-    for (int a = 0; a < 6; ++a)
-        for (int b = 0; b < 3; ++b) hcp[a * 3 + b] = h99(a, 6 + b);
-    for (int a = 0; a < 3; ++a)
-        for (int b = a; b < 3; ++b) hpp[sym3(a, b)] = h99(6 + a, 6 + b);
-    for (int k = 0; k < ni; ++k) {
-        for (int a = 0; a < 9; ++a) {
-            const double h = Jf[0][a] * WJ[0][9 + k] + Jf[1][a] * WJ[1][9 + k] + Jx[0][a] * Hm[0 * M + 3 + k] +
-                             Jx[1][a] * Hm[1 * M + 3 + k] + Jx[2][a] * Hm[2 * M + 3 + k];
-            if (a < 6) hck[a * ni + k] = h;
-            else hpk[(a - 6) * ni + k] = h;
-        }
-        for (int l = k; l < ni; ++l)
-            hkk[symn(ni, k, l)] = Jf[0][9 + k] * WJ[0][9 + l] + Jf[1][9 + k] * WJ[1][9 + l] + Hm[(3 + k) * M + 3 + l];
-    }
+    const int nl = 9 + ni;
     double* J = rec + Lo.jac();
-    for (int r = 0; r < 2; ++r)
-        for (int a = 0; a < nl; ++a) J[r * nl + a] = Jf[r][a];
+    hcc[sym6(0, 0)] = Hrr[0];
+    hcc[sym6(0, 1)] = Hrr[1];
+    hcc[sym6(0, 2)] = Hrr[2];
+    hcc[sym6(1, 1)] = Hrr[3];
+    hcc[sym6(1, 2)] = Hrr[4];
+    hcc[sym6(2, 2)] = Hrr[5];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            hcp[i * 3 + k] = s * Hrd[i][k];
+            if (k >= i) hpp[sym3(i, k)] = s * s * Hw[i][k];
+        }
+        for (int r = 0; r < 2; ++r) {
+            J[r * nl + i] = dot_v(i, Jw[r]);
+            J[r * nl + 6 + i] = s * Jw[r][i];
+        }
+    }
+    // centre columns: d moves by -e_k, or by -gb_k (tangent), whose sphere curves towards the anchor
+    if (!tangent) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                hcc[sym6(i, 3 + k)] = -Hrd[i][k];
+                if (i >= k) hcc[sym6(3 + k, 3 + i)] = Hw[k][i];
+                hcp[(3 + k) * 3 + i] = -s * Hw[k][i];
+            }
+            J[3 + k] = -Jw[0][k];
+            J[nl + 3 + k] = -Jw[1][k];
+        }
+    } else {
+        const double tt = (gw[0] * nvec[0] + gw[1] * nvec[1] + gw[2] * nvec[2]) / baseline;
+        for (int k = 0; k < 2; ++k) {
+            const double* b = gb + 3 * k;
+            double hb[3];
+            for (int i = 0; i < 3; ++i) {
+                hcc[sym6(i, 3 + k)] = -(Hrd[i][0] * b[0] + Hrd[i][1] * b[1] + Hrd[i][2] * b[2]);
+                hb[i] = Hw[i][0] * b[0] + Hw[i][1] * b[1] + Hw[i][2] * b[2];
+                hcp[(3 + k) * 3 + i] = -s * hb[i];
+            }
+            for (int q = k; q < 2; ++q)
+                hcc[sym6(3 + k, 3 + q)] = hb[0] * gb[3 * q] + hb[1] * gb[3 * q + 1] + hb[2] * gb[3 * q + 2] + (q == k ? tt : 0.0);
+            for (int r = 0; r < 2; ++r) J[r * nl + 3 + k] = -(Jw[r][0] * b[0] + Jw[r][1] * b[1] + Jw[r][2] * b[2]);
+        }
+        for (int i = 0; i < 6; ++i) hcc[sym6(i, 5)] = 0.0;
+        for (int i = 0; i < 3; ++i) hcp[15 + i] = 0.0;
+        J[5] = J[nl + 5] = 0.0;
+    }
+    // intrinsic columns: Jacobian, and per column the world vector q_k = R Hm[0:3, 3 + k] + Jw^T W2 J_k
+    double Ji[2][kNI + 1], WJi[2][kNI + 1];
+    {
+        const double aspect = c.fx > 0.0 ? c.fy / c.fx : 1.0;
+#pragma unroll
+        for (int k = 0; k < ni; ++k) {
+            intrinsic_column<double>(cols[k], p.x, p.y, p.r2, p.xd, p.yd, c.su, c.sv, c.su * c.fx, c.sv * c.fy, aspect,
+                                     Ji[0][k], Ji[1][k]);
+            WJi[0][k] = W00 * Ji[0][k] + W01 * Ji[1][k];
+            WJi[1][k] = W01 * Ji[0][k] + W11 * Ji[1][k];
+            J[9 + k] = Ji[0][k];
+            J[nl + 9 + k] = Ji[1][k];
+            double q[3];
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+                q[j] = c.R[3 * j] * Hm[3 + k] + c.R[3 * j + 1] * Hm[M + 3 + k] + c.R[3 * j + 2] * Hm[2 * M + 3 + k] +
+                       Jw[0][j] * WJi[0][k] + Jw[1][j] * WJi[1][k];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                hck[i * ni + k] = dot_v(i, q);
+                hpk[i * ni + k] = s * q[i];
+                if (!tangent) hck[(3 + i) * ni + k] = -q[i];
+                else hck[(3 + i) * ni + k] = i < 2 ? -(q[0] * gb[3 * i] + q[1] * gb[3 * i + 1] + q[2] * gb[3 * i + 2]) : 0.0;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < ni; ++k)
+#pragma unroll
+            for (int l = k; l < ni; ++l)
+                hkk[symn(ni, k, l)] = Ji[0][k] * WJi[0][l] + Ji[1][k] * WJi[1][l] + Hm[(3 + k) * M + 3 + l];
+    }
     double* w2 = rec + Lo.w2();
     w2[0] = W00;
     w2[1] = W01;
@@ -286,6 +370,7 @@ __device__ __forceinline__ void gauge_normal(const Shape& S, const DevPtrs& D, d
         for (int i = 0; i < 3; ++i) n[i] = e[i] / l;
 }
 
+template <int NI>
 __global__ void __launch_bounds__(128) k_adj_hessian(Shape S, DevPtrs D, AdjBuffers B) {
     const long long o = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (o >= S.nop) return;
@@ -293,12 +378,11 @@ __global__ void __launch_bounds__(128) k_adj_hessian(Shape S, DevPtrs D, AdjBuff
     DCam c;
     load_cam(D.cams_eff + static_cast<size_t>(cam) * kCamStride, c);
     const bool tangent = is_tangent(S, cam);
-    double n[3];
-    gauge_normal(S, D, n);
+    double n[3] = {0.0, 0.0, 0.0};
+    if (tangent) gauge_normal(S, D, n);
     double* rec = B.rec + static_cast<size_t>(o) * B.lay.stride;
-    if (!adj_obs_hessian(c, D.points + static_cast<size_t>(trk) * 3, D.pscale[trk], D.obs_u[o], D.obs_v[o], D.obs_w[o],
-                         S.loss, S.loss_scale, tangent, D.gauge_basis, n, S.gauge_baseline, S.ni, S.int_cols, B.lay,
-                         rec)) {
+    if (!adj_obs_hessian<NI>(c, D.points + static_cast<size_t>(trk) * 3, D.pscale[trk], D.obs_u[o], D.obs_v[o], D.obs_w[o],
+                             S.loss, S.loss_scale, tangent, D.gauge_basis, n, S.gauge_baseline, S.ni, S.int_cols, rec)) {
         for (int i = 0; i < B.lay.stride; ++i) rec[i] = 0.0;
         atomicOr(B.flags, 2);
     }
@@ -386,6 +470,8 @@ __device__ __forceinline__ void track_rhs(const Shape& S, const DevPtrs& D, cons
 }
 
 constexpr int kAdjThreads = 256;
+constexpr int kAdjRow = 19;  // shared-memory stride of a 6 x 3 block (odd: lanes on different observations)
+static_assert(kAdjThreads == 32 * kAssembleWarps, "the owner-gather schedule is planned for 8 warps");
 
 template <typename U>
 __device__ __forceinline__ U* carve(char*& ptr, size_t count) {
@@ -404,35 +490,42 @@ __device__ __forceinline__ U* carve(char*& ptr, size_t count) {
 //   rhs:                -sum_(o in c) Y_o b_t  and  -sum_t K_(t,g)^T V_t^-1 b_t
 // with W = H_cp (pose-point), K_(t,g) = sum over the track's observations of group g of H_pk,
 // V_t = sum H_pp and b_t = s(X) dL/dX of the track.
-__global__ void __launch_bounds__(kAdjThreads, 2)
+//
+// FP64-bound: a row of a pose block costs 18 FMAs a term, with Y formed once per observation.  The rows
+// run in the forward assembly's schedule (rows of one code path and similar length side by side, dealt
+// to the warps by work): an idle lane costs as much as a working one (60 cameras, 105 000 observations, 480
+// chunks: 563 -> 262 us).
+__global__ void __launch_bounds__(kAdjThreads, 3)
     k_adj_assemble(Shape S, DevPtrs D, AdjBuffers B, double* __restrict__ part_pair, double* __restrict__ part_cam,
                    double* __restrict__ part_chunk) {
     extern __shared__ __align__(16) char smem[];
     const AdjLayout& Lo = B.lay;
-    const int chunk = blockIdx.x, tid = threadIdx.x;
+    const int chunk = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int MO = S.max_obs, MT = S.max_tracks;
     const int ng = S.ng, ni = S.ni, nb = S.nb;
     char* ptr = smem;
-    double* s_W = carve<double>(ptr, static_cast<size_t>(MO) * 18);     // H_cp per observation
-    double* s_Vi = carve<double>(ptr, static_cast<size_t>(MT) * 12);    // V^-1 (9) and q = V^-1 b (3) per track
+    double* s_W = carve<double>(ptr, static_cast<size_t>(MO) * kAdjRow);  // H_cp per observation
+    double* s_Y = carve<double>(ptr, static_cast<size_t>(MO) * kAdjRow);  // H_pp (6), then Y = W V^-1
+    double* s_Vi = carve<double>(ptr, static_cast<size_t>(MT) * 12);     // V^-1 (9) and q = V^-1 b (3) per track
     double* s_K = carve<double>(ptr, static_cast<size_t>(MT) * nb * 3);  // K[(t, g*ni + c), j]
     int* s_info = carve<int>(ptr, MO);                                  // group + 1 | elim << 4 | slot << 8
     int* s_tfirst = carve<int>(ptr, MT + 1);
-    int* s_flag = carve<int>(ptr, 1);
+    int* s_next = carve<int>(ptr, 1);  // next intrinsic entry to take
     const int obs0 = D.ch_obs_begin[chunk], nobs = D.ch_obs_begin[chunk + 1] - obs0;
     const int trk0 = D.obs_trk[obs0];
     const int ntc = D.obs_trk[obs0 + nobs - 1] - trk0 + 1;
-    if (tid == 0) s_flag[0] = ntc > MT ? 1 : 0;
-    __syncthreads();
-    if (s_flag[0]) {
+    if (ntc > MT) {
         if (tid == 0) atomicOr(B.flags, 4);
         return;
     }
-    // per observation: H_cp into shared memory, group / elimination / track slot
+    // per observation: H_cp and H_pp (neighbours in the record) into shared memory, a warp per observation
+    for (int ob = wid; ob < nobs; ob += kAdjThreads / 32) {
+        const double* rec = B.rec + static_cast<size_t>(obs0 + ob) * Lo.stride + Lo.hcp();
+        if (lane < 24) (lane < 18 ? s_W + ob * kAdjRow : s_Y + ob * kAdjRow - 18)[lane] = rec[lane];
+    }
+    // group / elimination / track slot
     if (tid < nobs) {
         const int o = obs0 + tid;
-        const double* rec = B.rec + static_cast<size_t>(o) * Lo.stride + Lo.hcp();
-        for (int i = 0; i < 18; ++i) s_W[tid * 18 + i] = rec[i];
         const int cam = D.obs_cam[o], trk = D.obs_trk[o];
         const int g = ng > 0 ? D.cam_group[cam] : -1;
         const int elim = D.trk_block[trk] >= 0 ? 1 : 0;
@@ -440,18 +533,25 @@ __global__ void __launch_bounds__(kAdjThreads, 2)
         s_info[tid] = (g + 1) | (elim << 4) | (slot << 8);
         if (o == D.trk_obs_begin[trk]) s_tfirst[slot] = tid;
     }
-    if (tid == 0) s_tfirst[ntc] = nobs;
+    if (tid == 0) {
+        s_tfirst[ntc] = nobs;
+        s_next[0] = 0;
+    }
     __syncthreads();
-    // per track: V^-1 and q (FP64), also kept for the gradient kernel
+    // per track: V (a thread per term), then V^-1 and q (FP64), also kept for the gradient kernel
+    for (int e = tid; e < 6 * ntc; e += kAdjThreads) {
+        const int t = e / 6, i = e - 6 * t;
+        double v = 0.0;
+        for (int ob = s_tfirst[t]; ob < s_tfirst[t + 1]; ++ob) v += s_Y[ob * kAdjRow + i];
+        s_Vi[t * 12 + i] = v;
+    }
+    __syncthreads();
     if (tid < ntc) {
         const int trk = trk0 + tid;
         double Vi[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, q[3] = {0, 0, 0};
         if (D.trk_block[trk] >= 0) {
-            double V[6] = {0, 0, 0, 0, 0, 0};
-            for (int o = D.trk_obs_begin[trk]; o < D.trk_obs_begin[trk + 1]; ++o) {
-                const double* h = B.rec + static_cast<size_t>(o) * Lo.stride + Lo.hpp();
-                for (int i = 0; i < 6; ++i) V[i] += h[i];
-            }
+            double V[6];
+            for (int i = 0; i < 6; ++i) V[i] = s_Vi[tid * 12 + i];
             if (!sym3_inverse(V, Vi)) {
                 atomicOr(B.flags, 1);
                 for (int i = 0; i < 9; ++i) Vi[i] = 0.0;
@@ -465,6 +565,16 @@ __global__ void __launch_bounds__(kAdjThreads, 2)
             B.vinv[static_cast<size_t>(trk) * 9 + i] = Vi[i];
         }
         for (int i = 0; i < 3; ++i) s_Vi[tid * 12 + 9 + i] = q[i];
+    }
+    __syncthreads();
+    // rows of Y_o = W_o V_t^-1 (zero for a track that is not eliminated: its V^-1 is)
+    for (int e = tid; e < 6 * nobs; e += kAdjThreads) {
+        const int ob = e / 6, x = e - 6 * ob;
+        const double* Vi = s_Vi + (s_info[ob] >> 8) * 12;
+        const double* w = s_W + ob * kAdjRow + 3 * x;
+        double* y = s_Y + ob * kAdjRow + 3 * x;
+        const double w0 = w[0], w1 = w[1], w2 = w[2];
+        for (int j = 0; j < 3; ++j) y[j] = w0 * Vi[j] + w1 * Vi[3 + j] + w2 * Vi[6 + j];
     }
     // per track and group: K = sum of H_pk over the track's observations of the group
     if (nb > 0) {
@@ -489,19 +599,10 @@ __global__ void __launch_bounds__(kAdjThreads, 2)
     const int crow = 2 + ng * ni;
     const int chrec = nb * nb + 2 * nb;
     const int w_pair = npairs * 6, w_cam = ncams * crow;
-    const int w_total = w_pair + w_cam + chrec;
-    // row x of Y_o = W_o V_t^-1
-    auto yrow = [&](int ob, int x, double* y) {
-        const int info = s_info[ob];
-        if (!((info >> 4) & 1)) {
-            y[0] = y[1] = y[2] = 0.0;
-            return;
-        }
-        const double* Vi = s_Vi + (info >> 8) * 12;
-        const double* w = s_W + ob * 18 + 3 * x;
-        for (int j = 0; j < 3; ++j) y[j] = w[0] * Vi[j] + w[1] * Vi[3 + j] + w[2] * Vi[6 + j];
-    };
-    for (int wk = tid; wk < w_total; wk += blockDim.x) {
+    const int task_end = D.warp_task_begin[chunk * kAssembleWarps + wid + 1];
+    for (int pos = D.warp_task_begin[chunk * kAssembleWarps + wid] + lane; pos < task_end; pos += 32) {
+        const int wk = D.task_list[pos];
+        if (wk == kNoTask) continue;
         if (wk < w_pair) {
             const int sl = wk / 6, x = wk - sl * 6;
             const int pk = D.ch_pairs[pair0 + sl];
@@ -511,14 +612,16 @@ __global__ void __launch_bounds__(kAdjThreads, 2)
             for (int it = D.slot_item_begin[pair0 + sl]; it < i1; ++it) {
                 const unsigned item = D.slot_items[it];
                 const int oa = item & 0xFF, ob = item >> 8;
-                double y[3];
-                yrow(oa, x, y);
-                const double* wb = s_W + ob * 18;
+                const double* y = s_Y + oa * kAdjRow + 3 * x;
+                const double* wb = s_W + ob * kAdjRow;
                 if (oa == ob) {
                     const double* h = B.rec + static_cast<size_t>(obs0 + oa) * Lo.stride + Lo.hcc();
                     for (int q2 = 0; q2 < 6; ++q2) acc[q2] += h[x <= q2 ? sym6(x, q2) : sym6(q2, x)];
                 }
-                for (int q2 = 0; q2 < 6; ++q2) acc[q2] -= y[0] * wb[3 * q2] + y[1] * wb[3 * q2 + 1] + y[2] * wb[3 * q2 + 2];
+                const double y0 = -y[0], y1 = -y[1], y2 = -y[2];
+#pragma unroll
+                for (int q2 = 0; q2 < 6; ++q2)
+                    acc[q2] = fma(y2, wb[3 * q2 + 2], fma(y1, wb[3 * q2 + 1], fma(y0, wb[3 * q2], acc[q2])));
             }
             double* out = part_pair + static_cast<size_t>(pair0 + sl) * 36;
             for (int q2 = 0; q2 < 6; ++q2) {
@@ -549,8 +652,10 @@ __global__ void __launch_bounds__(kAdjThreads, 2)
                     }
                     if (!((info >> 4) & 1)) continue;
                     const double* q = s_Vi + (info >> 8) * 12 + 9;
-                    const double* w = s_W + ob * 18;
-                    for (int a = 0; a < 6; ++a) acc[a] -= w[3 * a] * q[0] + w[3 * a + 1] * q[1] + w[3 * a + 2] * q[2];
+                    const double* w = s_W + ob * kAdjRow;
+                    const double q0 = -q[0], q1 = -q[1], q2 = -q[2];
+                    for (int a = 0; a < 6; ++a)
+                        acc[a] = fma(w[3 * a + 2], q2, fma(w[3 * a + 1], q1, fma(w[3 * a], q0, acc[a])));
                 }
                 for (int a = 0; a < 6; ++a) out[a] = acc[a];
             } else if (row == 1) {
@@ -566,60 +671,69 @@ __global__ void __launch_bounds__(kAdjThreads, 2)
                     }
                     if ((info >> 4) & 1) {
                         const double* Kt = s_K + (static_cast<size_t>(info >> 8) * nb + gc) * 3;
-                        for (int a = 0; a < 6; ++a) {
-                            double y[3];
-                            yrow(ob, a, y);
-                            acc[a] -= y[0] * Kt[0] + y[1] * Kt[1] + y[2] * Kt[2];
-                        }
+                        const double* y = s_Y + ob * kAdjRow;
+                        const double k0 = -Kt[0], k1 = -Kt[1], k2 = -Kt[2];
+                        for (int a = 0; a < 6; ++a)
+                            acc[a] = fma(y[3 * a + 2], k2, fma(y[3 * a + 1], k1, fma(y[3 * a], k0, acc[a])));
                     }
                 }
                 for (int a = 0; a < 6; ++a) out[12 + (g * 6 + a) * ni + c2] = acc[a];
             }
-        } else {
-            const int e = wk - w_pair - w_cam;
-            double* out = part_chunk + static_cast<size_t>(chunk) * chrec;
-            double acc = 0.0;
-            if (e < nb * nb) {
-                const int i = e / nb, j = e - i * nb;
-                if (i > j) continue;
-                const int g1 = i / ni, c1 = i - g1 * ni, g2 = j / ni, c2 = j - g2 * ni;
-                if (g1 == g2)
-                    for (int ob = 0; ob < nobs; ++ob) {
-                        if ((s_info[ob] & 15) - 1 != g1) continue;
-                        const double* h = B.rec + static_cast<size_t>(obs0 + ob) * Lo.stride + Lo.hkk();
-                        acc += h[c1 <= c2 ? symn(ni, c1, c2) : symn(ni, c2, c1)];
-                    }
-                for (int t = 0; t < ntc; ++t) {
-                    if (!((s_info[s_tfirst[t]] >> 4) & 1)) continue;
-                    const double* K1 = s_K + (static_cast<size_t>(t) * nb + i) * 3;
-                    const double* K2 = s_K + (static_cast<size_t>(t) * nb + j) * 3;
-                    const double* Vi = s_Vi + t * 12;
-                    for (int r = 0; r < 3; ++r)
-                        acc -= K1[r] * (Vi[r * 3] * K2[0] + Vi[r * 3 + 1] * K2[1] + Vi[r * 3 + 2] * K2[2]);
+        }
+    }
+    // intrinsic entries: a warp each, its lanes striding over the chunk's observations and tracks, summed
+    // by a fixed shuffle tree; a warp takes the next entry when it is free
+    for (;;) {
+        int e = 0;
+        if (lane == 0) e = atomicAdd(s_next, 1);
+        e = __shfl_sync(0xffffffffu, e, 0);
+        if (e >= chrec) break;
+        double* out = part_chunk + static_cast<size_t>(chunk) * chrec;
+        double acc = 0.0;
+        if (e < nb * nb) {
+            const int i = e / nb, j = e - i * nb;
+            if (i > j) continue;
+            const int g1 = i / ni, c1 = i - g1 * ni, g2 = j / ni, c2 = j - g2 * ni;
+            if (g1 == g2)
+                for (int ob = lane; ob < nobs; ob += 32) {
+                    if ((s_info[ob] & 15) - 1 != g1) continue;
+                    const double* h = B.rec + static_cast<size_t>(obs0 + ob) * Lo.stride + Lo.hkk();
+                    acc += h[c1 <= c2 ? symn(ni, c1, c2) : symn(ni, c2, c1)];
                 }
+            for (int t = lane; t < ntc; t += 32) {
+                if (!((s_info[s_tfirst[t]] >> 4) & 1)) continue;
+                const double* K1 = s_K + (static_cast<size_t>(t) * nb + i) * 3;
+                const double* K2 = s_K + (static_cast<size_t>(t) * nb + j) * 3;
+                const double* Vi = s_Vi + t * 12;
+                for (int r = 0; r < 3; ++r)
+                    acc -= K1[r] * (Vi[r * 3] * K2[0] + Vi[r * 3 + 1] * K2[1] + Vi[r * 3 + 2] * K2[2]);
+            }
+            acc = warp_sum(acc);
+            if (lane == 0) {
                 out[e] = acc;
                 if (i != j) out[j * nb + i] = acc;
-            } else if (e < nb * nb + nb) {
-                const int col = e - nb * nb;
-                if (B.newton) {
-                    const int g = col / ni, c = col - g * ni;
-                    for (int ob = 0; ob < nobs; ++ob) {
-                        if ((s_info[ob] & 15) - 1 != g) continue;
-                        const double* rec = B.rec + static_cast<size_t>(obs0 + ob) * Lo.stride;
-                        const double* J = rec + Lo.jac();
-                        acc -= J[9 + c] * rec[Lo.w2() + 3] + J[9 + ni + 9 + c] * rec[Lo.w2() + 4];
-                    }
-                }
-                for (int t = 0; t < ntc; ++t) {
-                    if (!((s_info[s_tfirst[t]] >> 4) & 1)) continue;
-                    const double* K1 = s_K + (static_cast<size_t>(t) * nb + col) * 3;
-                    const double* q = s_Vi + t * 12 + 9;
-                    acc -= K1[0] * q[0] + K1[1] * q[1] + K1[2] * q[2];
-                }
-                out[e] = acc;
-            } else {
-                out[e] = 0.0;
             }
+        } else if (e < nb * nb + nb) {
+            const int col = e - nb * nb;
+            if (B.newton) {
+                const int g = col / ni, c = col - g * ni;
+                for (int ob = lane; ob < nobs; ob += 32) {
+                    if ((s_info[ob] & 15) - 1 != g) continue;
+                    const double* rec = B.rec + static_cast<size_t>(obs0 + ob) * Lo.stride;
+                    const double* J = rec + Lo.jac();
+                    acc -= J[9 + c] * rec[Lo.w2() + 3] + J[9 + ni + 9 + c] * rec[Lo.w2() + 4];
+                }
+            }
+            for (int t = lane; t < ntc; t += 32) {
+                if (!((s_info[s_tfirst[t]] >> 4) & 1)) continue;
+                const double* K1 = s_K + (static_cast<size_t>(t) * nb + col) * 3;
+                const double* q = s_Vi + t * 12 + 9;
+                acc -= K1[0] * q[0] + K1[1] * q[1] + K1[2] * q[2];
+            }
+            acc = warp_sum(acc);
+            if (lane == 0) out[e] = acc;
+        } else if (lane == 0) {
+            out[e] = 0.0;
         }
     }
 }
@@ -645,131 +759,213 @@ __global__ void k_adj_finalize(Shape S, DevPtrs D, RedOut<double> R, int newton)
     }
 }
 
-__global__ void __launch_bounds__(128) k_adj_gradient(Shape S, DevPtrs D, AdjBuffers B, const double* __restrict__ mu) {
+// mu over the primary variables of one camera (zero for a fixed one) and its group.
+__device__ __forceinline__ void primary_mu(const Shape& S, const DevPtrs& D, const double* __restrict__ mu, int cam,
+                                           int ni, double* mc, double* mk) {
+    const int b = D.cam_block[cam], g = S.ng > 0 ? D.cam_group[cam] : -1;
+#pragma unroll
+    for (int a = 0; a < 6; ++a) mc[a] = b >= 0 ? mu[6 * b + a] : 0.0;
+    for (int k = 0; k < ni; ++k) mk[k] = g >= 0 ? mu[6 * S.ncb + g * ni + k] : 0.0;
+}
+
+// The gradients in four kernels (one thread per track over all of its observations' records, and the
+// full second Hessian of a scale camera's observation within it, left most of the device waiting: 299 us for
+// 105 000 observations, against 9 + 9 + 12 + 20).  First, a thread per observation: its term H_cp^T mu_c + H_pk mu_k of the point sums.
+template <int NI>
+__global__ void __launch_bounds__(128) k_adj_terms(Shape S, DevPtrs D, AdjBuffers B, const double* __restrict__ mu) {
+    const long long o = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (o >= S.nop) return;
+    const int ni = NI < 0 ? S.ni : NI;
+    const double* rec = B.rec + static_cast<size_t>(o) * B.lay.stride;
+    const double* hcp = rec + B.lay.hcp();
+    const double* hpk = rec + B.lay.hpk();
+    double mc[6], mk[NI < 0 ? kMaxNI : NI + 1];
+    primary_mu(S, D, mu, D.obs_cam[o], ni, mc, mk);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        double v = 0.0;
+#pragma unroll
+        for (int a = 0; a < 6; ++a) v = fma(hcp[a * 3 + i], mc[a], v);
+        for (int k = 0; k < ni; ++k) v = fma(hpk[i * ni + k], mk[k], v);
+        B.terms[3 * static_cast<size_t>(o) + i] = v;
+    }
+}
+
+// A thread per track: the point part of mu, V^-1 (b_p - sum of the terms), or a fixed track's cross terms
+// -(sum of the terms) in the scaled point chart.
+__global__ void __launch_bounds__(64) k_adj_points(Shape S, DevPtrs D, AdjBuffers B) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= S.ntp) return;
-    const AdjLayout& Lo = B.lay;
-    const int ni = S.ni, nl = 9 + ni;
-    const int ob = D.trk_obs_begin[t], oe = D.trk_obs_begin[t + 1];
     const bool free_pt = D.trk_block[t] >= 0;
-    const double* mk_base = mu + 6 * S.ncb;
-    // point part of mu: V^-1 (b_p - sum_o (Hcp^T mu_c + Hpk mu_k))
-    double mp[3] = {0.0, 0.0, 0.0};
+    double acc[3] = {0.0, 0.0, 0.0};
+    if (free_pt) track_rhs(S, D, B, t, acc);
+    const int oe = D.trk_obs_begin[t + 1];
+#pragma unroll 4
+    for (int o = D.trk_obs_begin[t]; o < oe; ++o)
+        for (int i = 0; i < 3; ++i) acc[i] -= B.terms[3 * static_cast<size_t>(o) + i];
     if (free_pt) {
-        double acc[3];
-        track_rhs(S, D, B, t, acc);
-        for (int o = ob; o < oe; ++o) {
-            const double* rec = B.rec + static_cast<size_t>(o) * Lo.stride;
-            const int cam = D.obs_cam[o];
-            const int b = D.cam_block[cam], g = S.ng > 0 ? D.cam_group[cam] : -1;
-            if (b >= 0) {
-                const double* mc = mu + 6 * b;
-                const double* h = rec + Lo.hcp();
-                for (int a = 0; a < 6; ++a)
-                    for (int i = 0; i < 3; ++i) acc[i] -= h[a * 3 + i] * mc[a];
-            }
-            if (g >= 0) {
-                const double* h = rec + Lo.hpk();
-                for (int i = 0; i < 3; ++i)
-                    for (int k = 0; k < ni; ++k) acc[i] -= h[i * ni + k] * mk_base[g * ni + k];
-            }
-        }
         const double* Vi = B.vinv + static_cast<size_t>(t) * 9;
-        for (int i = 0; i < 3; ++i) mp[i] = Vi[i * 3] * acc[0] + Vi[i * 3 + 1] * acc[1] + Vi[i * 3 + 2] * acc[2];
-        for (int i = 0; i < 3; ++i) B.mu_p[static_cast<size_t>(t) * 3 + i] = mp[i];
-    }
-    double fixed_pt[3] = {0.0, 0.0, 0.0};
-    for (int o = ob; o < oe; ++o) {
-        const double* rec = B.rec + static_cast<size_t>(o) * Lo.stride;
-        const int cam = D.obs_cam[o];
-        const int b = D.cam_block[cam], g = S.ng > 0 ? D.cam_group[cam] : -1;
-        double mloc[9 + kMaxNI];  // mu over the observation's local variables
-        for (int a = 0; a < 6; ++a) mloc[a] = b >= 0 ? mu[6 * b + a] : 0.0;
-        for (int i = 0; i < 3; ++i) mloc[6 + i] = mp[i];
-        for (int k = 0; k < ni; ++k) mloc[9 + k] = g >= 0 ? mk_base[g * ni + k] : 0.0;
-        const double* J = rec + Lo.jac();
-        double j0 = 0.0, j1 = 0.0;
-        for (int a = 0; a < nl; ++a) {
-            j0 += J[a] * mloc[a];
-            j1 += J[nl + a] * mloc[a];
-        }
-        const double* w2 = rec + Lo.w2();
-        B.grad_obs[2 * static_cast<size_t>(o)] = w2[0] * j0 + w2[1] * j1;
-        B.grad_obs[2 * static_cast<size_t>(o) + 1] = w2[1] * j0 + w2[2] * j1;
-        if (b < 0) {
-            // fixed camera: -(H_c,pt mu_p + H_c,k mu_k)
-            const double* hcp = rec + Lo.hcp();
-            const double* hck = rec + Lo.hck();
-            for (int a = 0; a < 6; ++a) {
-                double v = hcp[a * 3] * mp[0] + hcp[a * 3 + 1] * mp[1] + hcp[a * 3 + 2] * mp[2];
-                for (int k = 0; k < ni; ++k) v += hck[a * ni + k] * mloc[9 + k];
-                if (v != 0.0) atomicAdd(B.grad_fixed_cam + static_cast<size_t>(cam) * 6 + a, -v);
-            }
-        }
-        if (!free_pt) {
-            // fixed track: -(H_pt,c mu_c + H_pt,k mu_k) in the scaled point chart
-            const double* hcp = rec + Lo.hcp();
-            const double* hpk = rec + Lo.hpk();
-            for (int i = 0; i < 3; ++i) {
-                double v = 0.0;
-                for (int a = 0; a < 6; ++a) v += hcp[a * 3 + i] * mloc[a];
-                for (int k = 0; k < ni; ++k) v += hpk[i * ni + k] * mloc[9 + k];
-                fixed_pt[i] -= v;
-            }
-        }
-        if (is_tangent(S, cam) && b >= 0) {
-            // gauge terms: the scale camera's observation in the Euclidean centre chart, with mu
-            // lifted to it (centre step = tangent basis * mu_t)
-            double frec[kAdjMaxStride];
-            DCam c;
-            load_cam(D.cams_eff + static_cast<size_t>(cam) * kCamStride, c);
-            double n[3];
-            gauge_normal(S, D, n);
-            if (!adj_obs_hessian(c, D.points + static_cast<size_t>(t) * 3, D.pscale[t], D.obs_u[o], D.obs_v[o], D.obs_w[o],
-                                 S.loss, S.loss_scale, false, D.gauge_basis, n, S.gauge_baseline, ni, S.int_cols, Lo,
-                                 frec)) {
-                atomicOr(B.flags, 2);
-                continue;
-            }
-            const double* gb = D.gauge_basis;
-            double ml[9 + kMaxNI];
-            for (int i = 0; i < 3; ++i) ml[i] = mloc[i];
-            for (int i = 0; i < 3; ++i) ml[3 + i] = gb[i] * mloc[3] + gb[3 + i] * mloc[4];
-            for (int i = 0; i < 3 + ni; ++i) ml[6 + i] = mloc[6 + i];
-            // hC = H[C rows, all] * ml
-            const double* hcc = frec + Lo.hcc();
-            const double* hcp = frec + Lo.hcp();
-            const double* hck = frec + Lo.hck();
-            double hC[3];
-            for (int i = 0; i < 3; ++i) {
-                const int r = 3 + i;
-                double v = 0.0;
-                for (int a = 0; a < 6; ++a) v += hcc[r <= a ? sym6(r, a) : sym6(a, r)] * ml[a];
-                for (int j = 0; j < 3; ++j) v += hcp[r * 3 + j] * ml[6 + j];
-                for (int k = 0; k < ni; ++k) v += hck[r * ni + k] * ml[9 + k];
-                hC[i] = v;
-            }
-            // gC = d phi / dC = lam^T J_C
-            const double* fJ = frec + Lo.jac();
-            const double* fw = frec + Lo.w2();
-            double gC[3];
-            for (int i = 0; i < 3; ++i) gC[i] = fw[3] * fJ[3 + i] + fw[4] * fJ[nl + 3 + i];
-            const double gt = gC[0] * ml[3] + gC[1] * ml[4] + gC[2] * ml[5];
-            for (int i = 0; i < 3; ++i) atomicAdd(B.gauge + i, -hC[i]);
-            atomicAdd(B.gauge + 3, -(n[0] * hC[0] + n[1] * hC[1] + n[2] * hC[2]) - gt / S.gauge_baseline);
-        }
-    }
-    if (!free_pt) {
+        for (int i = 0; i < 3; ++i)
+            B.mu_p[static_cast<size_t>(t) * 3 + i] = Vi[i * 3] * acc[0] + Vi[i * 3 + 1] * acc[1] + Vi[i * 3 + 2] * acc[2];
+    } else {
         const double s = D.pscale[t];
-        for (int i = 0; i < 3; ++i) B.grad_fixed_pt[static_cast<size_t>(t) * 3 + i] = fixed_pt[i] / s;
+        for (int i = 0; i < 3; ++i) B.grad_fixed_pt[static_cast<size_t>(t) * 3 + i] = acc[i] / s;
     }
+}
+
+// A thread per observation: dL/d(u, v) = W2 J mu, and a fixed camera's cross terms.  (mu_p is zero for a
+// fixed track.)
+template <int NI>
+__global__ void __launch_bounds__(128) k_adj_gradient(Shape S, DevPtrs D, AdjBuffers B, const double* __restrict__ mu) {
+    const long long o = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (o >= S.nop) return;
+    const AdjLayout& Lo = B.lay;
+    const int ni = NI < 0 ? S.ni : NI, nl = 9 + ni;
+    const int cam = D.obs_cam[o], t = D.obs_trk[o];
+    const double* rec = B.rec + static_cast<size_t>(o) * Lo.stride;
+    double mc[6], mp[3], mk[NI < 0 ? kMaxNI : NI + 1];
+    primary_mu(S, D, mu, cam, ni, mc, mk);
+    for (int i = 0; i < 3; ++i) mp[i] = B.mu_p[static_cast<size_t>(t) * 3 + i];
+    const double* J = rec + Lo.jac();
+    double j[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const double* Jr = J + r * nl;
+        double v = 0.0;
+#pragma unroll
+        for (int a = 0; a < 6; ++a) v = fma(Jr[a], mc[a], v);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) v = fma(Jr[6 + a], mp[a], v);
+        for (int k = 0; k < ni; ++k) v = fma(Jr[9 + k], mk[k], v);
+        j[r] = v;
+    }
+    const double* w2 = rec + Lo.w2();
+    B.grad_obs[2 * static_cast<size_t>(o)] = w2[0] * j[0] + w2[1] * j[1];
+    B.grad_obs[2 * static_cast<size_t>(o) + 1] = w2[1] * j[0] + w2[2] * j[1];
+    if (D.cam_block[cam] < 0) {
+        // fixed camera: -(H_c,pt mu_p + H_c,k mu_k)
+        const double* hcp = rec + Lo.hcp();
+        const double* hck = rec + Lo.hck();
+        for (int a = 0; a < 6; ++a) {
+            double v = hcp[a * 3] * mp[0] + hcp[a * 3 + 1] * mp[1] + hcp[a * 3 + 2] * mp[2];
+            for (int k = 0; k < ni; ++k) v += hck[a * ni + k] * mk[k];
+            if (v != 0.0) atomicAdd(B.grad_fixed_cam + static_cast<size_t>(cam) * 6 + a, -v);
+        }
+    }
+}
+
+// Gauge terms of one observation of the scale camera, added to sum[0..3]: the observation in the
+// Euclidean centre chart, with mu lifted to it (centre step = tangent basis * mu_t).
+template <int NI>
+__device__ __forceinline__ void gauge_terms(const Shape& S, const DevPtrs& D, const AdjBuffers& B,
+                                            const double* __restrict__ mu, long long o, double* sum) {
+    constexpr int kNI = NI < 0 ? kMaxNI : NI;
+    const int cam = D.obs_cam[o];
+    const int ni = NI < 0 ? S.ni : NI, nl = 9 + ni, t = D.obs_trk[o];
+    AdjLayout Lo;
+    Lo.ni = ni;
+    double mc[6], mk[kNI + 1];
+    primary_mu(S, D, mu, cam, ni, mc, mk);
+    double frec[68 + 11 * kNI + kNI * (kNI + 1) / 2];
+    DCam c;
+    load_cam(D.cams_eff + static_cast<size_t>(cam) * kCamStride, c);
+    double n[3];
+    gauge_normal(S, D, n);
+    if (!adj_obs_hessian<NI>(c, D.points + static_cast<size_t>(t) * 3, D.pscale[t], D.obs_u[o], D.obs_v[o], D.obs_w[o],
+                             S.loss, S.loss_scale, false, D.gauge_basis, n, S.gauge_baseline, ni, S.int_cols, frec)) {
+        atomicOr(B.flags, 2);
+        return;
+    }
+    const double* gb = D.gauge_basis;
+    double ml[9 + kNI];
+    for (int i = 0; i < 3; ++i) ml[i] = mc[i];
+    for (int i = 0; i < 3; ++i) ml[3 + i] = gb[i] * mc[3] + gb[3 + i] * mc[4];
+    for (int i = 0; i < 3; ++i) ml[6 + i] = B.mu_p[static_cast<size_t>(t) * 3 + i];
+    for (int k = 0; k < ni; ++k) ml[9 + k] = mk[k];
+    // hC = H[C rows, all] * ml
+    const double* hcc = frec + Lo.hcc();
+    const double* hcp = frec + Lo.hcp();
+    const double* hck = frec + Lo.hck();
+    double hC[3];
+    for (int i = 0; i < 3; ++i) {
+        const int r = 3 + i;
+        double v = 0.0;
+        for (int a = 0; a < 6; ++a) v += hcc[r <= a ? sym6(r, a) : sym6(a, r)] * ml[a];
+        for (int j = 0; j < 3; ++j) v += hcp[r * 3 + j] * ml[6 + j];
+        for (int k = 0; k < ni; ++k) v += hck[r * ni + k] * ml[9 + k];
+        hC[i] = v;
+    }
+    // gC = d phi / dC = lam^T J_C
+    const double* fJ = frec + Lo.jac();
+    const double* fw = frec + Lo.w2();
+    double gC[3];
+    for (int i = 0; i < 3; ++i) gC[i] = fw[3] * fJ[3 + i] + fw[4] * fJ[nl + 3 + i];
+    const double gt = gC[0] * ml[3] + gC[1] * ml[4] + gC[2] * ml[5];
+    for (int i = 0; i < 3; ++i) sum[i] -= hC[i];
+    sum[3] -= n[0] * hC[0] + n[1] * hC[1] + n[2] * hC[2] + gt / S.gauge_baseline;
+}
+
+// A block lists the scale camera's observations among its kGaugeSpan, then takes a thread per listed one
+// and adds the block's sums once (an atomic per observation queued on four addresses).
+constexpr int kGaugeThreads = 128, kGaugeSpan = 2048;
+template <int NI>
+__global__ void __launch_bounds__(kGaugeThreads) k_adj_gauge(Shape S, DevPtrs D, AdjBuffers B,
+                                                             const double* __restrict__ mu) {
+    __shared__ int s_list[kGaugeSpan];
+    __shared__ int s_count;
+    __shared__ double s_sum[4][kGaugeThreads / 32];
+    const int cam = S.gauge_scale, tid = threadIdx.x;
+    if (D.cam_block[cam] < 0) return;
+    if (tid == 0) s_count = 0;
+    __syncthreads();
+    const long long o0 = static_cast<long long>(blockIdx.x) * kGaugeSpan;
+    const int span = static_cast<int>(min(static_cast<long long>(kGaugeSpan), S.nop - o0));
+    for (int i = tid; i < span; i += kGaugeThreads)
+        if (D.obs_cam[o0 + i] == cam) s_list[atomicAdd(&s_count, 1)] = i;
+    __syncthreads();
+    const int count = s_count;
+    if (count == 0) return;
+    double sum[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int i = tid; i < count; i += kGaugeThreads) gauge_terms<NI>(S, D, B, mu, o0 + s_list[i], sum);
+    __syncwarp();
+    for (int k = 0; k < 4; ++k) {
+        const double v = warp_sum(sum[k]);
+        if ((tid & 31) == 0) s_sum[k][tid >> 5] = v;
+    }
+    __syncthreads();
+    if (tid < 4) {
+        double v = 0.0;
+        for (int w = 0; w < kGaugeThreads / 32; ++w) v += s_sum[tid][w];
+        atomicAdd(B.gauge + tid, v);
+    }
+}
+
+
+template <int NI>
+void hessian_of(const Shape& S, const DevPtrs& D, const AdjBuffers& B, cudaStream_t st) {
+    k_adj_hessian<NI><<<static_cast<unsigned>((S.nop + 127) / 128), 128, 0, st>>>(S, D, B);
+}
+
+template <int NI>
+void gradient_of(const Shape& S, const DevPtrs& D, const AdjBuffers& B, const double* mu, cudaStream_t st) {
+    const unsigned by_obs = static_cast<unsigned>((S.nop + 127) / 128);
+    if (by_obs) k_adj_terms<NI><<<by_obs, 128, 0, st>>>(S, D, B, mu);
+    k_adj_points<<<(S.ntp + 63) / 64, 64, 0, st>>>(S, D, B);
+    if (!by_obs) return;
+    k_adj_gradient<NI><<<by_obs, 128, 0, st>>>(S, D, B, mu);
+    if (S.gauge_scale >= 0 && S.gauge_anchor >= 0 && S.gauge_baseline > 0.0)
+        k_adj_gauge<NI><<<static_cast<unsigned>((S.nop + kGaugeSpan - 1) / kGaugeSpan), kGaugeThreads, 0, st>>>(S, D, B, mu);
 }
 
 }  // namespace
 
 void launch_adjoint_hessian(const Shape& S, const DevPtrs& D, const AdjBuffers& B, cudaStream_t st) {
     if (S.nop <= 0) return;
-    k_adj_hessian<<<static_cast<unsigned>((S.nop + 127) / 128), 128, 0, st>>>(S, D, B);
+    // a column count known to the compiler keeps the Hessian's intermediates in registers; no column and
+    // the eight of a self-calibration (f, cx, cy, k1-k3, p1, p2) are the usual ones
+    if (S.ni == 0) hessian_of<0>(S, D, B, st);
+    else if (S.ni == 8) hessian_of<8>(S, D, B, st);
+    else hessian_of<-1>(S, D, B, st);
 }
 
 void launch_adjoint_rhs(const Shape& S, const DevPtrs& D, const AdjBuffers& B, const RedOut<double>& R, cudaStream_t st) {
@@ -779,7 +975,7 @@ void launch_adjoint_rhs(const Shape& S, const DevPtrs& D, const AdjBuffers& B, c
 
 size_t adjoint_assemble_smem(const Shape& S) {
     const auto up = [](size_t b) { return (b + 15) & ~static_cast<size_t>(15); };
-    return up(static_cast<size_t>(S.max_obs) * 18 * sizeof(double)) + up(static_cast<size_t>(S.max_tracks) * 12 * sizeof(double)) +
+    return 2 * up(static_cast<size_t>(S.max_obs) * kAdjRow * sizeof(double)) + up(static_cast<size_t>(S.max_tracks) * 12 * sizeof(double)) +
            up(static_cast<size_t>(S.max_tracks) * S.nb * 3 * sizeof(double)) + up(static_cast<size_t>(S.max_obs) * sizeof(int)) +
            up(static_cast<size_t>(S.max_tracks + 1) * sizeof(int)) + up(sizeof(int));
 }
@@ -800,7 +996,8 @@ void launch_adjoint_schur(const Shape& S, const DevPtrs& D, const AdjBuffers& B,
 
 void launch_adjoint_gradient(const Shape& S, const DevPtrs& D, const AdjBuffers& B, const double* mu, cudaStream_t st) {
     if (S.ntp <= 0) return;
-    k_adj_gradient<<<(S.ntp + 127) / 128, 128, 0, st>>>(S, D, B, mu);
+    if (S.ni == 0) gradient_of<0>(S, D, B, mu, st);
+    else gradient_of<-1>(S, D, B, mu, st);
 }
 
 }  // namespace pb

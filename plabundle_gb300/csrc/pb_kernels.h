@@ -274,6 +274,7 @@ struct AdjBuffers {
     double* gcam;           // nc * 6 dL/d(final pose): rotation increment, world centre
     double* gint;           // ng * kP dL/d(group parameters)
     double* mu_p;           // ntp * 3 point part of the adjoint solution (point chart)
+    double* terms;          // nop * 3 per-observation terms of the point sums
     double* grad_obs;       // nop * 2 dL/d(u, v) (processing order)
     double* grad_fixed_cam; // nc * 6 cross terms of fixed cameras (zeroed by the caller)
     double* grad_fixed_pt;  // ntp * 3 cross terms of fixed tracks (world)

@@ -2169,6 +2169,7 @@ pb_status adjoint_core(pb_gpu_ctx* c, int newton, pb_adjoint_report* rep, float*
     const int nc = m.nc, ntp = S.ntp;
     AdjBuffers& B = c->adj;
     B.newton = newton;
+    B.terms = c->bs_terms;
     cudaEvent_t ev[4];
     for (auto& e : ev) check(cudaEventCreate(&e), "event");
     struct EvGuard {
@@ -2222,7 +2223,7 @@ pb_status adjoint_core(pb_gpu_ctx* c, int newton, pb_adjoint_report* rep, float*
     if (rc) return fail(c, PB_ERR_SINGULAR_BLOCK, "the exact Hessian is not positive definite (not a minimum?)");
     check(cudaEventRecord(ev[2], st), "event");
     launch_adjoint_gradient(S, D, B, c->step_c, st);
-    ++c->launches;
+    c->launches += 3 + (S.gauge_scale >= 0 && S.gauge_anchor >= 0 && S.gauge_baseline > 0.0 ? 1 : 0);
     check(cudaGetLastError(), "adjoint gradient launch");
     check(cudaEventRecord(ev[3], st), "event");
     cudaEventSynchronize(ev[3]);
