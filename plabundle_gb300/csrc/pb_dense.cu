@@ -175,12 +175,13 @@ __device__ __forceinline__ int owned_elements(int* ii, int* ll) {
 //
 // The factorisation is the unscaled right-looking elimination (after step j, column j holds
 // d_j * L_:j): every lower element (i, l) receives a_il = fma(-(a_ij a_lj), 1 / d_j, a_il) for
-// j < l in increasing j (one rounding of the product, one of the update, in every phase).  It runs in four panels of 16 columns so that the block synchronises 12 times instead of once
-// per column: warp 0 eliminates the panel's 16 x 16 diagonal block on its own (warp barriers) and
-// records 1 / d_j, then the rows below take the panel's steps in registers (16 lanes per row, the
-// row's pivot entries by shuffle), then every thread applies the panel's 16 steps, in order, to
-// its elements of the trailing block.  Each element sees the same updates in the same order as a
-// column-by-column elimination.  The inverse R = L^-1 (R = I, R_ic -= L_ij R_jc / L_jj for
+// j < l in increasing j (one rounding of the product, one of the update, in every phase).  It runs in
+// eight panels of eight columns: three warps take the rows of a panel, a lane per row with its eight
+// columns in registers (lanes 0-7 of each hold the panel's own rows, so that the pivot entries come by
+// shuffle and no warp waits for another), then every thread applies the panel's eight steps, in order,
+// to its elements of the trailing block.  Each element sees the same updates in the same order as a
+// column-by-column elimination.  (Against panels of sixteen columns, their own block on one warp and the
+// rows below it after a barrier: 354 unknowns 239 -> 220 us a factorisation, 114 unknowns 109 -> 94.)  The inverse R = L^-1 (R = I, R_ic -= L_ij R_jc / L_jj for
 // i > j >= c, then R_ic / L_ii) is independent per column: four lanes own a column (rows split
 // mod 4, held in registers) and pass row j between them by shuffle, with no block barrier.
 template <typename T>
@@ -192,59 +193,76 @@ __device__ void diag_factor_inverse(T* __restrict__ A, T* __restrict__ Dinv, int
     owned_elements(ii, ll);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __shared__ T s_inv[TS];  // 1 / d_j of the elimination, then 1 / L_jj of the inverse
-    constexpr int PW = 16;   // panel width
+    constexpr int PW = 8;    // panel width
     __syncthreads();
     for (int c0 = 0; c0 < TS; c0 += PW) {
-        // (a) the panel's diagonal block, warp 0, in registers: lane r holds columns 0-7 of row
-        // c0 + r, lane r + 16 its columns 8-15, and pivot entries reach the other lanes by shuffle
-        if (warp == 0) {
-            const int ri = lane & 15, half = lane >> 4;
-            T a[PW / 2];
+        // (a) the panel: row c0 + lane for lanes 0-7, then 24 of the rows below per warp
+        const int below = TS - c0 - PW;
+        T a[PW];
+        const int i = lane < PW ? c0 + lane : c0 + PW + 24 * warp + lane - PW;
+        const bool mine = i < TS;
+        if (warp < max(1, (below + 23) / 24)) {
 #pragma unroll
-            for (int q = 0; q < PW / 2; ++q) a[q] = sA[(c0 + ri) * TP + c0 + 8 * half + q];
+            for (int l = 0; l < PW; ++l) a[l] = mine ? sA[i * TP + c0 + l] : T(0);
+            // (no branch in the chain of pivots: the marks and reciprocals are written after it)
+            bool bad = false;
+            T my_inv = T(0);
 #pragma unroll
-            for (int rj = 0; rj < PW; ++rj) {
-                const int hj = rj >> 3;  // half holding column rj
-                const T d = __shfl_sync(0xffffffffu, a[rj & 7], rj + 16 * hj);
-                if (!(d > T(0))) {
-                    if (lane == 0) atomicOr(status, 2);
-                }
-                const T inv = d > T(0) ? T(1) / d : T(0);
-                if (lane == 0) s_inv[c0 + rj] = inv;
-                const T aij = __shfl_sync(0xffffffffu, a[rj & 7], ri + 16 * hj);
+            for (int j = 0; j < PW; ++j) {
+                const T d = __shfl_sync(0xffffffffu, a[j], j);
+                const bool pos = d > T(0);
+                const T inv = __frcp_rn(pos ? d : T(1)) * (pos ? T(1) : T(0));
+                bad |= !pos;
+                if (lane == j) my_inv = inv;
+                const T aij = a[j];
 #pragma unroll
-                for (int rl = 1; rl < PW; ++rl) {
-                    if (rl <= rj) continue;
-                    const T alj = __shfl_sync(0xffffffffu, a[rj & 7], rl + 16 * hj);
-                    if (half == (rl >> 3) && ri >= rl) a[rl & 7] = fma(-(aij * alj), inv, a[rl & 7]);
+                for (int l = j + 1; l < PW; ++l) {
+                    const T alj = __shfl_sync(0xffffffffu, aij, l);
+                    a[l] = fma(-(aij * alj), inv, a[l]);
                 }
             }
-#pragma unroll
-            for (int q = 0; q < PW / 2; ++q) sA[(c0 + ri) * TP + c0 + 8 * half + q] = a[q];
-        }
-        __syncthreads();
-        // (b) rows below the diagonal block, panel columns: two rows per warp, a lane per column
-        const int nbelow = TS - c0 - PW;
-        for (int task = warp; task < nbelow / 2; task += static_cast<int>(blockDim.x >> 5)) {
-            const int i = c0 + PW + 2 * task + (lane >> 4), l = c0 + (lane & 15);
-            T a = sA[i * TP + l];
-#pragma unroll
-            for (int j = c0; j < c0 + PW; ++j) {
-                const T aij = __shfl_sync(0xffffffffu, a, (lane & 16) | (j - c0));
-                if (l > j) a = fma(-(aij * sA[l * TP + j]), s_inv[j], a);
+            if (warp == 0) {
+                if (lane < PW) s_inv[c0 + lane] = my_inv;
+                if (lane == 0 && bad) atomicOr(status, 2);
             }
-            sA[i * TP + l] = a;
+            if (mine && lane >= PW)
+#pragma unroll
+                for (int l = 0; l < PW; ++l) sA[i * TP + c0 + l] = a[l];
         }
         __syncthreads();
-        // (c) the trailing block: elements (i, l), c0 + 16 <= l <= i < 64, the panel's steps in order
-        const int m = nbelow, ntrail = m * (m + 1) / 2;
-        for (int e = threadIdx.x; e < ntrail; e += blockDim.x) {
-            const int t = tri_row(e);
-            const int i = c0 + PW + t, l = c0 + PW + (e - t * (t + 1) / 2);
-            T a = sA[i * TP + l];
+        // the panel's own rows, from warp 0, once every warp has read them (the trailing block does not;
+        // entries above the diagonal are not read again)
+        if (warp == 0 && lane < PW)
 #pragma unroll
-            for (int j = c0; j < c0 + PW; ++j) a = fma(-(sA[i * TP + j] * sA[l * TP + j]), s_inv[j], a);
-            sA[i * TP + l] = a;
+            for (int l = 0; l < PW; ++l) sA[i * TP + c0 + l] = a[l];
+        // (b) the trailing block: elements (r, l), c0 + 8 <= l <= r < 64, the panel's steps in order; a lane
+        // per column (and the column 32 to the right), a warp every eighth row
+        {
+            T inv[PW], t0[PW], t1[PW];
+            const int l0 = c0 + PW + lane, l1 = l0 + 32;
+#pragma unroll
+            for (int j = 0; j < PW; ++j) {
+                inv[j] = s_inv[c0 + j];
+                t0[j] = l0 < TS ? sA[l0 * TP + c0 + j] : T(0);
+                t1[j] = l1 < TS ? sA[l1 * TP + c0 + j] : T(0);
+            }
+            for (int r = c0 + PW + warp; r < TS; r += 8) {
+                T rj[PW];
+#pragma unroll
+                for (int j = 0; j < PW; ++j) rj[j] = sA[r * TP + c0 + j];
+                if (l0 <= r) {
+                    T x = sA[r * TP + l0];
+#pragma unroll
+                    for (int j = 0; j < PW; ++j) x = fma(-(rj[j] * t0[j]), inv[j], x);
+                    sA[r * TP + l0] = x;
+                }
+                if (l1 <= r) {
+                    T x = sA[r * TP + l1];
+#pragma unroll
+                    for (int j = 0; j < PW; ++j) x = fma(-(rj[j] * t1[j]), inv[j], x);
+                    sA[r * TP + l1] = x;
+                }
+            }
         }
         __syncthreads();
     }
@@ -327,10 +345,20 @@ __device__ __forceinline__ void tile_product_store(T* __restrict__ C, int ldc, c
         }
 }
 
-template <typename T>
+// Barrier between the phases of a cooperative kernel: of the whole grid, or, for grids of at most sixteen
+// blocks, which one cluster holds, of the cluster (114 unknowns: CG solve 53.5 -> 45.0 us, FP32 factor 94 ->
+// 90, FP64 factor 145 -> 139).  Larger systems keep their blocks: 354 unknowns on sixteen blocks took 135 us a
+// solve against 121 on 45.  Either barrier orders the blocks' writes to global memory.
+constexpr int kClusterMax = 16;
+template <bool CLUSTER>
+__device__ __forceinline__ void phase_barrier() {
+    if constexpr (CLUSTER) cgk::this_cluster().sync();
+    else cgk::this_grid().sync();
+}
+
+template <typename T, bool CLUSTER>
 __global__ void __launch_bounds__(256) k_potrf_coop(T* __restrict__ A, T* __restrict__ X, T* __restrict__ Dinv, int np,
                                                    int nt, int* __restrict__ status) {
-    cgk::grid_group grid = cgk::this_grid();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* sA = reinterpret_cast<T*>(smem_raw);
     T* sB = sA + TS * TP;
@@ -340,9 +368,9 @@ __global__ void __launch_bounds__(256) k_potrf_coop(T* __restrict__ A, T* __rest
     for (int r = blockIdx.x; r < nrow; r += gridDim.x)
         for (int c = threadIdx.x; c < np; c += blockDim.x) X[static_cast<size_t>(r) * np + c] = r == c ? T(1) : T(0);
     (void)nthreads;
-    grid.sync();
+    phase_barrier<CLUSTER>();
     if (blockIdx.x == 0) diag_factor_inverse<T>(A, Dinv, np, 0, sA, sB, status);
-    grid.sync();
+    phase_barrier<CLUSTER>();
     for (int k = 0; k < nt; ++k) {
         const int m = nt - 1 - k;
         const T* Dk = Dinv + static_cast<size_t>(k) * TS * TS;
@@ -364,7 +392,7 @@ __global__ void __launch_bounds__(256) k_potrf_coop(T* __restrict__ A, T* __rest
             }
             __syncthreads();
         }
-        grid.sync();
+        phase_barrier<CLUSTER>();
         // Trailing update and R update.  Item 0 is the next diagonal tile (k+1, k+1): block 0
         // updates it and factors it at once (lookahead), while the other blocks share the rest.
         const int ntrail = m * (m + 1) / 2;
@@ -396,7 +424,7 @@ __global__ void __launch_bounds__(256) k_potrf_coop(T* __restrict__ A, T* __rest
                 diag_factor_inverse<T>(A, Dinv, np, k + 1, sA, sB, status);
             }
         }
-        grid.sync();
+        phase_barrier<CLUSTER>();
     }
     // X^T into the upper triangle of A (tile (j, i) = X_ij^T, j <= i).  The preconditioner is
     // applied as X^T (X u): forming X^T X explicitly in the factor's precision would square the
@@ -562,10 +590,10 @@ __device__ __forceinline__ int balanced32(int warp, int m) {
 // A (lower triangle, np x np with identity padding) -> X = L^-1 in X and X^T in the upper triangle of A;
 // nt tiles of 32.  The steps of k_potrf_coop: panel and inverse row, barrier, trailing and inverse
 // update with the next diagonal tile factored by the block that updates it, barrier.
+template <bool CLUSTER>
 __global__ void __launch_bounds__(kPotrf64Threads) k_potrf64_coop(double* __restrict__ A, double* __restrict__ X,
                                                                   double* __restrict__ Dinv, int np, int nt,
                                                                   int* __restrict__ status) {
-    cgk::grid_group grid = cgk::this_grid();
     extern __shared__ __align__(16) double smem64[];
     double* sA = smem64;
     double* sB = sA + TD * TDP;
@@ -582,7 +610,7 @@ __global__ void __launch_bounds__(kPotrf64Threads) k_potrf64_coop(double* __rest
         __syncthreads();
         diag_factor_inverse64(A, np, Dinv, sC, sA, sB, sT, s_d, status);
     }
-    grid.sync();
+    phase_barrier<CLUSTER>();
     for (int k = 0; k < nt; ++k) {
         const int m = nt - 1 - k;
         const double* Dk = Dinv + static_cast<size_t>(k) * TD * TD;
@@ -623,7 +651,7 @@ __global__ void __launch_bounds__(kPotrf64Threads) k_potrf64_coop(double* __rest
             }
             __syncthreads();
         }
-        grid.sync();
+        phase_barrier<CLUSTER>();
         // trailing update and R update; item 0 is the next diagonal tile, updated and factored by
         // block 0 while the other blocks share the rest
         const int ntrail = m * (m + 1) / 2;
@@ -683,7 +711,7 @@ __global__ void __launch_bounds__(kPotrf64Threads) k_potrf64_coop(double* __rest
             for (int q = 0; q < 4; ++q) dst[static_cast<size_t>(warp + 8 * q) * np + lane] = acc[q];
             __syncthreads();
         }
-        grid.sync();
+        phase_barrier<CLUSTER>();
     }
     for (int it = blockIdx.x; it < nt * (nt + 1) / 2; it += gridDim.x) {
         const int i = tri_row(it), j = it - i * (i + 1) / 2;
@@ -910,7 +938,7 @@ __device__ __forceinline__ double spmv_update(const PcgSystem<double>& sys, cons
 }
 
 // out: [0] iterations, [1] relative residual, [2] converged, [3] status (1: breakdown)
-template <typename T>
+template <typename T, bool CLUSTER>
 __global__ void __launch_bounds__(kCgThreads, 2) k_dense_cg(PcgSystem<double> sys, const T* __restrict__ X,
                                                          const T* __restrict__ XT, int np,
                                                          const double* __restrict__ dscale,
@@ -921,7 +949,6 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_dense_cg(PcgSystem<double> sy
                                                          T* __restrict__ u, T* __restrict__ w,
                                                          double* __restrict__ part, double* __restrict__ out,
                                                          double rel_tol, double abs_tol, int max_it) {
-    cgk::grid_group grid = cgk::this_grid();
     __shared__ double s_vals[kCgThreads];
     __shared__ double s_q[12];
     __shared__ double s_tot[kCgPart];
@@ -937,11 +964,11 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_dense_cg(PcgSystem<double> sy
         bb += b[i] * b[i];
     }
     block_partial(bb, s_vals, s_q, mypart + 0);
-    grid.sync();
+    phase_barrier<CLUSTER>();
     tri_rows<T, true>(X, np, n, u, w, nullptr, nullptr, nullptr);
-    grid.sync();
+    phase_barrier<CLUSTER>();
     block_partial(tri_rows<T, false>(XT, np, n, w, nullptr, z, dscale, b), s_vals, s_q, mypart + 1);
-    grid.sync();
+    phase_barrier<CLUSTER>();
     grid_totals<true>(part, 0, s_q, s_tot);
     const double bnorm = sqrt(s_tot[0]);
     double rz = s_tot[1];
@@ -959,7 +986,7 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_dense_cg(PcgSystem<double> sy
             p_cur = t;
         }
         block_partial(spmv_update(sys, z, beta, p_old, p_cur, qpart, pose_seg, border_seg), s_vals, s_q, mypart + 2);
-        grid.sync();
+        phase_barrier<CLUSTER>();
         grid_totals<false>(part, 2, s_q, s_tot);
         const double pq = s_tot[2];
         if (!(pq > 0.0) || !isfinite(pq) || !isfinite(rz)) {
@@ -988,7 +1015,7 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_dense_cg(PcgSystem<double> sy
             rr += rv * rv;
         }
         block_partial(rr, s_vals, s_q, mypart + 0);
-        grid.sync();
+        phase_barrier<CLUSTER>();
         ++it;
         grid_totals<false>(part, 0, s_q, s_tot);
         rn = sqrt(s_tot[0]);
@@ -1001,9 +1028,9 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_dense_cg(PcgSystem<double> sy
             break;
         }
         tri_rows<T, true>(X, np, n, u, w, nullptr, nullptr, nullptr);
-        grid.sync();
+        phase_barrier<CLUSTER>();
         block_partial(tri_rows<T, false>(XT, np, n, w, nullptr, z, dscale, r), s_vals, s_q, mypart + 1);
-        grid.sync();
+        phase_barrier<CLUSTER>();
         grid_totals<false>(part, 1, s_q, s_tot);
         const double rz_new = s_tot[1];
         beta = rz_new / rz;
@@ -1029,13 +1056,62 @@ size_t dense_bytes(int n) {
     return 2 * static_cast<size_t>(np) * np * sizeof(T) + static_cast<size_t>(np / TS) * TS * TS * sizeof(T);
 }
 
+// Launch of `grid` blocks as one cluster (more than eight need the non-portable size).
+static void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& at, int grid, int threads, size_t smem,
+                           cudaStream_t st) {
+    cfg = cudaLaunchConfig_t{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    at = cudaLaunchAttribute{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = static_cast<unsigned>(grid);
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+}
+
+// Largest cluster (0, 8 or kClusterMax blocks) of the kernel that the device can hold.
+static int largest_cluster(const void* kernel, int threads, size_t smem) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    for (int size : {kClusterMax, 8}) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at;
+        cluster_config(cfg, at, size, threads, smem, nullptr);
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0) return size;
+    }
+    cudaGetLastError();  // (a size that does not fit is not an error of the caller)
+    return 0;
+}
+
+// Launches a kernel of barrier-separated phases: as one cluster up to `cluster` blocks, else as a
+// cooperative grid.
+static cudaError_t launch_phased(const void* grid_kernel, const void* cluster_kernel, int cluster, int grid, int threads,
+                                 void** args, size_t smem, cudaStream_t st) {
+    if (grid > cluster) return cudaLaunchCooperativeKernel(grid_kernel, dim3(grid), dim3(threads), args, smem, st);
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at;
+    cluster_config(cfg, at, grid, threads, smem, st);
+    return cudaLaunchKernelExC(&cfg, cluster_kernel, args);
+}
+
 template <typename T>
 int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, cudaStream_t st, int* launches) {
     const int n = W.n, np = W.np, nt = W.nt;
     const size_t two_tiles = 2 * static_cast<size_t>(TS) * TP * sizeof(T);
-    static std::once_flag attrs;
-    if constexpr (sizeof(T) == 4)
-        std::call_once(attrs, [&] { set_smem<T>(reinterpret_cast<const void*>(&k_potrf_coop<T>), two_tiles); });
+    constexpr bool f64 = sizeof(T) == 8;
+    const void *kernel, *cluster_kernel;
+    if constexpr (f64) {
+        kernel = reinterpret_cast<const void*>(&k_potrf64_coop<false>);
+        cluster_kernel = reinterpret_cast<const void*>(&k_potrf64_coop<true>);
+    } else {
+        kernel = reinterpret_cast<const void*>(&k_potrf_coop<T, false>);
+        cluster_kernel = reinterpret_cast<const void*>(&k_potrf_coop<T, true>);
+    }
+    const int threads = f64 ? kPotrf64Threads : 256;
+    const size_t smem = f64 ? kPotrf64Smem : two_tiles;
     int L = 0;
     cudaMemsetAsync(W.status, 0, sizeof(int), st);
     cudaMemsetAsync(W.A, 0, static_cast<size_t>(np) * np * sizeof(T), st);
@@ -1045,13 +1121,10 @@ int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, cu
     if (nfill > 0) k_dense_fill<T><<<static_cast<unsigned>((nfill + 255) / 256), 256, 0, st>>>(sys, W.dscale, W.A, np);
     k_dense_diag<T><<<(np + 255) / 256, 256, 0, st>>>(W.A, n, np, shift);
     L += 3;
-    constexpr bool f64 = sizeof(T) == 8;
-    const void* kernel;
-    if constexpr (f64) kernel = reinterpret_cast<const void*>(&k_potrf64_coop);
-    else kernel = reinterpret_cast<const void*>(&k_potrf_coop<T>);
-    const int threads = f64 ? kPotrf64Threads : 256;
-    const size_t smem = f64 ? kPotrf64Smem : two_tiles;
     if (W.fact_grid == 0) {
+        set_smem<T>(kernel, smem);
+        set_smem<T>(cluster_kernel, smem);
+        W.fact_cluster = largest_cluster(cluster_kernel, threads, smem);
         int dev = 0, sms = 0, per_sm = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1067,7 +1140,7 @@ int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, cu
         void* args[] = {&A, &X, &Dv, &npv, &ntv, &stv};
         // one block per lower tile at most: small systems take a small grid
         const int fgrid = std::max(1, std::min(W.fact_grid, ntv * (ntv + 1) / 2));
-        if (cudaLaunchCooperativeKernel(kernel, dim3(fgrid), dim3(threads), args, smem, st) != cudaSuccess) return -1;
+        if (launch_phased(kernel, cluster_kernel, W.fact_cluster, fgrid, threads, args, smem, st) != cudaSuccess) return -1;
         ++L;
     }
     if (launches) *launches += L;
@@ -1091,12 +1164,14 @@ int dense_pcg(const PcgSystem<double>& sys, DenseWork<T>& W, const double* b, do
         int dev = 0, sms = 0, per_sm = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dense_cg<T>, kCgThreads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dense_cg<T, false>, kCgThreads, 0);
+        W.cg_cluster = largest_cluster(reinterpret_cast<const void*>(&k_dense_cg<T, true>), kCgThreads, 0);
         W.coop_grid = std::max(1, std::min(per_sm, 2) * sms);
     }
     // one warp per row of the triangular products: small systems (local windows) take a small
     // grid and leave the rest of the device to concurrent work
-    const int grid = std::max(1, std::min(W.coop_grid, (W.n + kCgWarps - 1) / kCgWarps));
+    const int rows = (W.n + kCgWarps - 1) / kCgWarps;
+    const int grid = std::max(1, std::min(W.coop_grid, rows));
     PcgSystem<double> s = sys;
     const T* X = W.X;
     const T* XT = W.A;
@@ -1107,9 +1182,10 @@ int dense_pcg(const PcgSystem<double>& sys, DenseWork<T>& W, const double* b, do
     int ps = W.pose_seg, bs = W.border_seg;
     void* args[] = {&s, &X, &XT, &np, &dscale, &b, &W.x, &W.r, &W.z, &W.p, &W.w, &W.qpart, &ps, &bs, &W.ut, &W.wt,
                     &W.part, &W.scal, &rt, &at, &mi};
-    const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&k_dense_cg<T>), dim3(grid),
-                                                      dim3(kCgThreads), args, 0, st);
-    if (e != cudaSuccess) return -1;
+    if (launch_phased(reinterpret_cast<const void*>(&k_dense_cg<T, false>),
+                      reinterpret_cast<const void*>(&k_dense_cg<T, true>), W.cg_cluster, grid, kCgThreads, args, 0, st) !=
+        cudaSuccess)
+        return -1;
     if (launches) *launches += 1;
     cudaMemcpyAsync(h_scal, W.scal, 4 * sizeof(double), cudaMemcpyDeviceToHost, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) return -1;

@@ -228,6 +228,7 @@ struct DenseWork {
     double* scal = nullptr;
     int coop_grid = 0;       // blocks of the cooperative CG launch
     int fact_grid = 0;       // blocks of the cooperative factorisation
+    int cg_cluster = 0, fact_cluster = 0;  // blocks that one cluster of the kernel can hold
 };
 
 template <typename T>
