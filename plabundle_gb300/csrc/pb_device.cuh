@@ -739,8 +739,13 @@ __device__ __forceinline__ float warp_sum(float v) {
 // scales and observation weights, written when the FP64 state changes.
 
 __host__ __device__ __forceinline__ float2 ff_pack(double d) {
+#if defined(__CUDA_ARCH__)
+    const ff v = ff_make_bits(d);
+    return make_float2(v.hi, v.lo);
+#else
     const float h = static_cast<float>(d);
     return make_float2(h, static_cast<float>(d - static_cast<double>(h)));
+#endif
 }
 __device__ __forceinline__ ff ffl(float2 v) { return {v.x, v.y}; }
 __device__ __forceinline__ ff ff_sub(ff a, ff b) { return a + (-b); }

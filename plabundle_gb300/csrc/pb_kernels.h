@@ -85,8 +85,13 @@ void pb_set_assemble_smem_f64(size_t bytes);
 void launch_effective(const Shape& S, const DevPtrs& D, cudaStream_t st);
 // Rig problems (pb_rig.cu): capture and sensor state, the chain maps of the camera blocks and the
 // reduced system over the rig's pose blocks (captures, then sensors).
-constexpr int kRigSegTerms = 64;  // pose terms summed by one warp before the per-block sum
-constexpr int kRigItemSeg = 32;   // camera blocks of a rig block summed by one warp (border, rhs)
+// Pose terms summed by one warp before the per-block sum: a warp's terms wait for one another (3000 cycles
+// each), the segments of a block are added in order afterwards.  64 when the terms fill the device several
+// times over, down to 16 for small rigs (150 cameras: 94 -> 29 us with 16 instead of 64; the sums 5 -> 9).
+inline int rig_seg_terms(long long terms) {
+    return static_cast<int>(std::min<long long>(64, std::max<long long>(16, terms / (152 * 32))));
+}
+constexpr int kRigItemSeg = 8;    // camera blocks of a rig block summed by one warp (border, rhs; 51 -> 20 us with 8 instead of 32)
 struct RigDev {
     int ncap, nsen, nrb, ncb, nup, nnzb;
     double* cap_state;   // ncap * 12: rotation (9), centre (3)
@@ -114,7 +119,7 @@ struct RigDev {
     int* term_begin;
     int* terms;          // 2 per term: camera-block CSR position, a << 2 | sensor row << 1 | sensor column
     const int* cb_col_idx;  // column indices of the camera-block CSR
-    // segments of the pose terms (consecutive terms of one upper block, at most kRigSegTerms):
+    // segments of the pose terms (consecutive terms of one upper block, at most rig_seg_terms):
     // seg_begin[s] first term of segment s (nseg + 1); up_seg_begin[u] first segment of upper
     // block u (nup + 1); seg_part the segments' partial sums (36 each)
     int nseg;

@@ -13,7 +13,7 @@
 // reduced system over the rig's blocks is S_rig[I][J] = sum M_aI^T S[a][b] M_bJ over the camera
 // blocks a, b chained to I and J, B_rig[I] = sum M_aI^T B[a], g_rig[I] = sum M_aI^T g[a].  The
 // sums follow host-built term lists in a fixed order: the pose terms of one rig block in
-// segments of kRigSegTerms consecutive terms (one warp each), then the segments in order; the
+// segments of rig_seg_terms consecutive terms (one warp each), then the segments in order; the
 // border and right-hand side over segments of kRigItemSeg camera blocks likewise.  The rig pose
 // diagonal is then damped as finalizePrimaryDiagonal(1 + damping, 1) damps every primary
 // diagonal, the solution is mapped
@@ -91,7 +91,7 @@ __global__ void k_rig_maps(RigDev R) {
         }
 }
 
-// Pose blocks, first pass: one warp per segment of at most kRigSeg terms of one upper rig block.
+// Pose blocks, first pass: one warp per segment of at most rig_seg_terms terms of one upper rig block.
 // Per term (camera-block CSR entry p = (a, b) and the sides of its chains) the warp forms
 // Y = S_ab M_b in shared memory and Z = M_a^T Y, and keeps the running sum of Z over the segment's
 // terms in order (lane e holds entries e and e + 32 of the 6x6 block); the partial goes to
@@ -162,6 +162,7 @@ __global__ void k_rig_pose_sum(RigDev R, double damping) {
     const int u = static_cast<int>(e / 36), rq = static_cast<int>(e - 36LL * u);
     const int r = rq / 6, q = rq - 6 * (rq / 6);
     double v = 0.0;
+#pragma unroll 8
     for (int g = R.up_seg_begin[u]; g < R.up_seg_begin[u + 1]; ++g) v += R.seg_part[static_cast<size_t>(g) * 36 + rq];
     const int tp = R.up_tpos[u];
     if (tp < 0 && r == q) v = v != 0.0 ? v * (1.0 + damping) : 1.0;
@@ -182,6 +183,7 @@ __global__ void __launch_bounds__(256) k_rig_border_seg(RigDev R, const double* 
     const int t0 = R.bseg_begin[g], t1 = R.bseg_begin[g + 1];
     for (int j = lane; j < w; j += 32) {
         double v = 0.0;
+#pragma unroll 2
         for (int t = t0; t < t1; ++t) {
             const int code = R.blk_items[t], a = code >> 1;
             const double* M = R.maps + static_cast<size_t>(a) * 72 + (code & 1) * 36;
@@ -205,6 +207,7 @@ __global__ void k_rig_border_sum(RigDev R, const double* __restrict__ rhs, int n
         const int row = static_cast<int>(e / w), j = static_cast<int>(e - static_cast<long long>(row) * w);
         const int I = row / 6, r = row - 6 * I;
         double v = 0.0;
+#pragma unroll 8
         for (int g = R.blk_seg_begin[I]; g < R.blk_seg_begin[I + 1]; ++g)
             v += R.bpart[(static_cast<size_t>(g) * 6 + r) * w + j];
         if (j < nbw) {

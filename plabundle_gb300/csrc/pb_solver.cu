@@ -485,10 +485,11 @@ void upload_structure(pb_gpu_ctx* c) {
         R.blk_begin = upload_new(A, rm.blk_begin, st);
         R.blk_items = upload_new(A, rm.blk_items, st);
         {
-            // segments of at most kRigSegTerms consecutive pose terms of one upper block
+            // segments of consecutive pose terms of one upper block
+            const int seg_terms = rig_seg_terms(rm.term_begin.empty() ? 0 : rm.term_begin.back());
             std::vector<int> sb, ub(1, 0);
             for (int u = 0; u < R.nup; ++u) {
-                for (int t = rm.term_begin[u]; t < rm.term_begin[u + 1]; t += kRigSegTerms) sb.push_back(t);
+                for (int t = rm.term_begin[u]; t < rm.term_begin[u + 1]; t += seg_terms) sb.push_back(t);
                 ub.push_back(static_cast<int>(sb.size()));
             }
             sb.push_back(rm.term_begin.empty() ? 0 : rm.term_begin.back());
