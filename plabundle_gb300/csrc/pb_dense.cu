@@ -358,7 +358,7 @@ __device__ __forceinline__ void phase_barrier() {
 
 template <typename T, bool CLUSTER>
 __global__ void __launch_bounds__(256) k_potrf_coop(T* __restrict__ A, T* __restrict__ X, T* __restrict__ Dinv, int np,
-                                                   int nt, int* __restrict__ status) {
+                                                   int nt, int* __restrict__ status, int* __restrict__ host_status) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* sA = reinterpret_cast<T*>(smem_raw);
     T* sB = sA + TS * TP;
@@ -426,6 +426,7 @@ __global__ void __launch_bounds__(256) k_potrf_coop(T* __restrict__ A, T* __rest
         }
         phase_barrier<CLUSTER>();
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *host_status = __ldcg(status);
     // X^T into the upper triangle of A (tile (j, i) = X_ij^T, j <= i).  The preconditioner is
     // applied as X^T (X u): forming X^T X explicitly in the factor's precision would square the
     // condition number of its rounding error.
@@ -593,7 +594,8 @@ __device__ __forceinline__ int balanced32(int warp, int m) {
 template <bool CLUSTER>
 __global__ void __launch_bounds__(kPotrf64Threads) k_potrf64_coop(double* __restrict__ A, double* __restrict__ X,
                                                                   double* __restrict__ Dinv, int np, int nt,
-                                                                  int* __restrict__ status) {
+                                                                  int* __restrict__ status,
+                                                                  int* __restrict__ host_status) {
     extern __shared__ __align__(16) double smem64[];
     double* sA = smem64;
     double* sB = sA + TD * TDP;
@@ -713,6 +715,7 @@ __global__ void __launch_bounds__(kPotrf64Threads) k_potrf64_coop(double* __rest
         }
         phase_barrier<CLUSTER>();
     }
+    if (blockIdx.x == 0 && tid == 0) *host_status = __ldcg(status);
     for (int it = blockIdx.x; it < nt * (nt + 1) / 2; it += gridDim.x) {
         const int i = tri_row(it), j = it - i * (i + 1) / 2;
         tile32_load(tile(X, i, j), np, sA);
@@ -1098,7 +1101,8 @@ static cudaError_t launch_phased(const void* grid_kernel, const void* cluster_ke
 }
 
 template <typename T>
-int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, cudaStream_t st, int* launches) {
+int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, int* h_status, cudaStream_t st,
+                 int* launches) {
     const int n = W.n, np = W.np, nt = W.nt;
     const size_t two_tiles = 2 * static_cast<size_t>(TS) * TP * sizeof(T);
     constexpr bool f64 = sizeof(T) == 8;
@@ -1137,7 +1141,7 @@ int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, cu
         T* Dv = W.Dinv;
         int npv = np, ntv = f64 ? (n + TD - 1) / TD : nt;
         int* stv = W.status;
-        void* args[] = {&A, &X, &Dv, &npv, &ntv, &stv};
+        void* args[] = {&A, &X, &Dv, &npv, &ntv, &stv, &h_status};
         // one block per lower tile at most: small systems take a small grid
         const int fgrid = std::max(1, std::min(W.fact_grid, ntv * (ntv + 1) / 2));
         if (launch_phased(kernel, cluster_kernel, W.fact_cluster, fgrid, threads, args, smem, st) != cudaSuccess) return -1;
@@ -1145,9 +1149,8 @@ int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, cu
     }
     if (launches) *launches += L;
     if (cudaGetLastError() != cudaSuccess) return -1;
-    int status = 0;
-    cudaMemcpyAsync(&status, W.status, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
+    const int status = *h_status;
     // opt-in trace (PB_GPU_TRACE=1): one line per factorisation
     static const bool trace = std::getenv("PB_GPU_TRACE") != nullptr;
     if (trace)
@@ -1181,13 +1184,12 @@ int dense_pcg(const PcgSystem<double>& sys, DenseWork<T>& W, const double* b, do
     int mi = max_it;
     int ps = W.pose_seg, bs = W.border_seg;
     void* args[] = {&s, &X, &XT, &np, &dscale, &b, &W.x, &W.r, &W.z, &W.p, &W.w, &W.qpart, &ps, &bs, &W.ut, &W.wt,
-                    &W.part, &W.scal, &rt, &at, &mi};
+                    &W.part, &h_scal, &rt, &at, &mi};
     if (launch_phased(reinterpret_cast<const void*>(&k_dense_cg<T, false>),
                       reinterpret_cast<const void*>(&k_dense_cg<T, true>), W.cg_cluster, grid, kCgThreads, args, 0, st) !=
         cudaSuccess)
         return -1;
     if (launches) *launches += 1;
-    cudaMemcpyAsync(h_scal, W.scal, 4 * sizeof(double), cudaMemcpyDeviceToHost, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
     *iterations = static_cast<int>(h_scal[0]);
     *relres = h_scal[1];
@@ -1200,8 +1202,8 @@ int dense_pcg(const PcgSystem<double>& sys, DenseWork<T>& W, const double* b, do
     return h_scal[3] != 0.0 ? 1 : 0;
 }
 
-template int dense_factor<float>(const PcgSystem<double>&, DenseWork<float>&, double, cudaStream_t, int*);
-template int dense_factor<double>(const PcgSystem<double>&, DenseWork<double>&, double, cudaStream_t, int*);
+template int dense_factor<float>(const PcgSystem<double>&, DenseWork<float>&, double, int*, cudaStream_t, int*);
+template int dense_factor<double>(const PcgSystem<double>&, DenseWork<double>&, double, int*, cudaStream_t, int*);
 template int dense_pcg<float>(const PcgSystem<double>&, DenseWork<float>&, const double*, double, double, int, int*,
                               double*, bool*, double*, cudaStream_t, int*);
 template int dense_pcg<double>(const PcgSystem<double>&, DenseWork<double>&, const double*, double, double, int, int*,

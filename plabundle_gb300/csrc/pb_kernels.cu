@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(256) k_reduce_sums(Shape S, DevPtrs D, ReduceA
 // finalizePrimaryDiagonal(1 + lambda, 1): positive diagonal entries scaled, empty ones set to 1.
 __global__ void k_finalize(Shape S, DevPtrs D, double* __restrict__ vals, double* __restrict__ Cm,
                            double* __restrict__ rhs_b, double* __restrict__ direct_b, double* __restrict__ result,
-                           double damping) {
+                           double* __restrict__ host_result, double damping) {
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     // rig problems damp the diagonal of the rig pose blocks after the map (pb_rig.cu) instead
     if (tid < S.ncb * 6 && !S.rig) {
@@ -245,7 +245,7 @@ __global__ void k_finalize(Shape S, DevPtrs D, double* __restrict__ vals, double
     }
     // priors of the intrinsic columns, a lane each (one thread after the other took 18 us for 16 columns);
     // their costs are added in column order
-    if (blockIdx.x == 0 && threadIdx.x < 32 && S.nb > 0) {
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
         double total = 0.0;
         for (int c0 = 0; c0 < S.nb; c0 += 32) {
             const int col = c0 + threadIdx.x;
@@ -264,7 +264,12 @@ __global__ void k_finalize(Shape S, DevPtrs D, double* __restrict__ vals, double
             }
             for (int i = 0; i < min(32, S.nb - c0); ++i) total += __shfl_sync(0xffffffffu, cost, i);
         }
-        if (threadIdx.x == 0) result[0] += total;
+        if (threadIdx.x == 0) {
+            const double cost = S.nb > 0 ? result[0] + total : result[0];
+            result[0] = cost;
+            host_result[0] = cost;
+            host_result[1] = result[1];
+        }
     }
 }
 
@@ -336,12 +341,11 @@ __global__ void k_effective(Shape S, DevPtrs D) {
 // BundleAdjustPlaMatrixAssembly.cpp:130-179; gauge tangent step :101-128; the plain
 // parameterisation's pose delta :1134-1136) and clamped intrinsic update (applyIntrinsicStep,
 // BundleAdjustPlaMatrixModel.cpp:248-269).
-__global__ void k_trial_cameras(Shape S, DevPtrs D, const double* __restrict__ step_c, const double* __restrict__ alphas,
-                                int n_alpha) {
+__global__ void k_trial_cameras(Shape S, DevPtrs D, const double* __restrict__ step_c, Alphas alphas, int n_alpha) {
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n_alpha * S.nc) return;
     const int a = idx / S.nc, c = idx - a * S.nc;
-    const double alpha = alphas[a];
+    const double alpha = alphas.v[a];
     // trial groups (each camera thread of the first ng cameras writes one group)
     double Gt[kGroupRec];
     const double* Gs = nullptr;
@@ -454,13 +458,13 @@ __global__ void k_trial_cameras(Shape S, DevPtrs D, const double* __restrict__ s
 // kMaxAlpha * gridDim.x on, the blocks' invalid-projection marks in the same order.
 constexpr int kCostThreads = 128;
 __global__ void __launch_bounds__(kCostThreads) k_cost_batch(Shape S, DevPtrs D, const double* __restrict__ step_p,
-                                                             const double* __restrict__ alphas, int use_trial, double c2,
+                                                             Alphas alphas, int use_trial, double c2,
                                                              double ic2, int plain, double* __restrict__ part) {
     __shared__ double s_c[kCostThreads / 32];
     __shared__ int s_bad[kCostThreads / 32];
     const int a = blockIdx.y;
     const double* cams = use_trial ? D.cams_trial + static_cast<size_t>(a) * S.nc * kCamStride : D.cams_eff;
-    const double alpha = use_trial ? alphas[a] : 0.0;
+    const double alpha = use_trial ? alphas.v[a] : 0.0;
     RobustSum acc;
     double targets = 0.0;  // control-point costs
     int bad = 0;
@@ -838,11 +842,11 @@ void launch_reduce_sums(const Shape& S, const DevPtrs& D, const AsmOut& O, const
 
 template <typename T>
 void launch_reduce(const Shape& S, const DevPtrs& D, const AsmOut& O, const RedOut<double>& R, double damping,
-                   cudaStream_t st) {
+                   double* host_result, cudaStream_t st) {
     launch_reduce_sums<T>(S, D, O, R, st);
     const int nf = std::max(S.ncb * 6, 1);
     k_finalize<<<(nf + 255) / 256, 256, 0, st>>>(S, D, R.vals, R.Cm, R.rhs + 6 * S.ncb, R.direct + 6 * S.ncb, R.result,
-                                                  damping);
+                                                  host_result, damping);
 }
 
 // The fixed-order sums of FP64 chunk partials of launch_reduce, without the damping and prior
@@ -902,7 +906,7 @@ static int cost_blocks(long long nop, int n_alpha) {
     return static_cast<int>(std::max<long long>(1, std::min<long long>(need, std::max(152, kCostMaxBlocks / n_alpha))));
 }
 
-void launch_cost(const Shape& S, const DevPtrs& D, const double* step_c, const double* step_p, const double* alphas,
+void launch_cost(const Shape& S, const DevPtrs& D, const double* step_c, const double* step_p, const Alphas& alphas,
                  int n_alpha, int use_trial, double* part, double* out, cudaStream_t st, const RigDev* rig) {
     if (use_trial) {
         const int n = n_alpha * S.nc;
@@ -1132,9 +1136,9 @@ void launch_quality(int nt, const signed char* active, const double* rms_before,
 }
 
 
-template void launch_reduce<float>(const Shape&, const DevPtrs&, const AsmOut&, const RedOut<double>&, double,
+template void launch_reduce<float>(const Shape&, const DevPtrs&, const AsmOut&, const RedOut<double>&, double, double*,
                                    cudaStream_t);
-template void launch_reduce<double>(const Shape&, const DevPtrs&, const AsmOut&, const RedOut<double>&, double,
+template void launch_reduce<double>(const Shape&, const DevPtrs&, const AsmOut&, const RedOut<double>&, double, double*,
                                     cudaStream_t);
 template void launch_back_substitute<float>(const Shape&, const DevPtrs&, const double*, const float*, const double*,
                                             double*, double*, double*, const double*, double*, cudaStream_t);

@@ -11,6 +11,13 @@
 namespace pb {
 
 constexpr int kMaxAlpha = 8;  // trial step lengths evaluated per objective pass
+// The scalars of a step (cost, flags, sums, CG outcome) are written by the kernels to the context's pinned
+// host memory and the trial step lengths travel as kernel parameters: a copy on the stream for a few
+// doubles cost more than the kernels of a small problem around it (solve step of 20 cameras and 2 000 points
+// 443 -> 409 us, a whole mixed solve of it 2.97 -> 2.82 ms, of 150 rig cameras 42.1 -> 38.8 ms).
+struct Alphas {
+    double v[kMaxAlpha];
+};
 constexpr int kCostMaxBlocks = 152 * 8;  // partials per step length of an objective pass, at most
 
 // Outputs of the assembly kernel (per-chunk partials) and per-track / per-observation data kept
@@ -66,7 +73,7 @@ template <typename T>
 void launch_assemble(const Shape& S, const DevPtrs& D, const AsmOut& O, double damping, size_t smem, cudaStream_t st);
 template <typename T>
 void launch_reduce(const Shape& S, const DevPtrs& D, const AsmOut& O, const RedOut<double>& R, double damping,
-                   cudaStream_t st);
+                   double* host_result, cudaStream_t st);
 void launch_reduce_sums64(const Shape& S, const DevPtrs& D, const AsmOut& O, const RedOut<double>& R, cudaStream_t st);
 // Observations in processing order (cam, u, v, weight and its float-float copy, track) gathered
 // from the original-order arrays through obs_orig and trk_obs_begin.
@@ -152,10 +159,10 @@ void launch_rig_transform(const RigDev& R, const double* vals, const double* bor
 // xr (6 nrb + nbw) -> R.xv (6 ncb + nbw), R.step_r = xr, R.sq = sum of xr^2 over 6 nrb + nglob.
 void launch_rig_expand(const RigDev& R, const double* xr, int nbw, int nglob, cudaStream_t st);
 // Trial captures, sensors and composed camera poses (pose entries 0-11 of the trial cameras).
-void launch_rig_trial(const RigDev& R, int nc, const double* alphas, int n_alpha, double* cams_trial, cudaStream_t st);
+void launch_rig_trial(const RigDev& R, int nc, const Alphas& alphas, int n_alpha, double* cams_trial, cudaStream_t st);
 void launch_rig_accept(const RigDev& R, int a, cudaStream_t st);
 
-void launch_cost(const Shape& S, const DevPtrs& D, const double* step_c, const double* step_p, const double* alphas,
+void launch_cost(const Shape& S, const DevPtrs& D, const double* step_c, const double* step_p, const Alphas& alphas,
                  int n_alpha, int use_trial, double* part, double* out, cudaStream_t st,
                  const RigDev* rig = nullptr);
 void launch_accept(const Shape& S, const DevPtrs& D, const double* step_p, double alpha, int a, cudaStream_t st);
@@ -164,10 +171,10 @@ void launch_accept(const Shape& S, const DevPtrs& D, const double* step_p, doubl
 // the camera / intrinsic step and the promoted point steps (`out`: their squared sum), and the
 // bars' cost of the trial states or of the current state.
 void launch_extend_system(const Shape& S, const DevPtrs& D, const RedOut<double>& R, const ExtSys& X, double damping,
-                          int* flags, double* bar_cost, cudaStream_t st);
+                          int* flags, double* bar_cost, int* host_flags, cudaStream_t st);
 void launch_ext_step(const Shape& S, const DevPtrs& D, const double* xsol, double* step_c, double* step_p, double* out,
                      cudaStream_t st);
-void launch_bar_cost(const Shape& S, const DevPtrs& D, const double* step_p, const double* alphas, int n_alpha,
+void launch_bar_cost(const Shape& S, const DevPtrs& D, const double* step_p, const Alphas& alphas, int n_alpha,
                      int use_trial, double* out, cudaStream_t st);
 void launch_strict_rms(const Shape& S, const DevPtrs& D, const double* cams, const double* init_points,
                        const int* proc_of_track, int use_state, int nt, double* out, cudaStream_t st);
@@ -230,7 +237,6 @@ struct DenseWork {
     double* qpart = nullptr;
     T *ut = nullptr, *wt = nullptr;  // scaled residual and X D r in the factor's type
     double* part = nullptr;  // per-block partials of the cooperative CG (grid * 4)
-    double* scal = nullptr;
     int coop_grid = 0;       // blocks of the cooperative CG launch
     int fact_grid = 0;       // blocks of the cooperative factorisation
     int cg_cluster = 0, fact_cluster = 0;  // blocks that one cluster of the kernel can hold
@@ -238,11 +244,13 @@ struct DenseWork {
 
 template <typename T>
 size_t dense_bytes(int n);
-// Returns 0 on success, a status bitmask when the scaled matrix is not positive definite at this
+// h_status: pinned host memory.  Returns 0 on success, a status bitmask when the scaled matrix is not positive definite at this
 // shift (bit 1: non-positive diagonal, bit 2: non-positive pivot), -1 on a CUDA error.
 template <typename T>
-int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, cudaStream_t st, int* launches);
-// CG on S x = b (FP64 S and vectors); the solution is left in W.x.  Returns 0, 1 on breakdown,
+int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, int* h_status, cudaStream_t st,
+                 int* launches);
+// CG on S x = b (FP64 S and vectors); the solution is left in W.x, its scalars in h_scal (pinned host
+// memory, four doubles).  Returns 0, 1 on breakdown,
 // -1 on a CUDA error.
 template <typename T>
 int dense_pcg(const PcgSystem<double>& sys, DenseWork<T>& W, const double* b, double rel_tol, double abs_tol,

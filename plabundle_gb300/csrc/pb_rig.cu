@@ -257,13 +257,13 @@ __global__ void k_rig_step_sq(RigDev R, const double* __restrict__ xr, int n) {
     if (threadIdx.x == 0) R.sq[0] = s[0];
 }
 
-__global__ void k_rig_trial(RigDev R, int nc, const double* __restrict__ alphas, int n_alpha,
+__global__ void k_rig_trial(RigDev R, int nc, Alphas alphas, int n_alpha,
                             double* __restrict__ cams_trial) {
     const int per = R.ncap + R.nsen + nc;
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= per * n_alpha) return;
     const int a = idx / per, i = idx - a * per;
-    const double alpha = alphas[a];
+    const double alpha = alphas.v[a];
     if (i < R.ncap) {
         rig_trial_record(R.cap_state + static_cast<size_t>(i) * 12, R.capture_block[i], R.step_r, alpha,
                          R.cap_trial + (static_cast<size_t>(a) * R.ncap + i) * 12);
@@ -314,7 +314,7 @@ void launch_rig_expand(const RigDev& R, const double* xr, int nbw, int nglob, cu
     k_rig_step_sq<<<1, 256, 0, st>>>(R, xr, 6 * R.nrb + nglob);
 }
 
-void launch_rig_trial(const RigDev& R, int nc, const double* alphas, int n_alpha, double* cams_trial, cudaStream_t st) {
+void launch_rig_trial(const RigDev& R, int nc, const Alphas& alphas, int n_alpha, double* cams_trial, cudaStream_t st) {
     const int n = (R.ncap + R.nsen + nc) * n_alpha;
     k_rig_trial<<<(n + 127) / 128, 128, 0, st>>>(R, nc, alphas, n_alpha, cams_trial);
 }

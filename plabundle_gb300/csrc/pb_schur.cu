@@ -352,7 +352,6 @@ void ensure_dense(SchurWork* w, int device) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     W.part = w->dense.alloc<double>(static_cast<size_t>(std::max(1, sms)) * 32 * 4);
-    W.scal = w->dense.alloc<double>(8);
     w->dense_n[idx] = w->n;
 }
 
@@ -504,7 +503,7 @@ int dense_solve(SchurWork* w, int device, const pb_schur_options& op, double tol
     double shift = sizeof(T) == 4 ? 1e-7 : 0.0;
     int fst = 0;
     for (int attempt = 0; attempt < 6; ++attempt) {
-        fst = dense_factor<T>(sys, W, shift, st, &launches);
+        fst = dense_factor<T>(sys, W, shift, reinterpret_cast<int*>(w->h_scal + 8), st, &launches);
         if (fst < 0) return -1;
         if (fst == 0 || (fst & 1)) break;
         shift = shift == 0.0 ? 1e-9 : shift * 10.0;

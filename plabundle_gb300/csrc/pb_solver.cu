@@ -83,6 +83,12 @@ void check(cudaError_t e, const char* what) {
     if (e != cudaSuccess) throw CudaError(std::string(what) + ": " + cudaGetErrorString(e));
 }
 
+// Slots (doubles) of a context's pinned host memory that the kernels write their scalars to; each has one
+// writer, and the host reads it after a synchronisation of the stream.
+constexpr int kSlotCost = 0, kSlotBacksub = 8, kSlotRigSq = 11, kSlotResult = 12, kSlotExtFlags = 14, kSlotBars = 16,
+              kSlotPcg = 30, kSlotCg = 40, kSlotFactor = 44, kSlotQuality = 48, kSlots = 64;
+static_assert(kSlotBacksub >= kSlotCost + kMaxAlpha && kSlotPcg >= kSlotBars + kMaxAlpha + 2, "slots overlap");
+
 // Assembly outputs of one arithmetic type (chunk partials, per-track factors, robust weights).
 template <typename T>
 struct PrecisionBuffers {
@@ -133,10 +139,9 @@ struct pb_gpu_ctx {
     double* res_out = nullptr;
     double* bs_part = nullptr;
     double* bs_terms = nullptr;  // per processed observation: its term of the point back-substitution
-    double* bs_out = nullptr;
+    double* bs_out = nullptr;    // pinned: directional decrease, sums of squared point and camera steps
     double* cost_part = nullptr;
-    double* cost_out = nullptr;
-    double* alphas_d = nullptr;
+    double* cost_out = nullptr;  // pinned: cost per step length
     double* pcg_part = nullptr;
     PcgResult* pcg_res = nullptr;
     int* pre_status = nullptr;
@@ -181,7 +186,7 @@ struct pb_gpu_ctx {
     ExtSys ext{};
     PcgSystem<double> sysx{};
     int* ext_flags = nullptr;
-    double* bar_d = nullptr;  // bar cost of the current state, then of the trial states
+    double* bar_d = nullptr;  // pinned: bar cost of the current state, of the trial states, the step sum
     // cost history of the last solve: the initial cost, then the cost after every accepted step,
     // with the LM iteration and the host time since the solve started
     std::vector<int> hist_it;
@@ -384,10 +389,9 @@ void upload_structure(pb_gpu_ctx* c) {
     const int bs_blocks = std::max(1, (ntp + 255) / 256);
     c->bs_part = A.alloc<double>(2 * static_cast<size_t>(bs_blocks));
     c->bs_terms = A.alloc<double>(3 * static_cast<size_t>(std::max<long long>(1, nop)));
-    c->bs_out = A.alloc<double>(4);
     c->cost_part = A.alloc<double>(static_cast<size_t>(kCostMaxBlocks) * kMaxAlpha * 2);
-    c->cost_out = A.alloc<double>(kMaxAlpha);
-    c->alphas_d = A.alloc<double>(kMaxAlpha);
+    c->cost_out = c->h_scratch + kSlotCost;
+    c->bs_out = c->h_scratch + kSlotBacksub;
     c->pcg_res = A.alloc<PcgResult>(1);
     c->pre_status = A.alloc<int>(1);
     c->rms_before_d = A.alloc<double>(nt);
@@ -442,7 +446,7 @@ void upload_structure(pb_gpu_ctx* c) {
         c->sysx.border_t = X.border_t;
         c->sysx.Cm = X.Cm;
         c->ext_flags = A.alloc<int>(1);
-        c->bar_d = A.alloc<double>(kMaxAlpha + 2);  // [0] current, [1 .. kMaxAlpha] trials, then the step sum
+        c->bar_d = c->h_scratch + kSlotBars;
     }
     c->rig_on = m.rig.on;
     if (c->rig_on) {
@@ -518,7 +522,7 @@ void upload_structure(pb_gpu_ctx* c) {
         R.rhs = A.alloc<double>(nr6 + nbw + 1);
         R.xv = A.alloc<double>(static_cast<size_t>(6) * m.ncb + nbw + 1);
         R.step_r = A.alloc<double>(nr6 + nbw + 1);
-        R.sq = A.alloc<double>(1);
+        R.sq = c->h_scratch + kSlotRigSq;
         check(cudaMemsetAsync(R.step_r, 0, (nr6 + nbw + 1) * sizeof(double), st), "memset");
         PcgSystem<double>& sr = c->sysr;
         sr = c->ext_on ? c->sysx : sy;
@@ -680,14 +684,13 @@ void assemble(pb_gpu_ctx* c, double damping, int precision, double* cost, int* f
     }
     {
         Timer t(c, 3);
-        launch_reduce<T>(S, D, B.out, c->red, damping, c->stream);
+        launch_reduce<T>(S, D, B.out, c->red, damping, c->h_scratch + kSlotResult, c->stream);
         c->launches += 2;  // k_reduce_sums, k_finalize
     }
     check(cudaGetLastError(), "assemble launch");
-    check(cudaMemcpyAsync(c->h_scratch, c->red.result, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H");
     check(cudaStreamSynchronize(c->stream), "assemble");
-    *cost = c->h_scratch[0];
-    *flags = static_cast<int>(c->h_scratch[1]);
+    *cost = c->h_scratch[kSlotResult];
+    *flags = static_cast<int>(c->h_scratch[kSlotResult + 1]);
     c->last_precision = precision;
     c->have_system = true;
     // scale bars: every assembly extends the reduced system by the promoted points and adds the
@@ -754,7 +757,6 @@ void ensure_dense(pb_gpu_ctx* c) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
     W.part = A.alloc<double>(static_cast<size_t>(std::max(1, sms)) * 32 * 4);
-    W.scal = A.alloc<double>(8);
     c->dense_ready[idx] = true;
 }
 
@@ -786,7 +788,7 @@ int solve_dense(pb_gpu_ctx* c, double rel, double abs_tol, int max_it, bool* con
         // about as much as a hundred CG iterations, so the kept factor is used until the CG
         // needs more than kReuseIterations on it.
         const int cap = std::min(max_it, std::max(kReuseIterations, 4 * c->f32_base_iters));
-        const int rc = dense_pcg<T>(sys, W, rhs, rel, abs_tol, cap, iterations, relres, converged, c->h_scratch + 40,
+        const int rc = dense_pcg<T>(sys, W, rhs, rel, abs_tol, cap, iterations, relres, converged, c->h_scratch + kSlotCg,
                                     c->stream, &c->launches);
         if (rc < 0) throw CudaError(std::string("dense CG failed: ") + cudaGetErrorString(cudaGetLastError()));
         if (rc == 0 && *converged) {
@@ -809,7 +811,7 @@ int solve_dense(pb_gpu_ctx* c, double rel, double abs_tol, int max_it, bool* con
     int attempts = 0;
     for (int attempt = 0; attempt < 6; ++attempt) {
         ++attempts;
-        st = dense_factor<T>(sys, W, shift, c->stream, &c->launches);
+        st = dense_factor<T>(sys, W, shift, reinterpret_cast<int*>(c->h_scratch + kSlotFactor), c->stream, &c->launches);
         if (st < 0) throw CudaError(std::string("dense factorisation failed: ") + cudaGetErrorString(cudaGetLastError()));
         if (st == 0 || (st & 1)) break;
         shift = shift == 0.0 ? 1e-9 : shift * 10.0;
@@ -817,7 +819,7 @@ int solve_dense(pb_gpu_ctx* c, double rel, double abs_tol, int max_it, bool* con
     const auto tf1 = std::chrono::steady_clock::now();
     if (st) return 1;
     if (f32) c->shift32 = shift;
-    const int rc = dense_pcg<T>(sys, W, rhs, rel, abs_tol, max_it, iterations, relres, converged, c->h_scratch + 40,
+    const int rc = dense_pcg<T>(sys, W, rhs, rel, abs_tol, max_it, iterations, relres, converged, c->h_scratch + kSlotCg,
                                 c->stream, &c->launches);
     if (trace)
         std::fprintf(stderr, "PB_GPU_TRACE dense n=%d factor_attempts=%d shift=%.1e factor_ms=%.3f cg_ms=%.3f cg_it=%d\n",
@@ -849,11 +851,11 @@ int solve_block_jacobi(pb_gpu_ctx* c, double rel, double abs_tol, int max_it, bo
     c->launches += 2;
     PcgResult res{};
     int pre = 0;
-    check(cudaMemcpyAsync(c->h_scratch, c->pre_status, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H");
-    check(cudaMemcpyAsync(c->h_scratch + 1, c->pcg_res, sizeof(PcgResult), cudaMemcpyDeviceToHost, st), "D2H");
+    check(cudaMemcpyAsync(c->h_scratch + kSlotPcg, c->pre_status, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H");
+    check(cudaMemcpyAsync(c->h_scratch + kSlotPcg + 1, c->pcg_res, sizeof(PcgResult), cudaMemcpyDeviceToHost, st), "D2H");
     check(cudaStreamSynchronize(st), "pcg");
-    std::memcpy(&pre, c->h_scratch, sizeof(int));
-    std::memcpy(&res, c->h_scratch + 1, sizeof(PcgResult));
+    std::memcpy(&pre, c->h_scratch + kSlotPcg, sizeof(int));
+    std::memcpy(&res, c->h_scratch + kSlotPcg + 1, sizeof(PcgResult));
     if (pre || res.status) return 1;
     check(cudaMemcpyAsync(c->step_c, c->pcg_x, c->S[0].n * sizeof(double), cudaMemcpyDeviceToDevice, st), "D2D");
     *converged = res.converged != 0;
@@ -929,43 +931,34 @@ void back_substitute(pb_gpu_ctx* c, double* dd, double* point_sq, double* cam_sq
                                       c->bs_part, c->direct64, c->bs_out, c->stream);
     c->launches += 3;
     check(cudaGetLastError(), "back-substitution launch");
-    check(cudaMemcpyAsync(c->h_scratch, c->bs_out, 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H");
-    if (c->rig_on)
-        check(cudaMemcpyAsync(c->h_scratch + 3, c->rig.sq, sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H");
     check(cudaStreamSynchronize(c->stream), "back-substitution");
-    *dd = c->h_scratch[0];
-    *point_sq = c->h_scratch[1];
+    *dd = c->bs_out[0];
+    *point_sq = c->bs_out[1];
     // the step RMS of a rig problem is taken over the rig's parameters, not the cameras'
-    *cam_sq = c->rig_on ? c->h_scratch[3] : c->h_scratch[2];
+    *cam_sq = c->rig_on ? *c->rig.sq : c->bs_out[2];
 }
 
 void eval_costs(pb_gpu_ctx* c, const double* alphas, int n, int use_trial, double* out) {
     const Shape& S = c->S[0];
     const DevPtrs& D = c->D[0];
-    if (use_trial) {
-        std::memcpy(c->h_scratch + 16, alphas, n * sizeof(double));
-        check(cudaMemcpyAsync(c->alphas_d, c->h_scratch + 16, n * sizeof(double), cudaMemcpyHostToDevice, c->stream), "H2D");
-    }
+    Alphas al{};
+    if (use_trial) std::copy(alphas, alphas + n, al.v);
     {
         Timer t(c, 2);
-        launch_cost(S, D, c->step_c, c->step_p, c->alphas_d, n, use_trial, c->cost_part, c->cost_out, c->stream,
+        launch_cost(S, D, c->step_c, c->step_p, al, n, use_trial, c->cost_part, c->cost_out, c->stream,
                     c->rig_on ? &c->rig : nullptr);
         c->launches += use_trial ? (c->rig_on ? 4 : 3) : 2;
         if (c->ext_on) {
-            launch_bar_cost(S, D, c->step_p, c->alphas_d, n, use_trial, c->bar_d + 1, c->stream);
+            launch_bar_cost(S, D, c->step_p, al, n, use_trial, c->bar_d + 1, c->stream);
             c->launches += 1;
         }
     }
     check(cudaGetLastError(), "cost launch");
-    check(cudaMemcpyAsync(c->h_scratch, c->cost_out, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H");
-    if (c->ext_on)
-        check(cudaMemcpyAsync(c->h_scratch + 8, c->bar_d + 1, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream),
-              "D2H");
     check(cudaStreamSynchronize(c->stream), "cost");
-    std::memcpy(out, c->h_scratch, n * sizeof(double));
+    std::copy(c->cost_out, c->cost_out + n, out);
     // the scale bars' robust cost (assembleScaleBars, BundleAdjustPlaMatrixAssemblySurvey.cpp:131-186)
     if (c->ext_on)
-        for (int i = 0; i < n; ++i) out[i] += c->h_scratch[8 + i];
+        for (int i = 0; i < n; ++i) out[i] += c->bar_d[1 + i];
 }
 
 // Scale bars: the reduced system of the last assembly extended by the promoted points; returns
@@ -973,16 +966,13 @@ void eval_costs(pb_gpu_ctx* c, const double* alphas, int n, int use_trial, doubl
 double extend_system(pb_gpu_ctx* c, double damping) {
     const Shape& S = c->S[0];
     check(cudaMemsetAsync(c->ext_flags, 0, sizeof(int), c->stream), "memset");
-    launch_extend_system(S, c->D[0], c->red, c->ext, damping, c->ext_flags, c->bar_d, c->stream);
+    int* host_flags = reinterpret_cast<int*>(c->h_scratch + kSlotExtFlags);
+    launch_extend_system(S, c->D[0], c->red, c->ext, damping, c->ext_flags, c->bar_d, host_flags, c->stream);
     c->launches += S.npr > 0 ? 4 : 3;
     check(cudaGetLastError(), "extension launch");
-    check(cudaMemcpyAsync(c->h_scratch, c->bar_d, sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H");
-    check(cudaMemcpyAsync(c->h_scratch + 1, c->ext_flags, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "D2H");
     check(cudaStreamSynchronize(c->stream), "extension");
-    int flags = 0;
-    std::memcpy(&flags, c->h_scratch + 1, sizeof(int));
-    if (flags & 2) throw std::runtime_error("linearisation produced an invalid projection");
-    return c->h_scratch[0];
+    if (*host_flags & 2) throw std::runtime_error("linearisation produced an invalid projection");
+    return c->bar_d[0];
 }
 
 // Scale bars: the promoted points' steps of the last extended solve into the point steps;
@@ -992,9 +982,8 @@ double promoted_steps(pb_gpu_ctx* c) {
     launch_ext_step(c->S[0], c->D[0], xsol, c->step_c, c->step_p, c->bar_d + kMaxAlpha + 1, c->stream);
     c->launches += 1;
     check(cudaGetLastError(), "promoted step launch");
-    check(cudaMemcpyAsync(c->h_scratch, c->bar_d + kMaxAlpha + 1, sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H");
     check(cudaStreamSynchronize(c->stream), "promoted steps");
-    return c->h_scratch[0];
+    return c->bar_d[kMaxAlpha + 1];
 }
 
 void reset_state(pb_gpu_ctx* c) {
@@ -1029,10 +1018,11 @@ void finalize_quality(pb_gpu_ctx* c, const pb_solve_options& op, pb_solve_report
     launch_quality(nt, c->active_d, c->rms_before_d, c->rms_after_d, op.enable_point_filter, op.filter_max_reproj_error,
                    op.filter_sigma_factor, c->valid_d, c->quality_part, c->quality_out, st);
     c->launches += 4;
-    check(cudaMemcpyAsync(c->h_scratch, c->quality_out, 5 * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H");
+    double* q = c->h_scratch + kSlotQuality;
+    check(cudaMemcpyAsync(q, c->quality_out, 5 * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H");
     check(cudaStreamSynchronize(st), "quality");
     c->quality_host_stale = true;
-    const double thr = c->h_scratch[0], kept_d = c->h_scratch[2], sb = c->h_scratch[3], sa = c->h_scratch[4];
+    const double thr = q[0], kept_d = q[2], sb = q[3], sa = q[4];
     const int kept = static_cast<int>(kept_d);
     rep->filter_threshold = thr;
     rep->optimized_tracks = kept;
@@ -1554,7 +1544,7 @@ pb_status pb_gpu_create(int32_t device, pb_gpu_ctx** out) {
     if (!c) return PB_ERR_CUDA;
     c->device = device;
     if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMallocHost(&c->h_scratch, 64 * sizeof(double)) != cudaSuccess ||
+        cudaMallocHost(&c->h_scratch, kSlots * sizeof(double)) != cudaSuccess ||
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess) {
         delete c;
         return PB_ERR_CUDA;

@@ -166,7 +166,8 @@ __global__ void __launch_bounds__(32) k_ext_points(Shape S, DevPtrs D, ExtSys X,
 // their terms on the promoted blocks and their cost at the current state; then the damping of the promoted
 // diagonals.
 __global__ void __launch_bounds__(32) k_ext_bars(Shape S, DevPtrs D, ExtSys X, double damping,
-                                                 double* __restrict__ bar_cost) {
+                                                 const int* __restrict__ flags, double* __restrict__ bar_cost,
+                                                 int* __restrict__ host_flags) {
     const int lane = threadIdx.x, nb = S.nb, nbx = X.nbx;
     double cost = 0.0;
     for (int i0 = 0; i0 < S.nbar; i0 += 32) {
@@ -212,7 +213,10 @@ __global__ void __launch_bounds__(32) k_ext_bars(Shape S, DevPtrs D, ExtSys X, d
             __syncwarp();
         }
     }
-    if (lane == 0) *bar_cost = cost;
+    if (lane == 0) {
+        *bar_cost = cost;
+        *host_flags = *flags;
+    }
     for (int e = lane; e < 3 * S.npr; e += 32) {
         double* d = X.Cm + static_cast<size_t>(nb + e) * nbx + nb + e;
         *d = *d != 0.0 ? *d * (1.0 + damping) : 1.0;
@@ -253,11 +257,11 @@ __global__ void k_ext_step(Shape S, DevPtrs D, const double* __restrict__ xsol, 
 
 // Scale-bar cost of each trial state (points + alpha step for the points that move) or of the
 // current state, one thread per step length, bars in order.
-__global__ void k_bar_cost(Shape S, DevPtrs D, const double* __restrict__ step_p, const double* __restrict__ alphas,
-                           int n_alpha, int use_trial, double* __restrict__ out) {
+__global__ void k_bar_cost(Shape S, DevPtrs D, const double* __restrict__ step_p, Alphas alphas, int n_alpha,
+                           int use_trial, double* __restrict__ out) {
     const int a = threadIdx.x;
     if (a >= n_alpha) return;
-    const double alpha = use_trial ? alphas[a] : 0.0;
+    const double alpha = use_trial ? alphas.v[a] : 0.0;
     double cost = 0.0;
     for (int i = 0; i < S.nbar; ++i) {
         const int ta = D.bar_pidx[2 * i], tb = D.bar_pidx[2 * i + 1];
@@ -285,10 +289,10 @@ __global__ void k_bar_cost(Shape S, DevPtrs D, const double* __restrict__ step_p
 }
 
 void launch_extend_system(const Shape& S, const DevPtrs& D, const RedOut<double>& R, const ExtSys& X, double damping,
-                          int* flags, double* bar_cost, cudaStream_t st) {
+                          int* flags, double* bar_cost, int* host_flags, cudaStream_t st) {
     k_ext_copy<<<std::max(1, 2 * 152), 256, 0, st>>>(S, R, X);
     if (S.npr > 0) k_ext_points<<<S.npr, 32, 0, st>>>(S, D, X, flags);
-    k_ext_bars<<<1, 32, 0, st>>>(S, D, X, damping, bar_cost);
+    k_ext_bars<<<1, 32, 0, st>>>(S, D, X, damping, flags, bar_cost, host_flags);
     k_ext_transpose<<<std::max(1, 2 * 152), 256, 0, st>>>(S, X);
 }
 
@@ -297,7 +301,7 @@ void launch_ext_step(const Shape& S, const DevPtrs& D, const double* xsol, doubl
     k_ext_step<<<std::max(1, (S.n + 255) / 256), 256, 0, st>>>(S, D, xsol, step_c, step_p, out);
 }
 
-void launch_bar_cost(const Shape& S, const DevPtrs& D, const double* step_p, const double* alphas, int n_alpha,
+void launch_bar_cost(const Shape& S, const DevPtrs& D, const double* step_p, const Alphas& alphas, int n_alpha,
                      int use_trial, double* out, cudaStream_t st) {
     k_bar_cost<<<1, 32, 0, st>>>(S, D, step_p, alphas, n_alpha, use_trial, out);
 }
