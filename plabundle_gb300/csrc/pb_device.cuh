@@ -452,34 +452,51 @@ __device__ __forceinline__ ff ff_make(double d) {
     return {h, static_cast<float>(d - static_cast<double>(h))};
 }
 // Conversions between FP64 and FP32 on the integer pipe, bit for bit those of the conversion
-// instructions, which take the FP64 pipe for 64 cycles a warp (the form below about ten).  Zero apart,
-// values outside the range of normal FP32 numbers go to the instruction.
+// instructions, which take the FP64 pipe for 64 cycles a warp (the forms below about twenty on the integer
+// pipe).
 __device__ __forceinline__ double f64_of(float f) {
-    const unsigned u = __float_as_uint(f), mag = u & 0x7fffffffu;
-    if (mag - 1u < 0x007fffffu || mag >= 0x7f800000u) return static_cast<double>(f);  // denormal, infinite, NaN
-    const unsigned hi = mag == 0u ? u : ((u & 0x80000000u) | ((mag >> 3) + 0x38000000u));
-    return __hiloint2double(static_cast<int>(hi), static_cast<int>(u << 29));
+    // No path may hold a conversion: predicated off it still takes its 64 cycles.
+    unsigned u = __float_as_uint(f), mag = u & 0x7fffffffu;
+    unsigned bias = 0x38000000u;  // (1023 - 127) << 20
+    if (mag < 0x00800000u) {      // zero and denormals: scaled by 2^24 they are zero or normal
+        u = __float_as_uint(f * 16777216.0f);
+        mag = u & 0x7fffffffu;
+        bias = mag == 0u ? 0u : 0x36800000u;  // (1023 - 127 - 24) << 20
+    } else if (mag >= 0x7f800000u) {
+        bias = 0x70000000u;  // infinities and NaNs keep their fraction
+    }
+    return __hiloint2double(static_cast<int>((u & 0x80000000u) | ((mag >> 3) + bias)), static_cast<int>(u << 29));
 }
 __device__ __forceinline__ double f64_of(double d) { return d; }
-// hi = RN(d), lo = RN(d - hi).  For 2^-74 <= |d| < 2^127 the difference is an integer of at most 29 bits
-// times 2^(e - 52) (e the exponent of d), rounded by its conversion to FP32; scaling it is exact.
+// hi = RN(d), lo = RN(d - hi), without a branch.  The difference is an integer of at most 29 bits times
+// 2^(e - 52) (e the exponent of d), rounded by its conversion to FP32; the scaling is exact.  Below 2^-74,
+// where the scale or the result would leave the normal FP32 numbers, the conversion is that of 2^100 d,
+// scaled back (only FP32 denormals may round twice); below 2^-174 both parts are zero.  Where hi is
+// infinite or NaN, so is every value made from it.
 __device__ __forceinline__ ff ff_make_bits(double d) {
     const unsigned hw = hi_word(d), lw = static_cast<unsigned>(__double2loint(d));
-    const unsigned ex = (hw >> 20) & 0x7ffu;
-    if (ex - 949u > 200u) {
-        const float h = static_cast<float>(d);
-        return {h, static_cast<float>(d - static_cast<double>(h))};
-    }
-    // sign, exponent - 896 and the upper 23 bits of the fraction, rounded to nearest even
-    unsigned u = (__funnelshift_l(lw, hw, 3) + 0x40000000u) | (hw & 0x80000000u);
+    const unsigned sign = hw & 0x80000000u, mag = hw & 0x7fffffffu;
+    const bool small = mag < (949u << 20), zero = mag < (849u << 20), large = mag >= (1151u << 20);
+    const unsigned ex = (mag >> 20) + (small ? 100u : 0u);
+    // exponent - 896 and the upper 23 bits of the fraction, rounded to nearest even
+    unsigned u = __funnelshift_l(lw, mag, 3) + (small ? 0x72000000u : 0x40000000u);
     int rest = static_cast<int>(lw & 0x1fffffffu);
-    if (rest + static_cast<int>(u & 1u) > 0x10000000) {
-        rest -= 0x20000000;
-        ++u;
+    const bool up = rest + static_cast<int>(u & 1u) > 0x10000000;
+    rest -= up ? 0x20000000 : 0;
+    u += up ? 1u : 0u;
+    if (zero) {
+        u = 0u;
+        rest = 0;
     }
-    if (hw & 0x80000000u) rest = -rest;
-    const float lo = static_cast<float>(rest) * __uint_as_float((ex - 948u) << 23);
-    return {__uint_as_float(u), lo};
+    float h = __uint_as_float(u | sign), l = static_cast<float>(sign ? -rest : rest) * __uint_as_float((ex - 948u) << 23);
+    const float back = small ? 0x1p-100f : 1.0f;
+    h *= back;
+    l *= back;
+    if (large) {
+        h = __uint_as_float(sign | 0x7f800000u | (mag > 0x7ff00000u || (mag == 0x7ff00000u && lw != 0u) ? 0x400000u : 0u));
+        l = -h;
+    }
+    return {h, l};
 }
 // __fmul_rn / __fadd_rn are never contracted into an FMA, which the error-free transformations
 // below depend on.

@@ -560,7 +560,9 @@ static_assert(kMaxNB <= kCostFinalThreads, "a thread per intrinsic column");
 // Back-substitution (recoverReferencePointSteps, ...ReferenceSchur.cpp:982-1082), one thread per
 // track:  dp = R^-T (q - R^-1 u),  u = sum_o w J_p^T (J_o dc).
 // Per observation o of an eliminated track: the term Y_o^T A_o dc (3 values) of its track's sum,
-// one thread per observation (records read by consecutive lanes, FP64 accumulation).
+// one thread per observation, FP64 accumulation.  The FP64 pipe bounds it, 2 (6 + ni) + 6 products an
+// observation; the mixed path's records widen on the integer pipe (500 cameras, 1.3 million observations:
+// 168 -> 83 us; the records staged in shared memory by consecutive lanes took the same).
 template <typename T>
 __global__ void __launch_bounds__(256) k_backsub_terms(Shape S, DevPtrs D, const T* __restrict__ obs_rec,
                                                        const double* __restrict__ step_c, double* __restrict__ terms) {
@@ -574,21 +576,21 @@ __global__ void __launch_bounds__(256) k_backsub_terms(Shape S, DevPtrs D, const
     if (b >= 0)
         for (int a = 0; a < 6; ++a) {
             const double dcv = step_c[6 * b + a];
-            e0 = fma(static_cast<double>(rec[a]), dcv, e0);
-            e1 = fma(static_cast<double>(rec[nA + a]), dcv, e1);
+            e0 = fma(f64_of(rec[a]), dcv, e0);
+            e1 = fma(f64_of(rec[nA + a]), dcv, e1);
         }
     const int g = S.ng > 0 ? D.cam_group[cam] : -1;
     if (g >= 0)
         for (int a = 0; a < S.ni; ++a) {
             const double dcv = step_c[6 * S.ncb + g * S.ni + a];
-            e0 = fma(static_cast<double>(rec[6 + a]), dcv, e0);
-            e1 = fma(static_cast<double>(rec[nA + 6 + a]), dcv, e1);
+            e0 = fma(f64_of(rec[6 + a]), dcv, e0);
+            e1 = fma(f64_of(rec[nA + 6 + a]), dcv, e1);
         }
     const T* Y = rec + 2 * nA;
     double* u = terms + static_cast<size_t>(o) * 3;
-    u[0] = static_cast<double>(Y[0]) * e0 + static_cast<double>(Y[3]) * e1;
-    u[1] = static_cast<double>(Y[1]) * e0 + static_cast<double>(Y[4]) * e1;
-    u[2] = static_cast<double>(Y[2]) * e0 + static_cast<double>(Y[5]) * e1;
+    u[0] = f64_of(Y[0]) * e0 + f64_of(Y[3]) * e1;
+    u[1] = f64_of(Y[1]) * e0 + f64_of(Y[4]) * e1;
+    u[2] = f64_of(Y[2]) * e0 + f64_of(Y[5]) * e1;
 }
 
 // track:  dp = R^-T (q - R^-1 u),  u = sum_o w J_p^T (J_o dc).
