@@ -840,8 +840,8 @@ __global__ void __launch_bounds__(128) k_adj_gradient(Shape S, DevPtrs D, AdjBuf
         j[r] = v;
     }
     const double* w2 = rec + Lo.w2();
-    B.grad_obs[2 * static_cast<size_t>(o)] = w2[0] * j[0] + w2[1] * j[1];
-    B.grad_obs[2 * static_cast<size_t>(o) + 1] = w2[1] * j[0] + w2[2] * j[1];
+    *reinterpret_cast<double2*>(B.grad_obs + 2 * static_cast<size_t>(D.obs_orig[o])) =
+        make_double2(w2[0] * j[0] + w2[1] * j[1], w2[1] * j[0] + w2[2] * j[1]);
     if (D.cam_block[cam] < 0) {
         // fixed camera: -(H_c,pt mu_p + H_c,k mu_k)
         const double* hcp = rec + Lo.hcp();

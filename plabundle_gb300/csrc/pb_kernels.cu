@@ -596,7 +596,8 @@ __global__ void __launch_bounds__(256) k_backsub_terms(Shape S, DevPtrs D, const
 // track:  dp = R^-T (q - R^-1 u),  u = sum_o w J_p^T (J_o dc).
 __global__ void __launch_bounds__(256) k_back_substitute(Shape S, DevPtrs D, const double* __restrict__ trk_data,
                                                          const double* __restrict__ terms,
-                                                         double* __restrict__ step_p, double* __restrict__ part) {
+                                                         double* __restrict__ step_p, double* __restrict__ step_e,
+                                                         double* __restrict__ part) {
     // Point steps dp = V^-1 (g_p - W^T dc) = R^-T (q - sum_o Y_o^T A_o dc) from the records the
     // assembly kept (A = [J_pose | J_intr] rows and Y = w Jp R^-T of every observation), with
     // FP64 accumulation (recoverReferencePointSteps, BundleAdjustPlaMatrixReferenceSchur.cpp:982-1082).
@@ -623,6 +624,12 @@ __global__ void __launch_bounds__(256) k_back_substitute(Shape S, DevPtrs D, con
         step_p[static_cast<size_t>(t) * 3 + 0] = p0;
         step_p[static_cast<size_t>(t) * 3 + 1] = p1;
         step_p[static_cast<size_t>(t) * 3 + 2] = p2;
+        if (step_e) {  // the caller's order (a scatter on the host: 200 000 points 1 220 -> 262 us a call)
+            double* e = step_e + static_cast<size_t>(D.trk_block[t]) * 3;
+            e[0] = p0;
+            e[1] = p1;
+            e[2] = p2;
+        }
         dd = td[9] * p0 + td[10] * p1 + td[11] * p2;
         ss = p0 * p0 + p1 * p1 + p2 * p2;
     } else if (t < S.ntp) {
@@ -859,12 +866,12 @@ void launch_reduce_sums64(const Shape& S, const DevPtrs& D, const AsmOut& O, con
 
 template <typename T>
 void launch_back_substitute(const Shape& S, const DevPtrs& D, const double* trk_data, const T* obs_rec, const double* step_c,
-                            double* step_p, double* terms, double* part, const double* direct64, double* out,
-                            cudaStream_t st) {
+                            double* step_p, double* step_e, double* terms, double* part, const double* direct64,
+                            double* out, cudaStream_t st) {
     const int nblk = std::max(1, (S.ntp + 255) / 256);
     if (S.nop > 0)
         k_backsub_terms<T><<<static_cast<unsigned>((S.nop + 255) / 256), 256, 0, st>>>(S, D, obs_rec, step_c, terms);
-    k_back_substitute<<<nblk, 256, 0, st>>>(S, D, trk_data, terms, step_p, part);
+    k_back_substitute<<<nblk, 256, 0, st>>>(S, D, trk_data, terms, step_p, step_e, part);
     k_backsub_final<<<1, 256, 0, st>>>(S, D, part, nblk, step_c, direct64, out);
 }
 
@@ -893,6 +900,50 @@ __global__ void k_gather_obs(long long nop, int ntp, DevPtrs D) {
 void launch_gather_obs(long long nop, int ntp, const DevPtrs& D, cudaStream_t st) {
     const long long n = std::max<long long>(std::max<long long>(nop, ntp), 1);
     k_gather_obs<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(nop, ntp, D);
+}
+
+// The dense symmetric matrix of a reduced system: pose blocks by their CSR row, the border in both
+// triangles, the intrinsic block; entries without a block are zero.  A CTA per row: its zeros and blocks
+// are written by consecutive lanes, so that the caller's copy is one transfer instead of a scatter on the
+// host (234 unknowns 75 -> 43 us a call).
+__global__ void __launch_bounds__(128) k_dense_rows(PcgSystem<double> A, double* __restrict__ out) {
+    const int r = blockIdx.x, n6 = 6 * A.ncb, n = n6 + A.nb, tid = threadIdx.x;
+    double* o = out + static_cast<size_t>(r) * n;
+    if (r >= n6) {
+        const int a = r - n6;
+        for (int c = tid; c < n; c += 128)
+            o[c] = c < n6 ? A.border[static_cast<size_t>(c) * A.nb + a] : A.Cm[static_cast<size_t>(a) * A.nb + c - n6];
+        return;
+    }
+    for (int c = tid; c < n; c += 128) o[c] = c < n6 ? 0.0 : A.border[static_cast<size_t>(r) * A.nb + c - n6];
+    __syncthreads();
+    const int i = r / 6, a = r - 6 * i;
+    const int p0 = A.row_ptr[i], m = 6 * (A.row_ptr[i + 1] - p0);
+    for (int e = tid; e < m; e += 128) {
+        const int p = p0 + e / 6, b = e % 6;
+        o[6 * A.col_idx[p] + b] = A.vals[static_cast<size_t>(p) * 36 + 6 * a + b];
+    }
+}
+
+void launch_dense_rows(const PcgSystem<double>& sys, double* out, cudaStream_t st) {
+    const int n = 6 * sys.ncb + sys.nb;
+    if (n > 0) k_dense_rows<<<n, 128, 0, st>>>(sys, out);
+}
+
+// The points of every track in the caller's order: the state of the processed tracks, the initial points of
+// the others.
+__global__ void __launch_bounds__(128) k_points_out(int nt, const int* __restrict__ proc_of_track,
+                                                    const double* __restrict__ points, const double* __restrict__ init,
+                                                    double* __restrict__ out) {
+    const long long i = static_cast<long long>(blockIdx.x) * 128 + threadIdx.x;
+    if (i >= 3ll * nt) return;
+    const int t = static_cast<int>(i / 3), p = proc_of_track[t];
+    out[i] = p >= 0 ? points[3ll * p + (i - 3ll * t)] : init[i];
+}
+
+void launch_points_out(int nt, const int* proc_of_track, const double* points, const double* init, double* out,
+                       cudaStream_t st) {
+    if (nt > 0) k_points_out<<<static_cast<unsigned>((3ll * nt + 127) / 128), 128, 0, st>>>(nt, proc_of_track, points, init, out);
 }
 
 void launch_effective(const Shape& S, const DevPtrs& D, cudaStream_t st) {
@@ -1143,9 +1194,9 @@ template void launch_reduce<float>(const Shape&, const DevPtrs&, const AsmOut&, 
 template void launch_reduce<double>(const Shape&, const DevPtrs&, const AsmOut&, const RedOut<double>&, double, double*,
                                     cudaStream_t);
 template void launch_back_substitute<float>(const Shape&, const DevPtrs&, const double*, const float*, const double*,
-                                            double*, double*, double*, const double*, double*, cudaStream_t);
+                                            double*, double*, double*, double*, const double*, double*, cudaStream_t);
 template void launch_back_substitute<double>(const Shape&, const DevPtrs&, const double*, const double*, const double*,
-                                             double*, double*, double*, const double*, double*, cudaStream_t);
+                                             double*, double*, double*, double*, const double*, double*, cudaStream_t);
 template void launch_linearize_export<float>(const Shape&, const DevPtrs&, double*, double*, double*, double*, double*,
                                              double*, signed char*, cudaStream_t);
 template void launch_linearize_export<double>(const Shape&, const DevPtrs&, double*, double*, double*, double*,

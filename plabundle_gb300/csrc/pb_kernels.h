@@ -79,11 +79,14 @@ void launch_reduce_sums64(const Shape& S, const DevPtrs& D, const AsmOut& O, con
 // from the original-order arrays through obs_orig and trk_obs_begin.
 void launch_gather_obs(long long nop, int ntp, const DevPtrs& D, cudaStream_t st);
 
-// terms: processed observations * 3 doubles (per-observation terms, summed per track in order)
+// terms: processed observations * 3 doubles (per-observation terms, summed per track in order); step_e: the
+// point steps by elimination block as well, or null
 template <typename T>
 void launch_back_substitute(const Shape& S, const DevPtrs& D, const double* trk_data, const T* obs_rec, const double* step_c,
-                            double* step_p, double* terms, double* part, const double* direct64, double* out,
-                            cudaStream_t st);
+                            double* step_p, double* step_e, double* terms, double* part, const double* direct64,
+                            double* out, cudaStream_t st);
+void launch_points_out(int nt, const int* proc_of_track, const double* points, const double* init, double* out,
+                       cudaStream_t st);
 template <typename T>
 void launch_linearize_export(const Shape& S, const DevPtrs& D, double* res, double* jp, double* jpose, double* ji,
                              double* nw, double* cost, signed char* valid, cudaStream_t st);
@@ -208,6 +211,8 @@ struct PcgResult {
     double bnorm;
 };
 
+void launch_dense_rows(const PcgSystem<double>& sys, double* out, cudaStream_t st);
+
 template <typename T>
 int pcg_precondition(const PcgSystem<T>& sys, int* d_status, cudaStream_t st);
 // Solves sys x = b with block-Jacobi PCG in one cooperative persistent kernel.
@@ -289,7 +294,7 @@ struct AdjBuffers {
     double* gint;           // ng * kP dL/d(group parameters)
     double* mu_p;           // ntp * 3 point part of the adjoint solution (point chart)
     double* terms;          // nop * 3 per-observation terms of the point sums
-    double* grad_obs;       // nop * 2 dL/d(u, v) (processing order)
+    double* grad_obs;       // 2 per uploaded observation: dL/d(u, v) in the caller's order, 0 where not processed
     double* grad_fixed_cam; // nc * 6 cross terms of fixed cameras (zeroed by the caller)
     double* grad_fixed_pt;  // ntp * 3 cross terms of fixed tracks (world)
     double* gauge;          // 4: cross terms of the anchor centre (3) and the gauge baseline (zeroed)

@@ -87,6 +87,14 @@ void check(cudaError_t e, const char* what) {
 // writer, and the host reads it after a synchronisation of the stream.
 constexpr int kSlotCost = 0, kSlotBacksub = 8, kSlotRigSq = 11, kSlotResult = 12, kSlotExtFlags = 14, kSlotBars = 16,
               kSlotPcg = 30, kSlotCg = 40, kSlotFactor = 44, kSlotQuality = 48, kSlots = 64;
+// Behind the slots, room to stage small arrays on their way to the caller (a copy to pageable memory waits
+// for its own end, several to pinned memory share one wait).
+constexpr size_t kStage = 4096;
+// A dense copy of at most this many values is laid out on the device (host scatter against this: 370
+// unknowns 119 / 58 us, 1 060 unknowns 451 / 238 us, 1 810 unknowns 975 / 621 us).  Beyond, the copy of
+// 32 MB and more into fresh pages costs more than the sparse blocks and the scatter (3 010 unknowns
+// 3 350 / 6 440 us).
+constexpr size_t kDenseOnDevice = size_t(1) << 22;
 static_assert(kSlotBacksub >= kSlotCost + kMaxAlpha && kSlotPcg >= kSlotBars + kMaxAlpha + 2, "slots overlap");
 
 // Assembly outputs of one arithmetic type (chunk partials, per-track factors, robust weights).
@@ -139,6 +147,7 @@ struct pb_gpu_ctx {
     double* res_out = nullptr;
     double* bs_part = nullptr;
     double* bs_terms = nullptr;  // per processed observation: its term of the point back-substitution
+    double* out_d = nullptr;     // results in the caller's order: points, point steps, rows of the dense system
     double* bs_out = nullptr;    // pinned: directional decrease, sums of squared point and camera steps
     double* cost_part = nullptr;
     double* cost_out = nullptr;  // pinned: cost per step length
@@ -170,6 +179,7 @@ struct pb_gpu_ctx {
     int solved = 0;
     // backward pass (exact-Hessian records and outputs) and the state snapshot
     DeviceArena aarena;
+    cudaEvent_t adj_ev[4] = {};  // phases of the backward pass
     AdjBuffers adj{};
     bool adj_ready = false;
     int adj_prec = 0;
@@ -390,6 +400,11 @@ void upload_structure(pb_gpu_ctx* c) {
     c->bs_part = A.alloc<double>(2 * static_cast<size_t>(bs_blocks));
     c->bs_terms = A.alloc<double>(3 * static_cast<size_t>(std::max<long long>(1, nop)));
     c->cost_part = A.alloc<double>(static_cast<size_t>(kCostMaxBlocks) * kMaxAlpha * 2);
+    {
+        const size_t nd = static_cast<size_t>(m.rig.on ? 6 * m.rig.nrb + S.nb : n);
+        const size_t dense = nd * nd <= kDenseOnDevice ? nd * nd : 0;
+        c->out_d = A.alloc<double>(std::max(static_cast<size_t>(3) * std::max(1, nt), dense));
+    }
     c->cost_out = c->h_scratch + kSlotCost;
     c->bs_out = c->h_scratch + kSlotBacksub;
     c->pcg_res = A.alloc<PcgResult>(1);
@@ -917,21 +932,59 @@ int solve_reduced(pb_gpu_ctx* c, const pb_solve_options& op, bool* converged, in
     return rc;
 }
 
-void back_substitute(pb_gpu_ctx* c, double* dd, double* point_sq, double* cam_sq) {
+// Device arrays on their way to the caller: small ones through the context's pinned stage, larger ones
+// straight; finish() waits for the stream and fills the caller's memory.
+class ReadBack {
+public:
+    explicit ReadBack(pb_gpu_ctx* ctx) : c(ctx) {}
+    void add(double* dst, const double* src, size_t n) {
+        if (n == 0) return;
+        double* to = dst;
+        if (used + n <= kStage && count < kItems) {
+            to = c->h_scratch + kSlots + used;
+            items[count++] = {dst, to, n};
+            used += n;
+        }
+        check(cudaMemcpyAsync(to, src, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H");
+    }
+    void finish() {
+        check(cudaStreamSynchronize(c->stream), "read back");
+        for (int i = 0; i < count; ++i) std::memcpy(items[i].dst, items[i].staged, items[i].n * sizeof(double));
+        count = 0;
+        used = 0;
+    }
+
+private:
+    static constexpr int kItems = 8;
+    struct Item {
+        double* dst;
+        const double* staged;
+        size_t n;
+    };
+    pb_gpu_ctx* c;
+    Item items[kItems];
+    int count = 0;
+    size_t used = 0;
+};
+
+// elim: the caller's array of the eliminated points' steps (3 per point block), or null.
+void back_substitute(pb_gpu_ctx* c, double* dd, double* point_sq, double* cam_sq, double* elim = nullptr) {
     const int precision = c->last_precision;
     const Shape& S = c->S[precision];
     const DevPtrs& D = c->D[precision];
     if (precision == PB_PRECISION_FP64)
         launch_back_substitute<double>(S, D, static_cast<const double*>(c->p64.out.trk_data_v),
                                        static_cast<const double*>(c->p64.out.obs_rec_v), c->step_c, c->step_p,
-                                       c->bs_terms, c->bs_part, c->direct64, c->bs_out, c->stream);
+                                       elim ? c->out_d : nullptr, c->bs_terms, c->bs_part, c->direct64, c->bs_out, c->stream);
     else
         launch_back_substitute<float>(S, D, static_cast<const double*>(c->p32.out.trk_data_v),
-                                      static_cast<const float*>(c->p32.out.obs_rec_v), c->step_c, c->step_p, c->bs_terms,
-                                      c->bs_part, c->direct64, c->bs_out, c->stream);
+                                      static_cast<const float*>(c->p32.out.obs_rec_v), c->step_c, c->step_p,
+                                      elim ? c->out_d : nullptr, c->bs_terms, c->bs_part, c->direct64, c->bs_out, c->stream);
     c->launches += 3;
     check(cudaGetLastError(), "back-substitution launch");
-    check(cudaStreamSynchronize(c->stream), "back-substitution");
+    ReadBack back(c);
+    if (elim) back.add(elim, c->out_d, static_cast<size_t>(3) * c->model.ntb);
+    back.finish();
     *dd = c->bs_out[0];
     *point_sq = c->bs_out[1];
     // the step RMS of a rig problem is taken over the rig's parameters, not the cameras'
@@ -1544,7 +1597,7 @@ pb_status pb_gpu_create(int32_t device, pb_gpu_ctx** out) {
     if (!c) return PB_ERR_CUDA;
     c->device = device;
     if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMallocHost(&c->h_scratch, kSlots * sizeof(double)) != cudaSuccess ||
+        cudaMallocHost(&c->h_scratch, (kSlots + kStage) * sizeof(double)) != cudaSuccess ||
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess) {
         delete c;
         return PB_ERR_CUDA;
@@ -1567,6 +1620,8 @@ pb_status pb_gpu_destroy(pb_gpu_ctx* c) {
     if (c->h_scratch) cudaFreeHost(c->h_scratch);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
+    for (cudaEvent_t e : c->adj_ev)
+        if (e) cudaEventDestroy(e);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
     return PB_OK;
@@ -1810,57 +1865,50 @@ pb_status pb_gpu_linearize_schur(pb_gpu_ctx* c, double lambda, int32_t precision
 pb_status pb_gpu_get_reduced(pb_gpu_ctx* c, double* dense, double* rhs, double* direct) {
     if (!c || !c->uploaded || !c->have_system) return fail(c, PB_ERR_STATE, "no reduced system assembled");
     try {
-        const HostModel& m = c->model;
-        const Shape& S = c->S[0];
         // rig problems: the system over the rig's pose blocks (the one that is solved); its
         // direct right-hand side is not formed and `direct` is left unwritten
         const bool rig = c->rig_on;
         if (rig && c->ext_on) return fail(c, PB_ERR_UNSUPPORTED, "the dense copy of a rig system with scale bars is not provided");
-        const int npose = rig ? m.rig.nrb : S.ncb;
-        const int nnzb = rig ? c->rig.nnzb : S.nnzb;
-        const std::vector<int>& row_ptr = rig ? m.rig.row_ptr : m.row_ptr;
-        const std::vector<int>& col_idx = rig ? m.rig.col_idx : m.col_idx;
-        const int nb = S.nb, n6 = 6 * npose, n = n6 + nb;
-        const size_t ts = 8;
-        std::vector<char> vals(static_cast<size_t>(std::max(1, nnzb)) * 36 * ts), border(static_cast<size_t>(std::max(1, npose)) * 6 * std::max(1, nb) * ts),
-            Cm(static_cast<size_t>(std::max(1, nb * nb)) * ts), r(n * ts), d(n * ts);
-        const void* src_vals = rig ? c->rig.vals : c->red.vals;
-        const void* src_border = rig ? c->rig.border : c->red.border;
-        const void* src_C = c->red.Cm;
-        const void* src_r = rig ? c->rig.rhs : c->red.rhs;
-        const void* src_d = c->red.direct;
-        check(cudaMemcpy(vals.data(), src_vals, static_cast<size_t>(nnzb) * 36 * ts, cudaMemcpyDeviceToHost), "D2H");
-        if (nb) {
-            check(cudaMemcpy(border.data(), src_border, static_cast<size_t>(npose) * 6 * nb * ts, cudaMemcpyDeviceToHost), "D2H");
-            check(cudaMemcpy(Cm.data(), src_C, static_cast<size_t>(nb) * nb * ts, cudaMemcpyDeviceToHost), "D2H");
+        const PcgSystem<double>& sys = rig ? c->sysr : c->sys;
+        const int n = 6 * sys.ncb + sys.nb;
+        ReadBack back(c);
+        std::vector<double> vals, border, Cm;
+        const bool on_device = static_cast<size_t>(n) * n <= kDenseOnDevice;
+        if (dense && on_device) {
+            launch_dense_rows(sys, c->out_d, c->stream);
+            check(cudaGetLastError(), "dense rows launch");
+            back.add(dense, c->out_d, static_cast<size_t>(n) * n);
+        } else if (dense) {
+            vals.resize(static_cast<size_t>(rig ? c->rig.nnzb : c->S[0].nnzb) * 36);
+            border.resize(static_cast<size_t>(6) * sys.ncb * sys.nb);
+            Cm.resize(static_cast<size_t>(sys.nb) * sys.nb);
+            back.add(vals.data(), sys.vals, vals.size());
+            back.add(border.data(), sys.border, border.size());
+            back.add(Cm.data(), sys.Cm, Cm.size());
         }
-        check(cudaMemcpy(r.data(), src_r, n * ts, cudaMemcpyDeviceToHost), "D2H");
-        if (!rig) check(cudaMemcpy(d.data(), src_d, n * ts, cudaMemcpyDeviceToHost), "D2H");
-        auto get = [&](const std::vector<char>& v, size_t i) {
-            return ts == 8 ? reinterpret_cast<const double*>(v.data())[i]
-                           : static_cast<double>(reinterpret_cast<const float*>(v.data())[i]);
-        };
-        if (dense) {
+        if (rhs) back.add(rhs, rig ? c->rig.rhs : c->red.rhs, n);
+        if (direct && !rig) back.add(direct, c->red.direct, n);
+        back.finish();
+        if (dense && !on_device) {
+            const HostModel& m = c->model;
+            const std::vector<int>& row_ptr = rig ? m.rig.row_ptr : m.row_ptr;
+            const std::vector<int>& col_idx = rig ? m.rig.col_idx : m.col_idx;
+            const int nb = sys.nb, n6 = 6 * sys.ncb;
             std::fill(dense, dense + static_cast<size_t>(n) * n, 0.0);
-            for (int i = 0; i < npose; ++i)
-                for (int p = row_ptr[i]; p < row_ptr[i + 1]; ++p) {
-                    const int j = col_idx[p];
+            for (int i = 0; i < sys.ncb; ++i)
+                for (int p = row_ptr[i]; p < row_ptr[i + 1]; ++p)
                     for (int a = 0; a < 6; ++a)
                         for (int b = 0; b < 6; ++b)
-                            dense[static_cast<size_t>(6 * i + a) * n + 6 * j + b] = get(vals, static_cast<size_t>(p) * 36 + a * 6 + b);
-                }
+                            dense[static_cast<size_t>(6 * i + a) * n + 6 * col_idx[p] + b] =
+                                vals[static_cast<size_t>(p) * 36 + a * 6 + b];
             for (int row = 0; row < n6; ++row)
                 for (int col = 0; col < nb; ++col) {
-                    const double v = get(border, static_cast<size_t>(row) * nb + col);
+                    const double v = border[static_cast<size_t>(row) * nb + col];
                     dense[static_cast<size_t>(row) * n + n6 + col] = v;
                     dense[static_cast<size_t>(n6 + col) * n + row] = v;
                 }
             for (int a = 0; a < nb; ++a)
-                for (int b = 0; b < nb; ++b) dense[static_cast<size_t>(n6 + a) * n + n6 + b] = get(Cm, static_cast<size_t>(a) * nb + b);
-        }
-        for (int i = 0; i < n; ++i) {
-            if (rhs) rhs[i] = get(r, i);
-            if (direct && !rig) direct[i] = get(d, i);
+                for (int b = 0; b < nb; ++b) dense[static_cast<size_t>(n6 + a) * n + n6 + b] = Cm[static_cast<size_t>(a) * nb + b];
         }
         return PB_OK;
     } catch (const std::exception& e) {
@@ -1883,12 +1931,10 @@ pb_status pb_gpu_solve_reduced(pb_gpu_ctx* c, double* step, int32_t* converged, 
         // the solution of the system pb_gpu_get_reduced copies: for a rig problem the rig step
         // (6 per rig block, then the intrinsic columns), else the camera-block step
         if (step) {
-            if (c->rig_on)
-                check(cudaMemcpy(step, c->rig.step_r, (6 * c->model.rig.nrb + c->S[0].nb) * sizeof(double),
-                                 cudaMemcpyDeviceToHost),
-                      "D2H");
-            else
-                check(cudaMemcpy(step, c->step_c, c->S[0].n * sizeof(double), cudaMemcpyDeviceToHost), "D2H");
+            ReadBack back(c);
+            if (c->rig_on) back.add(step, c->rig.step_r, 6 * static_cast<size_t>(c->model.rig.nrb) + c->S[0].nb);
+            else back.add(step, c->step_c, c->S[0].n);
+            back.finish();
         }
         if (rc) return fail(c, PB_ERR_SINGULAR_BLOCK, "reduced system is not numerically SPD (positive definite)");
         return PB_OK;
@@ -1901,19 +1947,9 @@ pb_status pb_gpu_back_substitute(pb_gpu_ctx* c, double* elim, double* dd, int32_
     if (!c || !c->uploaded || !c->have_system) return fail(c, PB_ERR_STATE, "no reduced system assembled");
     try {
         double d, ps, cs;
-        back_substitute(c, &d, &ps, &cs);
+        back_substitute(c, &d, &ps, &cs, elim);
         if (dd) *dd = d;
         if (success) *success = std::isfinite(d) ? 1 : 0;
-        if (elim) {
-            const HostModel& m = c->model;
-            std::vector<double> sp(m.trk_order.size() * 3);
-            check(cudaMemcpy(sp.data(), c->step_p, sp.size() * sizeof(double), cudaMemcpyDeviceToHost), "D2H");
-            for (size_t p = 0; p < m.trk_order.size(); ++p) {
-                const int tb = m.track_block[m.trk_order[p]];
-                if (tb < 0) continue;
-                for (int a = 0; a < 3; ++a) elim[static_cast<size_t>(tb) * 3 + a] = sp[p * 3 + a];
-            }
-        }
         return PB_OK;
     } catch (const std::exception& e) {
         return fail(c, PB_ERR_CUDA, e.what());
@@ -1977,15 +2013,14 @@ pb_status pb_gpu_download_state(pb_gpu_ctx* c, double* cams, double* pts, int8_t
     if (!c || !c->uploaded) return fail(c, PB_ERR_STATE, "no problem uploaded");
     try {
         const HostModel& m = c->model;
-        if (cams)
-            check(cudaMemcpy(cams, c->D[0].cams_eff, m.cams_in.size() * sizeof(double), cudaMemcpyDeviceToHost), "D2H");
+        ReadBack back(c);
+        if (cams) back.add(cams, c->D[0].cams_eff, m.cams_in.size());
         if (pts) {
-            std::vector<double> sp(m.trk_order.size() * 3);
-            check(cudaMemcpy(sp.data(), c->D[0].points, sp.size() * sizeof(double), cudaMemcpyDeviceToHost), "D2H");
-            std::copy(m.points_in.begin(), m.points_in.end(), pts);
-            for (size_t p = 0; p < m.trk_order.size(); ++p)
-                for (int a = 0; a < 3; ++a) pts[static_cast<size_t>(m.trk_order[p]) * 3 + a] = sp[p * 3 + a];
+            launch_points_out(m.nt, c->proc_of_track, c->D[0].points, c->init_points_all, c->out_d, c->stream);
+            check(cudaGetLastError(), "points launch");
+            back.add(pts, c->out_d, m.points_in.size());
         }
+        back.finish();
         if (valid || ra) fetch_quality(c);
         for (int t = 0; t < m.nt; ++t) {
             if (valid) valid[t] = c->solved && static_cast<size_t>(t) < c->valid.size() ? c->valid[t] : 0;
@@ -2147,6 +2182,9 @@ pb_status pb_gpu_set_observations(pb_gpu_ctx* c, int64_t n, const int64_t* index
 
 namespace {
 
+// The adjoint kernels' flags in pinned memory (the backward pass has no scale bars, whose slot this is).
+int* adjoint_flags(pb_gpu_ctx* c) { return reinterpret_cast<int*>(c->h_scratch + kSlotExtFlags); }
+
 // Exact-Hessian solve of the backward pass (newton == 0: H mu = dL/dz with dL/dz already in the
 // adjoint input buffers) or of a Newton step of the objective (newton == 1: H mu = -grad F).
 // Leaves mu in c->step_c (primary) and c->adj.mu_p (points), dL/d(u, v) and the cross terms in
@@ -2161,12 +2199,9 @@ pb_status adjoint_core(pb_gpu_ctx* c, int newton, pb_adjoint_report* rep, float*
     AdjBuffers& B = c->adj;
     B.newton = newton;
     B.terms = c->bs_terms;
-    cudaEvent_t ev[4];
-    for (auto& e : ev) check(cudaEventCreate(&e), "event");
-    struct EvGuard {
-        cudaEvent_t* e;
-        ~EvGuard() { for (int i = 0; i < 4; ++i) cudaEventDestroy(e[i]); }
-    } guard{ev};
+    cudaEvent_t* ev = c->adj_ev;
+    for (int i = 0; i < 4; ++i)
+        if (!ev[i]) check(cudaEventCreate(&ev[i]), "event");
     check(cudaEventRecord(ev[0], st), "event");
     // exact Hessian at the current state, reduced over the points
     const int n = S.n;
@@ -2183,9 +2218,10 @@ pb_status adjoint_core(pb_gpu_ctx* c, int newton, pb_adjoint_report* rep, float*
     c->launches += 6;
     check(cudaGetLastError(), "adjoint launch");
     check(cudaEventRecord(ev[1], st), "event");
-    int flags = 0;
-    check(cudaMemcpyAsync(&flags, B.flags, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H");
+    int* host_flags = adjoint_flags(c);
+    check(cudaMemcpyAsync(host_flags, B.flags, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H");
     check(cudaStreamSynchronize(st), "adjoint hessian");
+    const int flags = *host_flags;
     c->have_system = false;  // the reduced buffers now hold the exact Hessian, not an LM system
     if (rep) rep->point_blocks_singular = flags & 1;
     if (flags & 2) return fail(c, PB_ERR_INVALID_PROJECTION, "an observation does not project at this state");
@@ -2217,7 +2253,8 @@ pb_status adjoint_core(pb_gpu_ctx* c, int newton, pb_adjoint_report* rep, float*
     c->launches += 3 + (S.gauge_scale >= 0 && S.gauge_anchor >= 0 && S.gauge_baseline > 0.0 ? 1 : 0);
     check(cudaGetLastError(), "adjoint gradient launch");
     check(cudaEventRecord(ev[3], st), "event");
-    cudaEventSynchronize(ev[3]);
+    check(cudaMemcpyAsync(host_flags, B.flags, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H");
+    check(cudaStreamSynchronize(st), "adjoint gradient");
     cudaEventElapsedTime(&ms[0], ev[0], ev[1]);
     cudaEventElapsedTime(&ms[1], ev[1], ev[2]);
     cudaEventElapsedTime(&ms[2], ev[2], ev[3]);
@@ -2255,7 +2292,8 @@ pb_status adjoint_prepare(pb_gpu_ctx* c) {
     B.gcam = A.alloc<double>(static_cast<size_t>(nc) * 6);
     B.gint = A.alloc<double>(static_cast<size_t>(std::max(1, m.ng)) * kP);
     B.mu_p = A.alloc<double>(static_cast<size_t>(std::max(1, ntp)) * 3);
-    B.grad_obs = A.alloc<double>(static_cast<size_t>(std::max<long long>(1, nop)) * 2);
+    B.grad_obs = A.alloc<double>(static_cast<size_t>(std::max<long long>(1, m.no)) * 2);
+    check(cudaMemsetAsync(B.grad_obs, 0, static_cast<size_t>(std::max<long long>(1, m.no)) * 2 * sizeof(double), st), "memset");
     B.grad_fixed_cam = A.alloc<double>(static_cast<size_t>(nc) * 6);
     B.grad_fixed_pt = A.alloc<double>(static_cast<size_t>(std::max(1, ntp)) * 3);
     B.gauge = A.alloc<double>(4);
@@ -2297,46 +2335,54 @@ pb_status pb_gpu_backward(pb_gpu_ctx* c, const double* grad_cameras, const doubl
         const int nc = m.nc, ntp = S.ntp;
         const long long nop = S.nop;
         AdjBuffers& B = c->adj;
-        // inputs: dL/d(final state) (processing order for points)
-        std::vector<double> gcam(static_cast<size_t>(nc) * 6, 0.0), gpt(static_cast<size_t>(std::max(1, ntp)) * 3, 0.0),
-            gint(static_cast<size_t>(std::max(1, m.ng)) * kP, 0.0);
+        // inputs: dL/d(final state) (processing order for points); zero where the caller gives none
+        std::vector<double> gcam(static_cast<size_t>(nc) * 6, 0.0), gpt;
         if (grad_cameras) std::copy(grad_cameras, grad_cameras + gcam.size(), gcam.begin());
-        if (grad_points)
-            for (int p = 0; p < ntp; ++p)
-                for (int a = 0; a < 3; ++a) gpt[static_cast<size_t>(p) * 3 + a] = grad_points[static_cast<size_t>(m.trk_order[p]) * 3 + a];
-        if (grad_intrinsics && m.ng > 0) std::copy(grad_intrinsics, grad_intrinsics + static_cast<size_t>(m.ng) * kP, gint.begin());
         for (double v : gcam)
             if (!std::isfinite(v)) return fail(c, PB_ERR_INVALID_ARGUMENT, "non-finite camera gradient");
-        for (double v : gpt)
-            if (!std::isfinite(v)) return fail(c, PB_ERR_INVALID_ARGUMENT, "non-finite point gradient");
-        for (double v : gint)
-            if (!std::isfinite(v)) return fail(c, PB_ERR_INVALID_ARGUMENT, "non-finite intrinsic gradient");
+        if (grad_points) {
+            gpt.resize(static_cast<size_t>(ntp) * 3);
+            for (int p = 0; p < ntp; ++p)
+                for (int a = 0; a < 3; ++a) gpt[static_cast<size_t>(p) * 3 + a] = grad_points[static_cast<size_t>(m.trk_order[p]) * 3 + a];
+            for (double v : gpt)
+                if (!std::isfinite(v)) return fail(c, PB_ERR_INVALID_ARGUMENT, "non-finite point gradient");
+        }
+        const size_t n_gint = static_cast<size_t>(m.ng) * kP;
+        if (grad_intrinsics)
+            for (size_t i = 0; i < n_gint; ++i)
+                if (!std::isfinite(grad_intrinsics[i]))
+                    return fail(c, PB_ERR_INVALID_ARGUMENT, "non-finite intrinsic gradient");
         check(cudaMemcpyAsync(B.gcam, gcam.data(), gcam.size() * sizeof(double), cudaMemcpyHostToDevice, st), "H2D");
-        check(cudaMemcpyAsync(B.gpt, gpt.data(), gpt.size() * sizeof(double), cudaMemcpyHostToDevice, st), "H2D");
-        check(cudaMemcpyAsync(B.gint, gint.data(), gint.size() * sizeof(double), cudaMemcpyHostToDevice, st), "H2D");
+        if (!gpt.empty())
+            check(cudaMemcpyAsync(B.gpt, gpt.data(), gpt.size() * sizeof(double), cudaMemcpyHostToDevice, st), "H2D");
+        else
+            check(cudaMemsetAsync(B.gpt, 0, static_cast<size_t>(std::max(1, ntp)) * 3 * sizeof(double), st), "memset");
+        if (grad_intrinsics && n_gint)
+            check(cudaMemcpyAsync(B.gint, grad_intrinsics, n_gint * sizeof(double), cudaMemcpyHostToDevice, st), "H2D");
+        else
+            check(cudaMemsetAsync(B.gint, 0, static_cast<size_t>(std::max(1, m.ng)) * kP * sizeof(double), st), "memset");
         const int launches0 = c->launches;
         float ms[3] = {0.f, 0.f, 0.f};
         ps = adjoint_core(c, 0, rep, ms);
         if (ps != PB_OK) return ps;
-        int flags = 0;
-        std::vector<double> gobs(static_cast<size_t>(std::max<long long>(1, nop)) * 2), gfc(static_cast<size_t>(nc) * 6),
-            gfp(static_cast<size_t>(std::max(1, ntp)) * 3), gauge(4), cams(m.cams_in.size());
-        check(cudaMemcpyAsync(gobs.data(), B.grad_obs, gobs.size() * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H");
-        check(cudaMemcpyAsync(gfc.data(), B.grad_fixed_cam, gfc.size() * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H");
-        check(cudaMemcpyAsync(gfp.data(), B.grad_fixed_pt, gfp.size() * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H");
-        check(cudaMemcpyAsync(gauge.data(), B.gauge, 4 * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H");
-        check(cudaMemcpyAsync(cams.data(), D.cams_state, cams.size() * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H");
-        check(cudaMemcpyAsync(&flags, B.flags, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H");
-        check(cudaStreamSynchronize(st), "adjoint gradient");
-        if (flags & 2) return fail(c, PB_ERR_INVALID_PROJECTION, "an observation does not project at this state");
-        if (grad_observations) {
-            std::fill(grad_observations, grad_observations + static_cast<size_t>(m.no) * 2, 0.0);
-            for (long long p = 0; p < nop; ++p) {
-                const long long k = m.p_obs_orig[p];
-                grad_observations[2 * k] = gobs[2 * p];
-                grad_observations[2 * k + 1] = gobs[2 * p + 1];
-            }
+        if (*adjoint_flags(c) & 2) return fail(c, PB_ERR_INVALID_PROJECTION, "an observation does not project at this state");
+        // the gauge pair's centres, the cross terms and, where a track is fixed, its cross terms
+        const int sc = m.gauge_scale, an = m.gauge_anchor;
+        const bool gauge_pair = grad_initial_cameras && sc >= 0 && an >= 0 && m.gauge_baseline > 0.0 && m.camera_block[sc] >= 0;
+        const bool fixed_tracks = grad_initial_points && m.ntb < ntp;
+        std::vector<double> gfc(grad_initial_cameras ? static_cast<size_t>(nc) * 6 : 0),
+            gfp(fixed_tracks ? static_cast<size_t>(ntp) * 3 : 0);
+        double gauge[4] = {0, 0, 0, 0}, centre_sc[3] = {0, 0, 0}, centre_an[3] = {0, 0, 0};
+        ReadBack back(c);
+        back.add(gfc.data(), B.grad_fixed_cam, gfc.size());
+        if (gauge_pair) {
+            back.add(gauge, B.gauge, 4);
+            back.add(centre_sc, D.cams_state + static_cast<size_t>(sc) * kCamStride + 9, 3);
+            back.add(centre_an, D.cams_state + static_cast<size_t>(an) * kCamStride + 9, 3);
         }
+        back.add(gfp.data(), B.grad_fixed_pt, gfp.size());
+        if (grad_observations) back.add(grad_observations, B.grad_obs, static_cast<size_t>(m.no) * 2);
+        back.finish();
         if (grad_initial_cameras) {
             // fixed cameras: final pose = initial pose (direct term) plus the cross terms
             std::fill(grad_initial_cameras, grad_initial_cameras + static_cast<size_t>(nc) * 6, 0.0);
@@ -2345,11 +2391,10 @@ pb_status pb_gpu_backward(pb_gpu_ctx* c, const double* grad_cameras, const doubl
                     for (int a = 0; a < 6; ++a)
                         grad_initial_cameras[cam * 6 + a] = gcam[static_cast<size_t>(cam) * 6 + a] + gfc[static_cast<size_t>(cam) * 6 + a];
             // gauge: the scale camera's centre is anchor + b n(t), b = |C_scale^0 - C_anchor^0|
-            const int sc = m.gauge_scale, an = m.gauge_anchor;
-            if (sc >= 0 && an >= 0 && m.gauge_baseline > 0.0 && m.camera_block[sc] >= 0) {
+            if (gauge_pair) {
                 double nv[3], e0[3], l = 0.0, l0 = 0.0;
                 for (int i = 0; i < 3; ++i) {
-                    nv[i] = cams[static_cast<size_t>(sc) * kCamStride + 9 + i] - cams[static_cast<size_t>(an) * kCamStride + 9 + i];
+                    nv[i] = centre_sc[i] - centre_an[i];
                     e0[i] = m.cams_in[static_cast<size_t>(sc) * kCamStride + 9 + i] - m.cams_in[static_cast<size_t>(an) * kCamStride + 9 + i];
                     l += nv[i] * nv[i];
                     l0 += e0[i] * e0[i];
@@ -2368,7 +2413,7 @@ pb_status pb_gpu_backward(pb_gpu_ctx* c, const double* grad_cameras, const doubl
         }
         if (grad_initial_points) {
             std::fill(grad_initial_points, grad_initial_points + static_cast<size_t>(m.nt) * 3, 0.0);
-            for (int p = 0; p < ntp; ++p) {
+            for (int p = 0; fixed_tracks && p < ntp; ++p) {
                 const int t = m.trk_order[p];
                 if (m.track_block[t] >= 0) continue;
                 for (int a = 0; a < 3; ++a)

@@ -77,3 +77,19 @@ def test_reduced_system_and_point_steps(groups, refine, points, precision):
     tol = 1e-7 if precision == Precision.Fp64 else 2e-2
     assert np.linalg.norm(elim - oelim) <= tol * np.linalg.norm(oelim)
     assert abs(decrease - odecrease) <= (1e-7 if precision == Precision.Fp64 else 1e-5) * abs(odecrease)
+
+
+@pytest.mark.parametrize("n_along,n_lines", [(18, 18), (20, 17), (19, 18)])
+def test_dense_copy_on_either_side_of_its_size_rule(n_along, n_lines):
+    """1 954 unknowns are laid out on the device, 2 050 and 2 062 on the host.  The conjugate gradients stop at a
+    relative residual of 2e-10 on the device's own matrix; the copy, multiplied here, adds the rounding of
+    2 000 products a row."""
+    p = synth.aerial_grid_problem(seed=n_along, n_along=n_along, n_lines=n_lines, n_points=6000, n_groups=2)
+    ctx = Gb300Context(0)
+    assert ctx.upload(p, _options("fcr", False)) == 0
+    ctx.linearize_schur(1e-2, Precision.Fp64)
+    S, rhs, _ = ctx.reduced()
+    assert len(rhs) == 6 * (n_along * n_lines - 1) + 2 * ctx.sizes()["ni"] and np.array_equal(S, S.T)
+    step, converged, _, _ = ctx.solve_reduced()
+    assert converged
+    assert np.linalg.norm(S @ step - rhs) <= 1e-9 * np.linalg.norm(rhs)
