@@ -786,11 +786,12 @@ __device__ __forceinline__ ff ff_rsqrt(ff a) {
 // Float-float camera record: R (9), C (3), fx, fy, cx, cy, k1, k2, k3, p1, p2 (11), then the
 // signs su, sv and the depth flip as plain floats.
 constexpr int kCamFF = 24;
+__host__ __device__ __forceinline__ float2 camera_ff_value(int i, double c) {
+    if (i < 21) return ff_pack(c);
+    return make_float2(i < 23 ? (c < 0.0 ? -1.f : 1.f) : (c != 0.0 ? 1.f : 0.f), 0.f);
+}
 __host__ __device__ __forceinline__ void camera_ff(const double* c, float2* out) {
-    for (int i = 0; i < 21; ++i) out[i] = ff_pack(c[i]);
-    out[21] = make_float2(c[21] < 0.0 ? -1.f : 1.f, 0.f);
-    out[22] = make_float2(c[22] < 0.0 ? -1.f : 1.f, 0.f);
-    out[23] = make_float2(c[23] != 0.0 ? 1.f : 0.f, 0.f);
+    for (int i = 0; i < kCamFF; ++i) out[i] = camera_ff_value(i, c[i]);
 }
 
 struct LinFF {

@@ -341,11 +341,22 @@ __global__ void k_effective(Shape S, DevPtrs D) {
 // BundleAdjustPlaMatrixAssembly.cpp:130-179; gauge tangent step :101-128; the plain
 // parameterisation's pose delta :1134-1136) and clamped intrinsic update (applyIntrinsicStep,
 // BundleAdjustPlaMatrixModel.cpp:248-269).
-__global__ void k_trial_cameras(Shape S, DevPtrs D, const double* __restrict__ step_c, Alphas alphas, int n_alpha) {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= n_alpha * S.nc) return;
-    const int a = idx / S.nc, c = idx - a * S.nc;
+// Three lanes per camera, one rotation increment's sine and cosine each (a FP64 instruction takes the
+// pipe 64 cycles whatever the number of lanes: 20 cameras 10.1 -> 9.2 us), then the first of them.
+constexpr int kTrialCameras = 10;  // per warp
+__global__ void __launch_bounds__(32) k_trial_cameras(Shape S, DevPtrs D, const double* __restrict__ step_c, Alphas alphas, int n_alpha) {
+    const int lane = threadIdx.x & 31, lead = lane / 3 * 3;
+    const int idx = blockIdx.x * kTrialCameras + lane / 3;
+    const bool live = lane < 3 * kTrialCameras && idx < n_alpha * S.nc;
+    const int a = live ? idx / S.nc : 0, c = live ? idx - a * S.nc : 0;
     const double alpha = alphas.v[a];
+    const int b = live ? D.cam_block[c] : -1;
+    double sn = 0.0, cs = 1.0;
+    if (b >= 0 && S.ref_param) sincos(alpha * step_c[6 * b + lane - lead], &sn, &cs);
+    const double sx = __shfl_sync(0xffffffffu, sn, lead), cx = __shfl_sync(0xffffffffu, cs, lead);
+    const double sy = __shfl_sync(0xffffffffu, sn, (lead + 1) & 31), cy = __shfl_sync(0xffffffffu, cs, (lead + 1) & 31);
+    const double sz = __shfl_sync(0xffffffffu, sn, (lead + 2) & 31), cz = __shfl_sync(0xffffffffu, cs, (lead + 2) & 31);
+    if (!live || lane != lead) return;
     // trial groups (each camera thread of the first ng cameras writes one group)
     double Gt[kGroupRec];
     const double* Gs = nullptr;
@@ -373,7 +384,6 @@ __global__ void k_trial_cameras(Shape S, DevPtrs D, const double* __restrict__ s
     double pose[kCamStride];
     const double* st = D.cams_state + static_cast<size_t>(c) * kCamStride;
     for (int i = 0; i < kCamStride; ++i) pose[i] = st[i];
-    const int b = D.cam_block[c];
     if (b >= 0 && !S.ref_param) {
         // plain parameterisation: the camera's own pose delta (CameraState::applyDeltaPose,
         // BundleAdjustPlaMatrixAssembly.cpp:1134-1136), C2W' = Exp(alpha w) C2W by Rodrigues'
@@ -404,11 +414,6 @@ __global__ void k_trial_cameras(Shape S, DevPtrs D, const double* __restrict__ s
         for (int i = 0; i < 3; ++i) pose[9 + i] = st[9 + i] + alpha * d[3 + i];
     } else if (b >= 0) {
         const double* d = step_c + 6 * b;
-        const double dx = alpha * d[0], dy = alpha * d[1], dz = alpha * d[2];
-        double sx, cx, sy, cy, sz, cz;
-        sincos(dx, &sx, &cx);
-        sincos(dy, &sy, &cy);
-        sincos(dz, &sz, &cz);
         // E = Rx Ry Rz
         const double E[9] = {cy * cz, -cy * sz, sy,
                              sx * sy * cz + cx * sz, -sx * sy * sz + cx * cz, -sx * cy,
@@ -452,15 +457,34 @@ __global__ void k_trial_cameras(Shape S, DevPtrs D, const double* __restrict__ s
                  D.cams_trial + (static_cast<size_t>(a) * S.nc + c) * kCamStride);
 }
 
+// True in every thread of the block that is the last of `blocks` to come here: the partial results that the
+// others wrote before are visible to it.  The ticket is zero again afterwards.
+__device__ __forceinline__ bool last_block(unsigned* ticket, unsigned blocks) {
+    __shared__ unsigned s_ticket;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_ticket = atomicInc(ticket, blocks - 1);
+    }
+    __syncthreads();
+    if (s_ticket != blocks - 1) return false;
+    __threadfence();
+    return true;
+}
+
 // Objective of the trial states: image costs (FP64) per step length (blockIdx.y), block partials.
 // FP64-pipe-bound: see the objective in pb_device.cuh for the form of a term.  A thread takes every
 // (grid.x x block)-th observation; part holds the sums of step length a at a * gridDim.x and, from
-// kMaxAlpha * gridDim.x on, the blocks' invalid-projection marks in the same order.
+// kMaxAlpha * gridDim.x on, the blocks' invalid-projection marks in the same order.  The last block of a
+// step length adds them up in a fixed order (256 interleaved sums, two per thread) with the intrinsic priors
+// of the trial groups (assemblePrimaryPriors cost, BundleAdjustPlaMatrixAssemblySurvey.cpp:43-91); a kernel
+// of its own for it took as long as a small problem's objective (20 cameras: 7.6 + 3.5 us and the gap between them, now 10.2).
 constexpr int kCostThreads = 128;
 __global__ void __launch_bounds__(kCostThreads) k_cost_batch(Shape S, DevPtrs D, const double* __restrict__ step_p,
                                                              Alphas alphas, int use_trial, double c2,
-                                                             double ic2, int plain, double* __restrict__ part) {
-    __shared__ double s_c[kCostThreads / 32];
+                                                             double ic2, int plain, double* __restrict__ part,
+                                                             unsigned* __restrict__ tickets,
+                                                             double* __restrict__ out) {
+    __shared__ double s_c[kCostThreads / 16];
     __shared__ int s_bad[kCostThreads / 32];
     const int a = blockIdx.y;
     const double* cams = use_trial ? D.cams_trial + static_cast<size_t>(a) * S.nc * kCamStride : D.cams_eff;
@@ -513,49 +537,45 @@ __global__ void __launch_bounds__(kCostThreads) k_cost_batch(Shape S, DevPtrs D,
         part[at] = (s_c[0] + s_c[1]) + (s_c[2] + s_c[3]);
         part[static_cast<size_t>(kMaxAlpha) * gridDim.x + at] = s_bad[0] | s_bad[1] | s_bad[2] | s_bad[3];
     }
-}
-static_assert(kCostThreads == 128, "k_cost_batch adds the sums of four warps");
-
-// Final objective of step length blockIdx.x: block partials in fixed order plus the intrinsic priors of
-// the trial groups (assemblePrimaryPriors cost, BundleAdjustPlaMatrixAssemblySurvey.cpp:43-91).
-constexpr int kCostFinalThreads = 256;
-__global__ void __launch_bounds__(kCostFinalThreads) k_cost_final(Shape S, DevPtrs D, const double* __restrict__ part,
-                                                                  int nblocks, int use_trial, double* __restrict__ out) {
-    __shared__ double s_v[kCostFinalThreads / 32];
-    __shared__ int s_b[kCostFinalThreads / 32];
-    const int a = blockIdx.x, tid = threadIdx.x;
+    if (!last_block(tickets + a, gridDim.x)) return;
+    const int nblocks = gridDim.x, tid = threadIdx.x;
     const double* sums = part + static_cast<size_t>(a) * nblocks;
     const double* marks = part + static_cast<size_t>(kMaxAlpha + a) * nblocks;
-    double v = 0.0;
-    int bad = 0;
+    double half[2] = {0.0, 0.0};  // sums tid and tid + 128 of the 256
+    bad = 0;
 #pragma unroll 5
-    for (int i = tid; i < nblocks; i += kCostFinalThreads) {
-        v += sums[i];
-        bad |= __double_as_longlong(marks[i]) != 0;
+    for (int i = tid; i < nblocks; i += 2 * kCostThreads) {
+        half[0] += __ldcg(sums + i);
+        bad |= __double_as_longlong(__ldcg(marks + i)) != 0;
+        if (i + kCostThreads < nblocks) {
+            half[1] += __ldcg(sums + i + kCostThreads);
+            bad |= __double_as_longlong(__ldcg(marks + i + kCostThreads)) != 0;
+        }
     }
     if (tid < S.nb) {  // (at most 36 columns)
         const int g = tid / S.ni, p = S.int_cols[tid - g * S.ni];
         const double* G = (use_trial ? D.groups_trial + static_cast<size_t>(a) * S.ng * kGroupRec : D.groups) +
                           static_cast<size_t>(g) * kGroupRec;
         const double r = G[2 * kP + p] * (G[p] - G[kP + p]);
-        v = fma(0.5 * r, r, v);
+        half[0] = fma(0.5 * r, r, half[0]);
     }
-    v = warp_sum(v);
+    half[0] = warp_sum(half[0]);
+    half[1] = warp_sum(half[1]);
     bad = __any_sync(0xffffffffu, bad);
-    if ((tid & 31) == 0) {
-        s_v[tid >> 5] = v;
-        s_b[tid >> 5] = bad;
+    if (lane == 0) {
+        s_c[wid] = half[0];
+        s_c[wid + kCostThreads / 32] = half[1];
+        s_bad[wid] = bad;
     }
     __syncthreads();
     if (tid == 0) {
-        for (int w = 1; w < kCostFinalThreads / 32; ++w) {
-            v += s_v[w];
-            bad |= s_b[w];
-        }
-        out[a] = bad ? __longlong_as_double(0x7ff0000000000000ll) : v;
+        double total = half[0];
+        for (int w = 1; w < kCostThreads / 16; ++w) total += s_c[w];
+        bad = s_bad[0] | s_bad[1] | s_bad[2] | s_bad[3];
+        out[a] = bad ? __longlong_as_double(0x7ff0000000000000ll) : total;
     }
 }
-static_assert(kMaxNB <= kCostFinalThreads, "a thread per intrinsic column");
+static_assert(kCostThreads == 128 && kMaxNB <= kCostThreads, "four warps' sums; a thread per intrinsic column");
 
 // Back-substitution (recoverReferencePointSteps, ...ReferenceSchur.cpp:982-1082), one thread per
 // track:  dp = R^-T (q - R^-1 u),  u = sum_o w J_p^T (J_o dc).
@@ -594,10 +614,18 @@ __global__ void __launch_bounds__(256) k_backsub_terms(Shape S, DevPtrs D, const
 }
 
 // track:  dp = R^-T (q - R^-1 u),  u = sum_o w J_p^T (J_o dc).
-__global__ void __launch_bounds__(256) k_back_substitute(Shape S, DevPtrs D, const double* __restrict__ trk_data,
-                                                         const double* __restrict__ terms,
-                                                         double* __restrict__ step_p, double* __restrict__ step_e,
-                                                         double* __restrict__ part) {
+// The last block adds up the blocks' parts of the directional decrease and of the squared point steps and
+// the camera-side terms (dc . direct rhs, squared camera step), in a fixed order (20 cameras, 2 000 points: 9.1 + 5.1 us as two kernels, now 11.5).
+constexpr int kBacksubThreads = 128;
+__global__ void __launch_bounds__(kBacksubThreads) k_back_substitute(Shape S, DevPtrs D,
+                                                                     const double* __restrict__ trk_data,
+                                                                     const double* __restrict__ terms,
+                                                                     double* __restrict__ step_p,
+                                                                     double* __restrict__ step_e, double* __restrict__ part,
+                                                                     const double* __restrict__ step_c,
+                                                                     const double* __restrict__ direct64,
+                                                                     unsigned* __restrict__ ticket,
+                                                                     double* __restrict__ out) {
     // Point steps dp = V^-1 (g_p - W^T dc) = R^-T (q - sum_o Y_o^T A_o dc) from the records the
     // assembly kept (A = [J_pose | J_intr] rows and Y = w Jp R^-T of every observation), with
     // FP64 accumulation (recoverReferencePointSteps, BundleAdjustPlaMatrixReferenceSchur.cpp:982-1082).
@@ -607,7 +635,9 @@ __global__ void __launch_bounds__(256) k_back_substitute(Shape S, DevPtrs D, con
     double dd = 0.0, ss = 0.0;
     if (t < S.ntp && D.trk_block[t] >= 0) {
         double u0 = 0.0, u1 = 0.0, u2 = 0.0;
-        for (int o = D.trk_obs_begin[t]; o < D.trk_obs_begin[t + 1]; ++o) {
+        const int oe = D.trk_obs_begin[t + 1];
+#pragma unroll 4
+        for (int o = D.trk_obs_begin[t]; o < oe; ++o) {
             const double* u = terms + static_cast<size_t>(o) * 3;
             u0 += u[0];
             u1 += u[1];
@@ -637,76 +667,73 @@ __global__ void __launch_bounds__(256) k_back_substitute(Shape S, DevPtrs D, con
         step_p[static_cast<size_t>(t) * 3 + 1] = 0.0;
         step_p[static_cast<size_t>(t) * 3 + 2] = 0.0;
     }
-    __shared__ double s_d[8], s_s[8];
+    constexpr int kWarps = kBacksubThreads / 32;
+    __shared__ double s_sum[3][kWarps];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     dd = warp_sum(dd);
     ss = warp_sum(ss);
-    if ((threadIdx.x & 31) == 0) {
-        s_d[threadIdx.x >> 5] = dd;
-        s_s[threadIdx.x >> 5] = ss;
+    if (lane == 0) {
+        s_sum[0][wid] = dd;
+        s_sum[1][wid] = ss;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double a = 0.0, b = 0.0;
-        for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) {
-            a += s_d[w];
-            b += s_s[w];
-        }
-        part[2 * blockIdx.x] = a;
-        part[2 * blockIdx.x + 1] = b;
+    if (threadIdx.x == 0)
+        reinterpret_cast<double2*>(part)[blockIdx.x] =
+            make_double2((s_sum[0][0] + s_sum[0][1]) + (s_sum[0][2] + s_sum[0][3]),
+                         (s_sum[1][0] + s_sum[1][1]) + (s_sum[1][2] + s_sum[1][3]));
+    if (!last_block(ticket, gridDim.x)) return;
+    double sum[3] = {0.0, 0.0, 0.0};
+    const int nblocks = gridDim.x;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < nblocks; i += kBacksubThreads) {
+        const double2 v = __ldcg(reinterpret_cast<const double2*>(part) + i);
+        sum[0] += v.x;
+        sum[1] += v.y;
     }
-}
-
-// Fixed-order sum of block partials (pairs of values) plus the camera-side terms of the
-// directional decrease (dc . direct rhs) and of the step RMS.
-__global__ void k_backsub_final(Shape S, DevPtrs D, const double* __restrict__ part, int nblocks,
-                                const double* __restrict__ step_c, const double* __restrict__ direct64,
-                                double* __restrict__ out) {
-    __shared__ double s_a[256], s_b[256], s_c[256];
-    double a = 0.0, b = 0.0, c = 0.0;
-    for (int i = threadIdx.x; i < nblocks; i += blockDim.x) {
-        a += part[2 * i];
-        b += part[2 * i + 1];
+#pragma unroll 4
+    for (int i = threadIdx.x; i < S.n; i += kBacksubThreads) {
+        const double c = step_c[i];
+        sum[0] = fma(c, direct64[i], sum[0]);
+        sum[2] = fma(c, c, sum[2]);
     }
-    for (int i = threadIdx.x; i < S.n; i += blockDim.x) {
-        a += step_c[i] * direct64[i];
-        c += step_c[i] * step_c[i];
+    for (int i = 0; i < 3; ++i) {
+        const double v = warp_sum(sum[i]);
+        if (lane == 0) s_sum[i][wid] = v;
     }
-    s_a[threadIdx.x] = a;
-    s_b[threadIdx.x] = b;
-    s_c[threadIdx.x] = c;
     __syncthreads();
-    for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-        if (threadIdx.x < st) {
-            s_a[threadIdx.x] += s_a[threadIdx.x + st];
-            s_b[threadIdx.x] += s_b[threadIdx.x + st];
-            s_c[threadIdx.x] += s_c[threadIdx.x + st];
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        out[0] = s_a[0];  // directional decrease
-        out[1] = s_b[0];  // sum of squared point steps
-        out[2] = s_c[0];  // sum of squared camera/intrinsic steps
+    // directional decrease, sum of squared point steps, sum of squared camera and intrinsic steps
+    if (threadIdx.x < 3) {
+        const double* v = s_sum[threadIdx.x];
+        out[threadIdx.x] = (v[0] + v[1]) + (v[2] + v[3]);
     }
 }
+static_assert(kBacksubThreads == 128, "k_back_substitute adds the sums of four warps");
 
-// Accept trial `a`: poses and effective cameras from the trial, groups, points += s(X) alpha dp.
-__global__ void k_accept(Shape S, DevPtrs D, const double* __restrict__ step_p, double alpha, int a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < S.nc) {
-        const double* tr = D.cams_trial + (static_cast<size_t>(a) * S.nc + i) * kCamStride;
-        double* st = D.cams_state + static_cast<size_t>(i) * kCamStride;
-        double* ef = D.cams_eff + static_cast<size_t>(i) * kCamStride;
-        for (int q = 0; q < 12; ++q) st[q] = tr[q];
-        for (int q = 0; q < kCamStride; ++q) ef[q] = tr[q];
-        camera_ff(tr, D.cams_ff + static_cast<size_t>(i) * kCamFF);
+// Accept trial `a`: poses and effective cameras from the trial, groups, points += s(X) alpha dp.  The first
+// blocks take a camera per warp, a lane per value (a thread per camera went through 32 values and 21
+// conversions one after the other: 20 cameras 14.2 -> 5.8 us), the others a point or group value per thread.
+constexpr int kAcceptThreads = 64;
+__global__ void __launch_bounds__(kAcceptThreads) k_accept(Shape S, DevPtrs D, const double* __restrict__ step_p,
+                                                           double alpha, int a) {
+    constexpr int kCams = kAcceptThreads / 32;
+    const int cam_blocks = (S.nc + kCams - 1) / kCams;
+    if (static_cast<int>(blockIdx.x) < cam_blocks) {
+        const int c = blockIdx.x * kCams + (threadIdx.x >> 5), q = threadIdx.x & 31;
+        if (c >= S.nc) return;
+        const double* tr = D.cams_trial + (static_cast<size_t>(a) * S.nc + c) * kCamStride;
+        const double v = tr[q];
+        if (q < 12) D.cams_state[static_cast<size_t>(c) * kCamStride + q] = v;
+        D.cams_eff[static_cast<size_t>(c) * kCamStride + q] = v;
+        if (q < kCamFF) D.cams_ff[static_cast<size_t>(c) * kCamFF + q] = camera_ff_value(q, v);
         // the gauge tangent basis follows the accepted state (referenceGaugeTargetTangentBasis is
         // evaluated on the current cameras, BundleAdjustPlaMatrixAssembly.cpp:69-99, :110, :205);
         // read from the trial records, which this kernel does not write
-        if (i == S.gauge_scale && S.gauge_anchor >= 0 && S.gauge_baseline > 0.0)
+        if (q == 0 && c == S.gauge_scale && S.gauge_anchor >= 0 && S.gauge_baseline > 0.0)
             gauge_basis(D.cams_trial + (static_cast<size_t>(a) * S.nc + S.gauge_anchor) * kCamStride + 9, tr + 9,
                         D.gauge_basis + 6, D.gauge_basis);
+        return;
     }
+    const int i = (blockIdx.x - cam_blocks) * kAcceptThreads + threadIdx.x;
     if (i < S.ng * kGroupRec) D.groups[i] = D.groups_trial[static_cast<size_t>(a) * S.ng * kGroupRec + i];
     if (i < S.ntp && D.trk_free[i]) {
         double* X = D.points + static_cast<size_t>(i) * 3;
@@ -719,6 +746,7 @@ __global__ void k_accept(Shape S, DevPtrs D, const double* __restrict__ step_p, 
         D.pscale_ff[i] = ff_pack(sc);
     }
 }
+static_assert(kCamStride == 32, "a lane per value of a camera record");
 
 // Strict per-track RMS (strictTrackRms, BundleAdjustQuality.cpp:302-364) over the raw observations.
 // `proc_of_track` maps an original track to its processing index (-1: use the initial point).
@@ -864,15 +892,17 @@ void launch_reduce_sums64(const Shape& S, const DevPtrs& D, const AsmOut& O, con
     launch_reduce_sums<double>(S, D, O, R, st);
 }
 
+int backsub_blocks(int ntp) { return std::max(1, (ntp + kBacksubThreads - 1) / kBacksubThreads); }
+
 template <typename T>
 void launch_back_substitute(const Shape& S, const DevPtrs& D, const double* trk_data, const T* obs_rec, const double* step_c,
                             double* step_p, double* step_e, double* terms, double* part, const double* direct64,
-                            double* out, cudaStream_t st) {
-    const int nblk = std::max(1, (S.ntp + 255) / 256);
+                            unsigned* ticket, double* out, cudaStream_t st) {
+    const int nblk = backsub_blocks(S.ntp);
     if (S.nop > 0)
         k_backsub_terms<T><<<static_cast<unsigned>((S.nop + 255) / 256), 256, 0, st>>>(S, D, obs_rec, step_c, terms);
-    k_back_substitute<<<nblk, 256, 0, st>>>(S, D, trk_data, terms, step_p, step_e, part);
-    k_backsub_final<<<1, 256, 0, st>>>(S, D, part, nblk, step_c, direct64, out);
+    k_back_substitute<<<nblk, kBacksubThreads, 0, st>>>(S, D, trk_data, terms, step_p, step_e, part, step_c, direct64,
+                                                        ticket, out);
 }
 
 template <typename T>
@@ -960,23 +990,26 @@ static int cost_blocks(long long nop, int n_alpha) {
 }
 
 void launch_cost(const Shape& S, const DevPtrs& D, const double* step_c, const double* step_p, const Alphas& alphas,
-                 int n_alpha, int use_trial, double* part, double* out, cudaStream_t st, const RigDev* rig) {
+                 int n_alpha, int use_trial, double* part, unsigned* tickets, double* out, cudaStream_t st,
+                 const RigDev* rig) {
     if (use_trial) {
         const int n = n_alpha * S.nc;
-        k_trial_cameras<<<(n + 31) / 32, 32, 0, st>>>(S, D, step_c, alphas, n_alpha);
+        k_trial_cameras<<<(n + kTrialCameras - 1) / kTrialCameras, 32, 0, st>>>(S, D, step_c, alphas, n_alpha);
         // rig cameras: poses composed from the trial captures and sensors
         if (rig) launch_rig_trial(*rig, S.nc, alphas, n_alpha, D.cams_trial, st);
     }
     const int nblk = cost_blocks(S.nop, n_alpha);
     const double c2 = S.loss_scale * S.loss_scale, ic2 = 1.0 / c2;
     const int plain = S.loss != 0 && std::isnormal(c2) && std::isnormal(ic2) ? 1 : 0;
-    k_cost_batch<<<dim3(nblk, n_alpha), kCostThreads, 0, st>>>(S, D, step_p, alphas, use_trial, c2, ic2, plain, part);
-    k_cost_final<<<n_alpha, kCostFinalThreads, 0, st>>>(S, D, part, nblk, use_trial, out);
+    k_cost_batch<<<dim3(nblk, n_alpha), kCostThreads, 0, st>>>(S, D, step_p, alphas, use_trial, c2, ic2, plain, part,
+                                                                tickets, out);
 }
 
 void launch_accept(const Shape& S, const DevPtrs& D, const double* step_p, double alpha, int a, cudaStream_t st) {
-    const int n = std::max(std::max(S.nc, S.ntp), S.ng * kGroupRec);
-    k_accept<<<(n + 63) / 64, 64, 0, st>>>(S, D, step_p, alpha, a);
+    const int cam_blocks = (S.nc + kAcceptThreads / 32 - 1) / (kAcceptThreads / 32);
+    const int n = std::max(S.ntp, S.ng * kGroupRec);
+    const int blocks = cam_blocks + (n + kAcceptThreads - 1) / kAcceptThreads;
+    if (blocks > 0) k_accept<<<blocks, kAcceptThreads, 0, st>>>(S, D, step_p, alpha, a);
 }
 
 void launch_strict_rms(const Shape& S, const DevPtrs& D, const double* cams, const double* init_points,
@@ -1194,9 +1227,9 @@ template void launch_reduce<float>(const Shape&, const DevPtrs&, const AsmOut&, 
 template void launch_reduce<double>(const Shape&, const DevPtrs&, const AsmOut&, const RedOut<double>&, double, double*,
                                     cudaStream_t);
 template void launch_back_substitute<float>(const Shape&, const DevPtrs&, const double*, const float*, const double*,
-                                            double*, double*, double*, double*, const double*, double*, cudaStream_t);
+                                            double*, double*, double*, double*, const double*, unsigned*, double*, cudaStream_t);
 template void launch_back_substitute<double>(const Shape&, const DevPtrs&, const double*, const double*, const double*,
-                                             double*, double*, double*, double*, const double*, double*, cudaStream_t);
+                                             double*, double*, double*, double*, const double*, unsigned*, double*, cudaStream_t);
 template void launch_linearize_export<float>(const Shape&, const DevPtrs&, double*, double*, double*, double*, double*,
                                              double*, signed char*, cudaStream_t);
 template void launch_linearize_export<double>(const Shape&, const DevPtrs&, double*, double*, double*, double*,

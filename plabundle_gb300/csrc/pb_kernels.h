@@ -84,7 +84,8 @@ void launch_gather_obs(long long nop, int ntp, const DevPtrs& D, cudaStream_t st
 template <typename T>
 void launch_back_substitute(const Shape& S, const DevPtrs& D, const double* trk_data, const T* obs_rec, const double* step_c,
                             double* step_p, double* step_e, double* terms, double* part, const double* direct64,
-                            double* out, cudaStream_t st);
+                            unsigned* ticket, double* out, cudaStream_t st);
+int backsub_blocks(int ntp);  // pairs of doubles of `part`
 void launch_points_out(int nt, const int* proc_of_track, const double* points, const double* init, double* out,
                        cudaStream_t st);
 template <typename T>
@@ -166,7 +167,7 @@ void launch_rig_trial(const RigDev& R, int nc, const Alphas& alphas, int n_alpha
 void launch_rig_accept(const RigDev& R, int a, cudaStream_t st);
 
 void launch_cost(const Shape& S, const DevPtrs& D, const double* step_c, const double* step_p, const Alphas& alphas,
-                 int n_alpha, int use_trial, double* part, double* out, cudaStream_t st,
+                 int n_alpha, int use_trial, double* part, unsigned* tickets, double* out, cudaStream_t st,
                  const RigDev* rig = nullptr);
 void launch_accept(const Shape& S, const DevPtrs& D, const double* step_p, double alpha, int a, cudaStream_t st);
 // Scale bars (pb_survey.cu): the extended system of the current state (`flags` bit 2: a promoted

@@ -146,6 +146,7 @@ struct pb_gpu_ctx {
     double* r64 = nullptr;
     double* res_out = nullptr;
     double* bs_part = nullptr;
+    unsigned* tickets = nullptr;  // of the kernels whose last block finishes: the step lengths, the point steps
     double* bs_terms = nullptr;  // per processed observation: its term of the point back-substitution
     double* out_d = nullptr;     // results in the caller's order: points, point steps, rows of the dense system
     double* bs_out = nullptr;    // pinned: directional decrease, sums of squared point and camera steps
@@ -396,8 +397,9 @@ void upload_structure(pb_gpu_ctx* c) {
     c->x64 = A.alloc<double>(n);
     c->r64 = A.alloc<double>(n);
     c->res_out = A.alloc<double>(2 + static_cast<size_t>(std::max(1, (m.ncb + 7) / 8)) * kMaxNB);
-    const int bs_blocks = std::max(1, (ntp + 255) / 256);
-    c->bs_part = A.alloc<double>(2 * static_cast<size_t>(bs_blocks));
+    c->bs_part = A.alloc<double>(2 * static_cast<size_t>(backsub_blocks(ntp)));
+    c->tickets = A.alloc<unsigned>(kMaxAlpha + 1);
+    check(cudaMemsetAsync(c->tickets, 0, (kMaxAlpha + 1) * sizeof(unsigned), st), "memset");
     c->bs_terms = A.alloc<double>(3 * static_cast<size_t>(std::max<long long>(1, nop)));
     c->cost_part = A.alloc<double>(static_cast<size_t>(kCostMaxBlocks) * kMaxAlpha * 2);
     {
@@ -975,12 +977,14 @@ void back_substitute(pb_gpu_ctx* c, double* dd, double* point_sq, double* cam_sq
     if (precision == PB_PRECISION_FP64)
         launch_back_substitute<double>(S, D, static_cast<const double*>(c->p64.out.trk_data_v),
                                        static_cast<const double*>(c->p64.out.obs_rec_v), c->step_c, c->step_p,
-                                       elim ? c->out_d : nullptr, c->bs_terms, c->bs_part, c->direct64, c->bs_out, c->stream);
+                                       elim ? c->out_d : nullptr, c->bs_terms, c->bs_part, c->direct64, c->tickets + kMaxAlpha,
+                                      c->bs_out, c->stream);
     else
         launch_back_substitute<float>(S, D, static_cast<const double*>(c->p32.out.trk_data_v),
                                       static_cast<const float*>(c->p32.out.obs_rec_v), c->step_c, c->step_p,
-                                      elim ? c->out_d : nullptr, c->bs_terms, c->bs_part, c->direct64, c->bs_out, c->stream);
-    c->launches += 3;
+                                      elim ? c->out_d : nullptr, c->bs_terms, c->bs_part, c->direct64, c->tickets + kMaxAlpha,
+                                      c->bs_out, c->stream);
+    c->launches += 2;
     check(cudaGetLastError(), "back-substitution launch");
     ReadBack back(c);
     if (elim) back.add(elim, c->out_d, static_cast<size_t>(3) * c->model.ntb);
@@ -998,9 +1002,9 @@ void eval_costs(pb_gpu_ctx* c, const double* alphas, int n, int use_trial, doubl
     if (use_trial) std::copy(alphas, alphas + n, al.v);
     {
         Timer t(c, 2);
-        launch_cost(S, D, c->step_c, c->step_p, al, n, use_trial, c->cost_part, c->cost_out, c->stream,
+        launch_cost(S, D, c->step_c, c->step_p, al, n, use_trial, c->cost_part, c->tickets, c->cost_out, c->stream,
                     c->rig_on ? &c->rig : nullptr);
-        c->launches += use_trial ? (c->rig_on ? 4 : 3) : 2;
+        c->launches += use_trial ? (c->rig_on ? 3 : 2) : 1;
         if (c->ext_on) {
             launch_bar_cost(S, D, c->step_p, al, n, use_trial, c->bar_d + 1, c->stream);
             c->launches += 1;
