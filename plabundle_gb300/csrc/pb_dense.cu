@@ -1160,9 +1160,8 @@ int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, in
 }
 
 template <typename T>
-int dense_pcg(const PcgSystem<double>& sys, DenseWork<T>& W, const double* b, double rel_tol, double abs_tol,
-              int max_it, int* iterations, double* relres, bool* converged, double* h_scal, cudaStream_t st,
-              int* launches) {
+int dense_pcg_launch(const PcgSystem<double>& sys, DenseWork<T>& W, const double* b, double rel_tol, double abs_tol,
+                     int max_it, double* h_scal, cudaStream_t st, int* launches) {
     if (W.coop_grid == 0) {
         int dev = 0, sms = 0, per_sm = 0;
         cudaGetDevice(&dev);
@@ -1190,20 +1189,36 @@ int dense_pcg(const PcgSystem<double>& sys, DenseWork<T>& W, const double* b, do
         cudaSuccess)
         return -1;
     if (launches) *launches += 1;
-    if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
+    return 0;
+}
+
+int dense_pcg_result(const double* h_scal, int* iterations, double* relres, bool* converged) {
     *iterations = static_cast<int>(h_scal[0]);
     *relres = h_scal[1];
     *converged = h_scal[2] != 0.0;
     // opt-in trace (PB_GPU_TRACE=1): one line per CG launch
     static const bool trace = std::getenv("PB_GPU_TRACE") != nullptr;
     if (trace)
-        std::fprintf(stderr, "PB_GPU_CG precision=%d iterations=%d relres=%.3e converged=%d max_it=%d grid=%d\n",
-                     sizeof(T) == 4 ? 1 : 0, *iterations, *relres, *converged ? 1 : 0, max_it, grid);
+        std::fprintf(stderr, "PB_GPU_CG iterations=%d relres=%.3e converged=%d\n", *iterations, *relres,
+                     *converged ? 1 : 0);
     return h_scal[3] != 0.0 ? 1 : 0;
+}
+
+template <typename T>
+int dense_pcg(const PcgSystem<double>& sys, DenseWork<T>& W, const double* b, double rel_tol, double abs_tol,
+              int max_it, int* iterations, double* relres, bool* converged, double* h_scal, cudaStream_t st,
+              int* launches) {
+    if (dense_pcg_launch<T>(sys, W, b, rel_tol, abs_tol, max_it, h_scal, st, launches) != 0) return -1;
+    if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
+    return dense_pcg_result(h_scal, iterations, relres, converged);
 }
 
 template int dense_factor<float>(const PcgSystem<double>&, DenseWork<float>&, double, int*, cudaStream_t, int*);
 template int dense_factor<double>(const PcgSystem<double>&, DenseWork<double>&, double, int*, cudaStream_t, int*);
+template int dense_pcg_launch<float>(const PcgSystem<double>&, DenseWork<float>&, const double*, double, double, int,
+                                     double*, cudaStream_t, int*);
+template int dense_pcg_launch<double>(const PcgSystem<double>&, DenseWork<double>&, const double*, double, double, int,
+                                      double*, cudaStream_t, int*);
 template int dense_pcg<float>(const PcgSystem<double>&, DenseWork<float>&, const double*, double, double, int, int*,
                               double*, bool*, double*, cudaStream_t, int*);
 template int dense_pcg<double>(const PcgSystem<double>&, DenseWork<double>&, const double*, double, double, int, int*,

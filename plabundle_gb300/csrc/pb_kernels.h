@@ -262,6 +262,11 @@ template <typename T>
 int dense_pcg(const PcgSystem<double>& sys, DenseWork<T>& W, const double* b, double rel_tol, double abs_tol,
               int max_it, int* iterations, double* relres, bool* converged, double* h_scal, cudaStream_t st,
               int* launches);
+// The same in two halves: the launch, and its scalars once the stream has been waited for.
+template <typename T>
+int dense_pcg_launch(const PcgSystem<double>& sys, DenseWork<T>& W, const double* b, double rel_tol, double abs_tol,
+                     int max_it, double* h_scal, cudaStream_t st, int* launches);
+int dense_pcg_result(const double* h_scal, int* iterations, double* relres, bool* converged);
 
 // Backward pass (pb_adjoint.cu).  Per-observation record of the exact Hessian in the local chart
 // (pose 6 | point 3 | intrinsic columns ni): pose-pose (upper 6x6), pose-point (6x3), point-point
