@@ -528,7 +528,7 @@ pb_status pb_gpu_solve_damped_schur(pb_gpu_ctx* ctx, const pb_bne* equations, do
  *     is kept for the life of the process, so the call must not be used across a
  *     cudaDeviceReset of that device;
  *   - work is enqueued on `stream` (a cudaStream_t, NULL for the legacy default stream); the call
- *     copies its three totals back and synchronises `stream` before it returns;
+ *     brings its three totals back and synchronises `stream` before it returns;
  *   - an error already pending on the calling thread (cudaPeekAtLastError) is left in place and
  *     the call returns PB_ERR_CUDA without launching. */
 #define PB_NOALLOC_MAX_OBS 4194304
