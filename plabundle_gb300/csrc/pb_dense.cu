@@ -346,9 +346,8 @@ __device__ __forceinline__ void tile_product_store(T* __restrict__ C, int ldc, c
 }
 
 // Barrier between the phases of a cooperative kernel: of the whole grid, or, for grids of at most sixteen
-// blocks, which one cluster holds, of the cluster (114 unknowns: CG solve 53.5 -> 45.0 us, FP32 factor 94 ->
-// 90, FP64 factor 145 -> 139).  Larger systems keep their blocks: 354 unknowns on sixteen blocks took 135 us a
-// solve against 121 on 45.  Either barrier orders the blocks' writes to global memory.
+// blocks, which one cluster holds, of the cluster (114 unknowns: FP32 factor 94 -> 90 us, FP64 factor 145 ->
+// 139).  Either barrier orders the blocks' writes to global memory.
 constexpr int kClusterMax = 16;
 template <bool CLUSTER>
 __device__ __forceinline__ void phase_barrier() {
@@ -941,7 +940,7 @@ __device__ __forceinline__ double spmv_update(const PcgSystem<double>& sys, cons
 }
 
 // out: [0] iterations, [1] relative residual, [2] converged, [3] status (1: breakdown)
-template <typename T, bool CLUSTER>
+template <typename T>
 __global__ void __launch_bounds__(kCgThreads, 2) k_dense_cg(PcgSystem<double> sys, const T* __restrict__ X,
                                                          const T* __restrict__ XT, int np,
                                                          const double* __restrict__ dscale,
@@ -967,11 +966,11 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_dense_cg(PcgSystem<double> sy
         bb += b[i] * b[i];
     }
     block_partial(bb, s_vals, s_q, mypart + 0);
-    phase_barrier<CLUSTER>();
+    phase_barrier<false>();
     tri_rows<T, true>(X, np, n, u, w, nullptr, nullptr, nullptr);
-    phase_barrier<CLUSTER>();
+    phase_barrier<false>();
     block_partial(tri_rows<T, false>(XT, np, n, w, nullptr, z, dscale, b), s_vals, s_q, mypart + 1);
-    phase_barrier<CLUSTER>();
+    phase_barrier<false>();
     grid_totals<true>(part, 0, s_q, s_tot);
     const double bnorm = sqrt(s_tot[0]);
     double rz = s_tot[1];
@@ -989,7 +988,7 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_dense_cg(PcgSystem<double> sy
             p_cur = t;
         }
         block_partial(spmv_update(sys, z, beta, p_old, p_cur, qpart, pose_seg, border_seg), s_vals, s_q, mypart + 2);
-        phase_barrier<CLUSTER>();
+        phase_barrier<false>();
         grid_totals<false>(part, 2, s_q, s_tot);
         const double pq = s_tot[2];
         if (!(pq > 0.0) || !isfinite(pq) || !isfinite(rz)) {
@@ -1018,7 +1017,7 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_dense_cg(PcgSystem<double> sy
             rr += rv * rv;
         }
         block_partial(rr, s_vals, s_q, mypart + 0);
-        phase_barrier<CLUSTER>();
+        phase_barrier<false>();
         ++it;
         grid_totals<false>(part, 0, s_q, s_tot);
         rn = sqrt(s_tot[0]);
@@ -1031,9 +1030,9 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_dense_cg(PcgSystem<double> sy
             break;
         }
         tri_rows<T, true>(X, np, n, u, w, nullptr, nullptr, nullptr);
-        phase_barrier<CLUSTER>();
+        phase_barrier<false>();
         block_partial(tri_rows<T, false>(XT, np, n, w, nullptr, z, dscale, r), s_vals, s_q, mypart + 1);
-        phase_barrier<CLUSTER>();
+        phase_barrier<false>();
         grid_totals<false>(part, 1, s_q, s_tot);
         const double rz_new = s_tot[1];
         beta = rz_new / rz;
@@ -1044,6 +1043,213 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_dense_cg(PcgSystem<double> sy
         out[1] = bnorm > 0.0 ? rn / bnorm : 0.0;
         out[2] = converged ? 1.0 : 0.0;
         out[3] = status;
+    }
+}
+
+// The same iteration for systems of at most kCgClusterDim unknowns, on one cluster whose blocks all keep the
+// whole vectors in shared memory: a row's value goes from its warp to every block's copy, and what is not a
+// matrix product (the scalars, x, r, p and u) is done by every block for itself, the same bits in each, so
+// that an iteration takes three cluster barriers instead of four grid barriers and no vector or partial sum
+// goes through L2 between them (a solve of two iterations, call included: 114 unknowns 67 -> 52 us, 234
+// unknowns 69 -> 59, 380 unknowns 70 -> 67; 504 unknowns 74 on the grid against 88 here, sixteen blocks
+// being too few for the FP64 products, and without pose blocks 312 unknowns 642 against 637, 364 unknowns
+// 713 against 717 for a whole call).  An SpMV item is seg_blocks blocks of a block row, eight
+// blocks by three pairs of rows at a time over 24 lanes (twelve FP64 products a turn), or 256 entries of a
+// border row.  The matrices are read through L1, where a small system's shares stay.
+constexpr int kCgClusterDim = 384, kCgClusterDimBorder = 320;
+constexpr size_t kCgClusterSmem = 48 * 1024;
+struct CgClusterShape {
+    int seg_blocks, pose_seg, border_seg, items;  // items: sums of the SpMV items, 6 ncb pose_seg + nb border_seg
+};
+template <typename T>
+__host__ __device__ constexpr size_t cg_cluster_smem(int n, int np, int items) {
+    // u and w (padded, 16-byte rows), then r, z, p, scale, x, the item sums and the reduction's words
+    return 2 * static_cast<size_t>(np) * sizeof(T) + (5 * static_cast<size_t>(n) + items + 8) * sizeof(double);
+}
+
+// Sum over the first four warps (one per sub-partition), the same in every thread.
+__device__ __forceinline__ double four_warp_total(double v, double* s_red) {
+    const int warp = threadIdx.x >> 5;
+    __syncthreads();
+    if (warp < 4) {
+        v = warp_sum(v);
+        if ((threadIdx.x & 31) == 0) s_red[warp] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) s_red[4] = (s_red[0] + s_red[1]) + (s_red[2] + s_red[3]);
+    __syncthreads();
+    return s_red[4];
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kCgThreads) k_dense_cg_cluster(PcgSystem<double> sys, const T* __restrict__ X,
+                                                                 const T* __restrict__ XT, int np,
+                                                                 const double* __restrict__ dscale,
+                                                                 const double* __restrict__ b, double* __restrict__ x,
+                                                                 CgClusterShape shape, double* __restrict__ out,
+                                                                 double rel_tol, double abs_tol, int max_it) {
+    extern __shared__ __align__(16) unsigned char s_cg[];
+    using V = Vec16<T>;
+    using VV = typename V::type;
+    const cgk::cluster_group cluster = cgk::this_cluster();
+    const int n6 = 6 * sys.ncb, nb = sys.nb, n = n6 + nb;
+    const int tid = threadIdx.x, lane = tid & 31, C = gridDim.x;
+    const int gw = (tid >> 5) * C + blockIdx.x, nw = C * kCgWarps;  // consecutive rows go to different SMs
+    T* u = reinterpret_cast<T*>(s_cg);
+    T* w = u + np;
+    double* r = reinterpret_cast<double*>(w + np);
+    double* z = r + n;
+    double* p = z + n;
+    double* ds = p + n;
+    double* xs = ds + n;
+    double* q = xs + n;
+    double* s_red = q + shape.items;
+    double bb = 0.0;
+    for (int i = tid; i < np; i += kCgThreads) {
+        const double bi = i < n ? b[i] : 0.0, di = i < n ? dscale[i] : 0.0;
+        u[i] = static_cast<T>(di * bi);
+        w[i] = T(0);
+        if (i < n) {
+            r[i] = bi;
+            ds[i] = di;
+            p[i] = 0.0;
+            xs[i] = 0.0;
+        }
+    }
+    cluster.sync();
+    if (tid < 128)
+        for (int i = tid; i < n; i += 128) bb = fma(r[i], r[i], bb);
+    const double bnorm = sqrt(four_warp_total(bb, s_red));
+    const double tol = fmax(rel_tol * bnorm, abs_tol);
+    double rn = bnorm, rz = 0.0;
+    int it = 0, status = 0;
+    bool converged = rn <= tol;
+    T* w_to = lane < C ? cluster.map_shared_rank(w, lane) : nullptr;
+    double* z_to = lane < C ? cluster.map_shared_rank(z, lane) : nullptr;
+    double* q_to = lane < C ? cluster.map_shared_rank(q, lane) : nullptr;
+    while (!converged && it < max_it) {
+        // w = X u, z = D X^T w
+        for (int i = gw; i < n; i += nw) {
+            const VV* row = reinterpret_cast<const VV*>(X + static_cast<size_t>(i) * np);
+            const int q1 = (i + V::n) / V::n;
+            T acc = T(0);
+#pragma unroll 4
+            for (int k = lane; k < q1; k += 32) acc += V::dot(row[k], reinterpret_cast<const VV*>(u)[k]);
+            acc = warp_sum(acc);
+            if (w_to) w_to[i] = acc;
+        }
+        cluster.sync();
+        for (int i = gw; i < n; i += nw) {
+            const VV* row = reinterpret_cast<const VV*>(XT + static_cast<size_t>(i) * np);
+            const int q1 = (n + V::n - 1) / V::n;
+            T acc = T(0);
+#pragma unroll 4
+            for (int k = i / V::n + lane; k < q1; k += 32) acc += V::dot(row[k], reinterpret_cast<const VV*>(w)[k]);
+            acc = warp_sum(acc);
+            if (z_to) z_to[i] = static_cast<double>(acc) * ds[i];
+        }
+        cluster.sync();
+        double part = 0.0;
+        if (tid < 128)
+            for (int i = tid; i < n; i += 128) part = fma(r[i], z[i], part);
+        const double rz_new = four_warp_total(part, s_red);
+        const double beta = it == 0 ? 0.0 : rz_new / rz;
+        rz = rz_new;
+        if (tid < 128)
+            for (int i = tid; i < n; i += 128) p[i] = it == 0 ? z[i] : fma(beta, p[i], z[i]);
+        __syncthreads();
+        // item sums of S p
+        const int npose = sys.ncb * shape.pose_seg, nitems = npose + nb * shape.border_seg;
+        for (int t = gw; t < nitems; t += nw) {
+            if (t < npose) {
+                const int br = t / shape.pose_seg, sg = t - br * shape.pose_seg;
+                const int e0 = sys.row_ptr[br] + shape.seg_blocks * sg, e1 = min(sys.row_ptr[br + 1], e0 + shape.seg_blocks);
+                const int blk = lane >> 2, rows = lane & 3;
+                double a0 = 0.0, a1 = 0.0;
+                if (rows < 3) {
+                    for (int e = e0 + blk; e < e1; e += 8) {
+                        const double* pj = p + 6 * sys.col_idx[e];
+                        const double2* A = reinterpret_cast<const double2*>(sys.vals + static_cast<size_t>(e) * 36 + 12 * rows);
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) {
+                            const double2 m0 = A[c], m1 = A[3 + c];
+                            a0 = fma(m0.x, pj[2 * c], a0);
+                            a1 = fma(m1.x, pj[2 * c], a1);
+                            a0 = fma(m0.y, pj[2 * c + 1], a0);
+                            a1 = fma(m1.y, pj[2 * c + 1], a1);
+                        }
+                    }
+                    if (sg == 0) {
+                        const double* Bi = sys.border + static_cast<size_t>(6 * br + 2 * rows) * nb;
+                        for (int c = blk; c < nb; c += 8) {
+                            a0 = fma(Bi[c], p[n6 + c], a0);
+                            a1 = fma(Bi[nb + c], p[n6 + c], a1);
+                        }
+                    }
+                }
+                const bool up = lane & 16;
+                double v = (up ? a1 : a0) + __shfl_xor_sync(0xffffffffu, up ? a0 : a1, 16);
+                v += __shfl_xor_sync(0xffffffffu, v, 8);
+                v += __shfl_xor_sync(0xffffffffu, v, 4);
+                // the four lanes that hold a row's sum hand it to every fourth block
+                if (rows < 3)
+                    for (int k = blk & 3; k < C; k += 4) cluster.map_shared_rank(q, k)[6 * t + 2 * rows + (up ? 1 : 0)] = v;
+            } else {
+                const int k = t - npose, c = k / shape.border_seg, sg = k - c * shape.border_seg;
+                const double* Bc = sys.border_t + static_cast<size_t>(c) * n6;
+                const double* Cc = sys.Cm + static_cast<size_t>(c) * nb;
+                const int k1 = min(n, 256 * (sg + 1));
+                double v = 0.0;
+#pragma unroll 4
+                for (int j = 256 * sg + lane; j < k1; j += 32) v = fma(j < n6 ? Bc[j] : Cc[j - n6], p[j], v);
+                v = warp_sum(v);
+                if (q_to) q_to[6 * npose + k] = v;
+            }
+        }
+        cluster.sync();
+        // q from its items, p.q, and the updates
+        part = 0.0;
+        if (tid < 128)
+            for (int i = tid; i < n; i += 128) {
+                const double* qs = i < n6 ? q + 6 * (i / 6) * shape.pose_seg + i % 6 : q + 6 * npose + (i - n6) * shape.border_seg;
+                const int step = i < n6 ? 6 : 1, m = i < n6 ? shape.pose_seg : shape.border_seg;
+                double qi = qs[0];
+                for (int sg = 1; sg < m; ++sg) qi += qs[step * sg];
+                z[i] = qi;  // (z is free until the next product)
+                part = fma(p[i], qi, part);
+            }
+        const double pq = four_warp_total(part, s_red);
+        if (!(pq > 0.0) || !isfinite(pq) || !isfinite(rz)) {
+            status = 1;
+            break;
+        }
+        const double alpha = rz / pq;
+        part = 0.0;
+        if (tid < 128)
+            for (int i = tid; i < n; i += 128) {
+                xs[i] = fma(alpha, p[i], xs[i]);
+                const double rv = fma(-alpha, z[i], r[i]);
+                r[i] = rv;
+                u[i] = static_cast<T>(ds[i] * rv);
+                part = fma(rv, rv, part);
+            }
+        rn = sqrt(four_warp_total(part, s_red));
+        ++it;
+        if (!isfinite(rn)) {
+            status = 1;
+            break;
+        }
+        converged = rn <= tol;
+    }
+    if (blockIdx.x == 0) {
+        __syncthreads();
+        for (int i = tid; i < n; i += kCgThreads) x[i] = xs[i];
+        if (tid == 0) {
+            out[0] = it;
+            out[1] = bnorm > 0.0 ? rn / bnorm : 0.0;
+            out[2] = converged ? 1.0 : 0.0;
+            out[3] = status;
+        }
     }
 }
 
@@ -1166,13 +1372,34 @@ int dense_pcg_launch(const PcgSystem<double>& sys, DenseWork<T>& W, const double
         int dev = 0, sms = 0, per_sm = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dense_cg<T, false>, kCgThreads, 0);
-        W.cg_cluster = largest_cluster(reinterpret_cast<const void*>(&k_dense_cg<T, true>), kCgThreads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dense_cg<T>, kCgThreads, 0);
+        W.cg_cluster = largest_cluster(reinterpret_cast<const void*>(&k_dense_cg_cluster<T>), kCgThreads, kCgClusterSmem);
         W.coop_grid = std::max(1, std::min(per_sm, 2) * sms);
     }
     // one warp per row of the triangular products: small systems (local windows) take a small
     // grid and leave the rest of the device to concurrent work
     const int rows = (W.n + kCgWarps - 1) / kCgWarps;
+    // items of eight blocks each until every warp of the cluster has one, then longer ones
+    CgClusterShape shape{};
+    {
+        const int warps = kClusterMax * kCgWarps;
+        shape.seg_blocks = 8 * std::max(1, (sys.ncb * ((W.longest + 7) / 8) + warps - 1) / warps);
+        shape.pose_seg = sys.ncb > 0 ? std::max(1, (W.longest + shape.seg_blocks - 1) / shape.seg_blocks) : 0;
+        shape.border_seg = W.border_seg;
+        shape.items = 6 * sys.ncb * shape.pose_seg + sys.nb * shape.border_seg;
+    }
+    const size_t smem = cg_cluster_smem<T>(W.n, W.np, shape.items);
+    if (W.cg_cluster == kClusterMax && W.n <= (sys.ncb > 0 ? kCgClusterDim : kCgClusterDimBorder) && smem <= kCgClusterSmem) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at;
+        cluster_config(cfg, at, std::max(1, std::min(kClusterMax, rows)), kCgThreads, smem, st);
+        if (cudaLaunchKernelEx(&cfg, &k_dense_cg_cluster<T>, sys, static_cast<const T*>(W.X), static_cast<const T*>(W.A),
+                               W.np, static_cast<const double*>(W.dscale), b, W.x, shape, h_scal, rel_tol, abs_tol,
+                               max_it) != cudaSuccess)
+            return -1;
+        if (launches) *launches += 1;
+        return 0;
+    }
     const int grid = std::max(1, std::min(W.coop_grid, rows));
     PcgSystem<double> s = sys;
     const T* X = W.X;
@@ -1184,9 +1411,8 @@ int dense_pcg_launch(const PcgSystem<double>& sys, DenseWork<T>& W, const double
     int ps = W.pose_seg, bs = W.border_seg;
     void* args[] = {&s, &X, &XT, &np, &dscale, &b, &W.x, &W.r, &W.z, &W.p, &W.w, &W.qpart, &ps, &bs, &W.ut, &W.wt,
                     &W.part, &h_scal, &rt, &at, &mi};
-    if (launch_phased(reinterpret_cast<const void*>(&k_dense_cg<T, false>),
-                      reinterpret_cast<const void*>(&k_dense_cg<T, true>), W.cg_cluster, grid, kCgThreads, args, 0, st) !=
-        cudaSuccess)
+    if (cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&k_dense_cg<T>), dim3(grid), dim3(kCgThreads), args, 0,
+                                    st) != cudaSuccess)
         return -1;
     if (launches) *launches += 1;
     return 0;

@@ -240,6 +240,7 @@ struct DenseWork {
     // SpMV work items of the CG: pose_seg per pose block row (32 blocks each), border_seg per border
     // row (256 entries each); qpart holds their sums (6 ncb pose_seg + nb border_seg doubles)
     int pose_seg = 0, border_seg = 0;
+    int longest = 0;  // blocks of the longest pose block row
     double* qpart = nullptr;
     T *ut = nullptr, *wt = nullptr;  // scaled residual and X D r in the factor's type
     double* part = nullptr;  // per-block partials of the cooperative CG (grid * 4)

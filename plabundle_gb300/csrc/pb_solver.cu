@@ -768,6 +768,7 @@ void ensure_dense(pb_gpu_ctx* c) {
         // items per row), 256 entries of a border row per item
         int longest = 0;
         for (int r = 0; r < npose; ++r) longest = std::max(longest, prow[r + 1] - prow[r]);
+        W.longest = longest;
         W.pose_seg = npose > 0 ? std::max(1, (longest + 31) / 32) : 0;
         W.border_seg = nbsol > 0 ? (nsol + 255) / 256 : 0;
         W.qpart = A.alloc<double>(std::max<size_t>(1, 6 * static_cast<size_t>(npose) * W.pose_seg +
