@@ -65,30 +65,34 @@ __device__ void rig_trial_record(const double* __restrict__ state, int block, co
     }
 }
 
-__global__ void k_rig_maps(RigDev R) {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
+// Chain maps of camera block a: Mc = [I 0; -[L]x I] for its capture, Ms = diag(R, R) for its sensor, with
+// L = R c_sensor and R the capture's rotation.  A warp per camera block, a lane per entry (a thread per
+// block wrote 144 scattered values: 150 cameras 11.2 -> 4.0 us).
+__global__ void __launch_bounds__(64) k_rig_maps(RigDev R) {
+    const int a = blockIdx.x * 2 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (a >= R.ncb) return;
     const int c = R.cb_camera[a];
     const double* cp = R.cap_state + static_cast<size_t>(R.cam_capture[c]) * 12;
     const double* sp = R.sen_state + static_cast<size_t>(R.cam_sensor[c]) * 12;
     double L[3];
     for (int r = 0; r < 3; ++r) L[r] = cp[r * 3] * sp[9] + cp[r * 3 + 1] * sp[10] + cp[r * 3 + 2] * sp[11];
-    double* Mc = R.maps + static_cast<size_t>(a) * 72;
-    double* Ms = Mc + 36;
-    for (int i = 0; i < 36; ++i) Mc[i] = Ms[i] = 0.0;
-    for (int i = 0; i < 6; ++i) Mc[i * 7] = 1.0;
-    // rows 3-5, columns 0-2: -[L]x (column a is e_a x L)
-    Mc[3 * 6 + 1] = L[2];
-    Mc[3 * 6 + 2] = -L[1];
-    Mc[4 * 6 + 0] = -L[2];
-    Mc[4 * 6 + 2] = L[0];
-    Mc[5 * 6 + 0] = L[1];
-    Mc[5 * 6 + 1] = -L[0];
-    for (int r = 0; r < 3; ++r)
-        for (int q = 0; q < 3; ++q) {
-            Ms[r * 6 + q] = cp[r * 3 + q];
-            Ms[(3 + r) * 6 + 3 + q] = cp[r * 3 + q];
+    double* M = R.maps + static_cast<size_t>(a) * 72;
+    for (int e = lane; e < 72; e += 32) {
+        const int k = e % 36, r = k / 6, q = k - 6 * r;
+        double v = 0.0;
+        if (e < 36) {
+            if (r == q) v = 1.0;
+            // rows 3-5, columns 0-2: -[L]x (column a is e_a x L)
+            if (r >= 3 && q < 3 && r - 3 != q) {
+                const int o = 3 - (r - 3) - q;  // the axis that is neither
+                const double l = o == 0 ? L[0] : o == 1 ? L[1] : L[2];
+                v = (r - 3 + 1) % 3 == q ? l : -l;
+            }
+        } else if (r / 3 == q / 3) {
+            v = cp[(r % 3) * 3 + q % 3];
         }
+        M[e] = v;
+    }
 }
 
 // Pose blocks, first pass: one warp per segment of at most rig_seg_terms terms of one upper rig block.
@@ -257,33 +261,49 @@ __global__ void k_rig_step_sq(RigDev R, const double* __restrict__ xr, int n) {
     if (threadIdx.x == 0) R.sq[0] = s[0];
 }
 
-__global__ void k_rig_trial(RigDev R, int nc, Alphas alphas, int n_alpha,
-                            double* __restrict__ cams_trial) {
+// Trial captures, sensors and cameras.  Two lanes per record: of a camera the first moves its capture and
+// the second its sensor, in the same instructions (the FP64 pipe takes 64 cycles for a warp however few
+// lanes run), then the first composes them (150 cameras, two step lengths: 19.1 -> 10.9 us).
+constexpr int kRigTrialThreads = 64;
+__global__ void __launch_bounds__(kRigTrialThreads) k_rig_trial(RigDev R, int nc, Alphas alphas, int n_alpha,
+                                                                double* __restrict__ cams_trial) {
     const int per = R.ncap + R.nsen + nc;
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= per * n_alpha) return;
-    const int a = idx / per, i = idx - a * per;
-    const double alpha = alphas.v[a];
-    if (i < R.ncap) {
-        rig_trial_record(R.cap_state + static_cast<size_t>(i) * 12, R.capture_block[i], R.step_r, alpha,
-                         R.cap_trial + (static_cast<size_t>(a) * R.ncap + i) * 12);
-    } else if (i < R.ncap + R.nsen) {
-        const int s = i - R.ncap;
-        rig_trial_record(R.sen_state + static_cast<size_t>(s) * 12, R.sensor_block[s], R.step_r, alpha,
-                         R.sen_trial + (static_cast<size_t>(a) * R.nsen + s) * 12);
-    } else {
+    const int t = blockIdx.x * kRigTrialThreads + threadIdx.x, idx = t >> 1;
+    const bool second = t & 1, live = idx < per * n_alpha;
+    const int a = live ? idx / per : 0, i = live ? idx - a * per : 0;
+    const bool camera = live && i >= R.ncap + R.nsen;
+    int cap = -1, sen = -1;
+    if (camera) {
         const int c = i - R.ncap - R.nsen;
-        const int k = R.cam_capture[c], s = R.cam_sensor[c];
-        double cp[12], sp[12];
-        rig_trial_record(R.cap_state + static_cast<size_t>(k) * 12, R.capture_block[k], R.step_r, alpha, cp);
-        rig_trial_record(R.sen_state + static_cast<size_t>(s) * 12, R.sensor_block[s], R.step_r, alpha, sp);
+        if (second) sen = R.cam_sensor[c];
+        else cap = R.cam_capture[c];
+    } else if (live && !second) {
+        if (i < R.ncap) cap = i;
+        else sen = i - R.ncap;
+    }
+    double rec[12];
+    if (cap >= 0 || sen >= 0)
+        rig_trial_record(cap >= 0 ? R.cap_state + static_cast<size_t>(cap) * 12 : R.sen_state + static_cast<size_t>(sen) * 12,
+                         cap >= 0 ? R.capture_block[cap] : R.sensor_block[sen], R.step_r, alphas.v[a], rec);
+    else
+        for (int k = 0; k < 12; ++k) rec[k] = 0.0;
+    double sp[12];
+    for (int k = 0; k < 12; ++k) sp[k] = __shfl_down_sync(0xffffffffu, rec[k], 1);
+    if (!live || second) return;
+    if (camera) {
+        const int c = i - R.ncap - R.nsen;
+        const double* cp = rec;
         double* out = cams_trial + (static_cast<size_t>(a) * nc + c) * kCamStride;
         for (int r = 0; r < 3; ++r)
             for (int q = 0; q < 3; ++q)
                 out[r * 3 + q] = cp[r * 3] * sp[q] + cp[r * 3 + 1] * sp[3 + q] + cp[r * 3 + 2] * sp[6 + q];
         for (int r = 0; r < 3; ++r)
             out[9 + r] = cp[9 + r] + cp[r * 3] * sp[9] + cp[r * 3 + 1] * sp[10] + cp[r * 3 + 2] * sp[11];
+        return;
     }
+    double* out = cap >= 0 ? R.cap_trial + (static_cast<size_t>(a) * R.ncap + cap) * 12
+                           : R.sen_trial + (static_cast<size_t>(a) * R.nsen + sen) * 12;
+    for (int k = 0; k < 12; ++k) out[k] = rec[k];
 }
 
 __global__ void k_rig_accept(RigDev R, int a) {
@@ -295,7 +315,7 @@ __global__ void k_rig_accept(RigDev R, int a) {
 }  // namespace
 
 void launch_rig_maps(const RigDev& R, cudaStream_t st) {
-    if (R.ncb > 0) k_rig_maps<<<(R.ncb + 127) / 128, 128, 0, st>>>(R);
+    if (R.ncb > 0) k_rig_maps<<<(R.ncb + 1) / 2, 64, 0, st>>>(R);
 }
 
 void launch_rig_transform(const RigDev& R, const double* vals, const double* border, const double* rhs, int nbw,
@@ -315,8 +335,8 @@ void launch_rig_expand(const RigDev& R, const double* xr, int nbw, int nglob, cu
 }
 
 void launch_rig_trial(const RigDev& R, int nc, const Alphas& alphas, int n_alpha, double* cams_trial, cudaStream_t st) {
-    const int n = (R.ncap + R.nsen + nc) * n_alpha;
-    k_rig_trial<<<(n + 127) / 128, 128, 0, st>>>(R, nc, alphas, n_alpha, cams_trial);
+    const int n = 2 * (R.ncap + R.nsen + nc) * n_alpha;
+    k_rig_trial<<<(n + kRigTrialThreads - 1) / kRigTrialThreads, kRigTrialThreads, 0, st>>>(R, nc, alphas, n_alpha, cams_trial);
 }
 
 void launch_rig_accept(const RigDev& R, int a, cudaStream_t st) {

@@ -257,35 +257,44 @@ __global__ void k_ext_step(Shape S, DevPtrs D, const double* __restrict__ xsol, 
 
 // Scale-bar cost of each trial state (points + alpha step for the points that move) or of the
 // current state, one thread per step length, bars in order.
-__global__ void k_bar_cost(Shape S, DevPtrs D, const double* __restrict__ step_p, Alphas alphas, int n_alpha,
-                           int use_trial, double* __restrict__ out) {
-    const int a = threadIdx.x;
-    if (a >= n_alpha) return;
+// A warp per step length: the lanes evaluate the bars, whose costs are added in order (a thread per step
+// length took the bars' latencies one after the other: four bars 11.5 -> 6.6 us).
+__global__ void __launch_bounds__(32) k_bar_cost(Shape S, DevPtrs D, const double* __restrict__ step_p, Alphas alphas,
+                                                 int use_trial, double* __restrict__ out) {
+    const int a = blockIdx.x, lane = threadIdx.x;
     const double alpha = use_trial ? alphas.v[a] : 0.0;
     double cost = 0.0;
-    for (int i = 0; i < S.nbar; ++i) {
-        const int ta = D.bar_pidx[2 * i], tb = D.bar_pidx[2 * i + 1];
-        if (ta < 0 || tb < 0) continue;
-        double Xa[3], Xb[3];
-        for (int p = 0; p < 3; ++p) {
-            Xa[p] = D.points[static_cast<size_t>(ta) * 3 + p];
-            Xb[p] = D.points[static_cast<size_t>(tb) * 3 + p];
-        }
-        if (use_trial) {
-            if (D.trk_free[ta]) {
-                const double f = D.pscale[ta] * alpha;
-                for (int p = 0; p < 3; ++p) Xa[p] += f * step_p[static_cast<size_t>(ta) * 3 + p];
+    for (int i0 = 0; i0 < S.nbar; i0 += 32) {
+        const int i = i0 + lane, m = min(32, S.nbar - i0);
+        double cc = 0.0;
+        bool ok = false;
+        const int ta = lane < m ? D.bar_pidx[2 * i] : -1, tb = lane < m ? D.bar_pidx[2 * i + 1] : -1;
+        if (ta >= 0 && tb >= 0) {
+            double Xa[3], Xb[3];
+            for (int p = 0; p < 3; ++p) {
+                Xa[p] = D.points[static_cast<size_t>(ta) * 3 + p];
+                Xb[p] = D.points[static_cast<size_t>(tb) * 3 + p];
             }
-            if (D.trk_free[tb]) {
-                const double f = D.pscale[tb] * alpha;
-                for (int p = 0; p < 3; ++p) Xb[p] += f * step_p[static_cast<size_t>(tb) * 3 + p];
+            if (use_trial) {
+                if (D.trk_free[ta]) {
+                    const double f = D.pscale[ta] * alpha;
+                    for (int p = 0; p < 3; ++p) Xa[p] += f * step_p[static_cast<size_t>(ta) * 3 + p];
+                }
+                if (D.trk_free[tb]) {
+                    const double f = D.pscale[tb] * alpha;
+                    for (int p = 0; p < 3; ++p) Xb[p] += f * step_p[static_cast<size_t>(tb) * 3 + p];
+                }
             }
+            double r, J[3], w;
+            ok = bar_eval(Xa, Xb, D.bar_par[2 * i], D.bar_par[2 * i + 1], S.bar_huber, r, J, cc, w);
         }
-        double r, J[3], cc, w;
-        if (!bar_eval(Xa, Xb, D.bar_par[2 * i], D.bar_par[2 * i + 1], S.bar_huber, r, J, cc, w)) continue;
-        cost += cc;
+        const unsigned valid = __ballot_sync(0xffffffffu, ok);
+        for (int l = 0; l < m; ++l) {
+            const double c = __shfl_sync(0xffffffffu, cc, l);
+            if ((valid >> l) & 1u) cost += c;
+        }
     }
-    out[a] = cost;
+    if (lane == 0) out[a] = cost;
 }
 
 void launch_extend_system(const Shape& S, const DevPtrs& D, const RedOut<double>& R, const ExtSys& X, double damping,
@@ -303,7 +312,7 @@ void launch_ext_step(const Shape& S, const DevPtrs& D, const double* xsol, doubl
 
 void launch_bar_cost(const Shape& S, const DevPtrs& D, const double* step_p, const Alphas& alphas, int n_alpha,
                      int use_trial, double* out, cudaStream_t st) {
-    k_bar_cost<<<1, 32, 0, st>>>(S, D, step_p, alphas, n_alpha, use_trial, out);
+    k_bar_cost<<<n_alpha, 32, 0, st>>>(S, D, step_p, alphas, use_trial, out);
 }
 
 }  // namespace pb
