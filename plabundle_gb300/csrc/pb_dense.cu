@@ -454,8 +454,25 @@ __global__ void __launch_bounds__(256) k_potrf_coop(T* __restrict__ A, T* __rest
 namespace {
 constexpr int TD = 32, TDP = TD + 1;
 constexpr int kPotrf64Threads = 256;
-constexpr size_t kPotrf64Smem = (3 * static_cast<size_t>(TD) * TDP + TD * 9 + 3 * TD) * sizeof(double);
+constexpr size_t kPotrf64Smem = (4 * static_cast<size_t>(TD) * TDP + TD * 9 + 3 * TD) * sizeof(double);
 }  // namespace
+
+constexpr int kPanel = 4;
+
+// Pivot test on the integer pipe (an FP64 comparison and its predicate take about 100 cycles): the exponent
+// of a positive d in (-1000, 1000).
+__device__ __forceinline__ bool plain_pivot(double d) { return (hi_word(d) >> 20) - 24u <= 1998u; }
+// (out of line: not on the way of the ordinary pivots)
+__device__ __noinline__ double other_quotient(double a, double d) { return d > 0.0 ? a / d : 0.0; }
+__device__ __noinline__ double other_sqrt(double d) { return d > 0.0 ? sqrt(d) : 1.0; }
+// a / d for a plain pivot: x0 = 1 / d to 20 bits, e = 1 - d x0, and a (x0 (1 + e + e^2)), whose remainder e^3
+// is below the rounding.
+__device__ __forceinline__ double plain_quotient(double a, double d) {
+    double x0;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x0) : "d"(d));
+    const double e = fma(-d, x0, 1.0);
+    return a * fma(x0, fma(e, e, e), x0);
+}
 
 // Inverse of the 8 x 8 diagonal block b of the tile's factor from its unscaled columns, by one warp
 // (lane c < 8 a column): with L_ik = a_ik rs_k and z_k = rs_k x_k, x_i = -rs_i sum_k a_ik z_k.
@@ -463,81 +480,148 @@ __device__ __forceinline__ void inverse8(const double* sC, double* sX, const dou
                                          int b) {
     const int lane = threadIdx.x & 31, c = lane & 7, o = 8 * b;
     const double d = s_d[o + c];
-    const double sd = d > 0.0 ? sqrt64(d) : 1.0;
-    const double rs = rcp64(sd);
+    double sd, rs;
+    if (plain_pivot(d)) {
+        // rs = 1 / sqrt(d) from 20 bits by y (1 + e / 2 + 3 e^2 / 8), e = 1 - d y^2; sd from rs by one step
+        double y;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+        const double e = fma(-(d * y), y, 1.0);
+        rs = fma(y * e, fma(e, 0.375, 0.5), y);
+        const double s0 = d * rs;
+        sd = fma(fma(-s0, s0, d), 0.5 * rs, s0);
+    } else {
+        sd = other_sqrt(d);
+        rs = other_quotient(1.0, sd);
+    }
     if (lane < 8) {
         s_sd[o + c] = sd;
         s_rs[o + c] = rs;
     }
-    double z[8];
+    const double r2 = rs * rs;
+    double below[28], ri[8], ri2[8];  // the block below its diagonal by columns; all lanes' rs and r2
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        double t = 0.0;
+    for (int i = 0, q = 0; i < 8; ++i) {
+        ri[i] = __shfl_sync(0xffffffffu, rs, i);
+        ri2[i] = __shfl_sync(0xffffffffu, r2, i);
 #pragma unroll
-        for (int k = 0; k < i; ++k) t = fma(sC[(o + i) * TDP + o + k], z[k], t);
-        const double ri = __shfl_sync(0xffffffffu, rs, i);
-        const double x = i == c ? ri : (i > c ? -ri * t : 0.0);
-        z[i] = ri * x;
-        if (lane < 8) sX[(o + i) * TDP + o + c] = x;
+        for (int l = i + 1; l < 8; ++l, ++q) below[q] = sC[(o + l) * TDP + o + i];
     }
+    double t[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // sum_k a_ik z_k, grown column by column
+#pragma unroll
+    for (int i = 0, q = 0; i < 8; ++i) {
+        const double z = i == c ? ri2[i] : -ri2[i] * t[i];  // (t is zero above the diagonal)
+#pragma unroll
+        for (int l = i + 1; l < 8; ++l, ++q) t[l] = fma(below[q], z, t[l]);
+    }
+    if (lane < 8)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sX[(o + i) * TDP + o + c] = i == c ? ri[i] : -ri[i] * t[i];
 }
 
-// The diagonal tile in sC (lower triangle): L_kk into A (zeros above the diagonal) and D_k = L_kk^-1
-// into Dinv.  Unscaled elimination in four panels of eight columns: warp 0 takes the panel, a lane per
-// row with its eight columns in registers and the pivots passed by shuffle (a pivot costs a reciprocal
-// of three FP64 operations, a product and the updates: ~450 cycles a column, the chain that bounds the
-// tile), every warp then applies the panel to the rest; warp 1 inverts the previous panel's 8 x 8 block
-// meanwhile.  The square roots come once at the end, and the inverse grows from the 8 x 8 blocks by
-// doubling: X21 = -X22 (L21 X11).
-__device__ void diag_factor_inverse64(double* __restrict__ Akk, int np, double* __restrict__ D, double* sC, double* sX,
-                                      double* sP, double* sT, double* s_d, int* __restrict__ status) {
+// The diagonal tile in sC (lower triangle), less L L^T of the tile left of it when sL holds L^T: L_kk into A
+// (zeros above the diagonal) and D_k = L_kk^-1 into Dinv.  A dependent FP64 instruction takes 70 cycles, and
+// a column is four of them, the next column's update and shuffles, about 470 cycles, so that
+// warp 0 does nothing but the columns: panels of four, a lane per row with the columns in registers, where
+// it also applies the panel before.  Meanwhile the other warps apply the panel before to the columns behind
+// the current one, subtract L L^T from the columns that come up two panels later (these sums are the
+// largest part of the tile's work, and an SM takes 16 cycles for any FP64 instruction of a warp), and warp
+// 1 inverts the finished 8 x 8 blocks.  (A panel, its update of the rest and so on, after L L^T as a whole:
+// 66 000 cycles a tile, this 50 000; an FP64 step's solve,
+// with the panels' products shared by four blocks: 114 unknowns 208 -> 187 us, 380 unknowns 522 -> 450, 610
+// unknowns 925 -> 700, 1 210 unknowns 1 980 -> 1 700.)  The square roots come once at the end, and the inverse grows
+// from the 8 x 8 blocks by doubling: X21 = -X22 (L21 X11).
+__device__ void diag_factor_inverse64(double* __restrict__ Akk, int np, double* __restrict__ D, const double* sL, double* sC,
+                                      double* sX, double* sP, double* sT, double* s_d, int* __restrict__ status) {
     double* s_sd = s_d + TD;
     double* s_rs = s_sd + TD;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (sL && warp < kPanel && lane >= warp) {  // columns 0 .. 3: a warp per column
+        double v = sC[lane * TDP + warp];
+#pragma unroll 8
+        for (int l = 0; l < TD; ++l) v = fma(-sL[l * TDP + lane], sL[l * TDP + warp], v);
+        sC[lane * TDP + warp] = v;
+    }
     for (int e = tid; e < TD * TDP; e += kPotrf64Threads) sX[e] = 0.0;
     __syncthreads();
-    for (int b = 0; b < 4; ++b) {
-        const int c0 = 8 * b;
+    double tp[kPanel], ap[kPanel];  // warp 0: the panel before, multipliers and columns of the lane's row
+    bool bad = false;
+    for (int c0 = 0; c0 < TD; c0 += kPanel) {
+        const int toff = (c0 / kPanel) % 2 * kPanel;
         if (warp == 0) {
-            const int i = c0 + lane;
-            double a[8];
+            double a[kPanel], t[kPanel];
 #pragma unroll
-            for (int l = 0; l < 8; ++l) a[l] = i < TD ? sC[i * TDP + c0 + l] : 0.0;
+            for (int l = 0; l < kPanel; ++l) a[l] = sC[lane * TDP + c0 + l];
+            if (c0 > 0) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const double d = __shfl_sync(0xffffffffu, a[j], j);
-                const bool pos = d > 0.0;
-                const double inv = pos ? rcp64(d) : 0.0;
-                if (lane == j) {
-                    s_d[c0 + j] = d;
-                    if (!pos) atomicOr(status, 2);
-                }
-                const double t = a[j] * inv;
-                if (i < TD) sT[i * 9 + j] = t;
+                for (int j = 0; j < kPanel; ++j)
 #pragma unroll
-                for (int l = j + 1; l < 8; ++l) {
-                    const double alj = __shfl_sync(0xffffffffu, a[j], l);
-                    a[l] = fma(-t, alj, a[l]);
+                    for (int l = 0; l < kPanel; ++l) a[l] = fma(-tp[j], __shfl_sync(0xffffffffu, ap[j], c0 + l), a[l]);
+            }
+            double before[kPanel];
+            bool plain = true;
+#pragma unroll
+            for (int j = 0; j < kPanel; ++j) before[j] = a[j];
+#pragma unroll
+            for (int j = 0; j < kPanel; ++j) {
+                const double d = __shfl_sync(0xffffffffu, a[j], c0 + j);
+                plain = plain && plain_pivot(d);
+                t[j] = plain_quotient(a[j], d);
+#pragma unroll
+                for (int l = j + 1; l < kPanel; ++l) a[l] = fma(-t[j], __shfl_sync(0xffffffffu, a[j], c0 + l), a[l]);
+                if (lane == c0 + j) s_d[c0 + j] = d;
+            }
+            if (!plain) {  // a pivot that is not positive, or out of the quotient's range: the panel again
+#pragma unroll
+                for (int j = 0; j < kPanel; ++j) a[j] = before[j];
+#pragma unroll
+                for (int j = 0; j < kPanel; ++j) {
+                    const double d = __shfl_sync(0xffffffffu, a[j], c0 + j);
+                    t[j] = other_quotient(a[j], d);
+#pragma unroll
+                    for (int l = j + 1; l < kPanel; ++l) a[l] = fma(-t[j], __shfl_sync(0xffffffffu, a[j], c0 + l), a[l]);
+                    if (lane == c0 + j) s_d[c0 + j] = d;
+                    bad = bad || !(d > 0.0);
                 }
             }
-            if (i < TD)
+            if (lane >= c0)
 #pragma unroll
-                for (int l = 0; l < 8; ++l) sC[i * TDP + c0 + l] = a[l];
-        } else if (warp == 1 && b > 0) {
-            inverse8(sC, sX, s_d, s_sd, s_rs, b - 1);
-        }
-        __syncthreads();
-        const int m = TD - 8 - c0;
-        for (int e = tid; e < m * (m + 1) / 2; e += kPotrf64Threads) {
-            const int t = tri_row(e);
-            const int i = c0 + 8 + t, l = c0 + 8 + e - t * (t + 1) / 2;
-            double a = sC[i * TDP + l];
+                for (int l = 0; l < kPanel; ++l) {
+                    sC[lane * TDP + c0 + l] = a[l];
+                    sT[lane * 9 + toff + l] = t[l];
+                }
 #pragma unroll
-            for (int j = 0; j < 8; ++j) a = fma(-sT[i * 9 + j], sC[l * TDP + c0 + j], a);
-            sC[i * TDP + l] = a;
+            for (int l = 0; l < kPanel; ++l) {
+                ap[l] = a[l];
+                tp[l] = t[l];
+            }
+        } else if (warp == 1 && c0 > 0 && c0 % 8 == 0) {
+            inverse8(sC, sX, s_d, s_sd, s_rs, c0 / 8 - 1);
+        } else if (warp > 1 || c0 == 0) {
+            // columns c1 .. behind the panel: the panel before, and L L^T for the columns of the next but one
+            // panel (with the first panel, for those of the next one too)
+            const int c1 = c0 + kPanel, m = TD - c1;
+            const int l0 = c0 == 0 ? c1 : c1 + kPanel, l1 = c1 + 2 * kPanel;
+            const int first = c0 == 0 ? 32 : 64;
+            for (int e = tid - first; e < m * (m + 1) / 2; e += kPotrf64Threads - first) {
+                // by columns, so that a warp's elements share their kind: column c1 + q holds m - q of them
+                int q = 0, r = e;
+                while (r >= m - q) r -= m - q++;
+                const int l = c1 + q, i = l + r;
+                if (c0 == 0 && (!sL || l >= l1)) break;
+                double v = sC[i * TDP + l];
+                if (c0 > 0)
+#pragma unroll
+                    for (int j = 0; j < kPanel; ++j)
+                        v = fma(-sT[i * 9 + kPanel - toff + j], sC[l * TDP + c0 - kPanel + j], v);
+                if (sL && l >= l0 && l < l1)
+#pragma unroll 8
+                    for (int k = 0; k < TD; ++k) v = fma(-sL[k * TDP + i], sL[k * TDP + l], v);
+                sC[i * TDP + l] = v;
+            }
         }
         __syncthreads();
     }
+    if (bad && lane == 0) atomicOr(status, 2);
     if (warp == 1) inverse8(sC, sX, s_d, s_sd, s_rs, 3);
     __syncthreads();
     // L: columns times 1 / sqrt(pivot); the 8 x 8 blocks of the inverse are final already
@@ -550,21 +634,26 @@ __device__ void diag_factor_inverse64(double* __restrict__ Akk, int np, double* 
     __syncthreads();
 #pragma unroll
     for (int h = 8; h <= 16; h *= 2) {
-        // pairs of h x h blocks: rows r0 + h .. r0 + 2h - 1, columns r0 .. r0 + h - 1
-        const int per = h * h, pairs = TD / (2 * h);
-        const int pr = tid / per, e = tid % per, r = e / h, c = e % h, r0 = pr * 2 * h;
+        // pairs of h x h blocks: rows r0 + h .. r0 + 2h - 1, columns r0 .. r0 + h - 1.  Products with a
+        // triangular factor stop at its edge: a warp takes 32 / h columns (of L21 X11) or rows (of X22 P),
+        // long ones on the warps that share a sub-partition with short ones.
+        const int per = h * h, pairs = TD / (2 * h), wide = 32 / h, groups = h / wide;
+        const int pr = tid / per, e = tid % per, g = e >> 5, at = lane % h, r0 = pr * 2 * h;
+        const int line = (groups > 4 && g >= 4 ? groups + 3 - g : g) * wide + lane / h;
         if (pr < pairs) {
+            const int first = line / wide * wide;  // the same for the warp
             double t = 0.0;
-#pragma unroll
-            for (int k = 0; k < h; ++k) t = fma(sC[(r0 + h + r) * TDP + r0 + k], sX[(r0 + k) * TDP + r0 + c], t);
-            sP[(r0 + r) * TDP + c] = t;
+#pragma unroll 8
+            for (int k = first; k < h; ++k) t = fma(sC[(r0 + h + at) * TDP + r0 + k], sX[(r0 + k) * TDP + r0 + line], t);
+            sP[(r0 + at) * TDP + line] = t;
         }
         __syncthreads();
         if (pr < pairs) {
+            const int last = line / wide * wide + wide - 1;
             double t = 0.0;
-#pragma unroll
-            for (int k = 0; k < h; ++k) t = fma(sX[(r0 + h + r) * TDP + r0 + h + k], sP[(r0 + k) * TDP + c], t);
-            sX[(r0 + h + r) * TDP + r0 + c] = -t;
+#pragma unroll 8
+            for (int k = 0; k <= last; ++k) t = fma(sX[(r0 + h + line) * TDP + r0 + h + k], sP[(r0 + k) * TDP + at], t);
+            sX[(r0 + h + line) * TDP + r0 + at] = -t;
         }
         __syncthreads();
     }
@@ -599,48 +688,54 @@ __global__ void __launch_bounds__(kPotrf64Threads) k_potrf64_coop(double* __rest
     double* sA = smem64;
     double* sB = sA + TD * TDP;
     double* sC = sB + TD * TDP;
-    double* sT = sC + TD * TDP;
+    double* sX = sC + TD * TDP;
+    double* sT = sX + TD * TDP;
     double* s_d = sT + TD * 9;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     auto tile = [np](double* M, int i, int j) { return M + static_cast<size_t>(i) * TD * np + static_cast<size_t>(j) * TD; };
-    // R = 0 below the diagonal tiles (X_kk is D_k itself)
+    // R_ij (j < i) gathers in tile (j, i) of X, above the diagonal, and X_ij goes below it; L_ik goes to tile
+    // (k, i) of A.  No product is written over its operand, so that several blocks can share one.
     for (int r = blockIdx.x; r < nt * TD; r += gridDim.x)
-        for (int c = tid; c < (r / TD) * TD; c += kPotrf64Threads) X[static_cast<size_t>(r) * np + c] = 0.0;
+        for (int c = (r / TD + 1) * TD + tid; c < nt * TD; c += kPotrf64Threads) X[static_cast<size_t>(r) * np + c] = 0.0;
     if (blockIdx.x == 0) {
         tile32_load(A, np, sC);
         __syncthreads();
-        diag_factor_inverse64(A, np, Dinv, sC, sA, sB, sT, s_d, status);
+        diag_factor_inverse64(A, np, Dinv, nullptr, sC, sA, sB, sT, s_d, status);
     }
     phase_barrier<CLUSTER>();
     for (int k = 0; k < nt; ++k) {
         const int m = nt - 1 - k;
         const double* Dk = Dinv + static_cast<size_t>(k) * TD * TD;
-        for (int it = blockIdx.x; it < m + k + 1; it += gridDim.x) {
+        // L_ik = A_ik D_k^T (a lane per row) and X_kj = D_k R_kj (a lane per column).  A warp takes four
+        // columns (rows) whose lengths add up to 66; while four times the tiles fit the grid, four blocks
+        // share a tile, a warp taking one of the four and a sub-partition's two warps at most 37 products.
+        const int tiles = m + k + 1, parts = 4 * tiles <= static_cast<int>(gridDim.x) ? 4 : 1;
+        for (int it = blockIdx.x; it < tiles * parts; it += gridDim.x) {
+            const int tl = it / parts, pt = it - tl * parts;
+            const int q0 = parts == 1 ? 0 : (warp < 4 ? (pt + warp) & 3 : 3 - ((pt + warp) & 3));
+            const int q1 = parts == 1 ? 4 : q0 + 1;
             tile32_load(Dk, TD, sB);
-            if (it < m) {
-                // L_ik = A_ik D_k^T: a lane per row, columns of equal total length per warp
-                double* Aik = tile(A, k + 1 + it, k);
-                tile32_load(Aik, np, sA);
+            if (tl < m) {
+                tile32_load(tile(A, k + 1 + tl, k), np, sA);
                 __syncthreads();
+                double* L = tile(A, k, k + 1 + tl);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
+                    if (q < q0 || q >= q1) continue;
                     const int c = balanced32(warp, q);
                     double t = 0.0;
 #pragma unroll 8
                     for (int l = 0; l <= c; ++l) t = fma(sA[lane * TDP + l], sB[c * TDP + l], t);
-                    sC[lane * TDP + c] = t;
+                    L[static_cast<size_t>(c) * np + lane] = t;  // (transposed: rows of the tile are columns of L)
                 }
-                __syncthreads();
-                for (int e = tid; e < TD * TD; e += kPotrf64Threads)
-                    Aik[static_cast<size_t>(e / TD) * np + e % TD] = sC[(e / TD) * TDP + e % TD];
             } else {
-                // X_kj = D_k R_kj: a lane per column; X_kk = D_k
-                const int j = it - m;
-                double* Xkj = tile(X, k, j);
-                if (j < k) tile32_load(Xkj, np, sA);
+                const int j = tl - m;
+                if (j < k) tile32_load(tile(X, j, k), np, sA);
                 __syncthreads();
+                double* Xkj = tile(X, k, j);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
+                    if (q < q0 || q >= q1) continue;
                     const int r = balanced32(warp, q);
                     double t = 0.0;
                     if (j == k) t = sB[r * TDP + lane];
@@ -661,21 +756,12 @@ __global__ void __launch_bounds__(kPotrf64Threads) k_potrf64_coop(double* __rest
         const int stride = gridDim.x > 1 ? static_cast<int>(gridDim.x) - 1 : 1;
         for (int it = first_it; it < nitems; it = (it == 0 && gridDim.x > 1) ? nitems : it + stride) {
             if (it == 0) {
-                const double* Lk = tile(A, k + 1, k);
+                const double* Lk = tile(A, k, k + 1);
                 double* Akk = tile(A, k + 1, k + 1);
                 tile32_load(Lk, np, sA);
                 tile32_load(Akk, np, sC);
                 __syncthreads();
-                // the lower triangle alone: 528 elements
-                for (int e = tid; e < TD * (TD + 1) / 2; e += kPotrf64Threads) {
-                    const int r = tri_row(e), c = e - r * (r + 1) / 2;
-                    double t = sC[r * TDP + c];
-#pragma unroll 8
-                    for (int l = 0; l < TD; ++l) t = fma(-sA[r * TDP + l], sA[c * TDP + l], t);
-                    sC[r * TDP + c] = t;
-                }
-                __syncthreads();
-                diag_factor_inverse64(Akk, np, Dinv + static_cast<size_t>(k + 1) * TD * TD, sC, sA, sB, sT, s_d, status);
+                diag_factor_inverse64(Akk, np, Dinv + static_cast<size_t>(k + 1) * TD * TD, sA, sC, sX, sB, sT, s_d, status);
                 __syncthreads();
                 continue;
             }
@@ -685,28 +771,26 @@ __global__ void __launch_bounds__(kPotrf64Threads) k_potrf64_coop(double* __rest
                 // A_ij -= L_ik L_jk^T
                 const int t = tri_row(it);
                 const int i = k + 1 + t, j = k + 1 + (it - t * (t + 1) / 2);
-                tile32_load(tile(A, i, k), np, sA);
-                tile32_load(tile(A, j, k), np, sB);
+                tile32_load(tile(A, k, i), np, sA);
+                tile32_load(tile(A, k, j), np, sB);
                 dst = tile(A, i, j);
             } else {
                 // R_ij -= L_ik X_kj
                 const int q = it - ntrail;
                 const int i = k + 1 + q / (k + 1), j = q % (k + 1);
-                tile32_load(tile(A, i, k), np, sA);
+                tile32_load(tile(A, k, i), np, sA);
                 tile32_load(tile(X, k, j), np, sB);
-                dst = tile(X, i, j);
+                dst = tile(X, j, i);
             }
             double acc[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) acc[q] = dst[static_cast<size_t>(warp + 8 * q) * np + lane];
             __syncthreads();
-            const double* b = sB + (trail ? lane * TDP : lane);
-            const int bs = trail ? 1 : TDP;
 #pragma unroll 8
             for (int l = 0; l < TD; ++l) {
-                const double bv = b[l * bs];
+                const double bv = sB[l * TDP + lane];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) acc[q] = fma(-sA[(warp + 8 * q) * TDP + l], bv, acc[q]);
+                for (int q = 0; q < 4; ++q) acc[q] = fma(-sA[l * TDP + warp + 8 * q], bv, acc[q]);
             }
 #pragma unroll
             for (int q = 0; q < 4; ++q) dst[static_cast<size_t>(warp + 8 * q) * np + lane] = acc[q];
@@ -1348,8 +1432,8 @@ int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, in
         int npv = np, ntv = f64 ? (n + TD - 1) / TD : nt;
         int* stv = W.status;
         void* args[] = {&A, &X, &Dv, &npv, &ntv, &stv, &h_status};
-        // one block per lower tile at most: small systems take a small grid
-        const int fgrid = std::max(1, std::min(W.fact_grid, ntv * (ntv + 1) / 2));
+        // one block per lower tile, or four per tile of a panel, at most: small systems take a small grid
+        const int fgrid = std::max(1, std::min(W.fact_grid, std::max(ntv * (ntv + 1) / 2, f64 ? 4 * ntv : 0)));
         if (launch_phased(kernel, cluster_kernel, W.fact_cluster, fgrid, threads, args, smem, st) != cudaSuccess) return -1;
         ++L;
     }
