@@ -68,3 +68,28 @@ def test_block_schur_over_shapes(P, pb, E, views, mixed):
     assert np.linalg.norm(x - x_ref) <= 1e-10 * np.linalg.norm(x_ref)
     assert np.linalg.norm(y - y_ref) <= 1e-10 * np.linalg.norm(y_ref)
     ctx.close()
+
+
+@pytest.mark.parametrize("at", [0, 2, 3, 6, 14, 30, 32, 37, 46])
+def test_a_pivot_of_exactly_zero_is_shifted(at):
+    """Columns `at` and `at + 1` are equal and their scaled entries are exactly one, so that the second
+    pivot is exactly zero wherever it falls in a panel or tile: the factor is repeated with a small shift
+    and the solve reaches the consistent system's residual (1e-12 of the right-hand side, three entries of
+    rounding per row)."""
+    pb, P = 16, 3
+    eq = BlockNormalEquations(P, 1, pb, 3)
+    H, g = np.zeros((P * pb, P * pb)), np.zeros(P * pb)
+    rng = np.random.default_rng(at)
+    for b in range(P):
+        J = 2.0 * np.eye(pb)
+        c = at - b * pb
+        if 0 <= c < pb:
+            J[:, c + 1] = J[:, c]
+        r = rng.normal(size=pb)
+        eq.addPrimaryResidualBlock(b, J, r)
+        H[b * pb:(b + 1) * pb, b * pb:(b + 1) * pb] = J.T @ J
+        g[b * pb:(b + 1) * pb] = J.T @ r
+    eq.addEliminatedResidualBlock(0, np.eye(3), np.zeros(3))
+    ctx = Gb300Context(0)
+    x, _, _ = solve_damped_schur_complement(ctx, eq, 0.0, SchurComplementSolverOptions(useMixedPrecision=False))
+    assert np.linalg.norm(H @ x + g) <= 1e-11 * np.linalg.norm(g)
