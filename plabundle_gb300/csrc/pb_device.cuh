@@ -471,8 +471,9 @@ __device__ __forceinline__ double f64_of(double d) { return d; }
 // hi = RN(d), lo = RN(d - hi), without a branch.  The difference is an integer of at most 29 bits times
 // 2^(e - 52) (e the exponent of d), rounded by its conversion to FP32; the scaling is exact.  Below 2^-74,
 // where the scale or the result would leave the normal FP32 numbers, the conversion is that of 2^100 d,
-// scaled back (only FP32 denormals may round twice); below 2^-174 both parts are zero.  Where hi is
-// infinite or NaN, so is every value made from it.
+// scaled back (only FP32 denormals may round twice); below 2^-174 both parts are zero, by a scale of zero
+// too (the power of two's exponent runs out of its field there, and zero times an infinity is no number).
+// Where hi is infinite or NaN, so is every value made from it.
 __device__ __forceinline__ ff ff_make_bits(double d) {
     const unsigned hw = hi_word(d), lw = static_cast<unsigned>(__double2loint(d));
     const unsigned sign = hw & 0x80000000u, mag = hw & 0x7fffffffu;
@@ -488,7 +489,8 @@ __device__ __forceinline__ ff ff_make_bits(double d) {
         u = 0u;
         rest = 0;
     }
-    float h = __uint_as_float(u | sign), l = static_cast<float>(sign ? -rest : rest) * __uint_as_float((ex - 948u) << 23);
+    float h = __uint_as_float(u | sign),
+          l = static_cast<float>(sign ? -rest : rest) * __uint_as_float(zero ? 0u : (ex - 948u) << 23);
     const float back = small ? 0x1p-100f : 1.0f;
     h *= back;
     l *= back;
