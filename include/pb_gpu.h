@@ -204,6 +204,15 @@ typedef struct pb_solve_report {
     double mean_rms_after;
     double valid_track_ratio;
     double filter_threshold;
+    /* Phases of the iterations, in time on the solve's stream (the same on every path, whether the
+     * driver queues an iteration's phases behind one another or waits between them):
+     *   assembly_ms           linearisation, point elimination, the extension by scale bars;
+     *   linear_ms             from there to the point steps: a rig's transform onto its pose blocks,
+     *                         factorisations and conjugate gradients, with what was queued for nothing
+     *                         when a kept factor did not do;
+     *   back_substitution_ms  the point steps;
+     *   objective_ms          the trial states and their costs.
+     * total_ms is the host's time of the whole call. */
     double assembly_ms;
     double linear_ms;
     double back_substitution_ms;

@@ -687,9 +687,9 @@ struct Timer {
     }
 };
 
-// The kernels of an assembly: the reduced system, its extension by the promoted points of scale bars (every
-// assembly extends it and adds the bars' cost, so that every solve of this context sees the extended system)
-// and, for rigs, the transform onto the rig's pose blocks, damped there.
+// The kernels of an assembly: the reduced system and its extension by the promoted points of scale bars (every
+// assembly extends it and adds the bars' cost, so that every solve of this context sees the extended system).
+// For rigs, rig_transform follows.
 template <typename T>
 void enqueue_assembly(pb_gpu_ctx* c, double damping, int precision) {
     prepare_precision<T>(c, precision);
@@ -712,7 +712,6 @@ void enqueue_assembly(pb_gpu_ctx* c, double damping, int precision) {
     c->last_precision = precision;
     c->have_system = true;
     if (c->ext_on) enqueue_extension(c, damping);
-    if (c->rig_on) rig_transform(c, damping);
 }
 
 // After the stream has been waited for: cost and flags of the last assembly.
@@ -1177,6 +1176,7 @@ void enqueue_assembly(pb_gpu_ctx* c, double damping, int precision) {
 
 void do_assemble(pb_gpu_ctx* c, double damping, int precision, double* cost, int* flags) {
     enqueue_assembly(c, damping, precision);
+    if (c->rig_on) rig_transform(c, damping);
     check(cudaStreamSynchronize(c->stream), "assemble");
     read_assembly(c, cost, flags);
 }
@@ -1194,6 +1194,9 @@ struct Ahead {
     bool step = false;   // point steps and first objectives are
 };
 
+// Bounds of an iteration's phases on the solve's stream, which the report's times are taken from whether or
+// not the phases were queued behind one another: assembly 0 to 1, linear solve (with a rig's transform before
+// it) 1 to 2, point steps 2 to 3, objectives 3 to 4.
 void mark(pb_gpu_ctx* c, int i) {
     if (!c->lm_ev[i]) check(cudaEventCreate(&c->lm_ev[i]), "event");
     check(cudaEventRecord(c->lm_ev[i], c->stream), "event");
@@ -1204,7 +1207,7 @@ double between(pb_gpu_ctx* c, int i, int j) {
     return t;
 }
 
-// Point steps (events 2 to 3) and the objectives of n step lengths (3 to 4).
+// Point steps and the objectives of n step lengths.
 void enqueue_step(pb_gpu_ctx* c, const double* alphas, int n) {
     mark(c, 2);
     enqueue_back_substitution(c, false);
@@ -1220,6 +1223,7 @@ Ahead assemble_ahead(pb_gpu_ctx* c, const pb_solve_options& op, double damping, 
     mark(c, 0);
     enqueue_assembly(c, damping, precision);
     mark(c, 1);
+    if (c->rig_on) rig_transform(c, damping);
     ahead.solve = ahead.step = launch_kept_solve(c, op);
     if (ahead.step) enqueue_step(c, alphas, n);
     check(cudaStreamSynchronize(c->stream), "assemble");
@@ -1233,6 +1237,23 @@ void step_after_solve(pb_gpu_ctx* c, Ahead& ahead, const double* alphas, int n) 
     enqueue_step(c, alphas, n);
     check(cudaStreamSynchronize(c->stream), "step");
     ahead.step = true;
+}
+
+// Time of a linear solve that no step follows.
+double linear_alone(pb_gpu_ctx* c) {
+    mark(c, 2);
+    check(cudaEventSynchronize(c->lm_ev[2]), "linear solve");
+    return between(c, 1, 2);
+}
+
+// Further objectives of an iteration; returns their time.
+double more_costs(pb_gpu_ctx* c, const double* alphas, int n, double* costs) {
+    mark(c, 3);
+    enqueue_costs(c, alphas, n, 1);
+    mark(c, 4);
+    check(cudaStreamSynchronize(c->stream), "cost");
+    read_costs(c, n, costs);
+    return between(c, 3, 4);
 }
 
 // The LM / Armijo driver (online branch of optimizePointsWithPlaMatrix).
@@ -1334,11 +1355,9 @@ void lm_solve(pb_gpu_ctx* c, const pb_solve_options& op, pb_solve_report* rep) {
                 bool lconv = false;
                 int lit = 0, sweeps = 0;
                 double relres = 0.0;
-                auto tl = now();
-                const bool queued = ahead.solve;
                 const int lrc = solve_reduced(c, op, &lconv, &lit, &relres, &sweeps, &ahead.solve);
-                t_lin += ms(tl, now()) + (queued ? between(c, 1, 2) : 0.0);
                 ahead.step = ahead.step && ahead.solve;
+                if (lrc || !lconv) t_lin += linear_alone(c);
                 if (lrc) {
                     ++iterations;
                     ++rep->rejected_steps;
@@ -1356,6 +1375,7 @@ void lm_solve(pb_gpu_ctx* c, const pb_solve_options& op, pb_solve_report* rep) {
                 double dd, psq, csq;
                 step_after_solve(c, ahead, &full, n_first);
                 read_back_substitution(c, &dd, &psq, &csq);
+                t_lin += between(c, 1, 2);
                 t_bs += between(c, 2, 3);
                 t_obj += between(c, 3, 4);
                 if (!std::isfinite(dd)) {
@@ -1370,13 +1390,12 @@ void lm_solve(pb_gpu_ctx* c, const pb_solve_options& op, pb_solve_report* rep) {
                 int accepted_slot = -1;
                 double accepted_alpha = 1.0;
                 int k0 = 0;
-                auto tc = now();
                 while (k0 < op.line_search_steps && accepted_slot < 0) {
                     const int nbatch = std::min(k0 == 0 ? 1 : kMaxAlpha, op.line_search_steps - k0);
                     double al[kMaxAlpha], costs[kMaxAlpha];
                     for (int i = 0; i < nbatch; ++i) al[i] = std::ldexp(1.0, -(k0 + i));
                     if (k0 == 0) read_costs(c, 1, costs);  // evaluated with the point steps
-                    else eval_costs(c, al, nbatch, 1, costs);
+                    else t_obj += more_costs(c, al, nbatch, costs);
                     for (int i = 0; i < nbatch; ++i) {
                         ++rep->objective_evaluations;
                         cand = costs[i];
@@ -1390,7 +1409,6 @@ void lm_solve(pb_gpu_ctx* c, const pb_solve_options& op, pb_solve_report* rep) {
                     }
                     k0 += nbatch;
                 }
-                t_obj += ms(tc, now());
                 if (trace)
                     std::fprintf(stderr,
                                  "PB_GPU_TRACE it=%d precision=%d cost=%.15e lambda=%.3e lin_it=%d sweeps=%d "
@@ -1561,11 +1579,9 @@ void lm_solve_general(pb_gpu_ctx* c, const pb_solve_options& op, pb_solve_report
                 bool lconv = false;
                 int lit = 0, sweeps = 0;
                 double relres = 0.0;
-                auto tl = now();
-                const bool queued = ahead.solve;
                 const int lrc = solve_reduced(c, op, &lconv, &lit, &relres, &sweeps, &ahead.solve);
-                t_lin += ms(tl, now()) + (queued ? between(c, 1, 2) : 0.0);
                 ahead.step = ahead.step && ahead.solve;
+                if (lrc || !lconv) t_lin += linear_alone(c);
                 if (lrc) throw std::runtime_error("reduced system is not numerically SPD (positive definite)");
                 rep->linear_iterations += lit;
                 rep->refinement_sweeps += sweeps;
@@ -1579,6 +1595,7 @@ void lm_solve_general(pb_gpu_ctx* c, const pb_solve_options& op, pb_solve_report
                 step_after_solve(c, ahead, first, n_first);
                 read_back_substitution(c, &dd_bs, &psq, &csq);
                 if (c->ext_on) psq += c->bar_d[kMaxAlpha + 1];
+                t_lin += between(c, 1, 2);
                 t_bs += between(c, 2, 3);
                 t_obj += between(c, 3, 4);
                 const double rg = n_global > 0 ? std::sqrt(csq / n_global) : 0.0;
@@ -1587,7 +1604,6 @@ void lm_solve_general(pb_gpu_ctx* c, const pb_solve_options& op, pb_solve_report
                     converged = true;
                     continue;
                 }
-                auto tc = now();
                 // directional decrease by a forward difference of the objective along the step
                 double dd = 0.0;
                 double first_trial = kNaN;
@@ -1609,7 +1625,7 @@ void lm_solve_general(pb_gpu_ctx* c, const pb_solve_options& op, pb_solve_report
                     double al[kMaxAlpha], costs[kMaxAlpha];
                     for (int i = 0; i < nbatch; ++i) al[i] = std::ldexp(1.0, -(k0 + i));
                     if (k0 == 0) costs[0] = first_trial;  // evaluated with the point steps
-                    else eval_costs(c, al, nbatch, 1, costs);
+                    else t_obj += more_costs(c, al, nbatch, costs);
                     for (int i = 0; i < nbatch; ++i) {
                         ++rep->objective_evaluations;
                         cand = costs[i];
@@ -1624,7 +1640,6 @@ void lm_solve_general(pb_gpu_ctx* c, const pb_solve_options& op, pb_solve_report
                     }
                     k0 += nbatch;
                 }
-                t_obj += ms(tc, now());
                 // the last trial evaluated (the smallest step length) is accepted when it lowers
                 // the cost even without the Armijo condition
                 const bool accept = std::isfinite(cand) && cand < current;
