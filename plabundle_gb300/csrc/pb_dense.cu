@@ -1476,7 +1476,9 @@ int dense_pcg_launch(const PcgSystem<double>& sys, DenseWork<T>& W, const double
     if (W.cg_cluster == kClusterMax && W.n <= (sys.ncb > 0 ? kCgClusterDim : kCgClusterDimBorder) && smem <= kCgClusterSmem) {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute at;
-        cluster_config(cfg, at, std::max(1, std::min(kClusterMax, rows)), kCgThreads, smem, st);
+        W.cg_blocks = std::max(1, std::min(kClusterMax, rows));
+        W.cg_max_it = max_it;
+        cluster_config(cfg, at, W.cg_blocks, kCgThreads, smem, st);
         if (cudaLaunchKernelEx(&cfg, &k_dense_cg_cluster<T>, sys, static_cast<const T*>(W.X), static_cast<const T*>(W.A),
                                W.np, static_cast<const double*>(W.dscale), b, W.x, shape, h_scal, rel_tol, abs_tol,
                                max_it) != cudaSuccess)
@@ -1485,6 +1487,8 @@ int dense_pcg_launch(const PcgSystem<double>& sys, DenseWork<T>& W, const double
         return 0;
     }
     const int grid = std::max(1, std::min(W.coop_grid, rows));
+    W.cg_blocks = grid;
+    W.cg_max_it = max_it;
     PcgSystem<double> s = sys;
     const T* X = W.X;
     const T* XT = W.A;
@@ -1502,15 +1506,16 @@ int dense_pcg_launch(const PcgSystem<double>& sys, DenseWork<T>& W, const double
     return 0;
 }
 
-int dense_pcg_result(const double* h_scal, int* iterations, double* relres, bool* converged) {
+template <typename T>
+int dense_pcg_result(const DenseWork<T>& W, const double* h_scal, int* iterations, double* relres, bool* converged) {
     *iterations = static_cast<int>(h_scal[0]);
     *relres = h_scal[1];
     *converged = h_scal[2] != 0.0;
     // opt-in trace (PB_GPU_TRACE=1): one line per CG launch
     static const bool trace = std::getenv("PB_GPU_TRACE") != nullptr;
     if (trace)
-        std::fprintf(stderr, "PB_GPU_CG iterations=%d relres=%.3e converged=%d\n", *iterations, *relres,
-                     *converged ? 1 : 0);
+        std::fprintf(stderr, "PB_GPU_CG precision=%d iterations=%d relres=%.3e converged=%d max_it=%d grid=%d\n",
+                     sizeof(T) == 4 ? 1 : 0, *iterations, *relres, *converged ? 1 : 0, W.cg_max_it, W.cg_blocks);
     return h_scal[3] != 0.0 ? 1 : 0;
 }
 
@@ -1520,7 +1525,7 @@ int dense_pcg(const PcgSystem<double>& sys, DenseWork<T>& W, const double* b, do
               int* launches) {
     if (dense_pcg_launch<T>(sys, W, b, rel_tol, abs_tol, max_it, h_scal, st, launches) != 0) return -1;
     if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
-    return dense_pcg_result(h_scal, iterations, relres, converged);
+    return dense_pcg_result<T>(W, h_scal, iterations, relres, converged);
 }
 
 template int dense_factor<float>(const PcgSystem<double>&, DenseWork<float>&, double, int*, cudaStream_t, int*);
@@ -1529,6 +1534,8 @@ template int dense_pcg_launch<float>(const PcgSystem<double>&, DenseWork<float>&
                                      double*, cudaStream_t, int*);
 template int dense_pcg_launch<double>(const PcgSystem<double>&, DenseWork<double>&, const double*, double, double, int,
                                       double*, cudaStream_t, int*);
+template int dense_pcg_result<float>(const DenseWork<float>&, const double*, int*, double*, bool*);
+template int dense_pcg_result<double>(const DenseWork<double>&, const double*, int*, double*, bool*);
 template int dense_pcg<float>(const PcgSystem<double>&, DenseWork<float>&, const double*, double, double, int, int*,
                               double*, bool*, double*, cudaStream_t, int*);
 template int dense_pcg<double>(const PcgSystem<double>&, DenseWork<double>&, const double*, double, double, int, int*,

@@ -247,6 +247,7 @@ struct DenseWork {
     int coop_grid = 0;       // blocks of the cooperative CG launch
     int fact_grid = 0;       // blocks of the cooperative factorisation
     int cg_cluster = 0, fact_cluster = 0;  // blocks that one cluster of the kernel can hold
+    int cg_blocks = 0, cg_max_it = 0;      // of the last CG launch (trace)
 };
 
 template <typename T>
@@ -267,7 +268,8 @@ int dense_pcg(const PcgSystem<double>& sys, DenseWork<T>& W, const double* b, do
 template <typename T>
 int dense_pcg_launch(const PcgSystem<double>& sys, DenseWork<T>& W, const double* b, double rel_tol, double abs_tol,
                      int max_it, double* h_scal, cudaStream_t st, int* launches);
-int dense_pcg_result(const double* h_scal, int* iterations, double* relres, bool* converged);
+template <typename T>
+int dense_pcg_result(const DenseWork<T>& W, const double* h_scal, int* iterations, double* relres, bool* converged);
 
 // Backward pass (pb_adjoint.cu).  Per-observation record of the exact Hessian in the local chart
 // (pose 6 | point 3 | intrinsic columns ni): pose-pose (upper 6x6), pose-point (6x3), point-point

@@ -847,7 +847,7 @@ int solve_dense(pb_gpu_ctx* c, double rel, double abs_tol, int max_it, bool* con
             launch_kept_cg<T>(c, rel, abs_tol, max_it);
             check(cudaStreamSynchronize(c->stream), "dense CG");
         }
-        if (dense_pcg_result(c->h_scratch + kSlotCg, iterations, relres, converged) == 0 && *converged) {
+        if (dense_pcg_result<T>(W, c->h_scratch + kSlotCg, iterations, relres, converged) == 0 && *converged) {
             ++c->f32_age;
             if (!queued) copy_step(c, W.x);
             return 0;
