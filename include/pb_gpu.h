@@ -529,9 +529,9 @@ pb_status pb_gpu_solve_damped_schur(pb_gpu_ctx* ctx, const pb_bne* equations, do
  *     invalid_projections (host, may be NULL): how many did not (behind the camera, non-finite);
  *   - at most PB_NOALLOC_MAX_OBS observations, else PB_ERR_BOUNDS before any launch; a camera or
  *     point index out of range is skipped on the device and reported as PB_ERR_BOUNDS;
- *   - the scratch array is shared by all calls on a device: calls that overlap in time on one
- *     device race, so callers serialise them; nothing in it has to start at zero (every element
- *     read is written earlier in the same call);
+ *   - the scratch array is shared by all calls on a device: calls of several threads on one device
+ *     take turns, on whatever streams (a lock per device, held until the call returns); nothing in
+ *     it has to start at zero (every element read is written earlier in the same call);
  *   - the first call on a device resolves the array's address (cudaGetSymbolAddress, which may
  *     load the module), so that first call should come before any stream capture; the address
  *     is kept for the life of the process, so the call must not be used across a

@@ -10,8 +10,8 @@
 //   - at most PB_NOALLOC_MAX_OBS observations; larger inputs are rejected before any launch;
 //   - every element of the scratch array that the final sum reads is written earlier in the same
 //     call, so nothing has to start at zero;
-//   - the array is shared by all callers on a device: calls that overlap in time on one device
-//     race; callers serialise them (one stream, or host-side ordering);
+//   - the array and the host totals are shared by all callers on a device: a lock per device is held
+//     from the launch until the totals are read, so that threads take turns, whatever their streams;
 //   - the array's device address is resolved with cudaGetSymbolAddress on the first call on each
 //     device (that call may load the module), so that first call should come before any stream
 //     capture; the address is kept for the life of the process (not valid across a
@@ -169,21 +169,22 @@ __global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(kCluste
 // go straight to a file-scope host array; elsewhere they follow the scratch and are copied (a call of 2 001
 // observations: 33.6 -> 23.9 us).
 struct NoAllocDevice {
+    std::mutex turn;  // of the call that uses what follows
     double* scratch = nullptr;
     double* totals = nullptr;
     double* host = nullptr;  // the totals in host memory; null: copy them
 };
-NoAllocDevice noalloc_device() {
+NoAllocDevice* noalloc_device() {
     static std::mutex mu;
     static NoAllocDevice known[kNoAllocMaxDevices];
     alignas(64) static double host_totals[kNoAllocMaxDevices][8];
     int dev = -1;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kNoAllocMaxDevices) return {};
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kNoAllocMaxDevices) return nullptr;
     std::lock_guard<std::mutex> lock(mu);
     NoAllocDevice& d = known[dev];
     if (!d.scratch) {
         void* p = nullptr;
-        if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess) return {};
+        if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess) return nullptr;
         int reach = 0, tables = 0;
         cudaDeviceGetAttribute(&reach, cudaDevAttrPageableMemoryAccess, dev);
         cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev);
@@ -191,7 +192,7 @@ NoAllocDevice noalloc_device() {
         if (reach && tables) d.host = d.totals = host_totals[dev];
         else d.totals = d.scratch + 3 * static_cast<size_t>(kNoAllocMaxBlocks);
     }
-    return d;
+    return &d;
 }
 
 }  // namespace
@@ -217,8 +218,10 @@ extern "C" pb_status pb_gpu_objective_noalloc(const double* cameras, int32_t n_c
     }
     // an error pending from earlier work on this thread is not this call's: leave it in place
     if (cudaPeekAtLastError() != cudaSuccess) return PB_ERR_CUDA;
-    const NoAllocDevice d = noalloc_device();
-    if (!d.scratch) return PB_ERR_CUDA;
+    NoAllocDevice* const known = noalloc_device();
+    if (!known) return PB_ERR_CUDA;
+    NoAllocDevice& d = *known;
+    const std::lock_guard<std::mutex> turn(d.turn);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int nblocks = static_cast<int>(std::min<int64_t>((n_obs + kNoAllocThreads - 1) / kNoAllocThreads, kNoAllocMaxBlocks));
     const double c2 = robust_loss_scale * robust_loss_scale, ic2 = 1.0 / c2;
