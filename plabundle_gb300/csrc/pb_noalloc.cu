@@ -35,9 +35,10 @@ constexpr int kNoAllocThreads = 128;
 // most 1216 partials.
 constexpr int kNoAllocMaxBlocks = 152 * 8;
 constexpr int kClusterBlocks = 8, kClusterThreads = 256;
-// Up to two observations per thread of the cluster, one launch beats two (a call with its totals copied, 4 096 observations:
-// 35.0 against 36.7 us; 8 192: 46.3 against 37.0, eight SMs are then too few).
-constexpr long long kClusterMaxObs = 2LL * kClusterBlocks * kClusterThreads;
+// Up to one observation per thread of the cluster, one launch beats two (a call of 2 001 observations: 23.6
+// against 25.8 us); a second observation waits for the first on the same eight SMs (2 500: 27.1 against 25.7,
+// 4 096: 27.5 against 25.7, 8 192: 34.5 against 25.9).
+constexpr long long kClusterMaxObs = 1LL * kClusterBlocks * kClusterThreads;
 constexpr int kNoAllocMaxDevices = 64;
 
 // [0, B): cost partials; [B, 2B): invalid projections; [2B, 3B): index errors; [3B, 3B + 3): totals

@@ -19,7 +19,7 @@ def test_threads_take_turns(one_stream):
     L = native.load()
     shared = torch.cuda.Stream()
     jobs = []
-    for k, n in enumerate((65, 700, 3001, 4096, 4097, 9000)):  # one launch and two
+    for k, n in enumerate((65, 700, 2048, 2049, 4097, 9000)):  # one launch and two
         d = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in _inputs(n, 40 + k, False)]
         jobs.append((n, d, shared if one_stream else torch.cuda.Stream()))
     torch.cuda.synchronize()
