@@ -459,20 +459,9 @@ constexpr size_t kPotrf64Smem = (4 * static_cast<size_t>(TD) * TDP + TD * 9 + 3 
 
 constexpr int kPanel = 4;
 
-// Pivot test on the integer pipe (an FP64 comparison and its predicate take about 100 cycles): the exponent
-// of a positive d in (-1000, 1000).
-__device__ __forceinline__ bool plain_pivot(double d) { return (hi_word(d) >> 20) - 24u <= 1998u; }
 // (out of line: not on the way of the ordinary pivots)
 __device__ __noinline__ double other_quotient(double a, double d) { return d > 0.0 ? a / d : 0.0; }
 __device__ __noinline__ double other_sqrt(double d) { return d > 0.0 ? sqrt(d) : 1.0; }
-// a / d for a plain pivot: x0 = 1 / d to 20 bits, e = 1 - d x0, and a (x0 (1 + e + e^2)), whose remainder e^3
-// is below the rounding.
-__device__ __forceinline__ double plain_quotient(double a, double d) {
-    double x0;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x0) : "d"(d));
-    const double e = fma(-d, x0, 1.0);
-    return a * fma(x0, fma(e, e, e), x0);
-}
 
 // Inverse of the 8 x 8 diagonal block b of the tile's factor from its unscaled columns, by one warp
 // (lane c < 8 a column): with L_ik = a_ik rs_k and z_k = rs_k x_k, x_i = -rs_i sum_k a_ik z_k.
@@ -482,13 +471,7 @@ __device__ __forceinline__ void inverse8(const double* sC, double* sX, const dou
     const double d = s_d[o + c];
     double sd, rs;
     if (plain_pivot(d)) {
-        // rs = 1 / sqrt(d) from 20 bits by y (1 + e / 2 + 3 e^2 / 8), e = 1 - d y^2; sd from rs by one step
-        double y;
-        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-        const double e = fma(-(d * y), y, 1.0);
-        rs = fma(y * e, fma(e, 0.375, 0.5), y);
-        const double s0 = d * rs;
-        sd = fma(fma(-s0, s0, d), 0.5 * rs, s0);
+        plain_roots(d, sd, rs);
     } else {
         sd = other_sqrt(d);
         rs = other_quotient(1.0, sd);

@@ -93,8 +93,10 @@ __device__ __forceinline__ bool robust_loss(double s, int loss, double scale, do
 // and log1p of the CUDA library; about 48 in the form below (pb_gpu_objective_noalloc over 4 000 000
 // observations, Cauchy: 1021 -> 347 us a call).
 //   - comparisons and finiteness tests look at the bit patterns on the integer pipe;
-//   - the reciprocal and the square root take one third-order Householder step from the 20-bit
-//     hardware approximation of the operand's high word (error below 2^-59 before the last rounding);
+//   - the reciprocal and the square root take one third-order step from the 20-bit hardware
+//     approximation of the operand's high word (error below 2^-59 before the last rounding):
+//     Householder's for the reciprocal, the geometric series of 1 / (1 - e) to e^2, and Chebyshev's for
+//     the square root, the binomial series of (1 - e)^(-1/2) to e^2;
 //   - the principal point is subtracted from the pixel before the focal product is added;
 //   - a Cauchy sum takes one log1p per run of observations: sum log1p(x_i) = log1p(prod (1 + x_i) - 1),
 //     with the product kept as q = prod - 1 (q <- q + x (1 + q), relative precision also for tiny x).
@@ -130,6 +132,28 @@ __device__ __forceinline__ double sqrt64(double s) {
     const double n = s * y;
     const double e = fma(-n, y, 1.0);
     return fma(n, e * fma(0.375, e, 0.5), n);
+}
+
+// Pivots of the FP64 dense factor (pb_dense.cu), by the same two steps.  Pivot test on the integer pipe (an
+// FP64 comparison and its predicate take about 100 cycles): the exponent of a positive d in (-1000, 1000).
+__device__ __forceinline__ bool plain_pivot(double d) { return (hi_word(d) >> 20) - 24u <= 1998u; }
+// a / d for a plain pivot, within 2 ulp (the reciprocal and the product round once each): x0 = 1 / d to 20
+// bits, e = 1 - d x0, and a (x0 (1 + e + e^2)), whose remainder e^3 is below the rounding.
+__device__ __forceinline__ double plain_quotient(double a, double d) {
+    double x0;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x0) : "d"(d));
+    const double e = fma(-d, x0, 1.0);
+    return a * fma(x0, fma(e, e, e), x0);
+}
+// rs = 1 / sqrt(d) within 2 ulp from 20 bits y by y (1 + e / 2 + 3 e^2 / 8), e = 1 - d y^2; sd = sqrt(d)
+// within 1 ulp from d rs by one step of Newton's method.
+__device__ __forceinline__ void plain_roots(double d, double& sd, double& rs) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double e = fma(-(d * y), y, 1.0);
+    rs = fma(y * e, fma(e, 0.375, 0.5), y);
+    const double s0 = d * rs;
+    sd = fma(fma(-s0, s0, d), 0.5 * rs, s0);
 }
 
 // A camera record as the objective reads it (records of 32 doubles).  VEC: the records start on a

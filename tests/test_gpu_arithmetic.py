@@ -2,7 +2,14 @@
 
 Conversions between FP64 and FP32 on the integer pipe: the parts are those of the rounding conversions,
 hi = RN(d) and lo = RN(d - hi), bit for bit, except where a part is an FP32 denormal, which may round twice
-(one unit of 2^-149), and where hi overflows (both parts not finite, or hi infinite)."""
+(one unit of 2^-149), and where hi overflows (both parts not finite, or hi infinite).
+
+Reciprocals, quotients and roots: in units of the last place (ulp) of the exact value, taken in extended
+precision.  A series step from 20 bits leaves an error of 2^-59 before its one rounding (half an ulp), so
+that the reciprocal and the root stay within 1 ulp; a quotient rounds its reciprocal and its product, at
+most 2^-53 each, which is 2 ulp where the result's fraction is largest; the reciprocal root's product d y
+adds a quarter of its rounding to its own.  Outside the series' exponents the IEEE operation takes over,
+bit for bit."""
 import ctypes as C
 import os
 import subprocess
@@ -60,6 +67,49 @@ def test_fp64_to_float_pair(probe):
         same = (g.view(np.uint32) == want.view(np.uint32)) | ((g == 0) & (want == 0))
         near = (np.abs(want) < tiny) & (np.abs(g.astype(np.float64) - want) <= 2.0 ** -149)
         assert (same | near).all()
+
+
+def _ulps(got, want):
+    want64 = np.abs(want).astype(np.float64)
+    return np.abs(got.astype(np.longdouble) - want) / np.spacing(want64).astype(np.longdouble)
+
+
+def test_reciprocals_quotients_and_roots(probe):
+    assert np.finfo(np.longdouble).nmant >= 63
+    rng = np.random.default_rng(11)
+    frac = np.concatenate([np.array([0, 1, 2, 2 ** 52 - 1, 2 ** 52 - 2, 2 ** 51, 2 ** 32, 2 ** 32 - 1], np.uint64),
+                           rng.integers(0, 2 ** 52, 56, dtype=np.uint64)])
+    e = np.arange(2047, dtype=np.uint64) << np.uint64(52)
+    bits = (e[:, None] | frac[None, :]).ravel()[1:]  # (not zero)
+    x = np.concatenate([bits, bits | np.uint64(1 << 63)]).view(np.float64)
+    # the quotient's numerator: 40 binades around the divisor, and around one
+    with np.errstate(over="ignore"):
+        near = x * 2.0 ** rng.integers(-20, 21, x.size) * rng.uniform(-1, 1, x.size)
+    mid = np.abs(np.log2(np.abs(x))) < 900
+    y = np.where(mid, near, rng.uniform(-1, 1, x.size))
+    out = _apply_pairs(probe, x, y)
+    ex = (x.view(np.uint64) >> np.uint64(52)) & np.uint64(0x7ff)
+    xl, yl = x.astype(np.longdouble), y.astype(np.longdouble)
+    with np.errstate(over="ignore"):
+        inner = (ex >= 24) & (ex <= 2022)
+        assert np.array_equal(out[~inner, 0].view(np.uint64), (1.0 / x[~inner]).view(np.uint64))
+        assert _ulps(out[inner, 0], 1 / xl[inner]).max() <= 1
+    pos = x > 0
+    inner = pos & (ex >= 124) & (ex <= 1922)
+    assert np.array_equal(out[pos & ~inner, 1].view(np.uint64), np.sqrt(x[pos & ~inner]).view(np.uint64))
+    assert _ulps(out[inner, 1], np.sqrt(xl[inner])).max() <= 1
+    plain = pos & (ex >= 24) & (ex <= 2022)
+    assert (out[~plain, 2:] == -1).all()
+    q = yl[plain & mid] / xl[plain & mid]
+    assert _ulps(out[plain & mid, 2], q).max() <= 2
+    assert _ulps(out[plain, 3], 1 / np.sqrt(xl[plain])).max() <= 2
+    assert _ulps(out[plain, 4], np.sqrt(xl[plain])).max() <= 1
+
+
+def _apply_pairs(probe, x, y):
+    pairs, out = np.ascontiguousarray(np.stack([x, y], 1)), np.zeros((x.size, 5))
+    assert probe.probe_arith(C.c_int(x.size), C.c_void_p(pairs.ctypes.data), C.c_void_p(out.ctypes.data)) == 0
+    return out
 
 
 def test_fp32_to_fp64(probe):
