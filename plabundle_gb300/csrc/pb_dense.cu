@@ -98,12 +98,11 @@ __global__ void k_dense_diag(T* __restrict__ A, int n, int np, double shift) {
 
 // C (64x64) += A (64x64) * B (64x64): sA holds A row-major [r][k], sB holds B k-major [k][c];
 // 256 threads, thread (ty, tx) owns rows ty + 16 m and columns tx + 16 m'.
-template <typename T>
-__device__ __forceinline__ void tile_mma(const T* __restrict__ sA, const T* __restrict__ sB, T acc[4][4]) {
+__device__ __forceinline__ void tile_mma(const float* __restrict__ sA, const float* __restrict__ sB, float acc[4][4]) {
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll 8
     for (int kk = 0; kk < TS; ++kk) {
-        T a[4], b[4];
+        float a[4], b[4];
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
             a[m] = sA[(ty + 16 * m) * TP + kk];
@@ -137,9 +136,9 @@ struct Vec16<double> {
     __device__ static __forceinline__ double dot(const double2& a, const double2& b) { return a.x * b.x + a.y * b.y; }
 };
 
-template <typename T, bool TRANSPOSE>
-__device__ __forceinline__ void tile_load(const T* __restrict__ g, int np, T* __restrict__ s) {
-    using V = Vec16<T>;
+template <bool TRANSPOSE>
+__device__ __forceinline__ void tile_load(const float* __restrict__ g, int np, float* __restrict__ s) {
+    using V = Vec16<float>;
     constexpr int per_row = TS / V::n;
     for (int e = threadIdx.x; e < TS * per_row; e += blockDim.x) {
         const int r = e / per_row, c0 = (e % per_row) * V::n;
@@ -184,40 +183,39 @@ __device__ __forceinline__ int owned_elements(int* ii, int* ll) {
 // rows below it after a barrier: 354 unknowns 239 -> 220 us a factorisation, 114 unknowns 109 -> 94.)  The inverse R = L^-1 (R = I, R_ic -= L_ij R_jc / L_jj for
 // i > j >= c, then R_ic / L_ii) is independent per column: four lanes own a column (rows split
 // mod 4, held in registers) and pass row j between them by shuffle, with no block barrier.
-template <typename T>
-__device__ void diag_factor_inverse(T* __restrict__ A, T* __restrict__ Dinv, int np, int k, T* sA, T* sB,
-                                    int* __restrict__ status) {
-    T* Akk = A + static_cast<size_t>(k) * TS * np + static_cast<size_t>(k) * TS;
-    tile_load<T, false>(Akk, np, sA);
+__device__ void diag_factor_inverse(float* __restrict__ A, float* __restrict__ Dinv, int np, int k, float* sA,
+                                    float* sB, int* __restrict__ status) {
+    float* Akk = A + static_cast<size_t>(k) * TS * np + static_cast<size_t>(k) * TS;
+    tile_load<false>(Akk, np, sA);
     int ii[9], ll[9];
     owned_elements(ii, ll);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __shared__ T s_inv[TS];  // 1 / d_j of the elimination, then 1 / L_jj of the inverse
+    __shared__ float s_inv[TS];  // 1 / d_j of the elimination, then 1 / L_jj of the inverse
     constexpr int PW = 8;    // panel width
     __syncthreads();
     for (int c0 = 0; c0 < TS; c0 += PW) {
         // (a) the panel: row c0 + lane for lanes 0-7, then 24 of the rows below per warp
         const int below = TS - c0 - PW;
-        T a[PW];
+        float a[PW];
         const int i = lane < PW ? c0 + lane : c0 + PW + 24 * warp + lane - PW;
         const bool mine = i < TS;
         if (warp < max(1, (below + 23) / 24)) {
 #pragma unroll
-            for (int l = 0; l < PW; ++l) a[l] = mine ? sA[i * TP + c0 + l] : T(0);
+            for (int l = 0; l < PW; ++l) a[l] = mine ? sA[i * TP + c0 + l] : 0.f;
             // (no branch in the chain of pivots: the marks and reciprocals are written after it)
             bool bad = false;
-            T my_inv = T(0);
+            float my_inv = 0.f;
 #pragma unroll
             for (int j = 0; j < PW; ++j) {
-                const T d = __shfl_sync(0xffffffffu, a[j], j);
-                const bool pos = d > T(0);
-                const T inv = __frcp_rn(pos ? d : T(1)) * (pos ? T(1) : T(0));
+                const float d = __shfl_sync(0xffffffffu, a[j], j);
+                const bool pos = d > 0.f;
+                const float inv = __frcp_rn(pos ? d : 1.f) * (pos ? 1.f : 0.f);
                 bad |= !pos;
                 if (lane == j) my_inv = inv;
-                const T aij = a[j];
+                const float aij = a[j];
 #pragma unroll
                 for (int l = j + 1; l < PW; ++l) {
-                    const T alj = __shfl_sync(0xffffffffu, aij, l);
+                    const float alj = __shfl_sync(0xffffffffu, aij, l);
                     a[l] = fma(-(aij * alj), inv, a[l]);
                 }
             }
@@ -238,26 +236,26 @@ __device__ void diag_factor_inverse(T* __restrict__ A, T* __restrict__ Dinv, int
         // (b) the trailing block: elements (r, l), c0 + 8 <= l <= r < 64, the panel's steps in order; a lane
         // per column (and the column 32 to the right), a warp every eighth row
         {
-            T inv[PW], t0[PW], t1[PW];
+            float inv[PW], t0[PW], t1[PW];
             const int l0 = c0 + PW + lane, l1 = l0 + 32;
 #pragma unroll
             for (int j = 0; j < PW; ++j) {
                 inv[j] = s_inv[c0 + j];
-                t0[j] = l0 < TS ? sA[l0 * TP + c0 + j] : T(0);
-                t1[j] = l1 < TS ? sA[l1 * TP + c0 + j] : T(0);
+                t0[j] = l0 < TS ? sA[l0 * TP + c0 + j] : 0.f;
+                t1[j] = l1 < TS ? sA[l1 * TP + c0 + j] : 0.f;
             }
             for (int r = c0 + PW + warp; r < TS; r += 8) {
-                T rj[PW];
+                float rj[PW];
 #pragma unroll
                 for (int j = 0; j < PW; ++j) rj[j] = sA[r * TP + c0 + j];
                 if (l0 <= r) {
-                    T x = sA[r * TP + l0];
+                    float x = sA[r * TP + l0];
 #pragma unroll
                     for (int j = 0; j < PW; ++j) x = fma(-(rj[j] * t0[j]), inv[j], x);
                     sA[r * TP + l0] = x;
                 }
                 if (l1 <= r) {
-                    T x = sA[r * TP + l1];
+                    float x = sA[r * TP + l1];
 #pragma unroll
                     for (int j = 0; j < PW; ++j) x = fma(-(rj[j] * t1[j]), inv[j], x);
                     sA[r * TP + l1] = x;
@@ -266,12 +264,12 @@ __device__ void diag_factor_inverse(T* __restrict__ A, T* __restrict__ Dinv, int
         }
         __syncthreads();
     }
-    T v[9];
+    float v[9];
 #pragma unroll
     for (int s = 0; s < 9; ++s) {
         if (ii[s] < 0) continue;
-        const T d = sA[ll[s] * TP + ll[s]];
-        const T sd = d > T(0) ? sqrt(d) : T(1);
+        const float d = sA[ll[s] * TP + ll[s]];
+        const float sd = d > 0.f ? sqrt(d) : 1.f;
         v[s] = ii[s] == ll[s] ? sd : sA[ii[s] * TP + ll[s]] / sd;
     }
     __syncthreads();
@@ -279,24 +277,24 @@ __device__ void diag_factor_inverse(T* __restrict__ A, T* __restrict__ Dinv, int
     for (int s = 0; s < 9; ++s) {
         if (ii[s] < 0) continue;
         sA[ii[s] * TP + ll[s]] = v[s];
-        if (ii[s] != ll[s]) sA[ll[s] * TP + ii[s]] = T(0);
+        if (ii[s] != ll[s]) sA[ll[s] * TP + ii[s]] = 0.f;
     }
     __syncthreads();
     // 1 / L_jj once per row for the inverse
-    if (threadIdx.x < TS) s_inv[threadIdx.x] = T(1) / sA[threadIdx.x * TP + threadIdx.x];
+    if (threadIdx.x < TS) s_inv[threadIdx.x] = 1.f / sA[threadIdx.x * TP + threadIdx.x];
     __syncthreads();
     {
         // column c = 8 warp + lane / 4; this lane holds rows i = part + 4 q
         const int c = 8 * warp + (lane >> 2), part = lane & 3;
-        T r[TS / 4];
+        float r[TS / 4];
 #pragma unroll
-        for (int q = 0; q < TS / 4; ++q) r[q] = part + 4 * q == c ? T(1) : T(0);
+        for (int q = 0; q < TS / 4; ++q) r[q] = part + 4 * q == c ? 1.f : 0.f;
 #pragma unroll
         for (int j = 0; j < TS; ++j) {
             // row j of the column, final from the steps before j, from the lane that holds it
-            const T rj = __shfl_sync(0xffffffffu, r[j >> 2], (lane & ~3) | (j & 3));
+            const float rj = __shfl_sync(0xffffffffu, r[j >> 2], (lane & ~3) | (j & 3));
             if (8 * warp <= j) {  // some column of this warp has c <= j
-                const T inv = s_inv[j];
+                const float inv = s_inv[j];
 #pragma unroll
                 for (int q = 0; q < TS / 4; ++q) {
                     if (4 * q + 3 <= j) continue;  // every row of this slot is <= j
@@ -313,11 +311,11 @@ __device__ void diag_factor_inverse(T* __restrict__ A, T* __restrict__ Dinv, int
     for (int s = 0; s < 9; ++s)
         if (ii[s] >= 0) v[s] = sB[ii[s] * TP + ll[s]] / sA[ii[s] * TP + ii[s]];
     __syncthreads();
-    T* D = Dinv + static_cast<size_t>(k) * TS * TS;
+    float* D = Dinv + static_cast<size_t>(k) * TS * TS;
     for (int e = threadIdx.x; e < TS * TS; e += blockDim.x) {
         const int r = e / TS, c = e % TS;
         Akk[static_cast<size_t>(r) * np + c] = sA[r * TP + c];
-        D[e] = T(0);
+        D[e] = 0.f;
     }
     __syncthreads();
 #pragma unroll
@@ -326,21 +324,20 @@ __device__ void diag_factor_inverse(T* __restrict__ A, T* __restrict__ Dinv, int
 }
 
 // C = (accumulate ? C : 0) + alpha * sA sB over one 64x64 tile (row stride ldc).
-template <typename T>
-__device__ __forceinline__ void tile_product_store(T* __restrict__ C, int ldc, const T* sA, const T* sB, T alpha,
-                                                   bool accumulate) {
-    T acc[4][4];
+__device__ __forceinline__ void tile_product_store(float* __restrict__ C, int ldc, const float* sA, const float* sB,
+                                                   float alpha, bool accumulate) {
+    float acc[4][4];
 #pragma unroll
     for (int m = 0; m < 4; ++m)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) acc[m][q] = T(0);
-    tile_mma<T>(sA, sB, acc);
+        for (int q = 0; q < 4; ++q) acc[m][q] = 0.f;
+    tile_mma(sA, sB, acc);
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll
     for (int m = 0; m < 4; ++m)
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            T* c = C + static_cast<size_t>(ty + 16 * m) * ldc + tx + 16 * q;
+            float* c = C + static_cast<size_t>(ty + 16 * m) * ldc + tx + 16 * q;
             *c = accumulate ? *c + alpha * acc[m][q] : alpha * acc[m][q];
         }
 }
@@ -355,39 +352,38 @@ __device__ __forceinline__ void phase_barrier() {
     else cgk::this_grid().sync();
 }
 
-template <typename T, bool CLUSTER>
-__global__ void __launch_bounds__(256) k_potrf_coop(T* __restrict__ A, T* __restrict__ X, T* __restrict__ Dinv, int np,
-                                                   int nt, int* __restrict__ status, int* __restrict__ host_status) {
+template <bool CLUSTER>
+__global__ void __launch_bounds__(256) k_potrf_coop(float* __restrict__ A, float* __restrict__ X,
+                                                   float* __restrict__ Dinv, int np, int nt, int* __restrict__ status,
+                                                   int* __restrict__ host_status) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* sA = reinterpret_cast<T*>(smem_raw);
-    T* sB = sA + TS * TP;
-    auto tile = [np](T* M, int i, int j) { return M + static_cast<size_t>(i) * TS * np + static_cast<size_t>(j) * TS; };
+    float* sA = reinterpret_cast<float*>(smem_raw);
+    float* sB = sA + TS * TP;
+    auto tile = [np](float* M, int i, int j) { return M + static_cast<size_t>(i) * TS * np + static_cast<size_t>(j) * TS; };
     // X = I
-    const int nrow = np, nthreads = gridDim.x * blockDim.x;
-    for (int r = blockIdx.x; r < nrow; r += gridDim.x)
-        for (int c = threadIdx.x; c < np; c += blockDim.x) X[static_cast<size_t>(r) * np + c] = r == c ? T(1) : T(0);
-    (void)nthreads;
+    for (int r = blockIdx.x; r < np; r += gridDim.x)
+        for (int c = threadIdx.x; c < np; c += blockDim.x) X[static_cast<size_t>(r) * np + c] = r == c ? 1.f : 0.f;
     phase_barrier<CLUSTER>();
-    if (blockIdx.x == 0) diag_factor_inverse<T>(A, Dinv, np, 0, sA, sB, status);
+    if (blockIdx.x == 0) diag_factor_inverse(A, Dinv, np, 0, sA, sB, status);
     phase_barrier<CLUSTER>();
     for (int k = 0; k < nt; ++k) {
         const int m = nt - 1 - k;
-        const T* Dk = Dinv + static_cast<size_t>(k) * TS * TS;
+        const float* Dk = Dinv + static_cast<size_t>(k) * TS * TS;
         for (int it = blockIdx.x; it < m + k + 1; it += gridDim.x) {
             if (it < m) {
                 // L_ik = A_ik D_k^T
-                T* Aik = tile(A, k + 1 + it, k);
-                tile_load<T, false>(Aik, np, sA);
-                tile_load<T, true>(Dk, TS, sB);
+                float* Aik = tile(A, k + 1 + it, k);
+                tile_load<false>(Aik, np, sA);
+                tile_load<true>(Dk, TS, sB);
                 __syncthreads();
-                tile_product_store<T>(Aik, np, sA, sB, T(1), false);
+                tile_product_store(Aik, np, sA, sB, 1.f, false);
             } else {
                 // X_kj = D_k R_kj
-                T* Xkj = tile(X, k, it - m);
-                tile_load<T, false>(Dk, TS, sA);
-                tile_load<T, false>(Xkj, np, sB);
+                float* Xkj = tile(X, k, it - m);
+                tile_load<false>(Dk, TS, sA);
+                tile_load<false>(Xkj, np, sB);
                 __syncthreads();
-                tile_product_store<T>(Xkj, np, sA, sB, T(1), false);
+                tile_product_store(Xkj, np, sA, sB, 1.f, false);
             }
             __syncthreads();
         }
@@ -403,24 +399,24 @@ __global__ void __launch_bounds__(256) k_potrf_coop(T* __restrict__ A, T* __rest
                 // A_ij -= L_ik L_jk^T
                 const int t = tri_row(it);
                 const int i = k + 1 + t, j = k + 1 + (it - t * (t + 1) / 2);
-                tile_load<T, false>(tile(A, i, k), np, sA);
-                tile_load<T, true>(tile(A, j, k), np, sB);
+                tile_load<false>(tile(A, i, k), np, sA);
+                tile_load<true>(tile(A, j, k), np, sB);
                 __syncthreads();
-                tile_product_store<T>(tile(A, i, j), np, sA, sB, T(-1), true);
+                tile_product_store(tile(A, i, j), np, sA, sB, -1.f, true);
             } else {
                 // R_ij -= L_ik X_kj
                 const int q = it - ntrail;
                 const int i = k + 1 + q / (k + 1), j = q % (k + 1);
-                tile_load<T, false>(tile(A, i, k), np, sA);
-                tile_load<T, false>(tile(X, k, j), np, sB);
+                tile_load<false>(tile(A, i, k), np, sA);
+                tile_load<false>(tile(X, k, j), np, sB);
                 __syncthreads();
-                tile_product_store<T>(tile(X, i, j), np, sA, sB, T(-1), true);
+                tile_product_store(tile(X, i, j), np, sA, sB, -1.f, true);
             }
             __syncthreads();
             if (it == 0 && m > 0) {
                 // tile (k+1, k+1) is final: factor it for the next step
                 __threadfence_block();
-                diag_factor_inverse<T>(A, Dinv, np, k + 1, sA, sB, status);
+                diag_factor_inverse(A, Dinv, np, k + 1, sA, sB, status);
             }
         }
         phase_barrier<CLUSTER>();
@@ -431,9 +427,9 @@ __global__ void __launch_bounds__(256) k_potrf_coop(T* __restrict__ A, T* __rest
     // condition number of its rounding error.
     for (int it = blockIdx.x; it < nt * (nt + 1) / 2; it += gridDim.x) {
         const int i = tri_row(it), j = it - i * (i + 1) / 2;
-        tile_load<T, true>(tile(X, i, j), np, sA);
+        tile_load<true>(tile(X, i, j), np, sA);
         __syncthreads();
-        T* dst = tile(A, j, i);
+        float* dst = tile(A, j, i);
         for (int e = threadIdx.x; e < TS * TS; e += blockDim.x) {
             const int r = e / TS, c = e % TS;
             dst[static_cast<size_t>(r) * np + c] = sA[r * TP + c];
@@ -1357,8 +1353,8 @@ static int largest_cluster(const void* kernel, int threads, size_t smem) {
         cluster_config(cfg, at, size, threads, smem, nullptr);
         int clusters = 0;
         if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0) return size;
+        cudaGetLastError();  // (a size that does not fit is not an error of the caller)
     }
-    cudaGetLastError();  // (a size that does not fit is not an error of the caller)
     return 0;
 }
 
@@ -1377,15 +1373,15 @@ template <typename T>
 int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, int* h_status, cudaStream_t st,
                  int* launches) {
     const int n = W.n, np = W.np, nt = W.nt;
-    const size_t two_tiles = 2 * static_cast<size_t>(TS) * TP * sizeof(T);
+    const size_t two_tiles = 2 * static_cast<size_t>(TS) * TP * sizeof(float);
     constexpr bool f64 = sizeof(T) == 8;
     const void *kernel, *cluster_kernel;
     if constexpr (f64) {
         kernel = reinterpret_cast<const void*>(&k_potrf64_coop<false>);
         cluster_kernel = reinterpret_cast<const void*>(&k_potrf64_coop<true>);
     } else {
-        kernel = reinterpret_cast<const void*>(&k_potrf_coop<T, false>);
-        cluster_kernel = reinterpret_cast<const void*>(&k_potrf_coop<T, true>);
+        kernel = reinterpret_cast<const void*>(&k_potrf_coop<false>);
+        cluster_kernel = reinterpret_cast<const void*>(&k_potrf_coop<true>);
     }
     const int threads = f64 ? kPotrf64Threads : 256;
     const size_t smem = f64 ? kPotrf64Smem : two_tiles;
