@@ -418,18 +418,6 @@ __global__ void k_adj_rhs(Shape S, DevPtrs D, AdjBuffers B, double* __restrict__
     }
 }
 
-__device__ __forceinline__ int csr_find(const DevPtrs& D, int row, int col) {
-    int lo = D.row_ptr[row], hi = D.row_ptr[row + 1] - 1;
-    while (lo <= hi) {
-        const int mid = (lo + hi) >> 1;
-        const int v = D.col_idx[mid];
-        if (v == col) return mid;
-        if (v < col) lo = mid + 1;
-        else hi = mid - 1;
-    }
-    return -1;
-}
-
 // full 3x3 inverse of a symmetric matrix given by its upper triangle; false when singular
 // relative to its scale
 __device__ __forceinline__ bool sym3_inverse(const double* u, double* inv) {
@@ -866,7 +854,7 @@ __device__ __forceinline__ void gauge_terms(const Shape& S, const DevPtrs& D, co
     Lo.ni = ni;
     double mc[6], mk[kNI + 1];
     primary_mu(S, D, mu, cam, ni, mc, mk);
-    double frec[68 + 11 * kNI + kNI * (kNI + 1) / 2];
+    double frec[adj_stride(kNI)];
     DCam c;
     load_cam(D.cams_eff + static_cast<size_t>(cam) * kCamStride, c);
     double n[3];

@@ -455,7 +455,6 @@ __global__ void __launch_bounds__(kAssembleThreads, 2) k_assemble(Shape S, DevPt
     const int tslot = (wid >> 2) * 128 + lane * 4 + (wid & 3);
     const bool tact = tslot < ntc;
     const int tfirst = tact ? s_tfirst[tslot] : 0;
-    const int tk = tact ? s_tfirst[tslot + 1] - tfirst : 0;
     const int tobs = obs0 + tfirst;
     const bool telim = tact && (s_info[tfirst] & kElim);
     // control points of the track (linearizeTrack, BundleAdjustPlaMatrixReferenceSchur.cpp:331-346):

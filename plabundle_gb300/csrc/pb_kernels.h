@@ -275,6 +275,7 @@ int dense_pcg_result(const DenseWork<T>& W, const double* h_scal, int* iteration
 // (pose 6 | point 3 | intrinsic columns ni): pose-pose (upper 6x6), pose-point (6x3), point-point
 // (upper 3x3), pose-intrinsic (6 x ni), point-intrinsic (3 x ni), intrinsic (upper ni x ni), the
 // FP64 Jacobian rows (2 x (9 + ni)), W2 = 2 rho' w I + 4 rho'' w^2 r r^T (3) and lam = 2 rho' w r (2).
+__host__ __device__ constexpr int adj_stride(int ni) { return 68 + 11 * ni + ni * (ni + 1) / 2; }
 struct AdjLayout {
     int ni = 0, stride = 0;
     __host__ __device__ int hcc() const { return 0; }
@@ -288,11 +289,10 @@ struct AdjLayout {
     static AdjLayout make(int n_int) {
         AdjLayout L;
         L.ni = n_int;
-        L.stride = L.w2() + 5;
+        L.stride = adj_stride(n_int);
         return L;
     }
 };
-constexpr int kAdjMaxStride = 68 + 11 * kMaxNI + kMaxNI * (kMaxNI + 1) / 2;
 
 struct AdjBuffers {
     AdjLayout lay;

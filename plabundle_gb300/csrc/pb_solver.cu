@@ -2487,7 +2487,6 @@ pb_status pb_gpu_backward(pb_gpu_ctx* c, const double* grad_cameras, const doubl
         const DevPtrs& D = c->D[prec];
         cudaStream_t st = c->stream;
         const int nc = m.nc, ntp = S.ntp;
-        const long long nop = S.nop;
         AdjBuffers& B = c->adj;
         // inputs: dL/d(final state) (processing order for points); zero where the caller gives none
         std::vector<double> gcam(static_cast<size_t>(nc) * 6, 0.0), gpt;
