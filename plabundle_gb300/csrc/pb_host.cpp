@@ -1593,6 +1593,13 @@ int build_chunks(HostModel* m, int precision, size_t smem_budget, std::string* e
         for (int l = cs.cam_begin[c]; l < cs.cam_begin[c + 1]; ++l)
             cs.cam_contrib[fill_cam[m->camera_block[cs.cams[l]]]++] = l;
     }
+    // upper blocks by decreasing number of partials (a counting sort)
+    std::vector<int> at(static_cast<size_t>(cs.n()) + 2, 0);
+    auto shorter = [&](int u) { return std::max(0, cs.n() - (cs.up_contrib_begin[u + 1] - cs.up_contrib_begin[u])); };
+    for (int u = 0; u < nupper; ++u) ++at[shorter(u) + 1];
+    for (int i = 0; i <= cs.n(); ++i) at[i + 1] += at[i];
+    cs.up_order.resize(nupper);
+    for (int u = 0; u < nupper; ++u) cs.up_order[at[shorter(u)]++] = u;
     m->chunks_ready[precision] = true;
     return 0;
 }

@@ -38,6 +38,7 @@ struct Shape {
     double gauge_baseline;
     int int_cols[kMaxNI];
     int max_obs, max_cams, max_pairs, max_tracks;  // chunk limits of the active chunk set
+    long long pair_partials;  // chunk partials of pose blocks of the active chunk set
     // 1: the reference point parameterisation of image-only problems (point steps X + s(X) dX,
     // Euler target rotation steps); 0: plain X + dX and world-frame rotation-vector steps
     // (useReferencePointParameterization, BundleAdjustPlaMatrixAssembly.cpp:24-30)
@@ -121,6 +122,7 @@ struct DevPtrs {
     int* up_csr_t;          // nupper: CSR position of the transposed block (-1 on the diagonal)
     int* cam_contrib_begin; // ncb + 1
     int* cam_contrib;       // partial cam slots
+    int* up_order;          // upper pose blocks by decreasing number of partial slots
     // CSR pattern of pose blocks (both triangles)
     int* row_ptr;         // ncb + 1
     int* col_idx;         // nnzb
@@ -148,7 +150,7 @@ struct ChunkSet {
     std::vector<int> slot_item_begin, lcam_obs_begin;
     std::vector<unsigned short> slot_items;
     std::vector<unsigned char> lcam_obs;
-    std::vector<int> up_contrib_begin, up_contrib, cam_contrib_begin, cam_contrib;
+    std::vector<int> up_contrib_begin, up_contrib, cam_contrib_begin, cam_contrib, up_order;
     // owner-gather schedule of phase D of the assembly (see schedule_owner_tasks in pb_host.cpp)
     std::vector<int> warp_task_begin;
     std::vector<unsigned short> task_list;

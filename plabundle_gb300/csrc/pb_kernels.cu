@@ -18,10 +18,10 @@ namespace pb {
 
 // The three fixed-order sums below are independent of one another and each is latency-bound on
 // a small grid (the chunk-record sum has one CTA per 32 record entries), so one launch runs them
-// side by side over block ranges [pose pairs | cameras | chunk records + cost].  Each keeps the
+// side by side over block ranges [chunk records + cost | cameras | pose pairs].  Each keeps the
 // summation order of its own loop.  A list's merges are a serial chain of a few FP32 additions (one FP64
-// addition) each, and the lists are long (hundreds to thousands of chunks touch a camera), so the records
-// in flight per list decide.
+// addition) each, and the lists are long (hundreds of chunks touch a camera), so the records in flight per
+// list decide, unless the lists are short.
 template <typename T>
 struct ReduceArgs {
     using part_t = typename Acc<T>::part_type;
@@ -31,15 +31,30 @@ struct ReduceArgs {
     const double* part_cost;
     const int* part_flags;
     double *vals, *rhs, *direct, *border, *border_t, *Cm, *result;
-    unsigned chunk_blocks;
+    unsigned chunk_blocks;  // first block of the lists
+    unsigned list_blocks;   // ring: blocks of the lists; entries: blocks of the pose pairs
+    bool spread;            // ring: neighbouring lists to neighbouring blocks, not warps
 };
 
 // A warp sums up to 36 neighbouring entries of one list's records (lane l entries l and 32 + l) in the
 // order of the list.  The records stream through a ring of six stages of eight in shared memory by
 // asynchronous copies, their list indices loaded a vector of 32 ahead.  (A thread per entry with four
-// loads ahead left the longest lists waiting: 100 cameras, 4982 chunks, mixed 307 -> 160 us a launch; 500
-// cameras, 8301 chunks 211 -> 160 us; 40 cameras, FP64 47 -> 29 us.)
+// loads ahead leaves the longest lists waiting: this sum and k_finalize, 100 cameras and 120 000 points,
+// mixed 206 -> 104 us, FP64 270 -> 179; 500 cameras and 200 000 points 204 -> 101 and 358 -> 231; 40 cameras
+// and 9 001 points, FP64 36 -> 30.)
 constexpr int kRedWarps = 8, kRedEntries = 36, kRedStages = 6, kRedSlots = 8;
+// Beyond the resident blocks of the ring, pose-block lists of fewer records on average take a thread per entry
+// (500 cameras, this sum and k_finalize, ring against thread per entry: 7.8 records a list, mixed 27 / 20 us,
+// FP64 31 / 24; 16 records 32 / 30, 45 / 40; 24 records 38 / 43, 58 / 54; 750 rig cameras, 44 000 lists of 42
+// records 162 / 233, 302 / 310).  So many lists that either way keeps the device busy do so up to longer ones,
+// the ring taking two FP64 additions (lanes l and 32 + l) where a thread per entry takes 36 / 32 (1 800 rig
+// cameras, lists of 40: 463 / 475, 897 / 700; 3 000, 248 000 lists of 45: 930 / 831, 1843 / 1328; 3 000 nadir
+// cameras, 76 000 lists of 120: 700 / 1244, 1788 / 2012).
+template <typename T>
+static bool short_lists(const Shape& S) {
+    const bool fp64 = sizeof(T) == 8, many = S.nupper >= (fp64 ? 1 << 16 : 1 << 17);
+    return S.pair_partials < (many ? 64LL : fp64 ? 32LL : 20LL) * S.nupper;
+}
 constexpr int kRedPieces = kRedEntries / 2;  // 16-byte pieces of a full record tile
 constexpr size_t kRedSmem = static_cast<size_t>(kRedWarps) * kRedStages * kRedSlots * kRedEntries * 8;
 
@@ -99,6 +114,19 @@ __device__ __forceinline__ void reduce_list(Acc<T>* acc, const typename Acc<T>::
     }
 }
 
+// Entry e of camera block i's record: right-hand side, direct right-hand side, border.
+template <typename T>
+__device__ __forceinline__ void store_cam_sum(const Shape& S, const ReduceArgs<T>& R, int i, int e, double v) {
+    if (e < 6) R.rhs[i * 6 + e] = v;
+    else if (e < 12) R.direct[i * 6 + e - 6] = v;
+    else {
+        const int f = e - 12;  // (g * 6 + a) * ni + c
+        const int g = f / (6 * S.ni), rem = f - g * 6 * S.ni, a = rem / S.ni, c = rem - a * S.ni;
+        R.border[(static_cast<size_t>(i) * 6 + a) * S.nb + g * S.ni + c] = v;
+        R.border_t[static_cast<size_t>(g * S.ni + c) * 6 * S.ncb + i * 6 + a] = v;
+    }
+}
+
 // Sums of the chunk partials of every upper pose block, written to both CSR orientations, and of the
 // per-camera partials (rhs, direct rhs and the intrinsic border rows, in tiles of 36 entries): one warp
 // per block or tile.
@@ -109,10 +137,17 @@ __device__ __forceinline__ void reduce_lists(const Shape& S, const DevPtrs& D, c
     auto* ring = reinterpret_cast<typename Acc<T>::part_type*>(smem) +
                  static_cast<size_t>(wid) * kRedStages * kRedSlots * kRedEntries;
     const int camrec = 12 + S.ng * 6 * S.ni, tiles = (camrec + kRedEntries - 1) / kRedEntries;
-    const int unit = static_cast<int>(blk) * kRedWarps + wid;
+    // The cameras' lists first, then the pose blocks' by decreasing length (the diagonal blocks' are as long as
+    // the cameras').  While every block is resident (two on each of 152 SMs) neighbours go to different
+    // blocks, so that the long lists share the FP64 pipes evenly (60 cameras, FP64 58 -> 47 us).  Beyond, they
+    // share a block, which keeps its shared memory until its longest list is done: in the order of the
+    // reduced pattern the diagonal blocks' lists held up the short ones that came with them (750 rig cameras,
+    // 44 000 lists, 290 -> 162 us, FP64 430 -> 302; 250 cameras 83 -> 65, FP64 181 -> 123).
+    const int unit = static_cast<int>(R.spread ? wid * R.list_blocks + blk : blk * kRedWarps + wid), cams = S.ncb * tiles;
     Acc<T> acc[2];
-    if (unit < S.nupper) {
-        const int u = unit;
+    if (unit >= cams) {
+        if (unit >= cams + S.nupper) return;
+        const int u = D.up_order[unit - cams];
         reduce_list<T>(acc, R.part_pair, 36, 36, D.up_contrib, D.up_contrib_begin[u], D.up_contrib_begin[u + 1], ring);
         const int t = D.up_csr_t[u];
         double* vals = R.vals + static_cast<size_t>(D.up_csr[u]) * 36;
@@ -124,32 +159,52 @@ __device__ __forceinline__ void reduce_lists(const Shape& S, const DevPtrs& D, c
             vals[e] = v;
             if (t >= 0) R.vals[static_cast<size_t>(t) * 36 + (e % 6) * 6 + e / 6] = v;
         }
-    } else if (unit < S.nupper + S.ncb * tiles) {
-        const int i = (unit - S.nupper) / tiles, tile = unit - S.nupper - i * tiles, e0 = tile * kRedEntries;
+    } else {
+        const int i = unit / tiles, tile = unit - i * tiles, e0 = tile * kRedEntries;
         const int width = min(kRedEntries, camrec - e0);
         reduce_list<T>(acc, R.part_cam + e0, camrec, width, D.cam_contrib, D.cam_contrib_begin[i], D.cam_contrib_begin[i + 1],
                        ring);
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const int e = e0 + 32 * k + lane;
-            if (32 * k + lane >= width) continue;
-            const double v = acc[k].value64();
-            if (e < 6) R.rhs[i * 6 + e] = v;
-            else if (e < 12) R.direct[i * 6 + e - 6] = v;
-            else {
-                const int f = e - 12;  // (g * 6 + a) * ni + c
-                const int g = f / (6 * S.ni), rem = f - g * 6 * S.ni, a = rem / S.ni, c = rem - a * S.ni;
-                R.border[(static_cast<size_t>(i) * 6 + a) * S.nb + g * S.ni + c] = v;
-                R.border_t[static_cast<size_t>(g * S.ni + c) * 6 * S.ncb + i * 6 + a] = v;
-            }
-        }
+        for (int k = 0; k < 2; ++k)
+            if (32 * k + lane < width) store_cam_sum<T>(S, R, i, e0 + 32 * k + lane, acc[k].value64());
+    }
+}
+
+// The same sums with a thread per entry, four records of its list ahead: for short lists, whose start costs
+// more than their records, eight times as many threads in flight.  In the order of the reduced pattern,
+// whose neighbours share chunks.
+template <typename T>
+__device__ __forceinline__ void reduce_entries(const Shape& S, const DevPtrs& D, const ReduceArgs<T>& R, unsigned blk) {
+    const int width = 12 + S.ng * 6 * S.ni;
+    Acc<T> acc;
+    if (blk < R.list_blocks) {
+        const long long idx = static_cast<long long>(blk) * blockDim.x + threadIdx.x;
+        if (idx >= static_cast<long long>(S.nupper) * 36) return;
+        const int u = static_cast<int>(idx / 36), e = static_cast<int>(idx - static_cast<long long>(u) * 36);
+        const int c1 = D.up_contrib_begin[u + 1];
+#pragma unroll 4
+        for (int c = D.up_contrib_begin[u]; c < c1; ++c)
+            acc.merge_part(R.part_pair[static_cast<size_t>(D.up_contrib[c]) * 36 + e]);
+        const double v = acc.value64();
+        R.vals[static_cast<size_t>(D.up_csr[u]) * 36 + e] = v;
+        const int t = D.up_csr_t[u];
+        if (t >= 0) R.vals[static_cast<size_t>(t) * 36 + (e % 6) * 6 + e / 6] = v;
+    } else {
+        const long long idx = static_cast<long long>(blk - R.list_blocks) * blockDim.x + threadIdx.x;
+        if (idx >= static_cast<long long>(S.ncb) * width) return;
+        const int i = static_cast<int>(idx / width), e = static_cast<int>(idx - static_cast<long long>(i) * width);
+        const int c1 = D.cam_contrib_begin[i + 1];
+#pragma unroll 4
+        for (int c = D.cam_contrib_begin[i]; c < c1; ++c)
+            acc.merge_part(R.part_cam[static_cast<size_t>(D.cam_contrib[c]) * width + e]);
+        store_cam_sum<T>(S, R, i, e, acc.value64());
     }
 }
 
 // Chunk-level sums (intrinsic block, intrinsic rhs): one CTA per 32 record entries, its warps
 // striding over the chunks, merged in warp order.  The block after the last tile sums the costs
 // and flags.
-template <typename T>
+template <typename T, int kAhead>
 __device__ __forceinline__ void reduce_chunks(const Shape& S, const ReduceArgs<T>& R, unsigned blk) {
     const int nb = S.nb, chrec = nb * nb + 2 * nb;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -162,8 +217,7 @@ __device__ __forceinline__ void reduce_chunks(const Shape& S, const ReduceArgs<T
         const int e = blk * 32 + lane;
         Acc<T> acc;
         if (e < chrec) {
-            // sixteen records in registers while the next sixteen are on their way
-            constexpr int kAhead = 16;
+            // kAhead records in registers while the next ones are on their way
             const typename Acc<T>::part_type* src = R.part_chunk + e;
             typename Acc<T>::part_type v[kAhead];
             int c = wid;
@@ -222,12 +276,13 @@ __device__ __forceinline__ void reduce_chunks(const Shape& S, const ReduceArgs<T
 
 // 256 threads per block (the chunk-record sum's warp count and cost buffers assume it); the block
 // range decides the sum, uniformly per block: the chunk records first, they take longest.
-template <typename T>
-__global__ void __launch_bounds__(256) k_reduce_sums(Shape S, DevPtrs D, ReduceArgs<T> R) {
+template <typename T, bool RING>
+__global__ void __launch_bounds__(256, RING ? 2 : 8) k_reduce_sums(Shape S, DevPtrs D, ReduceArgs<T> R) {
     extern __shared__ __align__(16) unsigned char reduce_smem[];
     const unsigned b = blockIdx.x;
-    if (b < R.chunk_blocks) reduce_chunks<T>(S, R, b);
-    else reduce_lists<T>(S, D, R, b - R.chunk_blocks, reduce_smem);
+    if (b < R.chunk_blocks) reduce_chunks<T, RING ? 16 : 4>(S, R, b);
+    else if constexpr (RING) reduce_lists<T>(S, D, R, b - R.chunk_blocks, reduce_smem);
+    else reduce_entries<T>(S, D, R, b - R.chunk_blocks);
 }
 
 // Intrinsic priors (assembleReferencePriors, ...ReferenceSchur.cpp:492-536) and
@@ -872,9 +927,17 @@ void launch_reduce_sums(const Shape& S, const DevPtrs& D, const AsmOut& O, const
     int dev = 0;
     cudaGetDevice(&dev);
     std::call_once(once[dev & 63], [] {
-        cudaFuncSetAttribute(k_reduce_sums<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRedSmem));
+        cudaFuncSetAttribute(k_reduce_sums<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRedSmem));
     });
-    k_reduce_sums<T><<<A.chunk_blocks + list_blocks, 256, kRedSmem, st>>>(S, D, A);
+    A.list_blocks = list_blocks;
+    A.spread = list_blocks <= 2 * 152;
+    if (A.spread || !short_lists<T>(S)) {
+        k_reduce_sums<T, true><<<A.chunk_blocks + list_blocks, 256, kRedSmem, st>>>(S, D, A);
+        return;
+    }
+    A.list_blocks = static_cast<unsigned>((36LL * S.nupper + 255) / 256);
+    const unsigned cam_blocks = static_cast<unsigned>((static_cast<long long>(S.ncb) * (12 + S.ng * 6 * S.ni) + 255) / 256);
+    k_reduce_sums<T, false><<<A.chunk_blocks + A.list_blocks + cam_blocks, 256, 0, st>>>(S, D, A);
 }
 
 template <typename T>

@@ -591,6 +591,7 @@ void prepare_precision(pb_gpu_ctx* c, int precision) {
     S.max_cams = cs.max_cams;
     S.max_pairs = cs.max_pairs;
     S.max_tracks = cs.max_tracks;
+    S.pair_partials = static_cast<long long>(cs.n_pair_partials());
     D.ch_obs_begin = upload_new(A, cs.obs_begin, st);
     D.ch_cam_begin = upload_new(A, cs.cam_begin, st);
     D.ch_cams = upload_new(A, cs.cams, st);
@@ -600,6 +601,7 @@ void prepare_precision(pb_gpu_ctx* c, int precision) {
     D.up_contrib = upload_new(A, cs.up_contrib, st);
     D.cam_contrib_begin = upload_new(A, cs.cam_contrib_begin, st);
     D.cam_contrib = upload_new(A, cs.cam_contrib, st);
+    D.up_order = upload_new(A, cs.up_order, st);
     D.obs_lcam = upload_new(A, cs.obs_lcam, st);
     D.slot_item_begin = upload_new(A, cs.slot_item_begin, st);
     D.slot_items = upload_new(A, cs.slot_items, st);
@@ -1815,11 +1817,12 @@ pb_status pb_gpu_upload(pb_gpu_ctx* c, const pb_problem_desc* pr, const pb_solve
                 dst.ch_obs_begin = src.ch_obs_begin; dst.ch_cam_begin = src.ch_cam_begin; dst.ch_cams = src.ch_cams;
                 dst.ch_pair_begin = src.ch_pair_begin; dst.ch_pairs = src.ch_pairs;
                 dst.up_contrib_begin = src.up_contrib_begin; dst.up_contrib = src.up_contrib;
-                dst.cam_contrib_begin = src.cam_contrib_begin; dst.cam_contrib = src.cam_contrib; dst.obs_lcam = src.obs_lcam;
+                dst.cam_contrib_begin = src.cam_contrib_begin; dst.cam_contrib = src.cam_contrib; dst.up_order = src.up_order; dst.obs_lcam = src.obs_lcam;
                 dst.slot_item_begin = src.slot_item_begin; dst.slot_items = src.slot_items;
                 dst.lcam_obs_begin = src.lcam_obs_begin; dst.lcam_obs = src.lcam_obs;
                 dst.warp_task_begin = src.warp_task_begin; dst.task_list = src.task_list;
                 sd.nchunks = ss.nchunks; sd.max_obs = ss.max_obs; sd.max_cams = ss.max_cams; sd.max_pairs = ss.max_pairs; sd.max_tracks = ss.max_tracks;
+                sd.pair_partials = ss.pair_partials;
             };
             keep_chunks(c->D[0], d0, c->S[0], s0);
             keep_chunks(c->D[1], d1, c->S[1], s1);
