@@ -4,13 +4,15 @@
 // but badly conditioned: the focal-length / altitude mode of a nadir block gives a normalised
 // condition number near 1e7, where block-Jacobi PCG needs thousands of iterations.  Here the
 // Jacobi-scaled matrix Sn = D^-1/2 S D^-1/2 is factored densely (Sn + shift I = L L^T, blocked
-// right-looking Cholesky on 64x64 tiles), L is inverted (X = L^-1), and M^-1 = D^-1/2 X^T X D^-1/2
+// right-looking Cholesky on tiles of 64 in FP32, of 32 in FP64), L is inverted (X = L^-1), and
+// M^-1 = D^-1/2 X^T X D^-1/2
 // preconditions conjugate gradients whose matrix-vector products use the FP64 reduced matrix.
 // On the mixed path the factor and inverse are FP32 with a small shift that keeps the FP32
 // factorisation positive definite; the FP64 CG recovers the FP64 solution (it plays the role of
 // iterative refinement).  On the FP64 path the factor is FP64 and CG converges in one or two
-// iterations.  The factorisation with its inverse and the whole CG solve are each one cooperative
-// persistent kernel (grid barriers between phases, no host round trips).
+// iterations.  The factorisation with its inverse and the whole CG solve are each one persistent kernel
+// whose phases are separated by barriers, with no host round trips: of one thread-block cluster for small
+// systems, of a cooperative grid beyond.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -180,9 +182,10 @@ __device__ __forceinline__ int owned_elements(int* ii, int* ll) {
 // shuffle and no warp waits for another), then every thread applies the panel's eight steps, in order,
 // to its elements of the trailing block.  Each element sees the same updates in the same order as a
 // column-by-column elimination.  (Against panels of sixteen columns, their own block on one warp and the
-// rows below it after a barrier: 354 unknowns 239 -> 220 us a factorisation, 114 unknowns 109 -> 94.)  The inverse R = L^-1 (R = I, R_ic -= L_ij R_jc / L_jj for
-// i > j >= c, then R_ic / L_ii) is independent per column: four lanes own a column (rows split
-// mod 4, held in registers) and pass row j between them by shuffle, with no block barrier.
+// rows below it after a barrier: 354 unknowns 239 -> 220 us a factorisation, 114 unknowns 109 -> 94.)  The
+// inverse R = L^-1 (R = I, R_ic -= L_ij R_jc / L_jj for i > j >= c, then R_ic / L_ii) is independent per
+// column: four lanes own a column (rows split mod 4, held in registers) and pass row j between them by
+// shuffle, with no block barrier.
 __device__ void diag_factor_inverse(float* __restrict__ A, float* __restrict__ Dinv, int np, int k, float* sA,
                                     float* sB, int* __restrict__ status) {
     float* Akk = A + static_cast<size_t>(k) * TS * np + static_cast<size_t>(k) * TS;

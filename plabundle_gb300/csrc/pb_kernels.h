@@ -252,8 +252,9 @@ struct DenseWork {
 
 template <typename T>
 size_t dense_bytes(int n);
-// h_status: pinned host memory.  Returns 0 on success, a status bitmask when the scaled matrix is not positive definite at this
-// shift (bit 1: non-positive diagonal, bit 2: non-positive pivot), -1 on a CUDA error.
+// h_status: pinned host memory.  Returns 0 on success, a status bitmask when the scaled matrix is not
+// positive definite at this shift (bit 1: non-positive diagonal, bit 2: non-positive pivot), -1 on a CUDA
+// error.
 template <typename T>
 int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, int* h_status, cudaStream_t st,
                  int* launches);

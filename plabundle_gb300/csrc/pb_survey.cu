@@ -15,9 +15,10 @@
 //                          promoted point.
 // The extended system is solved like the reduced one (dense factor + CG).  Observation terms are
 // FP64 (linearize_obs<double>, the function of the FP64 assembly), one warp per promoted point, its
-// sums in processing order; the bars are applied in bar order, so every sum has a fixed order.  The promoted blocks are damped like every primary diagonal,
-// finalizePrimaryDiagonal(1 + damping, 1): a promoted point is not coupled to any eliminated
-// point, so its block is the same before and after the point elimination.
+// sums in processing order; the bars are applied in bar order, so every sum has a fixed order.  The
+// promoted blocks are damped like every primary diagonal, finalizePrimaryDiagonal(1 + damping, 1): a
+// promoted point is not coupled to any eliminated point, so its block is the same before and after the
+// point elimination.
 #include <cuda_runtime.h>
 
 #include "pb_device.cuh"
@@ -256,8 +257,7 @@ __global__ void k_ext_step(Shape S, DevPtrs D, const double* __restrict__ xsol, 
 }
 
 // Scale-bar cost of each trial state (points + alpha step for the points that move) or of the
-// current state, one thread per step length, bars in order.
-// A warp per step length: the lanes evaluate the bars, whose costs are added in order (a thread per step
+// current state, bars in order.  A warp per step length: the lanes evaluate the bars, whose costs are added in order (a thread per step
 // length took the bars' latencies one after the other: four bars 11.5 -> 6.6 us).
 __global__ void __launch_bounds__(32) k_bar_cost(Shape S, DevPtrs D, const double* __restrict__ step_p, Alphas alphas,
                                                  int use_trial, double* __restrict__ out) {
