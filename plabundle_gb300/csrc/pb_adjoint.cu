@@ -500,8 +500,9 @@ __global__ void __launch_bounds__(kAdjThreads, 3)
     int* s_tfirst = carve<int>(ptr, MT + 1);
     int* s_next = carve<int>(ptr, 1);  // next intrinsic entry to take
     const int obs0 = D.ch_obs_begin[chunk], nobs = D.ch_obs_begin[chunk + 1] - obs0;
-    const int trk0 = D.obs_trk[obs0];
-    const int ntc = D.obs_trk[obs0 + nobs - 1] - trk0 + 1;
+    // (a problem without a usable observation has one chunk, an empty one)
+    const int trk0 = nobs > 0 ? D.obs_trk[obs0] : 0;
+    const int ntc = nobs > 0 ? D.obs_trk[obs0 + nobs - 1] - trk0 + 1 : 0;
     if (ntc > MT) {
         if (tid == 0) atomicOr(B.flags, 4);
         return;
