@@ -1376,6 +1376,8 @@ template <typename T>
 int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, int* h_status, cudaStream_t st,
                  int* launches) {
     const int n = W.n, np = W.np, nt = W.nt;
+    // no unknowns: refused before any launch (a grid of no blocks is an error that a later query may clear)
+    if (n <= 0) return -1;
     const size_t two_tiles = 2 * static_cast<size_t>(TS) * TP * sizeof(float);
     constexpr bool f64 = sizeof(T) == 8;
     const void *kernel, *cluster_kernel;
