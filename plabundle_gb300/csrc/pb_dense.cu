@@ -1376,7 +1376,7 @@ template <typename T>
 int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, int* h_status, cudaStream_t st,
                  int* launches) {
     const int n = W.n, np = W.np, nt = W.nt;
-    // no unknowns: refused before any launch (a grid of no blocks is an error that a later query may clear)
+    // no unknowns: refused before any launch
     if (n <= 0) return -1;
     const size_t two_tiles = 2 * static_cast<size_t>(TS) * TP * sizeof(float);
     constexpr bool f64 = sizeof(T) == 8;
@@ -1390,15 +1390,7 @@ int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, in
     }
     const int threads = f64 ? kPotrf64Threads : 256;
     const size_t smem = f64 ? kPotrf64Smem : two_tiles;
-    int L = 0;
-    cudaMemsetAsync(W.status, 0, sizeof(int), st);
-    cudaMemsetAsync(W.A, 0, static_cast<size_t>(np) * np * sizeof(T), st);
-    k_dense_scale<<<(n + 255) / 256, 256, 0, st>>>(sys, W.dscale, W.status);
-    const long long nfill = static_cast<long long>(sys.row_ptr ? W.nnzb : 0) * 36 + 6LL * sys.ncb * sys.nb +
-                            static_cast<long long>(sys.nb) * sys.nb;
-    if (nfill > 0) k_dense_fill<T><<<static_cast<unsigned>((nfill + 255) / 256), 256, 0, st>>>(sys, W.dscale, W.A, np);
-    k_dense_diag<T><<<(np + 255) / 256, 256, 0, st>>>(W.A, n, np, shift);
-    L += 3;
+    // (before the launches: the query clears its own errors, and must not clear one of theirs)
     if (W.fact_grid == 0) {
         set_smem<T>(kernel, smem);
         set_smem<T>(cluster_kernel, smem);
@@ -1409,6 +1401,15 @@ int dense_factor(const PcgSystem<double>& sys, DenseWork<T>& W, double shift, in
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
         W.fact_grid = std::max(1, std::min(per_sm, 2) * sms);
     }
+    int L = 0;
+    cudaMemsetAsync(W.status, 0, sizeof(int), st);
+    cudaMemsetAsync(W.A, 0, static_cast<size_t>(np) * np * sizeof(T), st);
+    k_dense_scale<<<(n + 255) / 256, 256, 0, st>>>(sys, W.dscale, W.status);
+    const long long nfill = static_cast<long long>(sys.row_ptr ? W.nnzb : 0) * 36 + 6LL * sys.ncb * sys.nb +
+                            static_cast<long long>(sys.nb) * sys.nb;
+    if (nfill > 0) k_dense_fill<T><<<static_cast<unsigned>((nfill + 255) / 256), 256, 0, st>>>(sys, W.dscale, W.A, np);
+    k_dense_diag<T><<<(np + 255) / 256, 256, 0, st>>>(W.A, n, np, shift);
+    L += 3;
     {
         T* A = W.A;
         T* X = W.X;
